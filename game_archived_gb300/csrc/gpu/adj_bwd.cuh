@@ -157,7 +157,7 @@ __global__ void ba_pgrad(HGrid<double> g, AParams ap, AState<double> s, const do
         return d;
     };
     if (i < nw) {
-        const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc);
+        const int k = row_of(i, g.nc), c = (int)(i - (long long)k * g.nc);
         if (k == 0 || k == g.nl) return;
         const long long up = (long long)(k - 1) * g.nc + c, lo = (long long)k * g.nc + c;
         const double G = a_gv(g, s.ep, k, c);
@@ -172,7 +172,7 @@ __global__ void ba_pgrad(HGrid<double> g, AParams ap, AState<double> s, const do
         b_gv(g, ep_b, k, c, S * pb);
     } else {
         const long long j = i - nw;
-        const int l = (int)(j / g.ne), e = (int)(j - (long long)l * g.ne);
+        const int l = row_of(j, g.ne), e = (int)(j - (long long)l * g.ne);
         const int fr = g.from[e], to = g.to[e];
         const long long cf = (long long)l * g.nc + fr, ct = (long long)l * g.nc + to;
         const double G = a_grad_h(g, s.ep, l, e);
@@ -195,7 +195,7 @@ __global__ void ba_tri(HGrid<double> g, const double *tri_b, double *u_b)
     if (i >= n) return;
     const double tb = tri_b[i] / g.dual_area_t[i];
     if (tb == 0.0) return;
-    const int l = (int)(i / g.nt), t = (int)(i - (long long)l * g.nt);
+    const int l = row_of(i, g.nt), t = (int)(i - (long long)l * g.nt);
     for (int j = 0; j < 3; ++j) {
         const int e = g.vort_i[j * g.nt + t];
         const long long le = (long long)l * g.ne + e;
@@ -228,7 +228,7 @@ __global__ void ba_edge(HGrid<double> g, const double *u, const double *rho, con
     const long long n = (long long)(g.nl + 1) * g.ne;
     const long long i = gtid();
     if (i >= n) return;
-    const int k = (int)(i / g.ne), e = (int)(i - (long long)k * g.ne);
+    const int k = row_of(i, g.ne), e = (int)(i - (long long)k * g.ne);
     const int nl = g.nl, nc = g.nc, ne = g.ne;
     {
         const double zb = zh_b[i];
@@ -271,7 +271,7 @@ __global__ void ba_kin(HGrid<double> g, const double *u, const double *w, const 
     const long long ns = (long long)g.nl * g.nc;
     const long long i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const int n_edges = c < N_PENT ? 5 : 6;
     const double vb = v2_b[i];
     if (vb != 0.0) {
@@ -347,7 +347,7 @@ __global__ void ba_mom_h(HGrid<double> g, AParams ap, int adv, double new_w, dou
     const long long i = gtid();
     if (i >= n) return;
     const long long nw = (long long)(g.nl + 1) * g.nc, vi = nw + i;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     const double ub = u_new_b[i];
     u_old_b[i] += ub;
     const double tb = t_b[vi] + ap.dt * ub;
@@ -378,7 +378,7 @@ __global__ void ba_mom_v(HGrid<double> g, AParams ap, int adv, double new_w, dou
     const long long n = (long long)(g.nl + 1) * g.nc;
     const long long i = gtid();
     if (i >= n) return;
-    const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc);
+    const int k = row_of(i, g.nc), c = (int)(i - (long long)k * g.nc);
     const int nl = g.nl;
     double pb = pvt_b[i];
     if (k != 0 && k != nl) {
@@ -445,7 +445,7 @@ __global__ void ba_scalar(HGrid<double> g, const double *rho, const double *thet
     const double yb = st_rho_b[i], ytb = st_rt_b[i];
     if (yb == 0.0 && ytb == 0.0) return;
     const int nl = g.nl, n_oro = g.n_oro;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     const bool oro = l >= nl - n_oro - 1;
@@ -523,7 +523,7 @@ __global__ void ba_apply_layer(VGrid vg, AState<double> so, const double *wl, AS
     const int nc = vg.nc, nl = vg.nl;
     const long long ns = (long long)nl * nc, b = gtid();
     if (b >= ns) return;
-    const int j = (int)(b / nc);
+    const int j = row_of(b, nc);
     const double vol = vg.volume[b], gam = wl[WL_G * ns + b];
     const double rn = out.rho[b], rtn = out.rt[b];
     const double tpb = out_b.tp[b], epb = out_b.ep[b];
@@ -563,7 +563,7 @@ __global__ void ba_apply_rho(VGrid vg, AParams ap, const double *wr, const doubl
     const int nc = vg.nc, nl = vg.nl;
     const long long ns = (long long)nl * nc, b = gtid();
     if (b >= ns) return;
-    const int j = (int)(b / nc);
+    const int j = row_of(b, nc);
     const long long m = (long long)(nl - 1) * nc;
     const double dt = ap.dt, vol = vg.volume[b];
     const double rb = rn_b[b], rtb = rtn_b[b];
@@ -630,7 +630,7 @@ __global__ void ba_waves_rows(VGrid vg, AParams ap, AState<double> so, const dou
     const int nc = vg.nc, nl = vg.nl;
     const long long n = (long long)(nl - 1) * nc, q = gtid();
     if (q >= n) return;
-    const int j = (int)(q / nc);
+    const int j = row_of(q, nc);
     const long long ns = (long long)nl * nc;
     const long long b = q, lo = q + nc, wi = q + nc;
     const double dt = ap.dt, iw = ap.impl_thermo_weight, dt2 = dt * dt;

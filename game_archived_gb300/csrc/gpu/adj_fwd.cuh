@@ -160,7 +160,7 @@ __global__ void fa_pgrad(HGrid<double> g, AParams ap, AState<T> s, T *P)
         return 0.5 * (d_a + d_b);
     };
     if (i < nw) {
-        const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc);
+        const int k = row_of(i, g.nc), c = (int)(i - (long long)k * g.nc);
         if (k == 0 || k == g.nl) return;
         const long long up = (long long)(k - 1) * g.nc + c, lo = (long long)k * g.nc + c;
         T nl = a_gv(g, s.ep, k, c);
@@ -175,7 +175,7 @@ __global__ void fa_pgrad(HGrid<double> g, AParams ap, AState<T> s, T *P)
         P[i] = nl + lt;
     } else {
         const long long j = i - nw;
-        const int l = (int)(j / g.ne), e = (int)(j - (long long)l * g.ne);
+        const int l = row_of(j, g.ne), e = (int)(j - (long long)l * g.ne);
         const int fr = g.from[e], to = g.to[e];
         const long long cf = (long long)l * g.nc + fr, ct = (long long)l * g.nc + to;
         T nl = a_grad_h(g, s.ep, l, e);
@@ -198,7 +198,7 @@ __global__ void fa_tri(HGrid<double> g, const T *u, T *tri)
     const long long n = (long long)g.nl * g.nt;
     const long long i = gtid();
     if (i >= n) return;
-    const int l = (int)(i / g.nt), t = (int)(i - (long long)l * g.nt);
+    const int l = row_of(i, g.nt), t = (int)(i - (long long)l * g.nt);
     T acc = tzero<T>();
     for (int j = 0; j < 3; ++j) {
         const int e = g.vort_i[j * g.nt + t];
@@ -269,7 +269,7 @@ __global__ void fa_edge(HGrid<double> g, const T *u, const T *w, const T *rho, c
     const long long n = (long long)(g.nl + 1) * g.ne;
     const long long i = gtid();
     if (i >= n) return;
-    const int k = (int)(i / g.ne), e = (int)(i - (long long)k * g.ne);
+    const int k = row_of(i, g.ne), e = (int)(i - (long long)k * g.ne);
     const int nl = g.nl, nc = g.nc, ne = g.ne;
     zh[i] = (a_rel_tan(g, u, w, k, e) + g.f_vec[e]) / a_dens_tan(g, rho, k, e);
     if (k < nl) {
@@ -296,7 +296,7 @@ __global__ void fa_kin(HGrid<double> g, const T *u, const T *w, const T *rho, T 
     const long long ns = (long long)g.nl * g.nc;
     const long long i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const int n_edges = c < N_PENT ? 5 : 6;
     T acc = tzero<T>();
     for (int j = 0; j < n_edges; ++j) {
@@ -361,7 +361,7 @@ __global__ void fa_mom_h(HGrid<double> g, AParams ap, int adv, double new_w, dou
     const long long i = gtid();
     if (i >= n) return;
     const long long nw = (long long)(g.nl + 1) * g.nc, vi = nw + i;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     if (adv) {
         pvt[vi] = a_vflux_h(g, flux_h, flux_v, zh, zv, l, e);
         v2g[vi] = a_grad_h(g, v2, l, e);
@@ -383,7 +383,7 @@ __global__ void fa_mom_v(HGrid<double> g, AParams ap, int adv, double new_w, dou
     const long long n = (long long)(g.nl + 1) * g.nc;
     const long long i = gtid();
     if (i >= n) return;
-    const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc);
+    const int k = row_of(i, g.nc), c = (int)(i - (long long)k * g.nc);
     const int nl = g.nl;
     if (adv) {
         T acc = tzero<T>();
@@ -448,7 +448,7 @@ __global__ void fa_scalar(HGrid<double> g, const T *rho, const T *theta, const T
     const long long i = gtid();
     if (i >= ns) return;
     const int nl = g.nl, n_oro = g.n_oro;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     const bool oro = l >= nl - n_oro - 1;
@@ -547,7 +547,7 @@ __global__ void fa_waves_rows(VGrid vg, AParams ap, AState<T> so, const T *st_w,
     const int nc = vg.nc, nl = vg.nl;
     const long long n = (long long)(nl - 1) * nc, q = gtid();
     if (q >= n) return;
-    const int j = (int)(q / nc);
+    const int j = row_of(q, nc);
     const long long ns = (long long)nl * nc;
     const long long b = q, lo = q + nc, wi = q + nc;
     const double dt = ap.dt, iw = ap.impl_thermo_weight, dt2 = dt * dt;
@@ -619,7 +619,7 @@ __global__ void fa_waves_apply(VGrid vg, AParams ap, AState<T> so, const T *wl, 
     const int nc = vg.nc, nl = vg.nl;
     const long long ns = (long long)nl * nc, b = gtid();
     if (b >= ns) return;
-    const int j = (int)(b / nc);
+    const int j = row_of(b, nc);
     const long long m = (long long)(nl - 1) * nc;
     const double dt = ap.dt;
     const T *sol = wr + WR_SOL * m, *th_int = wr + WR_TH * m, *rio = wr + WR_RIO * m;

@@ -319,7 +319,7 @@ __global__ void fa_scalar_moist(HGrid<double> g, AParams ap, int rk, const T *rh
     const long long i = gtid();
     if (i >= ns) return;
     const int nl = g.nl, n_oro = g.n_oro, cond = ap.n_cond, n_const = ap.n_const;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     const bool oro = l >= nl - n_oro - 1;
@@ -447,7 +447,7 @@ __global__ void ba_scalar_moist(HGrid<double> g, AParams ap, int rk, const doubl
     const long long i = gtid();
     if (i >= ns) return;
     const int nl = g.nl, n_oro = g.n_oro, cond = ap.n_cond, n_const = ap.n_const;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     const bool oro = l >= nl - n_oro - 1;
@@ -642,7 +642,7 @@ __global__ void fa_tracer_solve(VGrid vg, StepParams p, AState<T> so, const T *w
     const long long q = gtid();
     const int n_tr = p.n_const - 1;
     if (q >= (long long)n_tr * nc) return;
-    const int slot = (int)(q / nc), i = (int)(q - (long long)slot * nc);
+    const int slot = row_of(q, nc), i = (int)(q - (long long)slot * nc);
     const int k = slot < p.n_cond ? slot : slot + 1;
     bool has_sink;
     const double vsink = sink_velocity(p, k, has_sink);

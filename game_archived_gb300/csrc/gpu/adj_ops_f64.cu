@@ -25,12 +25,12 @@ __global__ void kop_grad_adj(HGrid<double> g, const double *out_b, double *in_b)
     const double ob = out_b[i];
     if (ob == 0.0) return;
     if (i < nw) {
-        const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc);
+        const int k = row_of(i, g.nc), c = (int)(i - (long long)k * g.nc);
         if (k == 0 || k == g.nl) return;
         b_gv(g, in_b, k, c, ob);
     } else {
         const long long j = i - nw;
-        const int l = (int)(j / g.ne), e = (int)(j - (long long)l * g.ne);
+        const int l = row_of(j, g.ne), e = (int)(j - (long long)l * g.ne);
         b_grad_h(g, in_b, l, e, ob);
     }
 }
@@ -45,7 +45,7 @@ __global__ void kop_divv_adj(HGrid<double> g, const double *out_b, double *in_b_
     const double yb = out_b[i];
     if (yb == 0.0) return;
     const int nl = g.nl, n_oro = g.n_oro;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     const bool oro = l >= nl - n_oro - 1;
@@ -94,7 +94,7 @@ __global__ void kop_stv_adj(HGrid<double> g, const double *s, const double *v, c
     const double ob = out_b[i];
     if (ob == 0.0) return;
     if (i < nw) {
-        const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc);
+        const int k = row_of(i, g.nc), c = (int)(i - (long long)k * g.nc);
         if (k == 0 || k == g.nl) return;
         const long long up = (long long)(k - 1) * g.nc + c, lo = (long long)k * g.nc + c;
         acc(&v_b[i], 0.5 * (s[up] + s[lo]) * ob);
@@ -103,7 +103,7 @@ __global__ void kop_stv_adj(HGrid<double> g, const double *s, const double *v, c
         acc(&s_b[lo], q);
     } else {
         const long long j = i - nw;
-        const int l = (int)(j / g.ne), e = (int)(j - (long long)l * g.ne);
+        const int l = row_of(j, g.ne), e = (int)(j - (long long)l * g.ne);
         const long long ct = (long long)l * g.nc + g.to[e], cf = (long long)l * g.nc + g.from[e];
         acc(&v_b[i], 0.5 * (s[ct] + s[cf]) * ob);
         const double q = 0.5 * v[i] * ob;
@@ -121,7 +121,7 @@ __global__ void kop_inner_adj(HGrid<double> g, const double *a, const double *b,
     if (i >= ns) return;
     const double ob = out_b[i];
     if (ob == 0.0) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const int n_edges = c < N_PENT ? 5 : 6;
     const long long nw = (long long)(g.nl + 1) * g.nc;
     for (int j = 0; j < n_edges; ++j) {
@@ -147,7 +147,7 @@ __global__ void kop_vflux_h_adj(HGrid<double> g, const double *flux_v, const dou
     if (i >= n) return;
     const double ob = out_b_u[i];
     if (ob == 0.0) return;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     b_vflux_h(g, flux_h, flux_v, zh, zv, fh_b, fv_b, zh_b, zv_b, l, e, ob);
 }
 
@@ -160,7 +160,7 @@ __global__ void kop_vflux_v_adj(HGrid<double> g, const double *flux_h, const dou
     if (i >= n) return;
     const double pb = out_b_w[i];
     if (pb == 0.0) return;
-    const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc);
+    const int k = row_of(i, g.nc), c = (int)(i - (long long)k * g.nc);
     const int nl = g.nl, n_edges = c < N_PENT ? 5 : 6;
     const double vw = (k == 0 || k == nl) ? 1.0 : 0.5;
     const double *z = zh + (long long)k * g.ne;
@@ -195,7 +195,7 @@ __global__ void kop_divv_tracer_adj(HGrid<double> g, const double *density, cons
     const double yb = out_b[i];
     if (yb == 0.0) return;
     const int nl = g.nl, n_oro = g.n_oro;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     const double hb = yb / g.volume[i];
@@ -273,7 +273,7 @@ __global__ void ka_gen_densities(VGrid vg, StepParams p, DState so, DState sn, D
     const long long ns = (long long)nl * nc;
     const long long q = gtid();
     if (q >= (long long)(p.n_const - 1) * nc) return;
-    const int slot = (int)(q / nc), i = (int)(q - (long long)slot * nc);
+    const int slot = row_of(q, nc), i = (int)(q - (long long)slot * nc);
     const int k = slot < p.n_cond ? slot : slot + 1;
     const int cond = p.n_cond;
     const bool sink = k < cond, heat = rk == 0 && k < cond;

@@ -126,7 +126,7 @@ __global__ void kd_n2_adv(HGrid<R> g, SView<R> sv, DiffBufs b, DiffScratch<R> s)
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int nl = g.nl, l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int nl = g.nl, l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc;
     auto theta = [&](int ll) {
         const long long q = (long long)ll * nc + c;
@@ -188,7 +188,7 @@ __global__ void kd_hor_visc(HGrid<R> g, R eff_hor_res, int gas, const double *te
     const R visc = rg * tke2hor(tke, eff_hor_res);
     b.visc[i] = double(visc);
     if (WDV) {
-        const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+        const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
         s.wdv[i] = visc * R(divv_h_cell(g, sv.u, l, c));
     }
 }
@@ -201,7 +201,7 @@ __global__ void kd_zt(HGrid<R> g, int gas, SView<R> sv, DiffScratch<R> s)
     const long long n = (long long)g.nl * g.nt, i = gtid();
     if (i >= n) return;
     const long long ns = (long long)g.nl * g.nc;
-    const int l = (int)(i / g.nt), t = (int)(i - (long long)l * g.nt);
+    const int l = row_of(i, g.nt), t = (int)(i - (long long)l * g.nt);
     const long long sb = (long long)l * g.nc;
     const int e0 = g.vort_i[t], e1 = g.vort_i[g.nt + t], e2 = g.vort_i[2 * g.nt + t];
     const R *v = s.vint, *rg = sv.rho + gas * ns;
@@ -220,7 +220,7 @@ __global__ void kd_zr(HGrid<R> g, int gas, SView<R> sv, DiffScratch<R> s)
     const long long n = (long long)g.nl * g.ne, i = gtid();
     if (i >= n) return;
     const long long ns = (long long)g.nl * g.nc;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     const long long tf = (long long)l * g.nt + g.dual_from[e], tt = (long long)l * g.nt + g.dual_to[e];
     const R af = g.dual_area_t[tf], at = g.dual_area_t[tt];
     const R raw = (af * s.tri[tf] + at * s.tri[tt]) / (af + at);
@@ -308,7 +308,7 @@ __global__ void kd_fric_h(HGrid<R> g, DiffGrid<R> dg, int n_const, int gas, SVie
     const long long n = (long long)g.nl * g.ne, i = gtid();
     if (i >= n) return;
     const long long ns = (long long)g.nl * g.nc, nw = (long long)(g.nl + 1) * g.nc, nc = g.nc;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     const int fr = g.from[e], to = g.to[e];
     const long long f = (long long)l * nc + fr, t = (long long)l * nc + to;
     R fa;
@@ -341,7 +341,7 @@ __global__ void kd_wdiff_a(HGrid<R> g, DiffGrid<R> dg, int gas, SView<R> sv, Dif
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int nl = g.nl, l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int nl = g.nl, l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc;
     const R up = l == 0 ? R(0) : sv.w[(long long)l * nc + c];
     const R lo = l == nl - 1 ? R(0) : sv.w[(long long)(l + 1) * nc + c];
@@ -360,7 +360,7 @@ __global__ void kd_wdiff_b(HGrid<R> g, DiffBufs b, DiffScratch<R> s)
 {
     const long long n = (long long)g.nl * g.ne, i = gtid();
     if (i >= n) return;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     const long long o = (long long)l * g.nc;
     s.flx[i] = R(0.5) * (R(b.visc[o + g.from[e]]) + R(b.visc[o + g.to[e]])) * grad_h(g, s.s2, l, e);
 }
@@ -371,7 +371,7 @@ __global__ void kd_wdiff_c(HGrid<R> g, DiffScratch<R> s)
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     s.s3[i] = R(divv_h_cell(g, s.flx, l, c));
 }
 
@@ -383,7 +383,7 @@ __global__ void kd_wdiff_d(HGrid<R> g, int n_const, SView<R> sv, DiffBufs b, Dif
     const long long n = (long long)(g.nl - 1) * g.nc, i = gtid();
     if (i >= n) return;
     const long long ns = (long long)g.nl * g.nc, nc = g.nc;
-    const int k = (int)(i / nc) + 1, c = (int)(i - (long long)(k - 1) * nc);
+    const int k = row_of(i, nc) + 1, c = (int)(i - (long long)(k - 1) * nc);
     const long long up = (long long)(k - 1) * nc + c, lo = (long long)k * nc + c;
     R fa = (s.s1[up] - s.s1[lo]) / g.nd_v[(long long)k * nc + c];
     fa += R(0.5) * (s.s3[up] + s.s3[lo]);
@@ -397,7 +397,7 @@ __global__ void kd_dissipation(HGrid<R> g, int n_const, SView<R> sv, DiffBufs b)
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc, nw = (long long)(g.nl + 1) * nc;
     const int n_edges = c < N_PENT ? 5 : 6;
     R r = R(0);
@@ -423,7 +423,7 @@ __global__ void kd_pbl_hs_cell(HGrid<R> g, DiffGrid<R> dg, int gas, int moist, c
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int nl = g.nl, l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int nl = g.nl, l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const R exner = g.exner_bg[i] + sv.exner_pert[i];
     const R p = R(P_0) * pow(exner, R(C_D_P / R_D));
     s.hs_p[i] = p;
@@ -451,7 +451,7 @@ __global__ void kd_pbl_hs(HGrid<R> g, SView<R> sv, DiffBufs b, DiffScratch<R> s)
     const long long n = (long long)g.nl * g.ne, i = gtid();
     if (i >= n) return;
     const long long nw = (long long)(g.nl + 1) * g.nc;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     const long long o = (long long)l * g.nc;
     const R pressure = R(0.5) * (s.hs_p[o + g.from[e]] + s.hs_p[o + g.to[e]]);
     const R pressure_sfc = R(0.5) * (s.hs_ps[g.from[e]] + s.hs_ps[g.to[e]]);
@@ -485,7 +485,7 @@ __global__ void kd_hs_rad(long long ns, int nc, int gas, const double *lat, cons
 {
     const long long i = gtid();
     if (i >= ns) return;
-    const int c = (int)(i % nc);
+    const int c = (int)((unsigned)i % (unsigned)nc);
     if (!cov[c]) return;
     const double rg = so.rho[gas * ns + i], t = temperature[i];
     const double pressure = rg * R_D * t;
@@ -550,7 +550,7 @@ __global__ void kd_sdiff_flux(HGrid<R> g, SFields<R> sf, DiffScratch<R> s)
     const long long nc = g.nc;
     const int nl = g.nl;
     if (i < nh) {
-        const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+        const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
         const int fr = g.from[e], to = g.to[e];
         const long long o = (long long)l * nc;
         const R nd = g.nd_h[i];
@@ -588,7 +588,7 @@ __global__ void kd_sdiff_flux(HGrid<R> g, SFields<R> sf, DiffScratch<R> s)
         }
     } else if (i < nh + nv) {
         const long long rv = i - nh;
-        const int k = (int)(rv / nc) + 1, c = (int)(rv - (long long)(k - 1) * nc);
+        const int k = row_of(rv, nc) + 1, c = (int)(rv - (long long)(k - 1) * nc);
         const long long up = (long long)(k - 1) * nc + c, lo = (long long)k * nc + c;
         const R nd = g.nd_v[lo], rnd = EXACT ? R(0) : R(1) / nd;
         for (int q = 0; q < sf.nf; ++q) {
@@ -610,7 +610,7 @@ __global__ void kd_sdiff_div(HGrid<R> g, SFields<R> sf, DiffScratch<R> s)
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int nl = g.nl, n_oro = g.n_oro, l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int nl = g.nl, n_oro = g.n_oro, l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long nc = g.nc, ne = g.ne, nh = (long long)nl * ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     int ej[6];
@@ -704,7 +704,7 @@ void diffusion_momentum(Context *c, const StepParams &p, const HGrid<R> &g, cons
         }
         {
             ProfScope ps(c, "kd_tri_vort");
-            k_tri_vort<R><<<dnb((long long)c->nl * c->nt), 256, 0, st>>>(g, sv.u, s.tri);
+            k_tri_vort<R><<<dim3(dnb(c->nt), (unsigned)c->nl), 256, 0, st>>>(g, sv.u, s.tri);
         }
         {
             ProfScope ps(c, "kd_zt");

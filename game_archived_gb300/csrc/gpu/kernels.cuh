@@ -511,10 +511,10 @@ __global__ void k_make_shadow(long long n_rho, long long ns, long long nw, long 
 template <typename R>
 __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_tri_vort(HGrid<R> g, const R *u, R *tri_vort)
 {
-    const long long n = (long long)g.nl * g.nt;
-    const long long i = gtid();
-    if (i >= n) return;
-    const int l = (int)(i / g.nt), t = (int)(i - (long long)l * g.nt);
+    const LayerPoint pt_ = layer_point(g.nt);
+    if (!pt_.in) return;
+    const long long i = pt_.i;
+    const int l = pt_.l, t = pt_.x;
     R acc = R(0);
     for (int j = 0; j < 3; ++j) {
         const int e = g.vort_i[j * g.nt + t];
@@ -565,10 +565,10 @@ template <typename R>
 __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_edge_vort(HGrid<R> g, const R *u, const R *w, const R *rho_gas, const R *tri_vort, R *zh, R *zv,
                             R *flux_h)
 {
-    const long long n = (long long)(g.nl + 1) * g.ne;
-    const long long i = gtid();
-    if (i >= n) return;
-    const int k = (int)(i / g.ne), e = (int)(i - (long long)k * g.ne);
+    const LayerPoint pt_ = layer_point(g.ne);
+    if (!pt_.in) return;
+    const long long i = pt_.i;
+    const int k = pt_.l, e = pt_.x;
     const int nl = g.nl, nc = g.nc, ne = g.ne;
     const int fr = g.from[e], to = g.to[e];
     /* tangential component at level k */
@@ -616,9 +616,10 @@ template <typename R>
 __global__ void k_cell_kinetic(HGrid<R> g, const R *u, const R *w, const R *rho_gas, R *v2, R *flux_v)
 {
     const long long ns = (long long)g.nl * g.nc;
-    const long long i = gtid();
-    if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const LayerPoint pt_ = layer_point(g.nc);
+    if (!pt_.in) return;
+    const long long i = pt_.i;
+    const int l = pt_.l, c = pt_.x;
     const int n_edges = c < N_PENT ? 5 : 6;
     R acc = R(0);
     for (int j = 0; j < n_edges; ++j) {
@@ -811,10 +812,10 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
                              const R *flux_v, const R *zh, const R *zv, const R *v2, double new_w, double old_w,
                              const double *fric_u, const float4 *pc)
 {
-    const long long n = (long long)g.nl * g.ne;
-    const long long i = gtid();
-    if (i >= n) return;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const LayerPoint pt_ = layer_point(g.ne);
+    if (!pt_.in) return;
+    const long long i = pt_.i;
+    const int l = pt_.l, e = pt_.x;
     R P, pgo;
     if (PG) {
         if constexpr (sizeof(R) == sizeof(float))
@@ -860,10 +861,10 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
                              const R *flux_h, const R *zh, const R *v2, double new_w, double old_w,
                              const double *fric_w, const float4 *pc)
 {
-    const long long n = (long long)(g.nl + 1) * g.nc;
-    const long long i = gtid();
-    if (i >= n) return;
-    const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc);
+    const LayerPoint pt_ = layer_point(g.nc);
+    if (!pt_.in) return;
+    const long long i = pt_.i;
+    const int k = pt_.l, c = pt_.x;
     const int nl = g.nl;
     R pvt = R(0);
     if (ADV) {
@@ -1007,10 +1008,11 @@ __global__ void __launch_bounds__(128) k_scalar_tend2(HGrid<R> g, StepParams p, 
                                                       IrrTerms irr)
 {
     const long long ns = (long long)g.nl * g.nc;
-    const long long i = gtid();
-    if (i >= ns) return;
+    const LayerPoint pt_ = layer_point(g.nc);
+    if (!pt_.in) return;
+    const long long i = pt_.i;
     const int nl = g.nl, n_oro = g.n_oro;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = pt_.l, c = pt_.x;
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     const int cond = p.n_cond;

@@ -16,6 +16,30 @@ namespace {
 /* ------------------------------------------------------------ utilities */
 __device__ __forceinline__ long long gtid() { return (long long)blockIdx.x * blockDim.x + threadIdx.x; }
 
+/* The point of a kernel over [layer][entity] fields with a two-dimensional
+ * grid (layer_grid): y is the layer, x the entity, so no thread divides its
+ * index by the row length (a 64-bit division, some seventy instructions
+ * before the first load).  RES_ID 6, mixed: k_momentum_h 89.4 -> 78.7 us,
+ * k_edge_vort 63.9 -> 56.2 us, k_cell_kinetic 24.7 -> 21.7 us.  k_waves_apply
+ * and the sedimentation heat lose with it (43.7 -> 47.1, 43.4 -> 46.8 us: the
+ * shorter last block of every layer) and take row_of. */
+struct LayerPoint {
+    int l, x;    /* layer (or level), entity */
+    long long i; /* l * n + x */
+    bool in;
+};
+__device__ __forceinline__ LayerPoint layer_point(int n)
+{
+    const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x), l = (int)blockIdx.y;
+    return {l, x, (long long)l * n + x, x < n};
+}
+/* the row of index i in rows of n, for the kernels with a one-dimensional
+ * grid: a 32-bit division (every index is below 2^31: the index maps are
+ * 32-bit).  kd_sdiff_div 345 -> 216 us, kd_fric_h 197 -> 168 us, kd_n2_adv
+ * 104 -> 80 us (RES_ID 6, mixed).  The column kernels keep the 64-bit form,
+ * once per column: k_tracers_pcr was slower with the other (181 -> 216 us). */
+__device__ __forceinline__ int row_of(long long i, int n) { return (int)((unsigned)i / (unsigned)n); }
+
 /* FP64 reciprocal for the mixed path (the FP64 path divides exactly as the
  * reference).  The seed is the hardware's approximate reciprocal (PTX
  * rcp.approx.ftz.f64; relative error below 2^-20, measured on GB300 over

@@ -18,7 +18,7 @@ __global__ void k_op_grad_h(G g, const double *f, double *u, int with_correction
 {
     const long long n = (long long)g.nl * g.ne, i = gtid();
     if (i >= n) return;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     if (with_correction) {
         u[i] = grad_h(g, f, l, e);
     } else {
@@ -31,7 +31,7 @@ __global__ void k_op_grad_v(G g, const double *f, double *w)
 {
     const long long n = (long long)(g.nl - 1) * g.nc, i = gtid();
     if (i >= n) return;
-    const int k = (int)(i / g.nc) + 1, c = (int)(i - (long long)(k - 1) * g.nc);
+    const int k = row_of(i, g.nc) + 1, c = (int)(i - (long long)(k - 1) * g.nc);
     w[(long long)k * g.nc + c] = grad_v(g, f, k, c);
 }
 
@@ -40,7 +40,7 @@ __global__ void k_op_cov_to_con(G g, const double *w, double *u)
 {
     const long long n = (long long)g.n_oro * g.ne, i = gtid();
     if (i >= n) return;
-    const int l = (int)(i / g.ne) + (g.nl - g.n_oro), e = (int)(i % g.ne);
+    const int l = row_of(i, g.ne) + (g.nl - g.n_oro), e = (int)((unsigned)i % (unsigned)g.ne);
     const int fr = g.from[e], to = g.to[e];
     double c = ipw_at(g, 6, l, fr) * w[(long long)l * g.nc + fr];
     c += ipw_at(g, 6, l, to) * w[(long long)l * g.nc + to];
@@ -58,7 +58,7 @@ __global__ void k_op_stv_h(G g, const double *s, const double *v, double *out, i
 {
     const long long n = (long long)g.nl * g.ne, i = gtid();
     if (i >= n) return;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     const long long o = (long long)l * g.nc;
     double sv;
     if (upstream) sv = v[i] >= 0.0 ? s[o + g.from[e]] : s[o + g.to[e]];
@@ -82,7 +82,7 @@ __global__ void k_op_divv(G g, const double *in_u, const double *density, const 
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const int n_edges = c < N_PENT ? 5 : 6, nl = g.nl, n_oro = g.n_oro;
     const long long nc = g.nc;
     double comp_h = 0.0;
@@ -130,7 +130,7 @@ __global__ void k_op_inner(G g, const double *aw, const double *au, const double
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const int n_edges = c < N_PENT ? 5 : 6;
     double r = 0;
     for (int j = 0; j < n_edges; ++j) {
@@ -147,7 +147,7 @@ __global__ void k_op_rel_vort(G g, const double *u, const double *w, const doubl
 {
     const long long n = (long long)(g.nl + 1) * g.ne, i = gtid();
     if (i >= n) return;
-    const int k = (int)(i / g.ne), e = (int)(i - (long long)k * g.ne);
+    const int k = row_of(i, g.ne), e = (int)(i - (long long)k * g.ne);
     zh[i] = rel_vort_tangential(g, u, w, k, e);
     if (k < g.nl) {
         const int tf = g.dual_from[e], tt = g.dual_to[e];
@@ -163,7 +163,7 @@ __global__ void k_op_pot_vort(G g, const double *rzh, const double *rzv, const d
 {
     const long long n = (long long)(g.nl + 1) * g.ne, i = gtid();
     if (i >= n) return;
-    const int k = (int)(i / g.ne), e = (int)(i - (long long)k * g.ne);
+    const int k = row_of(i, g.ne), e = (int)(i - (long long)k * g.ne);
     const int nl = g.nl, nc = g.nc, ne = g.ne, fr = g.from[e], to = g.to[e];
     double pv = rzh[i] + g.f_vec[e];
     if (rho) {
@@ -199,7 +199,7 @@ __global__ void k_op_vflux_h(G g, const double *fw, const double *fu, const doub
 {
     const long long n = (long long)g.nl * g.ne, i = gtid();
     if (i >= n) return;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     out_u[i] = vorticity_flux_h(g, fu, fw, zh, zv, l, e);
 }
 
@@ -207,7 +207,7 @@ __global__ void k_op_vflux_v(G g, const double *fu, const double *zh, double *ou
 {
     const long long n = (long long)(g.nl + 1) * g.nc, i = gtid();
     if (i >= n) return;
-    const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc), nl = g.nl;
+    const int k = row_of(i, g.nc), c = (int)(i - (long long)k * g.nc), nl = g.nl;
     const int n_edges = c < N_PENT ? 5 : 6;
     const double vw = (k == 0 || k == nl) ? 1 : 0.5;
     const double *z = zh + (long long)k * g.ne;
@@ -254,7 +254,7 @@ __global__ void k_op_add_vertical_divv(G g, const double *w, double *out)
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const long long up = (long long)l * g.nc + c, lo = (long long)(l + 1) * g.nc + c;
     const double contra_upper = l == 0 ? 0.0 : w[up];
     const double contra_lower = l == g.nl - 1 ? 0.0 : w[lo];
@@ -321,7 +321,7 @@ void op_inner_product(Context *c, const double *a, const double *b, double *out)
 void op_rel_vort(Context *c, const double *wind, double *tri, double *curl)
 {
     const long long off = (long long)(c->nl + 1) * c->nc, coff = (long long)(c->nl + 1) * c->ne;
-    k_tri_vort<double><<<nb((long long)c->nl * c->nt), 256, 0, c->stream>>>(c->hg64, wind + off, tri);
+    k_tri_vort<double><<<dim3(nb(c->nt), (unsigned)c->nl), 256, 0, c->stream>>>(c->hg64, wind + off, tri);
     k_op_rel_vort<<<nb(coff), 256, 0, c->stream>>>(c->hg64, wind + off, wind, tri, curl, curl + coff);
     c->kernel_launches += 2;
 }

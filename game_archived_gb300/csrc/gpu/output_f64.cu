@@ -304,7 +304,7 @@ __global__ void k_curl_to_cells(G g, const double *zv, double *out)
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const int n_edges = c < N_PENT ? 5 : 6;
     double r = 0;
     for (int j = 0; j < n_edges; ++j) r += 0.5 * ipw_at(g, j, l, c) * zv[(long long)l * g.ne + g.adj[(long long)j * g.nc + c]];
@@ -316,7 +316,7 @@ __global__ void k_edges_to_cells(G g, const double *ue, double *out)
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const int n_edges = c < N_PENT ? 5 : 6;
     double r = 0;
     for (int j = 0; j < n_edges; ++j) r += 0.5 * ipw_at(g, j, l, c) * ue[(long long)l * g.ne + g.adj[(long long)j * g.nc + c]];
@@ -339,7 +339,7 @@ __global__ void k_uv_at_edge(G g, OutGrid og, const double *u, double *ue, doubl
 {
     const long long n = (long long)g.nl * g.ne, i = gtid();
     if (i >= n) return;
-    const int l = (int)(i / g.ne), e = (int)(i - (long long)l * g.ne);
+    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     const double w0 = u[i];
     const double w1 = tangential(g, u + (long long)l * g.ne, e);
     passive_turn(w0, w1, -og.direction[e], &ue[i], &ve[i]);
@@ -374,7 +374,7 @@ __global__ void k_epv_pv(G g, VGrid vg, const double *pzh, const double *pzv, do
     const double *zv = vg.z_v;
     if (i >= nw) {
         const long long ih = i - nw;
-        const int l = (int)(ih / ne), e = (int)(ih - (long long)l * ne);
+        const int l = row_of(ih, ne), e = (int)(ih - (long long)l * ne);
         const int f = g.from[e], t = g.to[e];
         const long long a = (long long)l * nc, b = (long long)(l + 1) * nc;
         const double zi = g.z_h[ih];
@@ -386,7 +386,7 @@ __global__ void k_epv_pv(G g, VGrid vg, const double *pzh, const double *pzv, do
         else lower = 0.5 * (zi - g.z_h[ih + ne]) / lt;
         out[i] = upper * pzh[(long long)l * ne + e] + lower * pzh[(long long)(l + 1) * ne + e];
     } else {
-        const int k = (int)(i / nc), c = (int)(i - (long long)k * nc);
+        const int k = row_of(i, nc), c = (int)(i - (long long)k * nc);
         double r = 0;
         if (k == 0) {
             for (int j = 0; j < 6; ++j) r += 0.5 * ipw_at(g, j, 0, c) * pzv[g.adj[(long long)j * nc + c]];
@@ -410,7 +410,7 @@ __global__ void k_inner_tangential(G g, const double *aw, const double *au, cons
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
-    const int l = (int)(i / g.nc), c = (int)(i - (long long)l * g.nc);
+    const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
     const double *bl = bu + (long long)l * g.ne, *al = au + (long long)l * g.ne;
     double r = 0;
     for (int j = 0; j < 6; ++j) {
@@ -503,7 +503,7 @@ __global__ void k_levels_to_ref(const int *c_n2o, int nc, const double *src, dou
 {
     const long long i = gtid();
     if (i >= (long long)N_PRESSURE_LEVELS * nc) return;
-    const int j = (int)(i / nc), c = (int)(i - (long long)j * nc);
+    const int j = row_of(i, nc), c = (int)(i - (long long)j * nc);
     dst[(long long)c_n2o[c] * N_PRESSURE_LEVELS + j] = src[i];
 }
 

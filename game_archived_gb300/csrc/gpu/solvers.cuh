@@ -136,9 +136,11 @@ __global__ void k_waves_layer(VGrid vg, StepParams p, DState so, DState sn, DSta
 __global__ void k_waves_rows(VGrid vg, StepParams p, DState so, DState st, WavesWork ww)
 {
     const int nc = vg.nc, nl = vg.nl;
-    const long long n = (long long)(nl - 1) * nc, q = gtid();
-    if (q >= n) return;
-    const int j = (int)(q / nc);
+    const long long n = (long long)(nl - 1) * nc;
+    const LayerPoint pt_ = layer_point(nc);
+    if (!pt_.in) return;
+    const long long q = pt_.i;
+    const int j = pt_.l;
     const long long ns = (long long)nl * nc, gp = p.n_cond * ns;
     const long long b = q, lo = q + nc, wi = q + nc;
     const double dt = p.dt, iw = p.impl_thermo_weight, dt2 = dt * dt;
@@ -178,9 +180,11 @@ __global__ void k_waves_rows(VGrid vg, StepParams p, DState so, DState st, Waves
 __global__ void k_waves_rows_mixed(VGrid vg, StepParams p, DState so, DState st, WavesWork ww)
 {
     const int nc = vg.nc, nl = vg.nl;
-    const long long n = (long long)(nl - 1) * nc, q = gtid();
-    if (q >= n) return;
-    const int j = (int)(q / nc);
+    const long long n = (long long)(nl - 1) * nc;
+    const LayerPoint pt_ = layer_point(nc);
+    if (!pt_.in) return;
+    const long long q = pt_.i;
+    const int j = pt_.l;
     const long long ns = (long long)nl * nc, gp = p.n_cond * ns;
     const long long b = q, lo = q + nc, wi = q + nc;
     const double dt = p.dt;
@@ -294,9 +298,10 @@ template <bool EXACT>
 __global__ void k_waves_apply(VGrid vg, StepParams p, DState so, DState sn, WavesWork ww, Shadow sh)
 {
     const int nc = vg.nc, nl = vg.nl;
-    const long long ns = (long long)nl * nc, b = gtid();
+    const long long ns = (long long)nl * nc;
+    const long long b = gtid();
     if (b >= ns) return;
-    const int j = (int)(b / nc);
+    const int j = row_of(b, nc);
     const long long gp = p.n_cond * ns;
     const double dt = p.dt;
     const double *sol = ww.r;

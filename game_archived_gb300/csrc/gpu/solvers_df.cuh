@@ -189,9 +189,10 @@ __global__ void k_tracers_sedheat_df(VGrid vg, StepParams p, DState so, DState s
                                      TracerWork tw, DfGrid dg, double *sed_heat)
 {
     const int nc = vg.nc, nl = vg.nl;
-    const long long ns = (long long)nl * nc, b = gtid();
+    const long long ns = (long long)nl * nc;
+    const long long b = gtid();
     if (b >= ns) return;
-    const int j = (int)(b / nc), i = (int)(b - (long long)j * nc);
+    const int j = row_of(b, nc), i = (int)(b - (long long)j * nc);
     const int n_cond = p.n_cond < SEDHEAT_MAX_COND ? p.n_cond : SEDHEAT_MAX_COND;
     /* enthalpy flux of constituent k at interface jj (below layer jj) */
     /* a condensate's flux is c_p T rho w A with rho its upstream density:
@@ -295,9 +296,11 @@ __global__ void k_waves_layer_df(VGrid vg, StepParams p, DState so, DState sn, D
 __global__ void k_waves_rows_df(VGrid vg, StepParams p, DState so, DState st, WavesWork ww, DfGrid dg)
 {
     const int nc = vg.nc, nl = vg.nl;
-    const long long n = (long long)(nl - 1) * nc, q = gtid();
-    if (q >= n) return;
-    const int j = (int)(q / nc);
+    const long long n = (long long)(nl - 1) * nc;
+    const LayerPoint pt_ = layer_point(nc);
+    if (!pt_.in) return;
+    const long long q = pt_.i;
+    const int j = pt_.l;
     const long long ns = (long long)nl * nc, gp = p.n_cond * ns;
     const long long b = q, lo = q + nc, wi = q + nc;
     const df dt = df_from_double(p.dt), inv_dt = df_from_double(p.inv_dt);
@@ -401,9 +404,10 @@ __global__ void __launch_bounds__(WAVES_BLOCK) k_waves_thomas_df(int nc, WavesWo
 __global__ void k_waves_apply_df(VGrid vg, StepParams p, DState so, DState sn, WavesWork ww, DfGrid dg, Shadow sh)
 {
     const int nc = vg.nc, nl = vg.nl;
-    const long long ns = (long long)nl * nc, b = gtid();
+    const long long ns = (long long)nl * nc;
+    const long long b = gtid();
     if (b >= ns) return;
-    const int j = (int)(b / nc);
+    const int j = row_of(b, nc);
     const long long gp = p.n_cond * ns;
     const df dt = df_from_double(p.dt);
     /* the new density as the FP64 old value plus the increment

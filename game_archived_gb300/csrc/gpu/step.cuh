@@ -15,6 +15,8 @@
 namespace game {
 
 inline unsigned nblocks(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
+/* the grid of a kernel over [layers][n] (layer_point) */
+inline dim3 layer_grid(int layers, int n, int bs) { return dim3(nblocks(n, bs), (unsigned)layers); }
 
 template <typename R>
 HGrid<R> &hgrid(Context *c);
@@ -112,7 +114,7 @@ static void launch_momentum_v(Context *c, const StepParams &p, const Views<R> &v
     ProfScope ps(c, "k_momentum_v");
     const double *fric_w = p.irr ? c->dbuf->fric : nullptr;
     const float4 *pc = sizeof(R) == sizeof(float) && PG ? c->pg_cell : nullptr;
-    k_momentum_v<R, ADV, PG><<<nblocks((long long)(c->nl + 1) * c->nc, 256), 256, 0, c->stream>>>(
+    k_momentum_v<R, ADV, PG><<<layer_grid(c->nl + 1, c->nc, 256), 256, 0, c->stream>>>(
         g, p, v.sv, st->ds.w, w.P_v, w.pvt_v, w.v2g_v, w.flux_h, w.zh, w.v2, new_w, old_w, fric_w, pc);
     c->kernel_launches++;
 }
@@ -126,7 +128,7 @@ static void launch_momentum_h(Context *c, const StepParams &p, const Views<R> &v
     ProfScope ps(c, "k_momentum_h");
     const double *fric_u = p.irr ? c->dbuf->fric + (long long)(c->nl + 1) * c->nc : nullptr;
     const float4 *pc = sizeof(R) == sizeof(float) && PG ? c->pg_cell : nullptr;
-    k_momentum_h<R, ADV, PG><<<nblocks((long long)c->nl * c->ne, 256), 256, 0, c->stream>>>(
+    k_momentum_h<R, ADV, PG><<<layer_grid(c->nl, c->ne, 256), 256, 0, c->stream>>>(
         g, p, v.sv, sn->ds.u, v.sh.u, so->ds.u, st->ds.u, w.P_h, w.pg_old_h, w.pvt_h, w.v2g_h, w.flux_h, w.flux_v,
         w.zh, w.zv, w.v2, new_w, old_w, fric_u, pc);
     c->kernel_launches++;
@@ -156,7 +158,7 @@ void launch_waves(Context *c, const StepParams &p, StateMirror *so, StateMirror 
             }
             {
                 ProfScope ps(c, "k_waves_rows");
-                k_waves_rows_df<<<nblocks((long long)(c->nl - 1) * c->nc, 256), 256, 0, c->stream>>>(
+                k_waves_rows_df<<<layer_grid(c->nl - 1, c->nc, 256), 256, 0, c->stream>>>(
                     c->vg, p, so->ds, st->ds, ww, c->dfg);
             }
             {
@@ -179,7 +181,7 @@ void launch_waves(Context *c, const StepParams &p, StateMirror *so, StateMirror 
     }
     {
         ProfScope ps(c, "k_waves_rows");
-        const unsigned nb = nblocks((long long)(c->nl - 1) * c->nc, 256);
+        const dim3 nb = layer_grid(c->nl - 1, c->nc, 256);
         if (EXACT)
             k_waves_rows<<<nb, 256, 0, c->stream>>>(c->vg, p, so->ds, st->ds, ww);
         else
@@ -308,16 +310,16 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
         if (adv) {
             {
                 ProfScope ps(c, "k_tri_vort");
-                k_tri_vort<R><<<nblocks((long long)c->nl * c->nt, bs), bs, 0, c->stream>>>(g, v.sv.u, w.tri_vort);
+                k_tri_vort<R><<<layer_grid(c->nl, c->nt, bs), bs, 0, c->stream>>>(g, v.sv.u, w.tri_vort);
             }
             {
                 ProfScope ps(c, "k_edge_vort");
-                k_edge_vort<R><<<nblocks((long long)(c->nl + 1) * c->ne, bs), bs, 0, c->stream>>>(
+                k_edge_vort<R><<<layer_grid(c->nl + 1, c->ne, bs), bs, 0, c->stream>>>(
                     g, v.sv.u, v.sv.w, rho_gas, w.tri_vort, w.zh, w.zv, w.flux_h);
             }
             {
                 ProfScope ps(c, "k_cell_kinetic");
-                k_cell_kinetic<R><<<nblocks(ns, bs), bs, 0, c->stream>>>(g, v.sv.u, v.sv.w, rho_gas, w.v2, w.flux_v);
+                k_cell_kinetic<R><<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(g, v.sv.u, v.sv.w, rho_gas, w.v2, w.flux_v);
             }
             c->kernel_launches += 3;
         }
@@ -347,11 +349,11 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
             ProfScope ps(c, "k_scalar_tend");
             if (p.irr) {
                 const DiffBufs &b = *c->dbuf;
-                k_scalar_tend2<R, true><<<nblocks(ns, 128), 128, 0, c->stream>>>(
+                k_scalar_tend2<R, true><<<layer_grid(c->nl, c->nc, 128), 128, 0, c->stream>>>(
                     g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, rk,
                     IrrTerms{b.hdiss, b.tdh, b.rad, b.mdt});
             } else {
-                k_scalar_tend2<R, false><<<nblocks(ns, 128), 128, 0, c->stream>>>(
+                k_scalar_tend2<R, false><<<layer_grid(c->nl, c->nc, 128), 128, 0, c->stream>>>(
                     g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, rk,
                     IrrTerms{});
             }

@@ -32,12 +32,12 @@ __global__ void k_sub_pgrad(HGrid<double> g, StepParams p, SView<double> s, doub
     if (i >= n) return;
     double nl, lt;
     if (i < nw) {
-        const int k = (int)(i / g.nc), c = (int)(i - (long long)k * g.nc);
+        const int k = row_of(i, g.nc), c = (int)(i - (long long)k * g.nc);
         if (k == 0 || k == g.nl) return;
         pgrad_v_parts(g, p, s, k, c, nl, lt);
     } else {
         const long long j = i - nw;
-        const int l = (int)(j / g.ne), e = (int)(j - (long long)l * g.ne);
+        const int l = row_of(j, g.ne), e = (int)(j - (long long)l * g.ne);
         pgrad_h_parts(g, p, s, l, e, nl, lt);
     }
     nl_out[i] = nl;
@@ -81,7 +81,7 @@ __global__ void k_sub_vec_tend(int nl, int nc, int ne, double *tend, const doubl
     const long long i = gtid();
     if (i >= n) return;
     if (i < nw) {
-        const int k = (int)(i / nc);
+        const int k = row_of(i, nc);
         if (k == 0 || k == nl) {
             tend[i] = 0.0;
             return;
@@ -148,7 +148,7 @@ void sub_scalar_tendencies(Context *c, const StepParams &p, StateMirror *sn, Sta
 {
     const Views<double> v = views<double>(c, sn);
     k_theta<double><<<nblocks(c->ns, 256), 256, 0, c->stream>>>(c->nl, c->nc, c->n_cond, v.sv, theta);
-    k_scalar_tend2<double, false><<<nblocks(c->ns, 128), 128, 0, c->stream>>>(
+    k_scalar_tend2<double, false><<<layer_grid(c->nl, c->nc, 128), 128, 0, c->stream>>>(
         c->hg64, p, v.sv, st->ds, theta, cp_ice, cp_water, pt_rates, pt_heat, sed_heat, c->inv_vol, rk, IrrTerms{});
     c->kernel_launches += 2;
 }
