@@ -97,6 +97,11 @@ StepParams params_from_config(Context *c, const void *config, double dt)
     p.inv_dt = 1.0 / dt;
     p.k_rows = 1.0 / (p.impl_thermo_weight * dt * dt * C_D_P);
     p.k_rows2 = 0.5 / (p.impl_thermo_weight * dt * C_D_P);
+    p.rows_a = p.impl_thermo_weight * (dt * dt) * C_D_P;
+    p.r_rows_a = 1.0 / p.rows_a;
+    p.rows_b = p.impl_thermo_weight * dt * C_D_P;
+    p.r_rows_b = 1.0 / p.rows_b;
+    p.half_inv_dt = 0.5 / dt;
     p.cur_hor = 0.5 + p.impl_thermo_weight;
     p.old_hor = 1.0 - (0.5 + p.impl_thermo_weight);
     p.cur_ver = 1.0 - p.impl_thermo_weight;

@@ -47,6 +47,7 @@
 #include "adj_ops.h"
 #include "diag.h"
 #include "ops.h"
+#include "solvers.cuh"
 
 namespace game {
 namespace {
@@ -86,11 +87,6 @@ __global__ void ku_dual_part(long long n, const Dual *in, double *d)
     const long long i = gtid();
     if (i < n) d[i] = in[i].d;
 }
-__global__ void ku_dden(long long n, double dt, const double *dc, double *dden)
-{
-    const long long i = gtid();
-    if (i < n) dden[i] = 1.0 + dt * dc[i];
-}
 /* flux_v levels 0 and L (never written by the step) */
 template <class T>
 __global__ void ku_fv_bounds(int nc, int nl, const double *src, T *fv)
@@ -126,7 +122,8 @@ struct AdjState {
     StepBufs<double> Z;          /* bars of one step */
     StepBufs<Dual> D;            /* tangent-linear run */
     double *rn_b = nullptr, *rtn_b = nullptr;
-    double *dden = nullptr, *fv_bounds = nullptr; /* (L+1) Nc */
+    double *dden = nullptr, *r_dden = nullptr; /* damping denominators and their reciprocals [L-1][Nc] */
+    double *fv_bounds = nullptr;               /* (L+1) Nc */
     /* checkpoints of every ck_every-th step start and of the window's end,
      * (state block + 3 Vt [+ S]) each, and one scratch slot for the start
      * of a step recomputed from the nearest checkpoint before it */
@@ -232,7 +229,8 @@ int ensure_adj(Context *c)
     a->nwi = (long long)(c->nl - 1) * c->nc;
     bool ok = alloc_step(a, a->B) && alloc_step(a, a->Z) && alloc_step(a, a->D);
     ok = ok && (a->rn_b = aalloc<double>(a, a->ns)) && (a->rtn_b = aalloc<double>(a, a->ns));
-    ok = ok && (a->dden = aalloc<double>(a, a->nwi)) && (a->fv_bounds = aalloc<double>(a, a->nw));
+    ok = ok && (a->dden = aalloc<double>(a, a->nwi)) && (a->r_dden = aalloc<double>(a, a->nwi))
+         && (a->fv_bounds = aalloc<double>(a, a->nw));
     ok = ok && (a->obj_w = aalloc<double>(a, c->nc)) && (a->obj_p = aalloc<double>(a, c->nc))
          && (a->obj_out = aalloc<double>(a, 1)) && (a->bar_state = aalloc<double>(a, a->nblk));
     for (int k = 0; k < 4; ++k)
@@ -272,6 +270,30 @@ bool moist_of(const AdjState *a) { return a->n_const > 1; }
  * and, moist, the sedimentation heat (S) */
 long long ck_stride(const AdjState *a) { return a->nblk + 3 * a->nv + (moist_of(a) ? a->ns : 0); }
 
+/* the sound-wave solve with the FP64 step's kernels, its work kept on the
+ * tape (wl, wr); the sweep also keeps the undamped solution, which the step
+ * does not */
+void waves_fwd(Context *c, AdjState *a, int rk, DState so, DState sn, DState tend, double *wl, double *wr, DState out)
+{
+    const long long ns = a->ns, m = a->nwi;
+    cudaStream_t st = c->stream;
+    WavesWork w{};
+    w.alpha = wl + WL_A * ns; w.beta = wl + WL_B * ns; w.gam = wl + WL_G * ns;
+    w.rho_expl = wl + WL_REXP * ns; w.rt_expl = wl + WL_RTEXP * ns; w.tp_expl = wl + WL_TPEXP * ns;
+    w.ep_expl = wl + WL_EPEXP * ns; w.thl = wl + WL_THL * ns;
+    w.c = wr + WR_C * m; w.d = wr + WR_D * m; w.e = wr + WR_E * m; w.r = wr + WR_R * m;
+    w.th_int = wr + WR_TH * m; w.rho_io = wr + WR_RIO * m; w.r_rho_io = wr + WR_RRIO * m;
+    k_waves_layer<true><<<nbk(ns), 256, 0, st>>>(c->vg, a->p, so, sn, tend, w, rk);
+    k_waves_rows<<<layer_grid(c->nl - 1, c->nc, 256), 256, 0, st>>>(c->vg, a->p, so, tend, w);
+    if (c->nl == 26)
+        fa_waves_thomas_fixed<26><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, a->dden, a->r_dden, wr);
+    else
+        fa_waves_thomas<double><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, wr);
+    w.r = wr + WR_SOL * m; /* what the step leaves in r */
+    k_waves_apply<true><<<nbk(ns), 256, 0, st>>>(c->vg, a->p, so, out, w, Shadow{});
+    fa_w_bounds<<<nbk(c->nc), 256, 0, st>>>(c->nc, c->nl, so.w, out.w);
+}
+
 /* ----------------------------------------------------------- step forward */
 /* the substage rk of a step: sn its input state (so at rk 0), out its
  * output (sn1, sn2); sed_prev the previous step's sedimentation heat */
@@ -287,7 +309,17 @@ void substage_fwd(Context *c, AdjState *a, StepBufs<T> &B, int rk, bool first, c
     AState<T> so = view(a, B.so), sn = view(a, rk ? B.sn1 : B.so), out = view(a, rk ? B.sn2 : B.sn1);
     const bool adv = rk == 1 || first;
     const double new_w = rk ? 0.5 : 1.0, old_w = 1.0 - new_w;
-    if (adv) {
+    /* the FP64 step's own kernels where they take their fields separately */
+    constexpr bool PLAIN = sizeof(T) == sizeof(double);
+    if constexpr (PLAIN) {
+        if (adv) {
+            k_tri_vort<double><<<layer_grid(c->nl, c->nt, 256), 256, 0, st>>>(g, sn.u, B.tri[rk]);
+            k_edge_vort<double><<<layer_grid(c->nl + 1, c->ne, 256), 256, 0, st>>>(g, sn.u, sn.w, sn.rho, B.tri[rk],
+                                                                                  B.zh[rk], B.zv[rk], B.fh[rk]);
+            k_cell_kinetic<double><<<layer_grid(c->nl, c->nc, 256), 256, 0, st>>>(g, sn.u, sn.w, sn.rho, B.v2[rk],
+                                                                                 B.fv[rk]);
+        }
+    } else if (adv) {
         fa_tri<T><<<nbk(a->ntri), 256, 0, st>>>(g, sn.u, B.tri[rk]);
         fa_edge<T><<<nbk(a->nzh), 256, 0, st>>>(g, sn.u, sn.w, sn.rho, B.tri[rk], B.zh[rk], B.zv[rk], B.fh[rk]);
         fa_kin<T><<<nbk(ns), 256, 0, st>>>(g, sn.u, sn.w, sn.rho, B.v2[rk], B.fv[rk]);
@@ -305,10 +337,16 @@ void substage_fwd(Context *c, AdjState *a, StepBufs<T> &B, int rk, bool first, c
     else
         fa_scalar<T><<<nbk(ns, 128), 128, 0, st>>>(g, sn.rho, B.theta[rk], out.u, B.str[rk], B.strt[rk]);
     const T *str_gas = B.str[rk] + (long long)a->n_cond * ns;
-    fa_waves_layer<T><<<nbk(ns), 256, 0, st>>>(vg, ap, rk, so, sn, str_gas, B.strt[rk], B.wl[rk]);
-    fa_waves_rows<T><<<nbk(a->nwi), 256, 0, st>>>(vg, ap, so, B.tend[rk], B.wl[rk], B.wr[rk]);
-    fa_waves_thomas<T><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, B.wr[rk]);
-    fa_waves_apply<T><<<nbk(ns), 256, 0, st>>>(vg, ap, so, B.wl[rk], B.wr[rk], out);
+    if constexpr (PLAIN) {
+        waves_fwd(c, a, rk, dview(a, B.so), dview(a, rk ? B.sn1 : B.so),
+                  DState{B.str[rk], B.strt[rk], nullptr, nullptr, B.tend[rk], nullptr}, B.wl[rk], B.wr[rk],
+                  dview(a, rk ? B.sn2 : B.sn1));
+    } else {
+        fa_waves_layer<T><<<nbk(ns), 256, 0, st>>>(vg, ap, rk, so, sn, str_gas, B.strt[rk], B.wl[rk]);
+        fa_waves_rows<T><<<nbk(a->nwi), 256, 0, st>>>(vg, ap, so, B.tend[rk], B.wl[rk], B.wr[rk]);
+        fa_waves_thomas<T><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, B.wr[rk]);
+        fa_waves_apply<T><<<nbk(ns), 256, 0, st>>>(vg, ap, so, B.wl[rk], B.wr[rk], out);
+    }
     c->kernel_launches += adv ? 11 : 8;
     if (moist) {
         if (rk == 0) {
@@ -335,7 +373,18 @@ void step_fwd(Context *c, AdjState *a, StepBufs<T> &B, const T *P_prev, const T 
         fa_prelude<T><<<nbk(a->ns), 256, 0, st>>>(c->vg, ap, so, B.pre);
         c->kernel_launches++;
     }
-    fa_pgrad<T><<<nbk(nv), 256, 0, st>>>(g, ap, so, B.P);
+    if constexpr (sizeof(T) == sizeof(double)) {
+        const DState d = dview(a, B.so);
+        const SView<double> sv{d.rho, d.rhotheta_v, d.theta_v_pert, d.exner_pert, d.w, d.u};
+        k_pg_cells64<<<layer_grid(c->nl, c->nc, 256), 256, 0, st>>>(g, a->p, sv, c->pg_cell64, c->grad_pi_v);
+        fd_pgrad_v<<<layer_grid(c->nl - 1, c->nc, 256), 256, 0, st>>>(g, c->pg_cell64, c->grad_pi_v,
+                                                                      a->n_const == 1, B.P);
+        fd_pgrad_h<<<layer_grid(c->nl, c->ne, 256), 256, 0, st>>>(g, c->pg_cell64, c->grad_pi_v, a->n_const == 1,
+                                                                  B.P + a->nw);
+        c->kernel_launches += 2;
+    } else {
+        fa_pgrad<T><<<nbk(nv), 256, 0, st>>>(g, ap, so, B.P);
+    }
     ku_neg<T><<<nbk(nv), 256, 0, st>>>(nv, first ? B.P : P_prev, B.pgo);
     if (!first) {
         ku_copy<T><<<nbk(nv), 256, 0, st>>>(nv, pvt_prev, B.pvt[0]);
@@ -588,7 +637,9 @@ int set_params(Context *c, AdjState *a, const StepParams &p)
     a->ap.n_const = a->n_const;
     a->ap.n_cond = a->n_cond;
     if (launch_damping_table(c, p)) return -1;
-    ku_dden<<<nbk(a->nwi), 256, 0, c->stream>>>(a->nwi, p.dt, c->damp_dc, a->dden);
+    const size_t n = (size_t)a->nwi * sizeof(double);
+    CK(cudaMemcpyAsync(a->dden, c->damp_den, n, cudaMemcpyDeviceToDevice, c->stream));
+    CK(cudaMemcpyAsync(a->r_dden, c->damp_inv, n, cudaMemcpyDeviceToDevice, c->stream));
     return 0;
 }
 
@@ -875,10 +926,7 @@ int adj_waves_backward(Context *c, StateMirror *so_m, StateMirror *sn_m, StateMi
     AState<double> so = view(a, so_m->dev), sn = view(a, sn_m->dev), out = view(a, a->B.sn2);
     double *wl = a->B.wl[0], *wr = a->B.wr[0], *wl_b = a->Z.wl[0], *wr_b = a->Z.wr[0];
     /* forward of the solver, keeping its work */
-    fa_waves_layer<double><<<nbk(ns), 256, 0, st>>>(vg, ap, rk, so, sn, st_m->ds.rho, st_m->ds.rhotheta_v, wl);
-    fa_waves_rows<double><<<nbk(a->nwi), 256, 0, st>>>(vg, ap, so, st_m->ds.w, wl, wr);
-    fa_waves_thomas<double><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, wr);
-    fa_waves_apply<double><<<nbk(ns), 256, 0, st>>>(vg, ap, so, wl, wr, out);
+    waves_fwd(c, a, rk, so_m->ds, sn_m->ds, st_m->ds, wl, wr, dview(a, a->B.sn2));
     /* bars: the output bar moves to a work block, the input bar starts with
      * the pass-through fields */
     double *ob = a->Z.sn2, *ib = sn_bar->dev;

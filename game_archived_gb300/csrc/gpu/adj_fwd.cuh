@@ -53,6 +53,9 @@ __device__ __forceinline__ Dual operator/(double a, Dual b)
 __device__ __forceinline__ Dual &operator+=(Dual &a, Dual b) { return a = a + b; }
 __device__ __forceinline__ Dual &operator-=(Dual &a, Dual b) { return a = a - b; }
 
+/* x / y with y a grid quantity and r its reciprocal (div_rcp) */
+__device__ __forceinline__ Dual div_rcp(Dual x, double y, double r) { return {div_rcp(x.v, y, r), div_rcp(x.d, y, r)}; }
+
 template <class T>
 __device__ __forceinline__ T tzero();
 template <>
@@ -100,7 +103,8 @@ __device__ __forceinline__ double ipw_d(const HGrid<double> &g, int j, int l, in
 template <class T>
 __device__ __forceinline__ T a_gv(const HGrid<double> &g, const T *f, int k, int c)
 {
-    return (f[(long long)(k - 1) * g.nc + c] - f[(long long)k * g.nc + c]) / g.nd_v[(long long)k * g.nc + c];
+    const long long i = (long long)k * g.nc + c;
+    return div_rcp(f[i - g.nc] - f[i], g.nd_v[i], g.r_nd_v[i]);
 }
 
 template <class T>
@@ -108,13 +112,33 @@ __device__ __forceinline__ T a_grad_h(const HGrid<double> &g, const T *f, int l,
 {
     const int fr = g.from[e], to = g.to[e];
     const long long le = (long long)l * g.ne + e;
-    T out = (f[(long long)l * g.nc + to] - f[(long long)l * g.nc + fr]) / g.nd_h[le];
-    if (l >= g.nl - g.n_oro) {
+    T out = div_rcp(f[(long long)l * g.nc + to] - f[(long long)l * g.nc + fr], g.nd_h[le], g.r_nd_h[le]);
+    if (l >= g.nl - g.n_oro && !zero_slope(g.slope_h[le])) {
         T c = ipw_d(g, 6, l, fr) * a_gv(g, f, l, fr);
         c += ipw_d(g, 6, l, to) * a_gv(g, f, l, to);
         if (l < g.nl - 1) {
             c += ipw_d(g, 7, l, fr) * a_gv(g, f, l + 1, fr);
             c += ipw_d(g, 7, l, to) * a_gv(g, f, l + 1, to);
+        }
+        c = 0.5 * c;
+        out += -g.slope_h[le] * c;
+    }
+    return out;
+}
+
+/* the same from the field's vertical gradients gv at the inner interfaces */
+template <class T>
+__device__ __forceinline__ T a_grad_h_pre(const HGrid<double> &g, const T *f, const T *gv, int l, int e)
+{
+    const int fr = g.from[e], to = g.to[e];
+    const long long le = (long long)l * g.ne + e, o = (long long)l * g.nc;
+    T out = div_rcp(f[o + to] - f[o + fr], g.nd_h[le], g.r_nd_h[le]);
+    if (l >= g.nl - g.n_oro && !zero_slope(g.slope_h[le])) {
+        T c = ipw_d(g, 6, l, fr) * gv[o + fr];
+        c += ipw_d(g, 6, l, to) * gv[o + to];
+        if (l < g.nl - 1) {
+            c += ipw_d(g, 7, l, fr) * gv[o + g.nc + fr];
+            c += ipw_d(g, 7, l, to) * gv[o + g.nc + to];
         }
         c = 0.5 * c;
         out += -g.slope_h[le] * c;
@@ -189,6 +213,21 @@ __global__ void fa_pgrad(HGrid<double> g, AParams ap, AState<T> s, T *P)
         }
         P[i] = nl + lt;
     }
+}
+
+/* the same in FP64 from the cell factors and vertical gradients of
+ * k_pg_cells64, the FP64 step's form */
+__global__ void fd_pgrad_v(HGrid<double> g, const Quad *pc, const double *grad_pi, bool dry, double *P)
+{
+    const LayerPoint p = layer_point(g.nc);
+    if (!p.in) return;
+    const long long i = p.i + g.nc; /* interface p.l + 1 */
+    P[i] = pgrad_v_cells(g, pc[i - g.nc], pc[i], grad_pi, i, dry);
+}
+__global__ void fd_pgrad_h(HGrid<double> g, const Quad *pc, const double *grad_pi, bool dry, double *P)
+{
+    const LayerPoint p = layer_point(g.ne);
+    if (p.in) P[p.i] = pgrad_h_cells(g, pc, grad_pi, p.l, p.x, dry);
 }
 
 /* relative vorticity on triangles (vorticities.c:167-222) */
@@ -351,6 +390,7 @@ __device__ __forceinline__ T a_vflux_h(const HGrid<double> &g, const T *flux_h, 
 
 /* horizontal momentum: advection terms (adv), tendency with weights
  * (vector_tendencies_expl.c:79-131) and the wind update (manage_rkhevi.c:67-75).
+ * Runs after fa_mom_v, whose vertical gradients of the kinetic energy it reads.
  * Vector fields in device layout; tend_out may alias nothing. */
 template <class T>
 __global__ void fa_mom_h(HGrid<double> g, AParams ap, int adv, double new_w, double old_w, const T *P, const T *pg_old,
@@ -364,7 +404,7 @@ __global__ void fa_mom_h(HGrid<double> g, AParams ap, int adv, double new_w, dou
     const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     if (adv) {
         pvt[vi] = a_vflux_h(g, flux_h, flux_v, zh, zv, l, e);
-        v2g[vi] = a_grad_h(g, v2, l, e);
+        v2g[vi] = a_grad_h_pre(g, v2, v2g, l, e);
     }
     const double cur_hor = 0.5 + ap.impl_thermo_weight, old_hor = 1.0 - (0.5 + ap.impl_thermo_weight);
     T y = old_hor * pg_old[vi] - cur_hor * P[vi] + pvt[vi] - 0.5 * v2g[vi];
@@ -502,10 +542,10 @@ __global__ void fa_scalar(HGrid<double> g, const T *rho, const T *theta, const T
 /* ---------------------------------------------- vertical sound-wave solver
  * (column_solvers.c:19-383, EXACT order).  Per-layer work wl = 8 x [L][Nc]:
  * alpha, beta, gam, rho_expl, rt_expl, tp_expl, ep_expl, thl; per-interface
- * work wr = 8 x [L-1][Nc]: c, d, e, r, x (undamped solution), sol (damped),
- * th_int, rho_io */
+ * work wr = 9 x [L-1][Nc]: c, d, e, r, x (undamped solution), sol (damped),
+ * th_int, rho_io and 1 / rho_io */
 enum { WL_A, WL_B, WL_G, WL_REXP, WL_RTEXP, WL_TPEXP, WL_EPEXP, WL_THL, WL_N };
-enum { WR_C, WR_D, WR_E, WR_R, WR_X, WR_SOL, WR_TH, WR_RIO, WR_N };
+enum { WR_C, WR_D, WR_E, WR_R, WR_X, WR_SOL, WR_TH, WR_RIO, WR_RRIO, WR_N };
 
 template <class T>
 __global__ void fa_waves_layer(VGrid vg, AParams ap, int rk, AState<T> so, AState<T> sn, const T *st_rho,
@@ -609,6 +649,44 @@ __global__ void fa_waves_thomas(int nc, int nl, const double *dden, T *wr)
         wr[WR_X * m + (long long)j * nc + i] = x;
         wr[WR_SOL * m + (long long)j * nc + i] = x / dden[(long long)j * nc + i];
     }
+}
+
+/* the same in FP64 with the layer count a compile-time constant: the sweep in
+ * registers, one reciprocal per row (k_waves_thomas) */
+template <int NL>
+__global__ void fa_waves_thomas_fixed(int nc, const double *dden, const double *r_dden, double *wr)
+{
+    const int i = (int)gtid();
+    if (i >= nc) return;
+    constexpr int n = NL - 1;
+    const long long m = (long long)n * nc;
+    double ep[n], rp[n];
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+        const long long q = (long long)j * nc + i;
+        const double dj = wr[WR_D * m + q], rj = wr[WR_R * m + q];
+        const double cm = j > 0 ? wr[WR_C * m + q - nc] : 0.0;
+        const double den = j > 0 ? dj - ep[j - 1] * cm : dj, inv = 1.0 / den;
+        if (j < n - 1) ep[j] = div_rcp(wr[WR_E * m + q], den, inv);
+        rp[j] = div_rcp(j > 0 ? rj - rp[j - 1] * cm : rj, den, inv);
+    }
+    double x = 0.0;
+#pragma unroll
+    for (int j = n - 1; j >= 0; --j) {
+        const long long q = (long long)j * nc + i;
+        x = j < n - 1 ? rp[j] - ep[j] * x : rp[j];
+        wr[WR_X * m + q] = x;
+        wr[WR_SOL * m + q] = div_rcp(x, dden[q], r_dden[q]);
+    }
+}
+
+/* TOA and surface w of the fused back-substitution's output */
+__global__ void fa_w_bounds(int nc, int nl, const double *w_old, double *w_new)
+{
+    const int i = (int)gtid();
+    if (i >= nc) return;
+    w_new[i] = w_old[i];
+    w_new[(long long)nl * nc + i] = w_old[(long long)nl * nc + i];
 }
 
 /* back-substitution into the new state (column_solvers.c:305-370); w at the

@@ -602,12 +602,17 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
     c->wv_rows = dalloc<double>(c, 7 * (size_t)(L - 1) * NC);
     c->damp_dc = dalloc<double>(c, (size_t)(L - 1) * NC);
     c->damp_inv = dalloc<double>(c, (size_t)(L - 1) * NC);
+    c->damp_den = dalloc<double>(c, (size_t)(L - 1) * NC);
+    c->pg_cell64 = dalloc<Quad>(c, NS);
+    c->grad_pi_v = dalloc<double>(c, (size_t)(L + 1) * NC);
     {
         std::vector<double> iv(h_vol.size()), ia(h_areav.size());
         for (size_t k = 0; k < iv.size(); ++k) iv[k] = 1.0 / h_vol[k];
         for (size_t k = 0; k < ia.size(); ++k) ia[k] = h_areav[k] != 0.0 ? 1.0 / h_areav[k] : 0.0;
         c->inv_vol = dupload(c, iv);
         c->inv_area_v = dupload(c, ia);
+        c->vg.r_volume = c->hg64.r_volume = c->inv_vol;
+        c->vg.r_area_v = c->hg64.r_area_v = c->inv_area_v;
         /* double-float (hi, lo) pairs of the tracer solver's tables */
         auto df_pairs = [](const std::vector<double> &x) {
             std::vector<float> out(2 * x.size());
@@ -654,8 +659,21 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
     };
     work(c->w64, double(0));
     work(c->w32, float(0));
+    {
+        /* the FP64 path's tables: reciprocals and products of grid quantities */
+        HGrid<double> &g = c->hg64;
+        g.r_nd_v = dalloc<double>(c, (size_t)(L + 1) * NC);
+        g.r_nd_h = dalloc<double>(c, (size_t)L * NE);
+        g.r_dual_area_h = dalloc<double>(c, (size_t)(L + 1) * NE);
+        g.r_dual_area_t = dalloc<double>(c, (size_t)L * NT);
+        g.r_dz_h = dalloc<double>(c, (size_t)(L + 1) * NE);
+        g.rhombus_area = dalloc<double>(c, (size_t)L * NE);
+        g.r_rhombus_area = dalloc<double>(c, (size_t)L * NE);
+        g.tri_circ = dalloc<double>(c, (size_t)3 * L * NT);
+    }
     for (auto &b : c->owned)
         if (!b.p) return fail("device allocation failed");
+    if (make_f64_tables(c)) return -1;
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));

@@ -99,6 +99,10 @@ struct Context {
     /* mixed path: pressure-gradient factors of the step start per (layer,
      * cell): Pi', c_p theta_v, c_p theta_v', rho_gas / rho_total (k_pg_cells) */
     float4 *pg_cell = nullptr;
+    /* FP64 path: the same factors in double, and the vertical gradient of
+     * Pi' at the inner interfaces [L+1][Nc] */
+    Quad *pg_cell64 = nullptr;
+    double *grad_pi_v = nullptr;
     double *gravity_potential = nullptr; /* [L][Nc] */
     /* global integrals: per-block (hi, lo) partial sums, one counter and one
      * result per field, and three energy-density fields [3][L][Nc] */
@@ -154,6 +158,7 @@ struct Context {
      * 1 / (1 + dt * coefficient) for the values in damp_key (start height,
      * maximum coefficient, dt) */
     double *damp_dc = nullptr, *damp_inv = nullptr;
+    double *damp_den = nullptr; /* 1 + dt * coefficient */
     float2 *damp_inv_df = nullptr; /* damp_inv as double-float pairs */
     double damp_key[3] = {-1.0, -1.0, -1.0};
     /* grid terms of the mixed-path sound-wave rows [6][L-1][Nc] */
@@ -250,6 +255,10 @@ int download_state_pinned(const void *host_state, StateMirror *m, int which_mask
 int upload_field(const double *host, double *dev, const int *map, long long n, long long host_len);
 int download_field(double *host, const double *dev, const int *map, long long n, long long host_len,
                    long long host_lo, long long host_hi);
+
+/* the FP64 path's reciprocal and product tables of the context's grid
+ * (tables_f64.cu), from the tables already on the device */
+int make_f64_tables(Context *c);
 
 /* the mixed step's lagged fields in its FP32 work arrays (aux.cu), from and to
  * device vector fields [w (L+1) Nc][u L Ne] of doubles: P the pressure

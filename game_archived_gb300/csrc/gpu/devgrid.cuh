@@ -75,6 +75,17 @@ struct HGrid {
     const int *vort_s;      /* [3][Nt] */
     const R *dual_area_t;   /* [L][Nt] */
     const R *dual_z_t;      /* [L][Nt] */
+    /* FP64 path only (null in the FP32 copy): reciprocals of grid quantities
+     * for div_rcp (0 where the quantity is 0), and products of grid
+     * quantities in the operators' order */
+    const R *r_nd_v, *r_area_v;             /* [L+1][Nc] */
+    const R *r_volume;                      /* [L][Nc] */
+    const R *r_nd_h;                        /* [L][Ne] */
+    const R *r_dual_area_h;                 /* [L+1][Ne] */
+    const R *r_dual_area_t;                 /* [L][Nt] */
+    const R *r_dz_h;                        /* [L+1][Ne] of z_h(k-1) - z_h(k) at the inner levels */
+    const R *rhombus_area, *r_rhombus_area; /* [L][Ne] sum of the two triangles' areas */
+    const R *tri_circ;                      /* [3][L][Nt] circulation weight of edge j: rescaled length times sign */
 };
 
 /* device tables of the output pass, built at initialisation (device order
@@ -97,6 +108,12 @@ struct VGrid {
     int nc, nl;
     const double *volume, *z_scalar, *exner_bg, *theta_v_bg; /* [L][Nc] */
     const double *area_v, *z_v;                             /* [L+1][Nc] */
+    const double *r_volume, *r_area_v;                      /* reciprocals (0 where the quantity is 0) */
+};
+
+/* four doubles moved by one 32-byte access */
+struct alignas(32) Quad {
+    double x, y, z, w;
 };
 
 /* one State in device layout (always double: the prognostic variables) */
@@ -154,13 +171,16 @@ struct StepParams {
     /* derived on the host for the mixed path: 1/dt, 1/(w dt^2 c_p), 0.5/(w dt c_p)
      * with w the implicit thermodynamic weight */
     double inv_dt, k_rows, k_rows2;
+    /* divisors of the sound-wave rows (column_solvers.c:142-189) and their
+     * reciprocals: w dt^2 c_p, w dt c_p; and 0.5 / dt */
+    double rows_a, r_rows_a, rows_b, r_rows_b, half_inv_dt;
     /* pressure-gradient weights of the momentum tendencies
      * (vector_tendencies_expl.c:79-83): 0.5 + w, 1 - (0.5 + w), 1 - w, in
      * double and rounded to float */
     double cur_hor, old_hor, cur_ver;
     float cur_hor_f, old_hor_f, cur_ver_f, pad_f;
 };
-static_assert(sizeof(StepParams) == 8 * sizeof(int) + 14 * sizeof(double) + 4 * sizeof(float),
+static_assert(sizeof(StepParams) == 8 * sizeof(int) + 19 * sizeof(double) + 4 * sizeof(float),
               "StepParams has padding");
 
 /* config switches of the diffusion branch (StepParams::diff) */

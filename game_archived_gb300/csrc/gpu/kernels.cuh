@@ -44,7 +44,43 @@ __device__ __forceinline__ R ipw_at(const HGrid<R> &g, int j, int l, int c)
 template <typename R, typename F>
 __device__ __forceinline__ R grad_v(const HGrid<R> &g, const F *f, int k, int c)
 {
-    return (R(f[(long long)(k - 1) * g.nc + c]) - R(f[(long long)k * g.nc + c])) / g.nd_v[(long long)k * g.nc + c];
+    const long long i = (long long)k * g.nc + c;
+    return div_tab(R(f[i - g.nc]) - R(f[i]), g.nd_v, g.r_nd_v, i);
+}
+
+/* the same for every inner interface of a field: formed once, where each is
+ * read by up to twelve edges' gradients (grad_h_pre) and by the interface's
+ * own momentum */
+__global__ void k_grad_v(HGrid<double> g, const double *f, double *out)
+{
+    const LayerPoint p = layer_point(g.nc);
+    if (p.in) out[p.i + g.nc] = grad_v(g, f, p.l + 1, p.x);
+}
+
+/* slopes are exactly 0 away from orography; no FP64 comparison */
+__device__ __forceinline__ bool zero_slope(double s) { return is_zero(s); }
+__device__ __forceinline__ bool zero_slope(float s) { return s == 0.0f; }
+
+/* horizontal gradient at edge e of layer l from the field and its vertical
+ * gradients gv (k_grad_v): grad_h's operations in its order */
+__device__ __forceinline__ double grad_h_pre(const HGrid<double> &g, double f_to, double f_fr, const double *gv, int l,
+                                             int e, int fr, int to)
+{
+    const long long le = (long long)l * g.ne + e;
+    double out = div_tab(f_to - f_fr, g.nd_h, g.r_nd_h, le);
+    if (l < g.nl - g.n_oro) return out;
+    const double slope = g.slope_h[le];
+    if (zero_slope(slope)) return out;
+    const double *gl = gv + (long long)l * g.nc;
+    double c = ipw_at(g, 6, l, fr) * gl[fr];
+    c += ipw_at(g, 6, l, to) * gl[to];
+    if (l < g.nl - 1) {
+        c += ipw_at(g, 7, l, fr) * gl[g.nc + fr];
+        c += ipw_at(g, 7, l, to) * gl[g.nc + to];
+    }
+    c = 0.5 * c;
+    out += -slope * c;
+    return out;
 }
 
 /* horizontal gradient at edge e of layer l, with the terrain-following
@@ -55,10 +91,10 @@ __device__ __forceinline__ R grad_h(const HGrid<R> &g, const F *f, int l, int e)
 {
     const int fr = g.from[e], to = g.to[e];
     const long long le = (long long)l * g.ne + e;
-    R out = (R(f[(long long)l * g.nc + to]) - R(f[(long long)l * g.nc + fr])) / g.nd_h[le];
+    R out = div_tab(R(f[(long long)l * g.nc + to]) - R(f[(long long)l * g.nc + fr]), g.nd_h, g.r_nd_h, le);
     if (l >= g.nl - g.n_oro) {
-        /* a zero slope adds -0: the mixed path skips it */
-        if (sizeof(R) == sizeof(float) && g.slope_h[le] == R(0)) return out;
+        /* a zero slope adds a zero */
+        if (zero_slope(g.slope_h[le])) return out;
         R c = ipw_at(g, 6, l, fr) * grad_v(g, f, l, fr);
         c += ipw_at(g, 6, l, to) * grad_v(g, f, l, to);
         if (l < g.nl - 1) {
@@ -79,8 +115,8 @@ __device__ __forceinline__ R hor_covariant(const HGrid<R> &g, const F *u, const 
     R r = R(u[le]);
     if (l >= g.nl - g.n_oro) {
         const R slope = g.slope_h[le];
-        /* a zero slope adds 0: the mixed path skips it */
-        if (sizeof(R) == sizeof(float) && slope == R(0)) return r;
+        /* a zero slope adds a zero */
+        if (zero_slope(slope)) return r;
         const int fr = g.from[e], to = g.to[e];
         R c = ipw_at(g, 6, l, fr) * R(w[(long long)l * g.nc + fr]);
         c += ipw_at(g, 6, l, to) * R(w[(long long)l * g.nc + to]);
@@ -513,9 +549,33 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_tri
 {
     const LayerPoint pt_ = layer_point(g.nt);
     if (!pt_.in) return;
-    const long long i = pt_.i;
+    const long long n = (long long)g.nl * g.nt, i = pt_.i;
     const int l = pt_.l, t = pt_.x;
     R acc = R(0);
+    if constexpr (sizeof(R) == sizeof(double)) {
+        /* FP64 issue bounds this kernel: the circulation weights come from a
+         * table and the vertical shear's denominator from its reciprocal, a
+         * third of the FP64 instructions (three divisions and two products
+         * less per edge) for three more streamed words: 96 -> 41 us at
+         * RES_ID 5 with the mountain, 345 -> 100 us at RES_ID 6 flat */
+        for (int j = 0; j < 3; ++j) {
+            const int e = g.vort_i[j * g.nt + t];
+            const long long le = (long long)l * g.ne + e;
+            double vel = u[le];
+            if (l >= g.nl - g.n_oro) {
+                const double zh = g.z_h[le], dz = g.dual_z_t[i] - zh;
+                if (!is_zero(dz)) {
+                    const bool above = __double_as_longlong(dz) > 0 || l == g.nl - 1;
+                    const long long lo_e = above ? le - g.ne : le + g.ne;
+                    const double r = above ? -g.r_dz_h[le] : g.r_dz_h[le + g.ne];
+                    vel += dz * div_rcp(vel - u[lo_e], zh - g.z_h[lo_e], r);
+                }
+            }
+            acc += g.tri_circ[j * n + i] * vel;
+        }
+        tri_vort[i] = div_tab(acc, g.dual_area_t, g.r_dual_area_t, i);
+        return;
+    }
     for (int j = 0; j < 3; ++j) {
         const int e = g.vort_i[j * g.nt + t];
         const long long le = (long long)l * g.ne + e;
@@ -544,7 +604,10 @@ __device__ __forceinline__ R rel_vort_tangential(const HGrid<R> &g, const R *u, 
 {
     const int nl = g.nl;
     if (k == 0) k = 1; /* no vertical shear of the tangential vorticity at the TOA */
-    const R inv_area = R(1) / g.dual_area_h[(long long)k * g.ne + e];
+    const long long ke = (long long)k * g.ne + e;
+    R inv_area;
+    if constexpr (sizeof(R) == sizeof(double)) inv_area = g.r_dual_area_h[ke];
+    else inv_area = R(1) / g.dual_area_h[ke];
     if (k == nl) {
         R c2 = hor_covariant(g, u, w, k - 1, e);
         return inv_area * g.nd_h[(long long)(k - 1) * g.ne + e] * c2;
@@ -597,7 +660,9 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_edg
         const int tf = g.dual_from[e], tt = g.dual_to[e];
         const long long kt = (long long)k * g.nt;
         R af = g.dual_area_t[kt + tf], at = g.dual_area_t[kt + tt];
-        R rel = (af * tri_vort[kt + tf] + at * tri_vort[kt + tt]) / (af + at);
+        R rel = af * tri_vort[kt + tf] + at * tri_vort[kt + tt];
+        if constexpr (sizeof(R) == sizeof(double)) rel = div_tab(rel, g.rhombus_area, g.r_rhombus_area, le);
+        else rel = rel / (af + at);
         R pv = rel + g.f_vec[ne + e];
         R dens = R(0);
         for (int j = 0; j < 4; ++j)
@@ -707,15 +772,6 @@ __device__ __forceinline__ void pgrad_h_parts(const HGrid<R> &g, const StepParam
     l_term = dec * l_term;
 }
 
-/* the sum nl + l, the only form the step reads */
-template <typename R>
-__device__ __forceinline__ R pgrad_h(const HGrid<R> &g, const StepParams &p, const SView<R> &s, int l, int e)
-{
-    R nl, l_term;
-    pgrad_h_parts(g, p, s, l, e, nl, l_term);
-    return nl + l_term;
-}
-
 /* the same at the inner interface k of cell c */
 template <typename R>
 __device__ __forceinline__ void pgrad_v_parts(const HGrid<R> &g, const StepParams &p, const SView<R> &s, int k, int c,
@@ -735,14 +791,6 @@ __device__ __forceinline__ void pgrad_v_parts(const HGrid<R> &g, const StepParam
     l_term = dec * l_term;
 }
 
-template <typename R>
-__device__ __forceinline__ R pgrad_v(const HGrid<R> &g, const StepParams &p, const SView<R> &s, int k, int c)
-{
-    R nl, l_term;
-    pgrad_v_parts(g, p, s, k, c, nl, l_term);
-    return nl + l_term;
-}
-
 /* Mixed path: the cell factors of the pressure gradient at the step start,
  * one float4 per (layer, cell): x = Pi', y = c_p (theta_v_bg + theta_v'),
  * z = c_p theta_v', w = rho_gas / (sum of all densities) -- the float
@@ -759,6 +807,53 @@ __global__ void k_pg_cells(HGrid<float> g, StepParams p, SView<float> s, float4 
     const float tp = s.theta_v_pert[i];
     pc[i] = make_float4(s.exner_pert[i], cdp * (g.theta_v_bg[i] + tp), cdp * tp,
                         s.rho[p.n_cond * ns + i] / density_total_r(s.rho, p.n_const, ns, i));
+}
+
+/* FP64 path: the same cell factors in double with the operations of
+ * pgrad_h_parts / pgrad_v_parts (the dry build's density ratio is rho / rho =
+ * 1 and is left out), and the vertical gradient of Pi' at the interface
+ * above the cell.  Formed once per cell instead of once per edge and
+ * interface that reads it (up to eight times). */
+__global__ void k_pg_cells64(HGrid<double> g, StepParams p, SView<double> s, Quad *pc, double *grad_pi)
+{
+    const LayerPoint pt = layer_point(g.nc);
+    if (!pt.in) return;
+    const long long ns = (long long)g.nl * g.nc, i = pt.i;
+    const double cdp = C_D_P, tp = s.theta_v_pert[i];
+    pc[i] = Quad{s.exner_pert[i], cdp * (g.theta_v_bg[i] + tp), cdp * tp,
+                 p.n_const > 1 ? s.rho[p.n_cond * ns + i] / density_total_r(s.rho, p.n_const, ns, i) : 1.0};
+    if (pt.l > 0) grad_pi[i] = grad_v(g, s.exner_pert, pt.l, pt.x);
+}
+
+__device__ __forceinline__ double pgrad_h_cells(const HGrid<double> &g, const Quad *pc, const double *grad_pi, int l,
+                                                int e, bool dry)
+{
+    const int fr = g.from[e], to = g.to[e];
+    const Quad a = pc[(long long)l * g.nc + fr], b = pc[(long long)l * g.nc + to];
+    double nl = grad_h_pre(g, b.x, a.x, grad_pi, l, e, fr, to);
+    nl = (0.5 * (b.y + a.y)) * nl;
+    double l_term = (0.5 * (b.z + a.z)) * g.exner_bg_grad_h[(long long)l * g.ne + e];
+    if (!dry) {
+        const double dec = 0.5 * (b.w + a.w);
+        nl = dec * nl;
+        l_term = dec * l_term;
+    }
+    return nl + l_term;
+}
+
+/* u, d: the factors of the cells above and below the interface i */
+__device__ __forceinline__ double pgrad_v_cells(const HGrid<double> &g, const Quad &u, const Quad &d,
+                                                const double *grad_pi, long long i, bool dry)
+{
+    double nl = grad_pi[i];
+    nl = (0.5 * (u.y + d.y)) * nl;
+    double l_term = (0.5 * (u.z + d.z)) * g.exner_bg_grad_v[i];
+    if (!dry) {
+        const double dec = 0.5 * (u.w + d.w);
+        nl = dec * nl;
+        l_term = dec * l_term;
+    }
+    return nl + l_term;
 }
 
 /* pgrad_h from the cell factors (mixed path, first substage) */
@@ -800,17 +895,35 @@ __device__ __forceinline__ float pgrad_v_packed(const HGrid<float> &g, float4 u,
     return nl + l_term;
 }
 
+/* what the momentum kernels read of the first substage's pressure gradient
+ * (mixed path: k_pg_cells; FP64 path: k_pg_cells64) and, FP64 path, of the
+ * kinetic energy's vertical gradient (k_grad_v) */
+template <typename R>
+struct PgCells;
+template <>
+struct PgCells<float> {
+    const float4 *cell;
+};
+template <>
+struct PgCells<double> {
+    const Quad *cell;
+    const double *grad_pi, *grad_v2;
+};
+
 /* ------------------------------------------------------- k_momentum_h
  * horizontal momentum: explicit tendency (vector_tendencies_expl.c:74-131) and
  * the wind update (manage_rkhevi.c:67-75).  ADV: the advection terms are
- * recomputed in this substage; PG: the pressure gradient is recomputed (on
- * the mixed path from the cell factors pc of k_pg_cells).  The wind update
+ * recomputed in this substage; PG: the pressure gradient is recomputed from
+ * the cell factors.  FP64 issue bounds the FP64 instantiation: with the
+ * vertical gradients and cell factors formed once, the zero slopes skipped
+ * and div_rcp for the distances it went from 182 to 101 us at RES_ID 5
+ * with the mountain (789 to 378 us at RES_ID 6, flat, moist).  The wind update
  * is FP64; u_shadow (mixed path) receives its FP32 copy. */
 template <typename R, bool ADV, bool PG>
 __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_momentum_h(HGrid<R> g, StepParams p, SView<R> sv, double *u_new, float *u_shadow, const double *u_old,
                              double *tend_u, R *P_h, R *pg_old_h, R *pvt_h, R *v2g_h, const R *flux_h,
                              const R *flux_v, const R *zh, const R *zv, const R *v2, double new_w, double old_w,
-                             const double *fric_u, const float4 *pc)
+                             const double *fric_u, PgCells<R> pg)
 {
     const LayerPoint pt_ = layer_point(g.ne);
     if (!pt_.in) return;
@@ -819,9 +932,9 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
     R P, pgo;
     if (PG) {
         if constexpr (sizeof(R) == sizeof(float))
-            P = pgrad_h_packed(g, pc, sv, l, e);
+            P = pgrad_h_packed(g, pg.cell, sv, l, e);
         else
-            P = pgrad_h(g, p, sv, l, e);
+            P = pgrad_h_cells(g, pg.cell, pg.grad_pi, l, e, p.n_const == 1);
         pgo = p.first_step ? -P : -P_h[i];
         P_h[i] = P;
         pg_old_h[i] = pgo;
@@ -832,7 +945,12 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
     R pvt, v2g;
     if (ADV) {
         pvt = vorticity_flux_h(g, flux_h, flux_v, zh, zv, l, e);
-        v2g = grad_h(g, v2, l, e);
+        if constexpr (sizeof(R) == sizeof(float)) {
+            v2g = grad_h(g, v2, l, e);
+        } else {
+            const int fr = g.from[e], to = g.to[e];
+            v2g = grad_h_pre(g, v2[(long long)l * g.nc + to], v2[(long long)l * g.nc + fr], pg.grad_v2, l, e, fr, to);
+        }
         pvt_h[i] = pvt;
         v2g_h[i] = v2g;
     } else {
@@ -859,7 +977,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
 template <typename R, bool ADV, bool PG>
 __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_momentum_v(HGrid<R> g, StepParams p, SView<R> sv, double *tend_w, R *P_v, R *pvt_v, R *v2g_v,
                              const R *flux_h, const R *zh, const R *v2, double new_w, double old_w,
-                             const double *fric_w, const float4 *pc)
+                             const double *fric_w, PgCells<R> pg)
 {
     const LayerPoint pt_ = layer_point(g.nc);
     if (!pt_.in) return;
@@ -888,31 +1006,29 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
         tend_w[i] = 0.0;
         return;
     }
-    /* the mixed path's first substage takes the pressure gradient and the
-     * condensate factors from the cell factors pc of k_pg_cells */
-    constexpr bool PACKED = PG && sizeof(R) == sizeof(float);
-    R P, v2g, d_up, d_lo;
-    if (PG) {
-        if constexpr (PACKED) {
-            const float4 fu = pc[(long long)(k - 1) * g.nc + c], fd = pc[(long long)k * g.nc + c];
-            P = pgrad_v_packed(g, fu, fd, k, c);
-            d_up = fu.w - 1.0f;
-            d_lo = fd.w - 1.0f;
-        } else {
-            P = pgrad_v(g, p, sv, k, c);
-        }
+    /* the first substage takes the pressure gradient and the condensate
+     * factors from the cell factors of k_pg_cells / k_pg_cells64 */
+    constexpr bool F = sizeof(R) == sizeof(float);
+    const bool dry = !F && p.n_const == 1;
+    R P, v2g, d_up = R(0), d_lo = R(0);
+    if constexpr (PG) {
+        const auto fu = pg.cell[i - g.nc], fd = pg.cell[i];
+        if constexpr (F) P = pgrad_v_packed(g, fu, fd, k, c);
+        else P = pgrad_v_cells(g, fu, fd, pg.grad_pi, i, dry);
+        d_up = fu.w - R(1);
+        d_lo = fd.w - R(1);
         P_v[i] = P;
     } else {
         P = P_v[i];
     }
-    if (ADV) {
+    if (!ADV) pvt = pvt_v[i];
+    if constexpr (ADV && F) {
         v2g = grad_v(g, v2, k, c);
         v2g_v[i] = v2g;
     } else {
-        pvt = pvt_v[i];
-        v2g = v2g_v[i];
+        v2g = v2g_v[i]; /* FP64 path: written by k_grad_v */
     }
-    if constexpr (!PACKED) {
+    if (!PG && !dry) {
         const long long ns = (long long)nl * g.nc;
         const long long up = (long long)(k - 1) * g.nc + c, lo = (long long)k * g.nc + c;
         d_up = sv.rho[p.n_cond * ns + up] / density_total_r(sv.rho, p.n_const, ns, up) - R(1);

@@ -33,6 +33,7 @@ __device__ __forceinline__ LayerPoint layer_point(int n)
     const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x), l = (int)blockIdx.y;
     return {l, x, (long long)l * n + x, x < n};
 }
+inline dim3 layer_grid(int layers, int n, int bs) { return dim3((unsigned)((n + bs - 1) / bs), (unsigned)layers); }
 /* the row of index i in rows of n, for the kernels with a one-dimensional
  * grid: a 32-bit division (every index is below 2^31: the index maps are
  * 32-bit).  kd_sdiff_div 345 -> 216 us, kd_fric_h 197 -> 168 us, kd_n2_adv
@@ -62,6 +63,28 @@ __device__ __forceinline__ double rcp_nr(double x)
     for (int s = 0; s < STEPS; ++s) r = fma(r, fma(-x, r, 1.0), r);
     return r;
 }
+
+/* x / y for a y whose reciprocal r = 1 / y is at hand (a grid quantity's from
+ * its table, or one reciprocal shared by several quotients): the quotient
+ * x r corrected once with its exact remainder (Markstein, "Computation of
+ * elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+ * Dev. 34, 1990; Brisebarre, Muller and Raina, "Accelerating correctly
+ * rounded floating-point division when the divisor is known in advance",
+ * IEEE Trans. Computers 53, 2004).  Equal to x / y for finite operands away
+ * from the ends of the exponent range (tested), in three FP64 issues
+ * instead of the division's eight or more, without its branch. */
+__device__ __forceinline__ double div_rcp(double x, double y, double r)
+{
+    const double q = __dmul_rn(x, r);
+    return __fma_rn(__fma_rn(-q, y, x), r, q);
+}
+/* x / tab[i] with the reciprocals of tab in rtab on the FP64 path; the mixed
+ * path divides in FP32 */
+__device__ __forceinline__ double div_tab(double x, const double *tab, const double *rtab, long long i)
+{
+    return div_rcp(x, tab[i], rtab[i]);
+}
+__device__ __forceinline__ float div_tab(float x, const float *tab, const float *, long long i) { return x / tab[i]; }
 
 /* x >= 0 for the solvers' branch and clip tests.  The FP64 path compares as
  * the reference does; the mixed path reads the sign bit on the integer pipe

@@ -35,13 +35,13 @@ struct WavesWork {
     /* per layer [L][Nc] */
     double *rho_expl, *rt_expl, *alpha, *beta, *gam, *tp_expl, *ep_expl, *thl;
     /* per inner interface [L-1][Nc] */
-    double *c, *d, *e, *r, *th_int, *rho_io, *dden;
+    double *c, *d, *e, *r, *th_int, *rho_io, *r_rho_io;
     /* mixed path: reciprocal grid metrics */
     const double *inv_vol;    /* [L][Nc] */
     const double *inv_area_v; /* [L+1][Nc] */
-    /* Klemp damping coefficient of the inner interfaces [L-1][Nc]; mixed
-     * path: 1 / (1 + dt * coefficient) for the current dt */
-    const double *damp_dc, *damp_inv;
+    /* 1 + dt * Klemp damping coefficient of the inner interfaces [L-1][Nc]
+     * for the current dt, and its reciprocal */
+    const double *damp_den, *damp_inv;
     /* mixed path: grid terms of the rows of inner interface j [6][L-1][Nc]:
      * dz = z(j) - z(j+1), H = (Pi_bg(j) - Pi_bg(j+1)) / 2, G1 = 2 / A_v,
      * G2 = (1/V(j+1) - 1/V(j)) / 2, Cz = dz / V(j), Ez = dz / V(j+1)
@@ -53,7 +53,7 @@ struct WavesWork {
  * (column_solvers.c:285-298).  It depends on the grid and the two damping
  * parameters only, so it is tabulated once per parameter pair instead of
  * once per substage. */
-__global__ void k_damping_table(VGrid vg, double start_height, double coeff_max, double dt, double *dc,
+__global__ void k_damping_table(VGrid vg, double start_height, double coeff_max, double dt, double *dc, double *den,
                                 double *inv_den, float2 *inv_den_df)
 {
     const long long n = (long long)(vg.nl - 1) * vg.nc, q = gtid();
@@ -66,10 +66,31 @@ __global__ void k_damping_table(VGrid vg, double start_height, double coeff_max,
         r = coeff_max * (s * s);
     }
     dc[q] = r;
-    const double inv = 1.0 / (1.0 + dt * r);
+    den[q] = 1.0 + dt * r;
+    const double inv = 1.0 / den[q];
     inv_den[q] = inv;
     const float hi = (float)inv;
     inv_den_df[q] = make_float2(hi, (float)(inv - (double)hi));
+}
+
+/* alpha, beta, gamma of a cell over its volume (column_solvers.c:102-139),
+ * FP64 path: every quotient correctly rounded as the reference's, the
+ * divisions by rho, rho^2 and the volume through one reciprocal each
+ * (div_rcp) */
+struct WaveCoeffs {
+    double alpha, beta, gam;
+};
+__device__ __forceinline__ WaveCoeffs wave_coeffs(int rk, double ro, double rto, double ebg, double epo, double rn,
+                                                  double rtn, double irn, double epn, double vol, double rv)
+{
+    const double pdw = 0.5, iro = 1.0 / ro;
+    const double ao = div_rcp(-rto, ro * ro, iro * iro);
+    const double go = R_D / (C_D_V * rto) * (ebg + epo);
+    if (rk == 0) return {div_rcp(ao, vol, rv), div_rcp(iro, vol, rv), div_rcp(go, vol, rv)};
+    const double an = div_rcp(-rtn, rn * rn, irn * irn);
+    const double gn = R_D / (C_D_V * rtn) * (ebg + epn);
+    return {div_rcp((1.0 - pdw) * ao + pdw * an, vol, rv), div_rcp((1.0 - pdw) * iro + pdw * irn, vol, rv),
+            div_rcp((1.0 - pdw) * go + pdw * gn, vol, rv)};
 }
 
 template <bool EXACT>
@@ -78,26 +99,25 @@ __global__ void k_waves_layer(VGrid vg, StepParams p, DState so, DState sn, DSta
     const long long ns = (long long)vg.nl * vg.nc, b = gtid();
     if (b >= ns) return;
     const long long gp = p.n_cond * ns;
-    const double dt = p.dt, pdw = 0.5;
+    const double dt = p.dt;
     const double vol = vg.volume[b];
     const double ro = so.rho[gp + b], rto = so.rhotheta_v[b];
-    double alpha, beta, gam;
     if (EXACT) {
-        if (rk == 0) {
-            alpha = -rto / (ro * ro) / vol;
-            beta = 1.0 / ro / vol;
-            gam = R_D / (C_D_V * rto) * (vg.exner_bg[b] + so.exner_pert[b]) / vol;
-        } else {
-            const double rn = sn.rho[gp + b];
-            const double ao = -rto / (ro * ro), bo = 1.0 / ro;
-            const double go = R_D / (C_D_V * rto) * (vg.exner_bg[b] + so.exner_pert[b]);
-            const double an = -sn.rhotheta_v[b] / (rn * rn), bn = 1.0 / rn;
-            const double gn = R_D / (C_D_V * sn.rhotheta_v[b]) * (vg.exner_bg[b] + sn.exner_pert[b]);
-            alpha = ((1.0 - pdw) * ao + pdw * an) / vol;
-            beta = ((1.0 - pdw) * bo + pdw * bn) / vol;
-            gam = ((1.0 - pdw) * go + pdw * gn) / vol;
-        }
+        const double rv = vg.r_volume[b];
+        const double rn = sn.rho[gp + b], rtn = sn.rhotheta_v[b], irn = 1.0 / rn;
+        const WaveCoeffs w = wave_coeffs(rk, ro, rto, vg.exner_bg[b], so.exner_pert[b], rn, rtn, irn,
+                                         rk == 0 ? 0.0 : sn.exner_pert[b], vol, rv);
+        const double str = st.rho[gp + b], strt = st.rhotheta_v[b], dtv = dt * vol;
+        ww.alpha[b] = w.alpha;
+        ww.beta[b] = w.beta;
+        ww.gam[b] = w.gam;
+        ww.rho_expl[b] = ro + dt * str;
+        ww.rt_expl[b] = rto + dt * strt;
+        ww.tp_expl[b] = so.theta_v_pert[b] + dtv * (w.alpha * str + w.beta * strt);
+        ww.ep_expl[b] = so.exner_pert[b] + dtv * w.gam * strt;
+        ww.thl[b] = div_rcp(rtn, rn, irn);
     } else {
+        double alpha, beta, gam;
         const double iv = ww.inv_vol[b], iro = rcp_nr<1>(ro);
         const double rn = sn.rho[gp + b], rtn = sn.rhotheta_v[b], irn = rk == 0 ? 0.0 : rcp_nr<1>(rn);
         const double go = (R_D / C_D_V) * (vg.exner_bg[b] + so.exner_pert[b]) * rcp_nr<1>(rto);
@@ -120,54 +140,54 @@ __global__ void k_waves_layer(VGrid vg, StepParams p, DState so, DState sn, DSta
         ww.tp_expl[b] = so.theta_v_pert[b] + dt * vol * (alpha * str + beta * strt);
         ww.ep_expl[b] = so.exner_pert[b] + dt * vol * gam * strt;
         ww.thl[b] = rtn * (rk == 0 ? rcp_nr<1>(rn) : irn);
-        return;
     }
-    ww.alpha[b] = alpha;
-    ww.beta[b] = beta;
-    ww.gam[b] = gam;
-    ww.rho_expl[b] = ro + dt * st.rho[gp + b];
-    ww.rt_expl[b] = rto + dt * st.rhotheta_v[b];
-    ww.tp_expl[b] = so.theta_v_pert[b] + dt * vol * (alpha * st.rho[gp + b] + beta * st.rhotheta_v[b]);
-    ww.ep_expl[b] = so.exner_pert[b] + dt * vol * gam * st.rhotheta_v[b];
-    ww.thl[b] = sn.rhotheta_v[b] / sn.rho[gp + b];
 }
 
-/* FP64 path: the rows in the reference's operation order */
+/* FP64 path: the rows in the reference's operation order.  Thread (interface
+ * j, column) forms d_j, r_j, the super-diagonal e_j of row j and the
+ * sub-diagonal c_{j-1} of row j - 1, whose theta_v, rho, w and heights are
+ * those of interface j: the two share their quotients.  FP64 issue bounds
+ * the kernel; one division per interface (1 / rho), the others by div_rcp:
+ * 96 -> 56 us at RES_ID 5, 360 -> 193 us at RES_ID 6. */
 __global__ void k_waves_rows(VGrid vg, StepParams p, DState so, DState st, WavesWork ww)
 {
     const int nc = vg.nc, nl = vg.nl;
-    const long long n = (long long)(nl - 1) * nc;
     const LayerPoint pt_ = layer_point(nc);
     if (!pt_.in) return;
     const long long q = pt_.i;
     const int j = pt_.l;
     const long long ns = (long long)nl * nc, gp = p.n_cond * ns;
     const long long b = q, lo = q + nc, wi = q + nc;
-    const double dt = p.dt, iw = p.impl_thermo_weight, dt2 = dt * dt;
-    const double rho_io = 0.5 * (so.rho[gp + b] + so.rho[gp + lo]);
+    const double dt = p.dt;
+    const double rho_io = 0.5 * (so.rho[gp + b] + so.rho[gp + lo]), r_rio = 1.0 / rho_io;
     const double rho_ie = 0.5 * (ww.rho_expl[b] + ww.rho_expl[lo]);
-    const double th = 0.5 * (ww.thl[b] + ww.thl[lo]);
+    const double tl_b = ww.thl[b], tl_lo = ww.thl[lo];
+    const double th = 0.5 * (tl_b + tl_lo);
     const double dz = vg.z_scalar[b] - vg.z_scalar[lo], dpi = vg.exner_bg[b] - vg.exner_bg[lo];
-    const double wo = so.w[wi];
+    const double half_dpi = 0.5 * dpi;
+    const double wo = so.w[wi], rv_b = vg.r_volume[b], rv_lo = vg.r_volume[lo];
     const double a0 = ww.alpha[b], a1 = ww.alpha[lo], b0 = ww.beta[b], b1 = ww.beta[lo];
     const double g0 = ww.gam[b], g1 = ww.gam[lo];
-    ww.d[q] = -(th * th) * (g0 + g1) + 0.5 * dpi * (a1 - a0 + th * (b1 - b0))
-              - dz / (iw * dt2 * C_D_P * rho_io) * (2.0 / vg.area_v[wi] + dt * wo * 0.5 * (-1.0 / vg.volume[b] + 1.0 / vg.volume[lo]));
-    ww.r[q] = -(wo + dt * st.w[wi]) * dz / (iw * dt2 * C_D_P) + th * (ww.ep_expl[b] - ww.ep_expl[lo]) / dt
-              + 0.5 / dt * (ww.tp_expl[b] + ww.tp_expl[lo]) * dpi - dz / (iw * dt2 * C_D_P) * wo * rho_ie / rho_io;
+    const double dz_a = div_rcp(dz, p.rows_a, p.r_rows_a);
+    ww.d[q] = -(th * th) * (g0 + g1) + half_dpi * (a1 - a0 + th * (b1 - b0))
+              - div_rcp(dz, p.rows_a * rho_io, p.r_rows_a * r_rio)
+                    * (2.0 * vg.r_area_v[wi] + dt * wo * 0.5 * (-rv_b + rv_lo));
+    ww.r[q] = div_rcp(-(wo + dt * st.w[wi]) * dz, p.rows_a, p.r_rows_a)
+              + div_rcp(th * (ww.ep_expl[b] - ww.ep_expl[lo]), dt, p.inv_dt)
+              + p.half_inv_dt * (ww.tp_expl[b] + ww.tp_expl[lo]) * dpi - div_rcp(dz_a * wo * rho_ie, rho_io, r_rio);
     ww.th_int[q] = th;
     ww.rho_io[q] = rho_io;
+    ww.r_rho_io[q] = r_rio;
+    /* the terms of c and e with the old w, before the layer's volume */
+    const double wt = div_rcp(dz, p.rows_b, p.r_rows_b) * 0.5 * wo;
     if (j < nl - 2) {
-        const long long lo2 = lo + nc;
-        const double th1 = 0.5 * (ww.thl[lo] + ww.thl[lo2]);
-        const double rho_io1 = 0.5 * (so.rho[gp + lo] + so.rho[gp + lo2]);
-        ww.c[q] = th1 * g1 * th + 0.5 * (vg.exner_bg[lo] - vg.exner_bg[lo2]) * (a1 + b1 * th)
-                  - (vg.z_scalar[lo] - vg.z_scalar[lo2]) / (iw * dt * C_D_P) * 0.5 * so.w[wi + nc] / (vg.volume[lo] * rho_io1);
-        ww.e[q] = th * g1 * th1 - 0.5 * dpi * (a1 + b1 * th1)
-                  + dz / (iw * dt * C_D_P) * 0.5 * wo / (vg.volume[lo] * rho_io);
+        const double th1 = 0.5 * (tl_lo + ww.thl[lo + nc]);
+        ww.e[q] = th * g1 * th1 - half_dpi * (a1 + b1 * th1) + div_rcp(wt, vg.volume[lo] * rho_io, rv_lo * r_rio);
     }
-    /* Klemp (2008) damping denominator of the solution at interface j + 1 */
-    ww.dden[q] = 1.0 + dt * ww.damp_dc[q];
+    if (j > 0) {
+        const double th0 = 0.5 * (ww.thl[b - nc] + tl_b);
+        ww.c[q - nc] = th * g0 * th0 + half_dpi * (a0 + b0 * th0) - div_rcp(wt, vg.volume[b] * rho_io, rv_b * r_rio);
+    }
 }
 
 /* Mixed path: the rows of column_solvers.c:142-189 rearranged so that every
@@ -231,8 +251,9 @@ __global__ void k_waves_thomas(int nc, WavesWork ww)
         const double dj = ww.d[q], rj = ww.r[q];
         if (j == 0) {
             if (EXACT) {
-                ep[0] = ww.e[q] / dj;
-                rp[0] = rj / dj;
+                const double inv = 1.0 / dj;
+                ep[0] = div_rcp(ww.e[q], dj, inv);
+                rp[0] = div_rcp(rj, dj, inv);
             } else {
                 const double inv = rcp_nr<2>(dj);
                 ep[0] = ww.e[q] * inv;
@@ -242,8 +263,9 @@ __global__ void k_waves_thomas(int nc, WavesWork ww)
             const double cm = ww.c[q - nc];
             const double den = dj - ep[j - 1] * cm;
             if (EXACT) {
-                if (j < n - 1) ep[j] = ww.e[q] / den;
-                rp[j] = (rj - rp[j - 1] * cm) / den;
+                const double inv = 1.0 / den;
+                if (j < n - 1) ep[j] = div_rcp(ww.e[q], den, inv);
+                rp[j] = div_rcp(rj - rp[j - 1] * cm, den, inv);
             } else {
                 const double inv = rcp_nr<2>(den);
                 if (j < n - 1) ep[j] = ww.e[q] * inv;
@@ -253,7 +275,9 @@ __global__ void k_waves_thomas(int nc, WavesWork ww)
     }
     /* damping: divide by 1 + dt * coefficient (mixed path: multiply by the
      * tabulated reciprocal) */
-    auto damp = [&](double x, long long q) { return EXACT ? x / ww.dden[q] : x * ww.damp_inv[q]; };
+    auto damp = [&](double x, long long q) {
+        return EXACT ? div_rcp(x, ww.damp_den[q], ww.damp_inv[q]) : x * ww.damp_inv[q];
+    };
     double x = rp[n - 1];
     ww.r[(long long)(n - 1) * nc + i] = damp(x, (long long)(n - 1) * nc + i);
 #pragma unroll
@@ -285,7 +309,9 @@ __global__ void k_waves_thomas_any(int nc, int nl, WavesWork ww)
             rp[j] = (rj - rp[j - 1] * cm) / den;
         }
     }
-    auto damp = [&](double x, long long q) { return EXACT ? x / ww.dden[q] : x * ww.damp_inv[q]; };
+    auto damp = [&](double x, long long q) {
+        return EXACT ? div_rcp(x, ww.damp_den[q], ww.damp_inv[q]) : x * ww.damp_inv[q];
+    };
     double x = rp[n - 1];
     ww.r[(long long)(n - 1) * nc + i] = damp(x, (long long)(n - 1) * nc + i);
     for (int j = n - 2; j >= 0; --j) {
@@ -312,14 +338,15 @@ __global__ void k_waves_apply(VGrid vg, StepParams p, DState so, DState sn, Wave
         if (jj == 0) num = sol[bb];
         else if (jj == nl - 1) num = -sol[bb - nc];
         else num = -sol[bb - nc] + sol[bb];
-        return EXACT ? ww.rho_expl[bb] + dt * (num) / ve : ww.rho_expl[bb] + dt * num * iv;
+        return EXACT ? ww.rho_expl[bb] + div_rcp(dt * num, ve, vg.r_volume[bb]) : ww.rho_expl[bb] + dt * num * iv;
     };
     const double r_new = rho_new(j, b);
     double num;
     if (j == 0) num = ww.th_int[b] * sol[b];
     else if (j == nl - 1) num = -ww.th_int[b - nc] * sol[b - nc];
     else num = -ww.th_int[b - nc] * sol[b - nc] + ww.th_int[b] * sol[b];
-    const double rt_new = EXACT ? ww.rt_expl[b] + dt * num / vg.volume[b] : ww.rt_expl[b] + dt * num * ww.inv_vol[b];
+    const double rt_new = EXACT ? ww.rt_expl[b] + div_rcp(dt * num, vg.volume[b], vg.r_volume[b])
+                                : ww.rt_expl[b] + dt * num * ww.inv_vol[b];
     const double tp_new = (EXACT ? rt_new / r_new : rt_new * rcp_nr<1>(r_new)) - vg.theta_v_bg[b];
     const double ep_new = so.exner_pert[b] + vg.volume[b] * ww.gam[b] * (rt_new - so.rhotheta_v[b]);
     sn.rho[gp + b] = r_new;
@@ -338,7 +365,8 @@ __global__ void k_waves_apply(VGrid vg, StepParams p, DState so, DState sn, Wave
         const double dint = 0.5 * (r_new + r_below);
         double wn;
         if (EXACT)
-            wn = (2.0 * sol[b] / vg.area_v[wi] - dint * so.w[wi]) / ww.rho_io[b];
+            wn = div_rcp(div_rcp(2.0 * sol[b], vg.area_v[wi], vg.r_area_v[wi]) - dint * so.w[wi], ww.rho_io[b],
+                         ww.r_rho_io[b]);
         else /* rho_io holds 1 / rho at the interface on the mixed path */
             wn = (2.0 * sol[b] * ww.inv_area_v[wi] - dint * so.w[wi]) * ww.rho_io[b];
         sn.w[wi] = wn;
@@ -650,7 +678,7 @@ __global__ void __launch_bounds__(32 * PCR_WARPS) k_waves_pcr(int nc, int nl, Wa
         const double *x = pcr_solution(s, n);
         for (int j = row0; j < n; j += 32) {
             const long long q = (long long)j * nc + i;
-            ww.r[q] = EXACT ? x[j] / ww.dden[q] : x[j] * ww.damp_inv[q];
+            ww.r[q] = EXACT ? div_rcp(x[j], ww.damp_den[q], ww.damp_inv[q]) : x[j] * ww.damp_inv[q];
         }
     }
 }

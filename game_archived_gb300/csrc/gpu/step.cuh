@@ -15,8 +15,6 @@
 namespace game {
 
 inline unsigned nblocks(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
-/* the grid of a kernel over [layers][n] (layer_point) */
-inline dim3 layer_grid(int layers, int n, int bs) { return dim3(nblocks(n, bs), (unsigned)layers); }
 
 template <typename R>
 HGrid<R> &hgrid(Context *c);
@@ -64,10 +62,10 @@ inline WavesWork waves_work(Context *c)
     w.rho_expl = a; w.rt_expl = a + ns; w.alpha = a + 2 * ns; w.beta = a + 3 * ns; w.gam = a + 4 * ns;
     w.tp_expl = a + 5 * ns; w.ep_expl = a + 6 * ns; w.thl = a + 7 * ns;
     w.c = b; w.d = b + ni; w.e = b + 2 * ni; w.r = b + 3 * ni; w.th_int = b + 4 * ni; w.rho_io = b + 5 * ni;
-    w.dden = b + 6 * ni;
+    w.r_rho_io = b + 6 * ni;
     w.inv_vol = c->inv_vol;
     w.inv_area_v = c->inv_area_v;
-    w.damp_dc = c->damp_dc;
+    w.damp_den = c->damp_den;
     w.damp_inv = c->damp_inv;
     w.geo = c->wv_geo;
     return w;
@@ -105,6 +103,19 @@ inline Views<float> views<float>(Context *c, StateMirror *sn)
     return v;
 }
 
+template <typename R>
+PgCells<R> pg_cells(Context *c);
+template <>
+inline PgCells<float> pg_cells<float>(Context *c)
+{
+    return {c->pg_cell};
+}
+template <>
+inline PgCells<double> pg_cells<double>(Context *c)
+{
+    return {c->pg_cell64, c->grad_pi_v, c->w64.v2g_v};
+}
+
 template <typename R, bool ADV, bool PG>
 static void launch_momentum_v(Context *c, const StepParams &p, const Views<R> &v, StateMirror *st, double new_w,
                               double old_w)
@@ -113,9 +124,9 @@ static void launch_momentum_v(Context *c, const StepParams &p, const Views<R> &v
     Work<R> &w = work<R>(c);
     ProfScope ps(c, "k_momentum_v");
     const double *fric_w = p.irr ? c->dbuf->fric : nullptr;
-    const float4 *pc = sizeof(R) == sizeof(float) && PG ? c->pg_cell : nullptr;
     k_momentum_v<R, ADV, PG><<<layer_grid(c->nl + 1, c->nc, 256), 256, 0, c->stream>>>(
-        g, p, v.sv, st->ds.w, w.P_v, w.pvt_v, w.v2g_v, w.flux_h, w.zh, w.v2, new_w, old_w, fric_w, pc);
+        g, p, v.sv, st->ds.w, w.P_v, w.pvt_v, w.v2g_v, w.flux_h, w.zh, w.v2, new_w, old_w, fric_w,
+        pg_cells<R>(c));
     c->kernel_launches++;
 }
 
@@ -127,10 +138,9 @@ static void launch_momentum_h(Context *c, const StepParams &p, const Views<R> &v
     Work<R> &w = work<R>(c);
     ProfScope ps(c, "k_momentum_h");
     const double *fric_u = p.irr ? c->dbuf->fric + (long long)(c->nl + 1) * c->nc : nullptr;
-    const float4 *pc = sizeof(R) == sizeof(float) && PG ? c->pg_cell : nullptr;
     k_momentum_h<R, ADV, PG><<<layer_grid(c->nl, c->ne, 256), 256, 0, c->stream>>>(
         g, p, v.sv, sn->ds.u, v.sh.u, so->ds.u, st->ds.u, w.P_h, w.pg_old_h, w.pvt_h, w.v2g_h, w.flux_h, w.flux_v,
-        w.zh, w.zv, w.v2, new_w, old_w, fric_u, pc);
+        w.zh, w.zv, w.v2, new_w, old_w, fric_u, pg_cells<R>(c));
     c->kernel_launches++;
 }
 
@@ -277,11 +287,14 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
         k_make_shadow<<<nblocks(pairs, bs), bs, 0, c->stream>>>(n_rho, ns, nw, nu, sn->ds, v.sh);
         c->kernel_launches++;
     }
-    if constexpr (!EXACT) {
+    {
         /* the first substage's pressure-gradient factors per cell (the
          * diffusion branch, which runs before it, changes none of its inputs) */
         ProfScope ps(c, "k_pg_cells");
-        k_pg_cells<<<nblocks(ns, bs), bs, 0, c->stream>>>(c->hg32, p, v.sv, c->pg_cell);
+        if constexpr (EXACT)
+            k_pg_cells64<<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(g, p, v.sv, c->pg_cell64, c->grad_pi_v);
+        else
+            k_pg_cells<<<nblocks(ns, bs), bs, 0, c->stream>>>(c->hg32, p, v.sv, c->pg_cell);
         c->kernel_launches++;
     }
     {
@@ -322,6 +335,11 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
                 k_cell_kinetic<R><<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(g, v.sv.u, v.sv.w, rho_gas, w.v2, w.flux_v);
             }
             c->kernel_launches += 3;
+            if constexpr (EXACT) {
+                ProfScope ps(c, "k_grad_v");
+                k_grad_v<<<layer_grid(c->nl - 1, c->nc, bs), bs, 0, c->stream>>>(g, w.v2, w.v2g_v);
+                c->kernel_launches++;
+            }
         }
         /* diffusion branch: momentum part on state_new before the wind update */
         if (rk == 0 && p.diff) launch_diffusion_momentum(c, p, v.sv);
