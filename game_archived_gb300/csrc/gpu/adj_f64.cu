@@ -47,7 +47,7 @@
 #include "adj_ops.h"
 #include "diag.h"
 #include "ops.h"
-#include "solvers.cuh"
+#include "step.cuh"
 
 namespace game {
 namespace {
@@ -330,7 +330,12 @@ void substage_fwd(Context *c, AdjState *a, StepBufs<T> &B, int rk, bool first, c
                                             B.zv[rk], B.v2[rk], B.pvt[rk], B.v2g[rk], B.tend[0], B.tend[rk], so.u,
                                             out.u);
     fa_theta<T><<<nbk(ns), 256, 0, st>>>(ns, sn.rho, sn.rt, B.theta[rk]);
-    if (moist)
+    if constexpr (PLAIN) {
+        const DState d = dview(a, rk ? B.sn1 : B.so);
+        const SView<double> sv{d.rho, d.rhotheta_v, d.theta_v_pert, d.exner_pert, d.w, out.u};
+        launch_scalar_tend64(c, a->p, sv, B.str[0], B.str[rk], B.strt[rk], B.theta[rk], B.pre + 7 * ns, B.pre + 8 * ns,
+                             B.pre + ns, B.pre + 6 * ns, rk == 0 ? sed_prev : B.sed, rk, IrrTerms{});
+    } else if (moist)
         fa_scalar_moist<T><<<nbk(ns, 128), 128, 0, st>>>(g, ap, rk, sn.rho_all, B.theta[rk], out.u, sn.ep, B.pre,
                                                           rk == 0 ? sed_prev : B.sed, B.str[0], B.str[rk],
                                                           B.strt[rk]);

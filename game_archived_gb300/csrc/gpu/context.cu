@@ -370,8 +370,8 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
     std::vector<double> h_ndh = edge_field(nd), h_areah = edge_field(area), h_zh = edge_field(zv),
                         h_slope = edge_field(slope), h_ebggh = edge_field(ebgg);
     /* cells none of whose edges slopes in any layer: there every
-     * terrain-following correction of the scalar tendencies vanishes, and the
-     * mixed path skips it (the FP64 path keeps the reference's operations) */
+     * terrain-following correction of the scalar tendencies vanishes and is
+     * skipped */
     std::vector<int> h_tilt(NC, 0);
     for (int i = 0; i < NC; ++i) {
         const int n_edges = i < N_PENT ? 5 : 6;
@@ -384,6 +384,7 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
                 }
         }
     }
+    for (int t : h_tilt) c->any_tilt |= t;
     std::vector<double> h_tw((size_t)10 * NE), h_rw((size_t)4 * NE), h_fvec((size_t)2 * NE);
     std::vector<int> h_ti((size_t)10 * NE), h_tm((size_t)10 * NE), h_ri((size_t)4 * NE);
     for (int e = 0; e < NE; ++e) {
@@ -670,6 +671,9 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
         g.rhombus_area = dalloc<double>(c, (size_t)L * NE);
         g.r_rhombus_area = dalloc<double>(c, (size_t)L * NE);
         g.tri_circ = dalloc<double>(c, (size_t)3 * L * NT);
+        g.corr_w = dalloc<double>(c, (size_t)6 * NS);
+        c->edge_flux64 = dalloc<double>(c, (size_t)2 * L * NE);
+        c->level_corr64 = dalloc<double>(c, (size_t)3 * (L + 1) * NC);
     }
     for (auto &b : c->owned)
         if (!b.p) return fail("device allocation failed");

@@ -50,6 +50,7 @@ struct StateMirror {
 
 struct Context {
     game_dims dims{};
+    int any_tilt = 0; /* some edge of the grid slopes */
     int nc = 0, ne = 0, nt = 0, nl = 0, n_oro = 0, n_const = 0, n_cond = 0, moist = 0;
     long long ns = 0, nv = 0, ndv = 0, ncurl = 0, state_len = 0;
     double radius = 0.0, toa = 0.0;
@@ -102,6 +103,10 @@ struct Context {
     /* FP64 path: the same factors in double, and the vertical gradient of
      * Pi' at the inner interfaces [L+1][Nc] */
     Quad *pg_cell64 = nullptr;
+    /* FP64 path: mass and rho theta_v fluxes of the edges [2][L][Ne], and the
+     * terrain corrections of both and of the wind at the levels [3][L+1][Nc],
+     * of the substage at hand (k_edge_flux, k_level_corr) */
+    double *edge_flux64 = nullptr, *level_corr64 = nullptr;
     double *grad_pi_v = nullptr;
     double *gravity_potential = nullptr; /* [L][Nc] */
     /* global integrals: per-block (hi, lo) partial sums, one counter and one

@@ -86,6 +86,7 @@ struct HGrid {
     const R *r_dz_h;                        /* [L+1][Ne] of z_h(k-1) - z_h(k) at the inner levels */
     const R *rhombus_area, *r_rhombus_area; /* [L][Ne] sum of the two triangles' areas */
     const R *tri_circ;                      /* [3][L][Nt] circulation weight of edge j: rescaled length times sign */
+    const R *corr_w;                        /* [6][L][Nc] terrain-correction weight of edge j: -ipw / 2 times slope */
 };
 
 /* device tables of the output pass, built at initialisation (device order

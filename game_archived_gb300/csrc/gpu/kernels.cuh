@@ -1288,6 +1288,176 @@ __global__ void __launch_bounds__(128) k_scalar_tend2(HGrid<R> g, StepParams p, 
     }
 }
 
+/* ---- the same tendencies on the FP64 path, in three kernels.  FP64 issue
+ * bounds them, so nothing is formed twice: the fluxes of an edge once
+ * (k_edge_flux) instead of by both its cells in up to three layer passes, the
+ * terrain corrections of a level once (k_level_corr) instead of by the cells
+ * above and below it, with tabulated weights, and only in columns with a
+ * sloping edge; constituents absent around an edge and zero heating are
+ * skipped (they add zeros).  Every accumulator receives the reference's terms
+ * in its order (layer k-1 before k, edges j = 0..5).
+ * RES_ID 5 with the mountain: 180 -> 72 us per substage; RES_ID 6 moist,
+ * flat: 1175 -> 486 us. */
+
+/* horizontal mass flux of the main gas and rho theta_v flux of every edge */
+__global__ void k_edge_flux(HGrid<double> g, const double *rho_gas, const double *theta, const double *u, double *flux_m,
+                            double *flux_t)
+{
+    const LayerPoint p = layer_point(g.ne);
+    if (!p.in) return;
+    const long long o = (long long)p.l * g.nc;
+    const int fr = g.from[p.x], to = g.to[p.x];
+    const double fm = (0.5 * (rho_gas[o + fr] + rho_gas[o + to])) * u[p.i];
+    flux_m[p.i] = fm;
+    flux_t[p.i] = (0.5 * (theta[o + fr] + theta[o + to])) * fm;
+}
+
+/* terrain corrections at level k (from layers k-1 and k, averaging.c:41-95)
+ * of the mass and rho theta_v fluxes, times the interface's area, and of the
+ * wind (WIND: for the tracers).  Grid: levels nl - n_oro .. nl - 1. */
+template <bool WIND>
+__global__ void k_level_corr(HGrid<double> g, const double *flux_m, const double *flux_t, const double *u,
+                             double *corr_m, double *corr_t, double *corr_w)
+{
+    const LayerPoint p = layer_point(g.nc);
+    if (!p.in || !g.tilt[p.x]) return;
+    const int c = p.x, k = p.l + g.nl - g.n_oro, n_edges = c < N_PENT ? 5 : 6;
+    const long long ns = (long long)g.nl * g.nc, kc = (long long)k * g.nc + c;
+    int e[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) e[j] = j < n_edges ? g.adj[j * g.nc + c] : 0;
+    double m = 0.0, t = 0.0, w = 0.0;
+    for (int ll = p.l > 0 ? k - 1 : k; ll <= k; ++ll) {
+        const double *cw = g.corr_w + (long long)ll * g.nc + c;
+        const long long lo = (long long)ll * g.ne;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            if (j >= n_edges) continue;
+            const double wc = cw[j * ns];
+            m += wc * flux_m[lo + e[j]];
+            t += wc * flux_t[lo + e[j]];
+            if (WIND) w += wc * u[lo + e[j]];
+        }
+    }
+    const double area = g.area_v[kc];
+    corr_m[kc] = m * area;
+    corr_t[kc] = t * area;
+    if (WIND) corr_w[kc] = w;
+}
+
+/* the tendencies of a cell from them; rho_prev: the tendencies of the
+ * previous substage (old weight 1/2 at rk 1, non-main constituents) */
+template <bool IRR>
+__global__ void __launch_bounds__(128)
+    k_scalar_tend64(HGrid<double> g, StepParams p, SView<double> sv, const double *rho_prev, double *st_rho,
+                    double *st_rt, const double *flux_m, const double *flux_t, const double *corr, const double *theta,
+                    const double *cp_ice, const double *cp_water, const double *pt_rates, const double *pt_heat,
+                    const double *sed_heat, int rk, IrrTerms irr)
+{
+    const LayerPoint pt_ = layer_point(g.nc);
+    if (!pt_.in) return;
+    const long long i = pt_.i, nc = g.nc, ne = g.ne, ns = (long long)g.nl * nc, nw = ns + nc;
+    const int l = pt_.l, c = pt_.x, nl = g.nl, n_oro = g.n_oro, cond = p.n_cond;
+    const int n_edges = c < N_PENT ? 5 : 6;
+    /* corrections at the level above (up) and below (lo) the layer */
+    const bool oro = l >= nl - n_oro - 1 && g.tilt[c];
+    const bool up = oro && l >= nl - n_oro, lo = oro && l < nl - 1;
+    const double inv_vol = g.r_volume[i];
+    int ej[6];
+    bool sfj[6];
+    double arj[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const bool on = j < n_edges;
+        ej[j] = on ? g.adj[j * nc + c] : 0;
+        sfj[j] = on && g.adj_sign[j * nc + c] > 0;
+        arj[j] = on ? g.area_h[(long long)l * ne + ej[j]] : 0.0;
+    }
+    auto comp_v = [&](const double *cr) {
+        const double a = up ? cr[i] : 0.0, b = lo ? cr[i + nc] : 0.0;
+        return up ? (lo ? a - b : a) : -b;
+    };
+    const long long lo_e = (long long)l * ne;
+    {
+        double hm = 0.0, ht = 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            if (j >= n_edges) continue;
+            const double am = flux_m[lo_e + ej[j]] * arj[j], at = flux_t[lo_e + ej[j]] * arj[j];
+            hm += sfj[j] ? am : -am;
+            ht += sfj[j] ? at : -at;
+        }
+        double y = -(inv_vol * (oro ? hm + comp_v(corr) : hm));
+        double yt = -(inv_vol * (oro ? ht + comp_v(corr + nw) : ht));
+        double rate = p.moist ? pt_rates[cond * ns + i] : 0.0;
+        if (IRR) y = y + irr.mass_diff[cond * ns + i];
+        if (p.moist) y = y + rate;
+        st_rho[cond * ns + i] = y;
+        if (p.moist || IRR) {
+            /* diabatic heating: c_v-weighted, divided by c_p * Pi */
+            double heat = pt_heat[i] + sed_heat[i];
+            if (IRR) {
+                heat = irr.heating_diss[i] + irr.temp_diff_heating[i] + irr.radiation[i] + pt_heat[i] + sed_heat[i];
+                rate = pt_rates[cond * ns + i] + irr.mass_diff[cond * ns + i];
+            }
+            if (!is_zero(heat)) {
+                const double rg = sv.rho[cond * ns + i];
+                double cv = 0.0;
+                for (int kk = 0; kk < cond; ++kk) {
+                    const double r = sv.rho[kk * ns + i];
+                    if (!is_zero(r)) cv += r * ((kk % 2 == 0) ? cp_ice[i] : cp_water[i]);
+                }
+                cv += rg * C_D_V;
+                if (p.moist) cv += sv.rho[(cond + 1) * ns + i] * C_V_V;
+                yt = yt + C_D_V * rg / cv * heat / (C_D_P * (g.exner_bg[i] + sv.exner_pert[i]));
+            }
+            yt = yt + rate * theta[i];
+        }
+        st_rt[i] = yt;
+    }
+    if (p.n_const == 1) return;
+    /* the other constituents: upstream flux */
+    int nbj[6];
+    double uj[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const bool on = j < n_edges;
+        uj[j] = on ? sv.u[lo_e + ej[j]] : 0.0;
+        /* the upstream cell: the cell itself where the wind leaves it (u =
+         * -0 picks the other one, whose product is a zero as well) */
+        nbj[j] = on && nonneg<false>(uj[j]) != sfj[j] ? g.adj_nbr[j * nc + c] : c;
+    }
+    const double w_up = up ? corr[2 * nw + i] : 0.0, w_lo = lo ? corr[2 * nw + i + nc] : 0.0;
+    const double area_up = oro ? g.area_v[i] : 0.0, area_lo = oro ? g.area_v[i + nc] : 0.0;
+    const double *fl = sv.rho + (long long)l * nc;
+#pragma unroll 1
+    for (int k = 0; k < p.n_const; ++k, fl += ns) {
+        if (k == cond) continue;
+        double h = 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            if (j >= n_edges) continue;
+            const double d = fl[nbj[j]];
+            if (is_zero(d)) continue;
+            const double a = d * uj[j] * arj[j];
+            h += sfj[j] ? a : -a;
+        }
+        if (oro) {
+            const double d_up = up ? (w_up <= 0.0 ? fl[c - nc] : fl[c]) : 0.0;
+            const double d_lo = lo ? (w_lo <= 0.0 ? fl[c] : fl[c + nc]) : 0.0;
+            double cv;
+            if (!up) cv = -d_lo * w_lo * area_lo;
+            else if (!lo) cv = d_up * w_up * area_up;
+            else cv = d_up * w_up * area_up - d_lo * w_lo * area_lo;
+            h = h + cv;
+        }
+        double y = -(inv_vol * h);
+        if (IRR) y = y + irr.mass_diff[k * ns + i];
+        if (p.moist) y = y + pt_rates[(k == cond + 1 ? k - 1 : k) * ns + i];
+        st_rho[k * ns + i] = rk == 0 ? y : 0.5 * rho_prev[k * ns + i] + 0.5 * y;
+    }
+}
+
 /* per-thread column sweeps of the adjoint hold at most this many layers */
 constexpr int MAX_L = 64;
 

@@ -103,6 +103,36 @@ inline Views<float> views<float>(Context *c, StateMirror *sn)
     return v;
 }
 
+/* the FP64 path's scalar tendencies; theta: rho theta_v / rho_gas */
+inline void launch_scalar_tend64(Context *c, const StepParams &p, const SView<double> &sv, const double *rho_prev,
+                                 double *st_rho, double *st_rt, const double *theta, const double *cp_ice,
+                                 const double *cp_water, const double *pt_rates, const double *pt_heat,
+                                 const double *sed_heat, int rk, const IrrTerms &irr)
+{
+    const HGrid<double> &g = c->hg64;
+    const long long nu = (long long)c->nl * c->ne, nw = (long long)(c->nl + 1) * c->nc;
+    double *fm = c->edge_flux64, *ft = fm + nu, *cr = c->level_corr64;
+    cudaStream_t s = c->stream;
+    k_edge_flux<<<layer_grid(c->nl, c->ne, 256), 256, 0, s>>>(g, sv.rho + (long long)c->n_cond * c->ns, theta, sv.u, fm,
+                                                             ft);
+    c->kernel_launches += 2;
+    if (c->any_tilt) {
+        const dim3 nb = layer_grid(c->n_oro, c->nc, 256);
+        if (p.n_const > 1)
+            k_level_corr<true><<<nb, 256, 0, s>>>(g, fm, ft, sv.u, cr, cr + nw, cr + 2 * nw);
+        else
+            k_level_corr<false><<<nb, 256, 0, s>>>(g, fm, ft, sv.u, cr, cr + nw, cr + 2 * nw);
+        c->kernel_launches++;
+    }
+    const dim3 nb = layer_grid(c->nl, c->nc, 128);
+    if (p.irr)
+        k_scalar_tend64<true><<<nb, 128, 0, s>>>(g, p, sv, rho_prev, st_rho, st_rt, fm, ft, cr, theta, cp_ice, cp_water,
+                                                 pt_rates, pt_heat, sed_heat, rk, irr);
+    else
+        k_scalar_tend64<false><<<nb, 128, 0, s>>>(g, p, sv, rho_prev, st_rho, st_rt, fm, ft, cr, theta, cp_ice, cp_water,
+                                                  pt_rates, pt_heat, sed_heat, rk, irr);
+}
+
 template <typename R>
 PgCells<R> pg_cells(Context *c);
 template <>
@@ -365,18 +395,22 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
         }
         {
             ProfScope ps(c, "k_scalar_tend");
-            if (p.irr) {
-                const DiffBufs &b = *c->dbuf;
+            IrrTerms irr{};
+            if (p.irr) irr = {c->dbuf->hdiss, c->dbuf->tdh, c->dbuf->rad, c->dbuf->mdt};
+            if constexpr (EXACT) {
+                launch_scalar_tend64(c, p, v.sv, st->ds.rho, st->ds.rho, st->ds.rhotheta_v, theta, cpi, cpw, c->pt_rates,
+                                     c->pt_heat, c->sed_heat, rk, irr);
+            } else if (p.irr) {
                 k_scalar_tend2<R, true><<<layer_grid(c->nl, c->nc, 128), 128, 0, c->stream>>>(
                     g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, rk,
-                    IrrTerms{b.hdiss, b.tdh, b.rad, b.mdt});
+                    irr);
             } else {
                 k_scalar_tend2<R, false><<<layer_grid(c->nl, c->nc, 128), 128, 0, c->stream>>>(
                     g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, rk,
-                    IrrTerms{});
+                    irr);
             }
         }
-        c->kernel_launches += 2;
+        c->kernel_launches += EXACT ? 1 : 2; /* launch_scalar_tend64 counts its own */
         /* the tendency is final from here on: a host-in/host-out call copies
          * it out while the solvers run */
         if (rk == 1) {

@@ -52,6 +52,18 @@ __global__ void k_tri_circ(HGrid<double> g, double *w)
     }
 }
 
+/* weights of the terrain corrections (averaging.c:41-95) */
+__global__ void k_corr_w(HGrid<double> g, double *w)
+{
+    const LayerPoint p = layer_point(g.nc);
+    if (!p.in) return;
+    const long long ns = (long long)g.nl * g.nc;
+    const int n_edges = p.x < N_PENT ? 5 : 6;
+    for (int j = 0; j < 6; ++j)
+        w[j * ns + p.i] =
+            j < n_edges ? -0.5 * ipw_at(g, j, p.l, p.x) * g.slope_h[(long long)p.l * g.ne + g.adj[j * g.nc + p.x]] : 0.0;
+}
+
 }  // namespace
 
 int make_f64_tables(Context *c)
@@ -70,6 +82,7 @@ int make_f64_tables(Context *c)
     k_rhombus_area<<<layer_grid(c->nl, c->ne, 256), 256>>>(g, const_cast<double *>(g.rhombus_area),
                                               const_cast<double *>(g.r_rhombus_area));
     k_tri_circ<<<layer_grid(c->nl, c->nt, 256), 256>>>(g, const_cast<double *>(g.tri_circ));
+    k_corr_w<<<layer_grid(c->nl, c->nc, 256), 256>>>(g, const_cast<double *>(g.corr_w));
     CK(cudaDeviceSynchronize());
     CK(cudaGetLastError());
     return 0;
