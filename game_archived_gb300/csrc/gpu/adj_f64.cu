@@ -375,7 +375,11 @@ void step_fwd(Context *c, AdjState *a, StepBufs<T> &B, const T *P_prev, const T 
     const long long nv = a->nv;
     AState<T> so = view(a, B.so);
     if (moist_of(a)) {
-        fa_prelude<T><<<nbk(a->ns), 256, 0, st>>>(c->vg, ap, so, B.pre);
+        if constexpr (sizeof(T) == sizeof(double))
+            k_cell_prepare<<<nbk(a->ns), 256, 0, st>>>(c->vg, a->p, dview(a, B.so), B.pre, B.pre + a->ns,
+                                                       B.pre + 6 * a->ns, B.pre + 7 * a->ns, B.pre + 8 * a->ns);
+        else
+            fa_prelude<T><<<nbk(a->ns), 256, 0, st>>>(c->vg, ap, so, B.pre);
         c->kernel_launches++;
     }
     if constexpr (sizeof(T) == sizeof(double)) {

