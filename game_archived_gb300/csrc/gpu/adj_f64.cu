@@ -294,6 +294,25 @@ void waves_fwd(Context *c, AdjState *a, int rk, DState so, DState sn, DState ten
     fa_w_bounds<<<nbk(c->nc), 256, 0, st>>>(c->nc, c->nl, so.w, out.w);
 }
 
+/* the tracer solve (per-thread sweeps whatever the solver setting, as the
+ * adjoint transposes them) and at rk 0 the sedimentation heat */
+void tracers_fwd(Context *c, AdjState *a, int rk, DState so, DState out, double *str, const double *pre, double *sed)
+{
+    const long long ns = a->ns, nsys = (long long)(a->n_const - 1) * c->nc;
+    cudaStream_t st = c->stream;
+    const TracerWork tw{pre + 7 * ns, pre + 8 * ns, c->inv_vol};
+    if (rk == 0) {
+        k_tracers_sedheat64<<<layer_grid(c->nl, c->nc, 128), 128, 0, st>>>(c->vg, a->p, so, out, pre, tw, sed);
+        c->kernel_launches++;
+    }
+    const DState tend{str, nullptr, nullptr, nullptr, nullptr, nullptr};
+    if (c->nl == 26)
+        k_tracers_solve<26, 26, true><<<nbk(nsys, 64), 64, 0, st>>>(c->vg, a->p, so, out, tend, tw, nullptr);
+    else
+        k_tracers_solve<0, MAX_L, true><<<nbk(nsys, 64), 64, 0, st>>>(c->vg, a->p, so, out, tend, tw, nullptr);
+    c->kernel_launches++;
+}
+
 /* ----------------------------------------------------------- step forward */
 /* the substage rk of a step: sn its input state (so at rk 0), out its
  * output (sn1, sn2); sed_prev the previous step's sedimentation heat */
@@ -354,6 +373,10 @@ void substage_fwd(Context *c, AdjState *a, StepBufs<T> &B, int rk, bool first, c
     }
     c->kernel_launches += adv ? 11 : 8;
     if (moist) {
+        if constexpr (PLAIN) {
+            tracers_fwd(c, a, rk, dview(a, B.so), dview(a, rk ? B.sn2 : B.sn1), B.str[rk], B.pre, B.sed);
+            return;
+        }
         if (rk == 0) {
             fa_sedheat<T><<<nbk(c->nc, 128), 128, 0, st>>>(vg, a->p, so, out.w, B.pre, B.sed);
             c->kernel_launches++;

@@ -266,9 +266,12 @@ void launch_tracers(Context *c, const StepParams &p, StateMirror *so, StateMirro
         if (!EXACT && p.dfloat)
             k_tracers_sedheat_df<<<nblocks(ns, 128), 128, 0, strm>>>(c->vg, p, so->ds, sn->ds, temperature, tw,
                                                                      c->dfg, sed_heat);
+        else if (EXACT)
+            k_tracers_sedheat64<<<layer_grid(c->nl, c->nc, 128), 128, 0, strm>>>(c->vg, p, so->ds, sn->ds, temperature,
+                                                                                 tw, sed_heat);
         else
-            k_tracers_sedheat<EXACT><<<nblocks(c->nc, 128), 128, 0, strm>>>(c->vg, p, so->ds, sn->ds, temperature,
-                                                                                tw, sed_heat);
+            k_tracers_sedheat<<<nblocks(c->nc, 128), 128, 0, strm>>>(c->vg, p, so->ds, sn->ds, temperature, tw,
+                                                                     sed_heat);
         c->kernel_launches++;
     }
     ProfScope ps(c, "k_tracers_solve");
