@@ -121,7 +121,8 @@ struct AdjState {
     StepBufs<double> B;          /* forward tape of one step */
     StepBufs<double> Z;          /* bars of one step */
     StepBufs<Dual> D;            /* tangent-linear run */
-    double *rn_b = nullptr, *rtn_b = nullptr;
+    double *rn_b = nullptr, *rtn_b = nullptr; /* work of the wave solver's adjoint */
+    double *db = nullptr, *br = nullptr;
     double *dden = nullptr, *r_dden = nullptr; /* damping denominators and their reciprocals [L-1][Nc] */
     double *fv_bounds = nullptr;               /* (L+1) Nc */
     /* checkpoints of every ck_every-th step start and of the window's end,
@@ -228,7 +229,8 @@ int ensure_adj(Context *c)
     a->nzh = (long long)(c->nl + 1) * c->ne;
     a->nwi = (long long)(c->nl - 1) * c->nc;
     bool ok = alloc_step(a, a->B) && alloc_step(a, a->Z) && alloc_step(a, a->D);
-    ok = ok && (a->rn_b = aalloc<double>(a, a->ns)) && (a->rtn_b = aalloc<double>(a, a->ns));
+    ok = ok && (a->rn_b = aalloc<double>(a, a->ns)) && (a->rtn_b = aalloc<double>(a, a->ns))
+         && (a->db = aalloc<double>(a, a->nwi)) && (a->br = aalloc<double>(a, BR_N * a->nwi));
     ok = ok && (a->dden = aalloc<double>(a, a->nwi)) && (a->r_dden = aalloc<double>(a, a->nwi))
          && (a->fv_bounds = aalloc<double>(a, a->nw));
     ok = ok && (a->obj_w = aalloc<double>(a, c->nc)) && (a->obj_p = aalloc<double>(a, c->nc))
@@ -427,6 +429,26 @@ void step_fwd(Context *c, AdjState *a, StepBufs<T> &B, const T *P_prev, const T 
     substage_fwd<T>(c, a, B, 1, first, sed_prev);
 }
 
+/* adjoint of the sound-wave solve (waves_fwd) of substage rk */
+void waves_bwd(Context *c, AdjState *a, int rk, AState<double> so, AState<double> sn, AState<double> out,
+               const double *str, const double *strt, const double *wl, const double *wr, AState<double> out_b,
+               AState<double> so_b, AState<double> sn_b, double *str_b, double *strt_b, double *tend_w_b)
+{
+    const VGrid &vg = c->vg;
+    cudaStream_t st = c->stream;
+    double *wl_b = a->Z.wl[0], *wr_b = a->Z.wr[0];
+    const dim3 cells = layer_grid(c->nl, c->nc, 256);
+    ba_apply_state<<<cells, 256, 0, st>>>(vg, so, wl, wr, out, out_b, a->rn_b, a->rtn_b, a->db, so_b, wl_b, wr_b);
+    ba_apply_rho<<<cells, 256, 0, st>>>(vg, a->p.dt, wr, a->rn_b, a->rtn_b, a->db, wl_b, wr_b);
+    if (c->nl == 26)
+        ba_thomas<26, 26><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, a->r_dden, wr, wr_b);
+    else
+        ba_thomas<0, MAX_L><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, a->r_dden, wr, wr_b);
+    ba_waves_rows<<<layer_grid(c->nl - 1, c->nc, 256), 256, 0, st>>>(vg, a->p, so, wl, wr, wr_b, a->br, so_b, tend_w_b);
+    ba_waves_layer<<<cells, 256, 0, st>>>(vg, a->p.dt, rk, so, sn, str, strt, wl, wl_b, a->br, so_b, sn_b, str_b,
+                                          strt_b);
+}
+
 /* ---------------------------------------------------------- step backward
  * s2b: bar of the step's end state (modified); P_next_b, pvt_next_b,
  * v2g_next_b, sed_next_b: bars of this step's lagged outputs from the next
@@ -469,8 +491,6 @@ void step_bwd(Context *c, AdjState *a, bool first, double *s2b, const double *P_
         zero(Z.theta[r], ns);
         zero(Z.str[r], a->nrho);
         zero(Z.strt[r], ns);
-        zero(Z.wl[r], WL_N * ns);
-        zero(Z.wr[r], WR_N * a->nwi);
     }
     if (pvt_next_b) ku_copy<double><<<nbk(nv), 256, 0, st>>>(nv, pvt_next_b, Z.pvt[1]);
     if (v2g_next_b) ku_copy<double><<<nbk(nv), 256, 0, st>>>(nv, v2g_next_b, Z.v2g[1]);
@@ -497,15 +517,9 @@ void step_bwd(Context *c, AdjState *a, bool first, double *s2b, const double *P_
             if (adj_gen_densities(c, a->p, &mso, &msn, &mst, B.pre, rk, Z.sed, &mso_b, &msn_b, &mst_b, Z.pre))
                 return;
         }
-        ba_apply_layer<<<nbk(ns), 256, 0, st>>>(vg, so, B.wl[rk], out, out_b, a->rn_b, a->rtn_b, sob_v, Z.wl[rk]);
-        ba_apply_w<<<nbk(a->nwi), 256, 0, st>>>(vg, so, B.wr[rk], out, out_b, a->rn_b, sob_v, Z.wr[rk]);
-        ba_apply_rho<<<nbk(ns), 256, 0, st>>>(vg, ap, B.wr[rk], a->rn_b, a->rtn_b, Z.wl[rk], Z.wr[rk]);
-        ba_thomas<<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, B.wr[rk], Z.wr[rk]);
-        ba_waves_rows<<<nbk(a->nwi), 256, 0, st>>>(vg, ap, so, B.wl[rk], B.wr[rk], Z.wr[rk], Z.wl[rk], sob_v,
-                                                   Z.tend[rk]);
         const long long gas = (long long)a->n_cond * ns;
-        ba_waves_layer<<<nbk(ns), 256, 0, st>>>(vg, ap, rk, so, sn, B.str[rk] + gas, B.strt[rk], B.wl[rk], Z.wl[rk],
-                                                sob_v, sn_b, Z.str[rk] + gas, Z.strt[rk]);
+        waves_bwd(c, a, rk, so, sn, out, B.str[rk] + gas, B.strt[rk], B.wl[rk], B.wr[rk], out_b, sob_v, sn_b,
+                  Z.str[rk] + gas, Z.strt[rk], Z.tend[rk]);
         /* scalar tendencies: densities and theta_v of sn, the wind of out */
         if (moist)
             ba_scalar_moist<<<nbk(ns, 128), 128, 0, st>>>(g, ap, rk, sn.rho_all, B.theta[rk], out.u, sn.ep, B.pre,
@@ -956,7 +970,7 @@ int adj_waves_backward(Context *c, StateMirror *so_m, StateMirror *sn_m, StateMi
     const AParams ap = a->ap;
     const long long ns = a->ns;
     AState<double> so = view(a, so_m->dev), sn = view(a, sn_m->dev), out = view(a, a->B.sn2);
-    double *wl = a->B.wl[0], *wr = a->B.wr[0], *wl_b = a->Z.wl[0], *wr_b = a->Z.wr[0];
+    double *wl = a->B.wl[0], *wr = a->B.wr[0];
     /* forward of the solver, keeping its work */
     waves_fwd(c, a, rk, so_m->ds, sn_m->ds, st_m->ds, wl, wr, dview(a, a->B.sn2));
     /* bars: the output bar moves to a work block, the input bar starts with
@@ -967,15 +981,8 @@ int adj_waves_backward(Context *c, StateMirror *so_m, StateMirror *sn_m, StateMi
     AState<double> out_b = view(a, ob), in_b = view(a, ib), so_b = view(a, so_bar->dev);
     ku_waves_passthrough<<<nbk(std::max<long long>(a->nu, c->nc)), 256, 0, st>>>(c->nc, c->nl, a->nu, out_b.w,
                                                                                    out_b.u, in_b.w, in_b.u);
-    cudaMemsetAsync(wl_b, 0, (size_t)WL_N * ns * sizeof(double), st);
-    cudaMemsetAsync(wr_b, 0, (size_t)WR_N * a->nwi * sizeof(double), st);
-    ba_apply_layer<<<nbk(ns), 256, 0, st>>>(vg, so, wl, out, out_b, a->rn_b, a->rtn_b, so_b, wl_b);
-    ba_apply_w<<<nbk(a->nwi), 256, 0, st>>>(vg, so, wr, out, out_b, a->rn_b, so_b, wr_b);
-    ba_apply_rho<<<nbk(ns), 256, 0, st>>>(vg, ap, wr, a->rn_b, a->rtn_b, wl_b, wr_b);
-    ba_thomas<<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, wr, wr_b);
-    ba_waves_rows<<<nbk(a->nwi), 256, 0, st>>>(vg, ap, so, wl, wr, wr_b, wl_b, so_b, st_bar->ds.w);
-    ba_waves_layer<<<nbk(ns), 256, 0, st>>>(vg, ap, rk, so, sn, st_m->ds.rho, st_m->ds.rhotheta_v, wl, wl_b, so_b,
-                                            in_b, st_bar->ds.rho, st_bar->ds.rhotheta_v);
+    waves_bwd(c, a, rk, so, sn, out, st_m->ds.rho, st_m->ds.rhotheta_v, wl, wr, out_b, so_b, in_b, st_bar->ds.rho,
+              st_bar->ds.rhotheta_v, st_bar->ds.w);
     c->kernel_launches += 12;
     CK(cudaGetLastError());
     return 0;
