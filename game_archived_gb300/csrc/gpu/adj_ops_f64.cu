@@ -255,125 +255,173 @@ __device__ double d_cpT(int id, double t)
     return dcp * t + c_p_cond(id, t);
 }
 
-/* three_band_solver_gen_densities (column_solvers.c:385-639) in reverse mode;
- * thread = (tracer slot, column).  The column's rows and unclipped solution
- * are rebuilt, the transposed tridiagonal system gives the bar of the
- * right-hand side, and the bars of the rows move to the inputs: the old
- * density and tendency of the tracer (owned by the thread), the old and new
- * vertical wind and, at rk 0, the temperature through the sedimentation heat
- * (shared by the tracer slots: atomic).  Upwind picks and flux-sign branches
- * are held fixed; clipped outputs carry no derivative.  The thread takes the
- * bar of its tracer's new density and leaves it zero (the forward overwrites
- * that field without reading it). */
-template <int CAP>
-__global__ void ka_gen_densities(VGrid vg, StepParams p, DState so, DState sn, DState st, const double *temperature,
-                                 int rk, const double *sed_b, DState so_b, DState sn_b, DState st_b, double *t_b)
+/* three_band_solver_gen_densities (column_solvers.c:385-639) in reverse mode,
+ * in three kernels over its (tracer, column) systems: the rows per (tracer,
+ * layer, column), the two tridiagonal solves per (tracer, column) -- the
+ * unclipped solution x and the bar y of the right-hand side, the transposed
+ * system's -- and the bars of the inputs per (tracer, layer, column) again:
+ * the old density and tendency of the tracer, the old and new vertical wind
+ * and, at rk 0, the temperature through the sedimentation heat.  One kernel
+ * with a column per thread did all of it in local memory with 200 blocks of
+ * work at RES_ID 4: 551 -> 152 us.  Upwind picks and flux-sign branches are
+ * held fixed; clipped outputs carry no derivative.  The bar of the new
+ * density is taken and left zero (the forward overwrites that field without
+ * reading it).
+ * work: 4 arrays [C-1][L][Nc]: c, d (x after the solve), e, r (y after it). */
+struct TracerRows {
+    double *c, *d, *e, *r;
+};
+struct TracerSlot {
+    int k;       /* constituent */
+    bool sink;   /* sediments */
+    double vs;   /* its velocity */
+};
+__device__ __forceinline__ TracerSlot tracer_slot(const StepParams &p, int slot)
 {
-    const int nc = vg.nc, nl = vg.nl;
-    const long long ns = (long long)nl * nc;
+    const int cond = p.n_cond, k = slot < cond ? slot : slot + 1;
+    const bool sink = k < cond;
+    return {k, sink,
+            k < cond / 4 ? p.snow_velocity : k < cond / 2 ? p.rain_velocity : sink ? p.cloud_velocity : 0.0};
+}
+
+/* grid: x cells, y layers, z tracer slots */
+__global__ void ka_gen_rows(VGrid vg, StepParams p, DState so, DState sn, DState st, TracerRows w)
+{
+    const LayerPoint pt = layer_point(vg.nc);
+    if (!pt.in) return;
+    const int nc = vg.nc, nl = vg.nl, j = pt.l;
+    const long long ns = (long long)nl * nc, b = pt.i, o = (long long)blockIdx.z * ns + b;
+    const TracerSlot s = tracer_slot(p, blockIdx.z);
+    const double *ro = so.rho + s.k * ns;
+    const double dt = p.dt, h = 0.5 * dt, v = vg.volume[b], rv = vg.r_volume[b];
+    const double g = div_rcp(h, v, rv);
+    double c = 0.0, d = 1.0, e = 0.0, r = ro[b] + dt * st.rho[s.k * ns + b];
+    if (j < nl - 1) {
+        const long long wi = b + nc;
+        const double ar = vg.area_v[wi], f = ar * (so.w[wi] - s.vs), bw = ar * (sn.w[wi] - s.vs);
+        const double fr = (nonneg<true>(bw) ? ro[wi] : ro[b]) * bw;
+        if (nonneg<true>(f)) {
+            e = -g * f;
+        } else {
+            c = div_rcp(h, vg.volume[wi], vg.r_volume[wi]) * f;
+            d -= g * f;
+        }
+        r += div_rcp(h * fr, v, rv);
+    }
+    if (j > 0) {
+        const double ar = vg.area_v[b], f = ar * (so.w[b] - s.vs), bw = ar * (sn.w[b] - s.vs);
+        const double fr = (nonneg<true>(bw) ? ro[b] : ro[b - nc]) * bw;
+        if (nonneg<true>(f)) d += g * f;
+        r -= div_rcp(h * fr, v, rv);
+    }
+    if (j == nl - 1 && s.sink) {
+        const double a = h * s.vs * vg.area_v[b + nc];
+        d += div_rcp(a, v, rv);
+        r -= div_rcp(a * ro[b], v, rv);
+    }
+    w.c[o] = c;
+    w.d[o] = d;
+    w.e[o] = e;
+    w.r[o] = r;
+}
+
+/* x over d, y over r.  NL > 0: the layer count is a compile-time constant and
+ * the sweeps stay in registers; else the layer count is nl (at most CAP) */
+template <int NL, int CAP>
+__global__ void ka_gen_solve(int nc, int nl_arg, int n_tr, int n_cond, TracerRows w, DState sn_b)
+{
     const long long q = gtid();
-    if (q >= (long long)(p.n_const - 1) * nc) return;
+    if (q >= (long long)n_tr * nc) return;
+    const int nl = NL > 0 ? NL : nl_arg;
     const int slot = row_of(q, nc), i = (int)(q - (long long)slot * nc);
-    const int k = slot < p.n_cond ? slot : slot + 1;
-    const int cond = p.n_cond;
-    const bool sink = k < cond, heat = rk == 0 && k < cond;
-    const double vs = k < cond / 4 ? p.snow_velocity : k < cond / 2 ? p.rain_velocity : sink ? p.cloud_velocity : 0.0;
-    const double dt = p.dt, iw = 0.5, ew = 0.5;
-    const double *ro = so.rho + k * ns, *tr = st.rho + k * ns;
-    double *ro_b = so_b.rho + k * ns, *tr_b = st_b.rho + k * ns, *rn_b = sn_b.rho + k * ns;
-    const long long bot = i + ns - nc;
-    const double a_sfc = vg.area_v[(long long)nl * nc + i];
-    auto vol = [&](int j) { return vg.volume[i + (long long)j * nc]; };
-    auto fi = [&](int j) { const long long wi = i + (long long)(j + 1) * nc; return vg.area_v[wi] * (so.w[wi] - vs); };
-    auto bw = [&](int j) { const long long wi = i + (long long)(j + 1) * nc; return vg.area_v[wi] * (sn.w[wi] - vs); };
-    auto io = [&](int j) { return bw(j) >= 0.0 ? i + (long long)(j + 1) * nc : i + (long long)j * nc; };
-    double cc[CAP], dd[CAP], ee[CAP], xx[CAP], ep[CAP], rp[CAP];
-    /* rows */
+    const long long ns = (long long)nl * nc;
+    const double *cc = w.c + slot * ns + i, *ee = w.e + slot * ns + i;
+    double *dx = w.d + slot * ns + i, *ry = w.r + slot * ns + i;
+    double *rn_b = sn_b.rho + (slot < n_cond ? slot : slot + 1) * ns + i;
+    double ep[NL > 0 ? NL : CAP], rp[NL > 0 ? NL : CAP], dd[NL > 0 ? NL : CAP];
+#pragma unroll
     for (int j = 0; j < nl; ++j) {
-        const double v = vol(j);
-        double d = 1.0, r = ro[i + (long long)j * nc] + dt * tr[i + (long long)j * nc];
-        if (j < nl - 1) {
-            const double f = fi(j), fr = ro[io(j)] * bw(j);
-            ee[j] = f >= 0.0 ? -iw * dt / v * f : 0.0;
-            cc[j] = f < 0.0 ? iw * dt / vol(j + 1) * f : 0.0;
-            if (f < 0.0) d -= iw * dt / v * f;
-            r += ew * dt * fr / v;
-        }
-        if (j > 0) {
-            const double f = fi(j - 1), fr = ro[io(j - 1)] * bw(j - 1);
-            if (f >= 0.0) d += iw * dt / v * f;
-            r -= ew * dt * fr / v;
-        }
-        if (j == nl - 1 && sink) {
-            d += iw * vs * dt * a_sfc / v;
-            r -= ew * vs * dt * ro[bot] * a_sfc / v;
-        }
-        dd[j] = d;
-        /* forward elimination */
-        if (j == 0) {
-            ep[0] = nl > 1 ? ee[0] / d : 0.0;
-            rp[0] = r / d;
-        } else {
-            const double den = d - ep[j - 1] * cc[j - 1];
-            if (j < nl - 1) ep[j] = ee[j] / den;
-            rp[j] = (r - rp[j - 1] * cc[j - 1]) / den;
-        }
+        const long long o = (long long)j * nc;
+        dd[j] = dx[o];
+        const double cm = j > 0 ? cc[o - nc] : 0.0, r = ry[o];
+        const double den = j > 0 ? dd[j] - ep[j - 1] * cm : dd[j], inv = 1.0 / den;
+        ep[j] = j < nl - 1 ? div_rcp(ee[o], den, inv) : 0.0;
+        rp[j] = div_rcp(j > 0 ? r - rp[j - 1] * cm : r, den, inv);
     }
-    xx[nl - 1] = rp[nl - 1];
-    for (int j = nl - 2; j >= 0; --j) xx[j] = rp[j] - ep[j] * xx[j + 1];
-    /* transposed system A^T y = xbar (sub-diagonal ee, super-diagonal cc) */
+    double x = 0.0;
+#pragma unroll
+    for (int j = nl - 1; j >= 0; --j) {
+        x = j < nl - 1 ? rp[j] - ep[j] * x : rp[j];
+        dx[(long long)j * nc] = x;
+        rp[j] = x; /* its sign clips the bar below */
+    }
+    /* transposed system A^T y = xbar (sub-diagonal e, super-diagonal c) */
+#pragma unroll
     for (int j = 0; j < nl; ++j) {
-        const long long b = i + (long long)j * nc;
-        const double g = xx[j] < 0.0 ? 0.0 : rn_b[b];
-        rn_b[b] = 0.0;
-        if (j == 0) {
-            ep[0] = nl > 1 ? cc[0] / dd[0] : 0.0;
-            rp[0] = g / dd[0];
-        } else {
-            const double den = dd[j] - ep[j - 1] * ee[j - 1];
-            if (j < nl - 1) ep[j] = cc[j] / den;
-            rp[j] = (g - rp[j - 1] * ee[j - 1]) / den;
+        const long long o = (long long)j * nc;
+        const double g = rp[j] < 0.0 ? 0.0 : rn_b[o];
+        rn_b[o] = 0.0;
+        const double sub = j > 0 ? ee[o - nc] : 0.0;
+        const double den = j > 0 ? dd[j] - ep[j - 1] * sub : dd[j], inv = 1.0 / den;
+        ep[j] = j < nl - 1 ? div_rcp(cc[o], den, inv) : 0.0;
+        rp[j] = div_rcp(j > 0 ? g - rp[j - 1] * sub : g, den, inv);
+    }
+    double y = 0.0;
+#pragma unroll
+    for (int j = nl - 1; j >= 0; --j) {
+        y = j < nl - 1 ? rp[j] - ep[j] * y : rp[j];
+        ry[(long long)j * nc] = y;
+    }
+}
+
+/* grid: x cells, y layers, z tracer slots; a layer's thread takes the interface
+ * below it too.  The wind and the temperature are shared by the tracers, the
+ * upstream density by a layer's two interfaces: atomic. */
+__global__ void ka_gen_bars(VGrid vg, StepParams p, DState so, DState sn, const double *temperature, int rk,
+                            const double *sed_b, TracerRows w, DState so_b, DState sn_b, DState st_b, double *t_b)
+{
+    const LayerPoint pt = layer_point(vg.nc);
+    if (!pt.in) return;
+    const int nc = vg.nc, nl = vg.nl, j = pt.l;
+    const long long ns = (long long)nl * nc, b = pt.i, o = (long long)blockIdx.z * ns + b;
+    const TracerSlot s = tracer_slot(p, blockIdx.z);
+    const bool heat = rk == 0 && s.sink;
+    const double *ro = so.rho + s.k * ns;
+    double *ro_b = so_b.rho + s.k * ns;
+    const double dt = p.dt, h = 0.5 * dt, y = w.r[o], rv = vg.r_volume[b], yv = div_rcp(y, vg.volume[b], rv);
+    st_b.rho[s.k * ns + b] += dt * y;
+    double own = y; /* bar of this layer's old density */
+    if (j == nl - 1) {
+        if (s.sink) {
+            const double a_sfc = vg.area_v[b + nc];
+            own -= h * s.vs * a_sfc * yv;
+            if (heat) {
+                const double hb = div_rcp(sed_b[b], vg.volume[b], rv) * a_sfc, tb = temperature[b];
+                own -= s.vs * c_p_cond(s.k, tb) * tb * hb;
+                acc(&t_b[b], -s.vs * d_cpT(s.k, tb) * ro[b] * hb);
+            }
         }
+        acc(&ro_b[b], own);
+        return;
     }
-    for (int j = nl - 2; j >= 0; --j) rp[j] = rp[j] - ep[j] * rp[j + 1];
-    const double *y = rp;
-    /* bars of the inputs */
-    for (int j = 0; j < nl; ++j) {
-        const long long b = i + (long long)j * nc;
-        ro_b[b] += y[j];
-        tr_b[b] += dt * y[j];
+    const long long wi = b + nc;
+    const double ar = vg.area_v[wi], f = ar * (so.w[wi] - s.vs), bw = ar * (sn.w[wi] - s.vs);
+    const bool below = nonneg<true>(bw);
+    const long long id = below ? wi : b;
+    const double rv1 = vg.r_volume[wi], v1 = vg.volume[wi], y1v = div_rcp(w.r[o + nc], v1, rv1), dio = ro[id];
+    double frb = h * (yv - y1v);
+    if (heat) {
+        const double hb = div_rcp(sed_b[b], vg.volume[b], rv) - div_rcp(sed_b[wi], v1, rv1), t = temperature[id];
+        frb += c_p_cond(s.k, t) * t * hb;
+        acc(&t_b[id], d_cpT(s.k, t) * dio * bw * hb);
     }
-    if (sink) {
-        const double v = vol(nl - 1);
-        double rb = -ew * vs * dt * a_sfc / v * y[nl - 1];
-        if (heat) {
-            const double hb = sed_b[bot], tb = temperature[bot];
-            rb += -vs * c_p_cond(k, tb) * tb * a_sfc / v * hb;
-            acc(&t_b[bot], -vs * d_cpT(k, tb) * ro[bot] * a_sfc / v * hb);
-        }
-        ro_b[bot] += rb;
-    }
-    for (int j = 0; j < nl - 1; ++j) {
-        const double vj = vol(j), vj1 = vol(j + 1);
-        const long long wi = i + (long long)(j + 1) * nc, id = io(j);
-        const double f = fi(j), b_ = bw(j), dio = ro[id];
-        double frb = ew * dt * (y[j] / vj - y[j + 1] / vj1);
-        if (heat) {
-            const double hb = sed_b[i + (long long)j * nc] / vj - sed_b[i + (long long)(j + 1) * nc] / vj1;
-            const double t = temperature[id];
-            frb += c_p_cond(k, t) * t * hb;
-            acc(&t_b[id], d_cpT(k, t) * dio * b_ * hb);
-        }
-        ro_b[id] += b_ * frb;
-        acc(&sn_b.w[wi], vg.area_v[wi] * dio * frb);
-        /* rows j (e, d) and j + 1 (c, d) */
-        double fb;
-        if (f >= 0.0)
-            fb = -iw * dt / vj * (-y[j] * xx[j + 1]) + iw * dt / vj1 * (-y[j + 1] * xx[j + 1]);
-        else
-            fb = iw * dt / vj1 * (-y[j + 1] * xx[j]) - iw * dt / vj * (-y[j] * xx[j]);
-        acc(&so_b.w[wi], vg.area_v[wi] * fb);
-    }
+    if (below) acc(&ro_b[wi], bw * frb);
+    else own += bw * frb;
+    acc(&ro_b[b], own);
+    acc(&sn_b.w[wi], ar * dio * frb);
+    /* rows j (e, d) and j + 1 (c, d) */
+    const double xs = nonneg<true>(f) ? w.d[o + nc] : w.d[o];
+    acc(&so_b.w[wi], ar * (h * (yv - y1v) * xs));
 }
 
 }  // namespace
@@ -436,16 +484,24 @@ int adj_gen_densities(Context *c, const StepParams &p, StateMirror *so, StateMir
                       StateMirror *st_b, double *t_b)
 {
     if (c->n_const <= 1) return 0;
-    const long long nsys = (long long)(c->n_const - 1) * c->nc;
-    if (c->nl <= 64)
-        ka_gen_densities<64><<<nb(nsys, 64), 64, 0, c->stream>>>(c->vg, p, so->ds, sn->ds, st->ds, temperature, rk,
-                                                                 sed_b, so_b->ds, sn_b->ds, st_b->ds, t_b);
-    else if (c->nl <= 256)
-        ka_gen_densities<256><<<nb(nsys, 64), 64, 0, c->stream>>>(c->vg, p, so->ds, sn->ds, st->ds, temperature, rk,
-                                                                  sed_b, so_b->ds, sn_b->ds, st_b->ds, t_b);
+    if (c->nl > 256) return -1;
+    const int n_tr = c->n_const - 1;
+    const long long nsys = (long long)n_tr * c->nc, len = (long long)n_tr * c->ns;
+    double *work = tracer_adj_work(c);
+    if (!work) return -1;
+    const TracerRows w{work, work + len, work + 2 * len, work + 3 * len};
+    const dim3 boxes(nb(c->nc, 128), (unsigned)c->nl, (unsigned)n_tr);
+    ka_gen_rows<<<boxes, 128, 0, c->stream>>>(c->vg, p, so->ds, sn->ds, st->ds, w);
+    const unsigned cols = nb(nsys, 64);
+    if (c->nl == 26)
+        ka_gen_solve<26, 26><<<cols, 64, 0, c->stream>>>(c->nc, c->nl, n_tr, c->n_cond, w, sn_b->ds);
+    else if (c->nl <= 64)
+        ka_gen_solve<0, 64><<<cols, 64, 0, c->stream>>>(c->nc, c->nl, n_tr, c->n_cond, w, sn_b->ds);
     else
-        return -1;
-    c->kernel_launches++;
+        ka_gen_solve<0, 256><<<cols, 64, 0, c->stream>>>(c->nc, c->nl, n_tr, c->n_cond, w, sn_b->ds);
+    ka_gen_bars<<<boxes, 128, 0, c->stream>>>(c->vg, p, so->ds, sn->ds, temperature, rk, sed_b, w, so_b->ds, sn_b->ds,
+                                              st_b->ds, t_b);
+    c->kernel_launches += 3;
     /* the forward overwrites the sedimentation heat at rk 0 */
     if (rk == 0 && cudaMemsetAsync(sed_b, 0, (size_t)c->ns * sizeof(double), c->stream) != cudaSuccess) return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;

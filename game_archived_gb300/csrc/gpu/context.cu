@@ -787,6 +787,15 @@ int ensure_diff_buffers(Context *c)
     return 0;
 }
 
+double *tracer_adj_work(Context *c)
+{
+    if (c->tracer_adj) return c->tracer_adj;
+    c->tracer_adj = dalloc<double>(c, 4 * (size_t)(c->n_const - 1) * (size_t)c->ns);
+    if (!c->tracer_adj) fail("device allocation of the tracer adjoint's work array failed");
+    else if (cudaDeviceSynchronize() != cudaSuccess) return nullptr; /* cleared before the stream uses it */
+    return c->tracer_adj;
+}
+
 int ensure_sub_buffers(Context *c)
 {
     Context::SubBuffers &b = c->sub;

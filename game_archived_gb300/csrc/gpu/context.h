@@ -185,6 +185,9 @@ struct Context {
     struct OutBufs *obuf = nullptr;
     void (*obuf_release)(Context *) = nullptr;
     int use_graphs = 1;
+    /* rows and solutions of the tracer adjoint's column systems
+     * [4][C-1][L][Nc], allocated on first use */
+    double *tracer_adj = nullptr;
     int column_solver = 0; /* 0 by layer count, 1 per-thread sweeps, 2 warp cyclic reduction */
     /* arithmetic of the mixed path's vertical eliminations: 0 FP64, 1
      * double-float (default) */
@@ -247,6 +250,7 @@ StateMirror *mirror(const void *host_state, int create);
 void set_mirror_views(Context *c, StateMirror &m);
 int ensure_sub_buffers(Context *c);
 int ensure_diff_buffers(Context *c);
+double *tracer_adj_work(Context *c); /* null on failure */
 /* the library's own pinned host allocations (game_gpu_host_alloc) and
  * their device addresses: States inside them are copied by kernels that read
  * and write host memory directly over NVLink-C2C */
