@@ -97,42 +97,52 @@ __device__ __forceinline__ bool nonneg(double x)
     return EXACT ? x >= 0.0 : __double2hiint(x) >= 0;
 }
 
-/* double -> float rounded to nearest even, by integer operations for values
- * whose float is a normal number (or overflows to infinity by rounding) and
- * for zeros; subnormal results, infinities and NaNs go through the conversion
- * instruction.  The same bits as float(x); used by the mixed path where it
- * writes its FP32 shadow from FP64 results, to keep the conversion off the
- * FP64 pipe (zeros included: constituents absent from a run are zero
- * everywhere, and each conversion instruction costs an FP64-pipe issue). */
+/* double -> float rounded to nearest even, by integer operations alone: the same
+ * bits as float(x), zeros, subnormal results, overflows, infinities and NaNs
+ * included (tested).  Used by the mixed path where it writes its FP32 shadow
+ * from FP64 results, to keep the conversion off the FP64 pipe (one warp
+ * instruction per 16 cycles).  No case may use the conversion instruction: the
+ * compiler runs it ahead of the test that guards it, so a fallback costs every
+ * value its FP64 issue.  Without it k_make_shadow's FP64 issue falls from 16 us
+ * to 0 and its time from 37 to 34 us, k_cell_prepare_f32's from 31 to 5 us and
+ * 59.5 to 57.7 us, the scalar tendencies take 141 us for 147 (RES_ID 6). */
 __device__ __forceinline__ float to_float(double x)
 {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x), m = b & 0xfffffffffffffULL;
+    const unsigned e = (unsigned)(b >> 52) & 0x7ffu, sign = (unsigned)(b >> 63) << 31;
     if (e - 897u <= 253u) { /* float exponent field e - 896 in [1, 254] */
-        const unsigned long long m = b & 0xfffffffffffffULL;
-        unsigned r = ((unsigned)(b >> 63) << 31) | ((e - 896u) << 23) | (unsigned)(m >> 29);
+        unsigned r = sign | ((e - 896u) << 23) | (unsigned)(m >> 29);
         const unsigned rem = (unsigned)(m & 0x1fffffffULL), half = 0x10000000u;
         r += (rem > half || (rem == half && (r & 1u))) ? 1u : 0u;
         return __uint_as_float(r);
     }
-    if ((b << 1) == 0ULL) return __uint_as_float((unsigned)(b >> 63) << 31); /* +-0 */
-    return __double2float_rn(x);
+    if (e > 896u) /* beyond the float range, infinity, NaN */
+        return __uint_as_float(sign | 0x7f800000u | (e == 0x7ffu && m != 0ULL ? 0x400000u | (unsigned)(m >> 29) : 0u));
+    const unsigned shift = 926u - e; /* to units of the smallest subnormal float */
+    if (shift > 54u) return __uint_as_float(sign);
+    const unsigned long long v = m | 0x10000000000000ULL, rem = v & ((1ULL << shift) - 1ULL), half = 1ULL << (shift - 1u);
+    unsigned r = (unsigned)(v >> shift);
+    r += (rem > half || (rem == half && (r & 1u))) ? 1u : 0u;
+    return __uint_as_float(sign | r);
 }
 
-/* float -> double (exact) by integer operations for normal numbers and
- * zeros; subnormals, infinities and NaNs through the conversion instruction.
- * The same bits as double(x); the mixed path widens its FP32 sums and
- * products with it before the FP64 accumulation, keeping the conversion off
- * the FP64 pipe.  wide() is the identity on double. */
+/* float -> double (exact) by integer operations alone, for the same reason:
+ * the same bits as double(x) except a NaN's payload.  The mixed path widens
+ * its FP32 sums and products with it before the FP64 accumulation.  wide() is
+ * the identity on double. */
 __device__ __forceinline__ double to_double(float x)
 {
-    const unsigned u = __float_as_uint(x);
+    const unsigned u = __float_as_uint(x), sign = u & 0x80000000u;
     const unsigned fe = (u >> 23) & 0xffu;
     if (fe - 1u <= 253u) /* normal */
-        return __hiloint2double((int)((u & 0x80000000u) | ((fe + 896u) << 20) | ((u >> 3) & 0xfffffu)),
-                                (int)(u << 29));
-    if ((u & 0x7fffffffu) == 0u) return __hiloint2double((int)(u & 0x80000000u), 0);
-    return (double)x;
+        return __hiloint2double((int)(sign | ((fe + 896u) << 20) | ((u >> 3) & 0xfffffu)), (int)(u << 29));
+    const unsigned m = u & 0x7fffffu;
+    if (fe != 0u) /* infinity, NaN */
+        return __hiloint2double((int)(sign | 0x7ff00000u | (m ? 0x80000u : 0u) | (m >> 3)), (int)(m << 29));
+    if (m == 0u) return __hiloint2double((int)sign, 0);
+    const int p = 31 - __clz((int)m); /* m 2^-149 = 1.f 2^(p - 149) */
+    const unsigned long long f = ((unsigned long long)m << (52 - p)) & 0xfffffffffffffULL;
+    return __hiloint2double((int)(sign | ((unsigned)(p + 874) << 20) | (unsigned)(f >> 32)), (int)(unsigned)f);
 }
 /* x == +-0 by an integer test (an FP64 comparison would issue on the FP64
  * pipe) */
