@@ -309,9 +309,9 @@ void tracers_fwd(Context *c, AdjState *a, int rk, DState so, DState out, double 
     }
     const DState tend{str, nullptr, nullptr, nullptr, nullptr, nullptr};
     if (c->nl == 26)
-        k_tracers_solve<26, 26, true><<<nbk(nsys, 64), 64, 0, st>>>(c->vg, a->p, so, out, tend, tw, nullptr);
+        k_tracers_solve<26, 26, true><<<nbk(nsys, 64), 64, 0, st>>>(c->vg, a->p, so, out, tend, tw, nullptr, Present{});
     else
-        k_tracers_solve<0, MAX_L, true><<<nbk(nsys, 64), 64, 0, st>>>(c->vg, a->p, so, out, tend, tw, nullptr);
+        k_tracers_solve<0, MAX_L, true><<<nbk(nsys, 64), 64, 0, st>>>(c->vg, a->p, so, out, tend, tw, nullptr, Present{});
     c->kernel_launches++;
 }
 

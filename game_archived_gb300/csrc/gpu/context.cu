@@ -384,7 +384,11 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
                 }
         }
     }
-    for (int t : h_tilt) c->any_tilt |= t;
+    std::vector<int> h_tilt_cells;
+    for (int i = 0; i < NC; ++i)
+        if (h_tilt[i]) h_tilt_cells.push_back(i);
+    c->n_tilt = (int)h_tilt_cells.size();
+    c->tilt_cells = dupload(c, h_tilt_cells);
     std::vector<double> h_tw((size_t)10 * NE), h_rw((size_t)4 * NE), h_fvec((size_t)2 * NE);
     std::vector<int> h_ti((size_t)10 * NE), h_tm((size_t)10 * NE), h_ri((size_t)4 * NE);
     for (int e = 0; e < NE; ++e) {
@@ -590,6 +594,8 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
      * 30 * 4^RES_ID edges) */
     if (NC % 2 != 0 || NE % 2 != 0) return fail("grid with an odd number of cells or edges");
     c->shadow = dalloc<float>(c, (size_t)(c->n_const + 3) * NS + (size_t)(L + 1) * NC + (size_t)L * NE);
+    c->present.by_layer = dalloc<int>(c, (size_t)L + 8 * c->n_const);
+    c->present.by_const = (unsigned *)(c->present.by_layer + L);
     c->theta32 = dalloc<float>(c, NS);
     c->pg_cell = dalloc<float4>(c, NS);
     c->cp32_ice = dalloc<float>(c, NS);

@@ -50,7 +50,8 @@ struct StateMirror {
 
 struct Context {
     game_dims dims{};
-    int any_tilt = 0; /* some edge of the grid slopes */
+    int n_tilt = 0; /* columns with a sloping edge, and their list */
+    int *tilt_cells = nullptr;
     int nc = 0, ne = 0, nt = 0, nl = 0, n_oro = 0, n_const = 0, n_cond = 0, moist = 0;
     long long ns = 0, nv = 0, ndv = 0, ncurl = 0, state_len = 0;
     double radius = 0.0, toa = 0.0;
@@ -96,6 +97,7 @@ struct Context {
     double *cp_ice = nullptr, *cp_water = nullptr; /* c_p of ice / liquid water at T, [L][Nc] */
     /* mixed path: FP32 shadow of state_new and FP32 copies of per-step fields */
     float *shadow = nullptr;          /* [rho C*S][rhotheta S][theta' S][Pi' S][w (L+1)Nc][u L*Ne] */
+    Present present{}; /* which constituents the shadow's layers hold */
     float *theta32 = nullptr, *cp32_ice = nullptr, *cp32_water = nullptr;
     /* mixed path: pressure-gradient factors of the step start per (layer,
      * cell): Pi', c_p theta_v, c_p theta_v', rho_gas / rho_total (k_pg_cells) */

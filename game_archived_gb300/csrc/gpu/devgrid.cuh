@@ -151,10 +151,24 @@ struct DfGrid {
     const float2 *damp_inv;
 };
 
+/* which layers may hold a nonzero density of which constituent in the FP32
+ * shadow: cleared at the start of a mixed step, set for the step-start state
+ * per layer (a bit per constituent) and by the tracer solve per constituent
+ * (a bit per layer, 32 layers a word) */
+struct Present {
+    int *by_layer;     /* [L] */
+    unsigned *by_const; /* [C][8] */
+    __device__ __forceinline__ bool holds(int k, int l) const
+    {
+        return ((by_layer[l] >> k) & 1) || ((by_const[8 * k + (l >> 5)] >> (l & 31)) & 1u);
+    }
+};
+
 /* FP32 shadow of state_new (mixed path); kernels that write the FP64 state
  * also write the shadow.  All pointers null on the FP64 path. */
 struct Shadow {
     float *rho, *rhotheta_v, *theta_v_pert, *exner_pert, *w, *u;
+    Present present;
 };
 
 /* run configuration of one step (no padding: compared bytewise as a key) */

@@ -804,15 +804,30 @@ __device__ __forceinline__ void pgrad_v_parts(const HGrid<R> &g, const StepParam
  * substage's gradients gather two float4 per edge (or interface) instead of
  * some twenty scalars.  Read from the FP32 shadow of state_new, which the
  * first substage's pressure gradient reads. */
-__global__ void k_pg_cells(HGrid<float> g, StepParams p, SView<float> s, float4 *pc)
+__global__ void k_pg_cells(HGrid<float> g, StepParams p, SView<float> s, float4 *pc, Present present)
 {
-    const long long ns = (long long)g.nl * g.nc;
-    const long long i = gtid();
-    if (i >= ns) return;
-    const float cdp = float(C_D_P);
-    const float tp = s.theta_v_pert[i];
-    pc[i] = make_float4(s.exner_pert[i], cdp * (g.theta_v_bg[i] + tp), cdp * tp,
-                        s.rho[p.n_cond * ns + i] / density_total_r(s.rho, p.n_const, ns, i));
+    const LayerPoint pt = layer_point(g.nc);
+    const long long ns = (long long)g.nl * g.nc, i = pt.i;
+    int held = 0; /* constituents with a density here */
+    if (pt.in) {
+        const float cdp = float(C_D_P);
+        const float tp = s.theta_v_pert[i];
+        pc[i] = make_float4(s.exner_pert[i], cdp * (g.theta_v_bg[i] + tp), cdp * tp,
+                            s.rho[p.n_cond * ns + i] / density_total_r(s.rho, p.n_const, ns, i));
+        for (int k = 0; k < p.n_const; ++k) held |= (s.rho[k * ns + i] != 0.f) << k;
+    }
+    if (p.n_const == 1) return;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) held |= __shfl_xor_sync(0xffffffffu, held, d);
+    __shared__ int any;
+    if (threadIdx.x == 0) any = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0 && held) atomicOr(&any, held);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int *row = present.by_layer + pt.l;
+        if (any & ~*(volatile int *)row) atomicOr(row, any);
+    }
 }
 
 /* FP64 path: the same cell factors in double with the operations of
@@ -1049,7 +1064,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
     tend_w[i] = t;
 }
 
-/* ------------------------------------------------------ k_scalar_tend2
+/* ------------------------------------------------------ k_scalar_tend32
  * explicit mass and rho*theta_v tendencies (scalar_tendencies_expl.c:90-178)
  * at (cell, layer) */
 
@@ -1104,67 +1119,219 @@ struct FluxSum<float> {
         hi = t;
         lo += err;
     }
+    __device__ __forceinline__ bool zero() const { return hi == 0.f && lo == 0.f; }
     __device__ __forceinline__ double value() const { return to_double(hi) + to_double(lo); }
 };
 
-/* Explicit mass and rho*theta_v tendencies (scalar_tendencies_expl.c:90-178)
- * at (cell, layer).  The cell's edges are streamed one layer at a time
- * (layer l-1, l, l+1) so that only one layer's fluxes are live; every
- * accumulator still receives its terms in the reference's order (layer
- * l-1 before l, edges j = 0..5), so with R = double every sum and product is
- * the reference's, bit for bit.  The main mass flux is reused for the
- * rho*theta_v flux; the terrain correction of the wind is computed once for
- * all tracers.  Edge fluxes are products in R, divergences accumulate in
- * double (FluxSum) and tendencies are formed in double. */
 /* irreversible terms of the tendencies (scalar_tendencies_expl.c:125-176):
  * dissipative and diffusive heating, radiation, mass diffusion [C][L][Nc] */
 struct IrrTerms {
     const double *heating_diss, *temp_diff_heating, *radiation, *mass_diff;
 };
 
-template <typename R, bool IRR>
-__global__ void __launch_bounds__(128) k_scalar_tend2(HGrid<R> g, StepParams p, SView<R> sv, DState st,
-                                                      const R *theta, const R *cp_ice, const R *cp_water,
-                                                      const double *pt_rates, const double *pt_heat,
-                                                      const double *sed_heat, const double *inv_vol_tab, int rk,
-                                                      IrrTerms irr)
+/* FP64 operations that stay behind the test that guards them: the compiler runs
+ * plain ones ahead of it and selects, and each issue holds the FP64 pipe for 16
+ * cycles */
+__device__ __forceinline__ double guarded_mul(double a, double b)
+{
+    double r;
+    asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+}
+__device__ __forceinline__ double guarded_add(double a, double b)
+{
+    double r;
+    asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+}
+__device__ __forceinline__ double guarded_fma(double a, double b, double c)
+{
+    double r;
+    asm volatile("fma.rn.f64 %0, %1, %2, %3;" : "=d"(r) : "d"(a), "d"(b), "d"(c));
+    return r;
+}
+
+/* half of x exactly, without an FP64 instruction for normal numbers whose half
+ * is normal, and zeros */
+__device__ __forceinline__ double half_of(double x)
+{
+    const int hi = __double2hiint(x);
+    if (((unsigned)(hi >> 20) & 0x7ffu) - 2u <= 2044u) return __hiloint2double(hi - 0x100000, __double2loint(x));
+    return is_zero(x) ? x : guarded_mul(0.5, x);
+}
+
+/* The mixed path's tendencies at (cell, layer) of the columns without a sloping
+ * edge (all of them on a flat grid), where the terrain corrections vanish.
+ * Edge fluxes are FP32 products, their divergences double-word FP32 sums
+ * (FluxSum), the tendencies FP64.  The cell's edges, neighbours, orientation,
+ * wind and face areas are loaded once for all constituents.
+ *
+ * Bounds: load latency of the gathers, then FP64 issue (one warp instruction
+ * per 16 cycles).  Hence: a constituent absent from the layer (present: set
+ * by k_pg_cells and the tracer solve) is neither gathered nor
+ * summed; a zero flux and a zero rate leave the tendency without FP64
+ * arithmetic; sums with exact zeros are left out, the rk 1 mean takes one
+ * addition.  RES_ID 6 moist, cloud-free: 141 -> 85 us per launch. */
+template <bool IRR>
+__global__ void __launch_bounds__(128) k_scalar_tend32(HGrid<float> g, StepParams p, SView<float> sv, DState st,
+                                                       const float *theta, const float *cp_ice, const float *cp_water,
+                                                       const double *pt_rates, const double *pt_heat,
+                                                       const double *sed_heat, const double *inv_vol_tab,
+                                                       Present present, int rk, IrrTerms irr)
 {
     const long long ns = (long long)g.nl * g.nc;
     const LayerPoint pt_ = layer_point(g.nc);
     if (!pt_.in) return;
     const long long i = pt_.i;
-    const int nl = g.nl, n_oro = g.n_oro;
-    const int l = pt_.l, c = pt_.x;
+    const int nl = g.nl, l = pt_.l, c = pt_.x;
+    if (g.tilt[c]) return; /* k_scalar_tend_tilt */
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     const int cond = p.n_cond;
-    /* terrain-following corrections: in the orography layers (on the mixed
-     * path only where the cell's edges slope; elsewhere they are zero) */
-    const bool oro = l >= nl - n_oro - 1 && (sizeof(R) == sizeof(double) || g.tilt[c]);
+    const double inv_vol = inv_vol_tab[i];
+    int ej[6], nbj[6];
+    bool sfj[6];
+    float uj[6], arj[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const bool on = j < n_edges;
+        ej[j] = on ? g.adj[j * nc + c] : 0;
+        nbj[j] = on ? g.adj_nbr[j * nc + c] : c;
+        sfj[j] = on && g.adj_sign[j * nc + c] > 0;
+    }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const bool on = j < n_edges;
+        uj[j] = on ? sv.u[(long long)l * ne + ej[j]] : 0.f;
+        arj[j] = on ? g.area_h[(long long)l * ne + ej[j]] : 0.f;
+    }
+    /* the main gas: centred mass flux and, from it, the rho*theta_v flux
+     * (new weight 1 in both substages) */
+    {
+        const float *f = sv.rho + cond * ns;
+        FluxSum<float> hm, ht;
+        const long long o = (long long)l * nc;
+        const float fs = f[o + c], ts = theta[o + c];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            if (j >= n_edges) continue;
+            const float fm = (0.5f * (fs + f[o + nbj[j]])) * uj[j];
+            const float ft = (0.5f * (ts + theta[o + nbj[j]])) * fm;
+            const float am = fm * arj[j], at = ft * arj[j];
+            hm.add(sfj[j] ? am : -am);
+            ht.add(sfj[j] ? at : -at);
+        }
+        const double dm = hm.value(), dt_ = ht.value();
+        const double div = inv_vol * dm;
+        double y = -div;
+        if (IRR) y = y + irr.mass_diff[cond * ns + i];
+        if (p.moist) y = y + pt_rates[cond * ns + i];
+        st.rho[cond * ns + i] = y;
+        const double div_t = inv_vol * dt_;
+        double yt = -div_t;
+        if (p.moist || IRR) {
+            /* diabatic heating: c_v-weighted, divided by c_p * Pi */
+            float cv = 0.f;
+            for (int kk = 0; kk < cond; ++kk) cv += sv.rho[kk * ns + i] * ((kk % 2 == 0) ? cp_ice[i] : cp_water[i]);
+            cv += sv.rho[cond * ns + i] * float(C_D_V);
+            if (p.moist) cv += sv.rho[(cond + 1) * ns + i] * float(C_V_V);
+            double heat = pt_heat[i] + sed_heat[i], rate = pt_rates[cond * ns + i];
+            if (IRR) {
+                heat = irr.heating_diss[i] + irr.temp_diff_heating[i] + irr.radiation[i] + pt_heat[i] + sed_heat[i];
+                rate = pt_rates[cond * ns + i] + irr.mass_diff[cond * ns + i];
+            }
+            const float fac = float(C_D_V) * sv.rho[cond * ns + i] / cv / (float(C_D_P) * (g.exner_bg[i] + sv.exner_pert[i]));
+            yt = yt + wide(fac) * heat + rate * wide(theta[i]);
+        }
+        st.rhotheta_v[i] = yt;
+    }
+    if (p.n_const == 1) return;
+    /* the other constituents: upstream flux */
+    const long long o = (long long)l * nc;
+#pragma unroll 1
+    for (int k = 0; k < p.n_const; ++k) {
+        if (k == cond) continue;
+        const float *f = sv.rho + k * ns;
+        double sum = 0.0;
+        if (present.holds(k, l)) {
+            FluxSum<float> h;
+            const float fs = f[o + c];
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                if (j >= n_edges) continue;
+                const float ue = uj[j];
+                const float fv = ((ue >= 0.f) == sfj[j] ? fs : f[o + nbj[j]]) * ue;
+                const float a = fv * arj[j];
+                h.add(sfj[j] ? a : -a);
+            }
+            if (!h.zero()) sum = guarded_add(to_double(h.hi), to_double(h.lo));
+        }
+        double rate = 0.0;
+        if (p.moist) rate = pt_rates[(k == cond + 1 ? k - 1 : k) * ns + i];
+        double y = 0.0;
+        if (IRR || !is_zero(sum) || !is_zero(rate)) {
+            if (IRR) {
+                y = guarded_fma(-inv_vol, sum, irr.mass_diff[k * ns + i]);
+                if (p.moist) y = guarded_add(y, rate);
+            } else {
+                y = guarded_mul(-inv_vol, sum);
+                if (p.moist) y = guarded_add(y, rate);
+            }
+        }
+        if (rk != 0) {
+            const double old = st.rho[k * ns + i];
+            if (!is_zero(old) || !is_zero(y)) y = half_of(guarded_add(old, y));
+        }
+        st.rho[k * ns + i] = y;
+    }
+}
+
+/* the same in the columns with a sloping edge (tilt_cells), with the terrain
+ * corrections: the cell's edges are streamed one layer at a time, every
+ * accumulator in the reference's order (layer l-1 before l, edges j = 0..5) */
+template <bool IRR>
+__global__ void __launch_bounds__(128) k_scalar_tend_tilt(HGrid<float> g, StepParams p, SView<float> sv,
+                                                          DState st, const float *theta, const float *cp_ice,
+                                                          const float *cp_water,
+                                                      const double *pt_rates, const double *pt_heat,
+                                                      const double *sed_heat, const double *inv_vol_tab, int rk,
+                                                      IrrTerms irr, const int *tilt_cells, int n_tilt)
+{
+    const long long ns = (long long)g.nl * g.nc;
+    const LayerPoint pt_ = layer_point(n_tilt);
+    if (!pt_.in) return;
+    const int nl = g.nl, n_oro = g.n_oro;
+    const int l = pt_.l, c = tilt_cells[pt_.x];
+    const long long i = (long long)l * g.nc + c;
+    const long long nc = g.nc, ne = g.ne;
+    const int n_edges = c < N_PENT ? 5 : 6;
+    const int cond = p.n_cond;
+    /* terrain-following corrections: in the orography layers */
+    const bool oro = l >= nl - n_oro - 1;
     const bool up_corr = oro && l >= nl - n_oro;            /* contra_corr at level l needed   */
     const bool lo_corr = oro && l < nl - 1;                 /* contra_corr at level l+1 needed */
     const bool up_has_prev = up_corr && l > nl - n_oro;     /* level l sums layer l-1, then l  */
     const bool lo_has_curr = lo_corr && l + 1 > nl - n_oro; /* level l+1 sums layer l, then l+1 */
-    const double inv_vol = sizeof(R) == sizeof(double) ? 1.0 / double(g.volume[i]) : inv_vol_tab[i];
-    const R area_up = g.area_v[(long long)l * nc + c], area_lo = g.area_v[(long long)(l + 1) * nc + c];
+    const double inv_vol = inv_vol_tab[i];
+    const float area_up = g.area_v[(long long)l * nc + c], area_lo = g.area_v[(long long)(l + 1) * nc + c];
     auto edge = [&](int j) { return g.adj[j * nc + c]; };
     auto wcorr = [&](int ll, int j) {
-        return R(-0.5) * ipw_at(g, j, ll, c) * g.slope_h[(long long)ll * ne + edge(j)];
+        return float(-0.5) * ipw_at(g, j, ll, c) * g.slope_h[(long long)ll * ne + edge(j)];
     };
     auto uval = [&](int ll, int j) { return sv.u[(long long)ll * ne + edge(j)]; };
-    auto comp_v = [&](R up, R lo) -> double {
+    auto comp_v = [&](float up, float lo) -> double {
         if (!oro) return 0.0;
         if (l == nl - n_oro - 1) return wide(-lo * area_lo);
         if (l == nl - 1) return wide(up * area_up);
         return wide(up * area_up - lo * area_lo);
     };
     /* terrain correction of the wind at levels l and l+1 (shared by the tracers) */
-    R w_up = R(0), w_lo = R(0);
+    float w_up = float(0), w_lo = float(0);
     if (oro) {
         if (up_has_prev)
             for (int j = 0; j < n_edges; ++j) w_up += wcorr(l - 1, j) * uval(l - 1, j);
         for (int j = 0; j < n_edges; ++j) {
-            const R t = wcorr(l, j) * uval(l, j);
+            const float t = wcorr(l, j) * uval(l, j);
             if (up_corr) w_up += t;
             if (lo_has_curr) w_lo += t;
         }
@@ -1174,25 +1341,25 @@ __global__ void __launch_bounds__(128) k_scalar_tend2(HGrid<R> g, StepParams p, 
     /* the main gas: centred mass flux and, from it, the rho*theta_v flux
      * (new weight 1 in both substages) */
     {
-        const R *f = sv.rho + cond * ns;
-        FluxSum<R> hm, ht;
-        R um = R(0), ut = R(0), lm = R(0), lt = R(0);
+        const float *f = sv.rho + cond * ns;
+        FluxSum<float> hm, ht;
+        float um = float(0), ut = float(0), lm = float(0), lt = float(0);
         auto layer_pass = [&](int ll, bool to_h, bool to_up, bool to_lo) {
             const long long o = (long long)ll * nc;
-            const R fs = f[o + c], ts = theta[o + c];
+            const float fs = f[o + c], ts = theta[o + c];
             for (int j = 0; j < n_edges; ++j) {
                 const int nb = g.adj_nbr[j * nc + c];
-                const R fm = (R(0.5) * (fs + f[o + nb])) * uval(ll, j);
-                const R ft = (R(0.5) * (ts + theta[o + nb])) * fm;
+                const float fm = (float(0.5) * (fs + f[o + nb])) * uval(ll, j);
+                const float ft = (float(0.5) * (ts + theta[o + nb])) * fm;
                 if (to_h) {
-                    const R ar = g.area_h[(long long)ll * ne + edge(j)];
+                    const float ar = g.area_h[(long long)ll * ne + edge(j)];
                     const bool self_from = g.adj_sign[j * nc + c] > 0;
-                    const R am = fm * ar, at = ft * ar;
+                    const float am = fm * ar, at = ft * ar;
                     hm.add(self_from ? am : -am);
                     ht.add(self_from ? at : -at);
                 }
                 if (to_up || to_lo) {
-                    const R wc = wcorr(ll, j);
+                    const float wc = wcorr(ll, j);
                     if (to_up) {
                         um += wc * fm;
                         ut += wc * ft;
@@ -1211,30 +1378,24 @@ __global__ void __launch_bounds__(128) k_scalar_tend2(HGrid<R> g, StepParams p, 
         double y = -div;
         if (IRR) y = y + irr.mass_diff[cond * ns + i];
         if (p.moist) y = y + pt_rates[cond * ns + i];
-        st.rho[cond * ns + i] = rk == 0 ? y : 0.0 * st.rho[cond * ns + i] + 1.0 * y;
+        st.rho[cond * ns + i] = y;
         const double div_t = inv_vol * (ht.value() + comp_v(ut, lt));
         double yt = -div_t;
         if (p.moist || IRR) {
             /* diabatic heating: c_v-weighted, divided by c_p * Pi */
-            R cv = R(0);
+            float cv = float(0);
             for (int kk = 0; kk < cond; ++kk) cv += sv.rho[kk * ns + i] * ((kk % 2 == 0) ? cp_ice[i] : cp_water[i]);
-            cv += sv.rho[cond * ns + i] * R(C_D_V);
-            if (p.moist) cv += sv.rho[(cond + 1) * ns + i] * R(C_V_V);
+            cv += sv.rho[cond * ns + i] * float(C_D_V);
+            if (p.moist) cv += sv.rho[(cond + 1) * ns + i] * float(C_V_V);
             double heat = pt_heat[i] + sed_heat[i], rate = pt_rates[cond * ns + i];
             if (IRR) {
                 heat = irr.heating_diss[i] + irr.temp_diff_heating[i] + irr.radiation[i] + pt_heat[i] + sed_heat[i];
                 rate = pt_rates[cond * ns + i] + irr.mass_diff[cond * ns + i];
             }
-            if (sizeof(R) == sizeof(double)) {
-                yt = yt + C_D_V * double(sv.rho[cond * ns + i]) / double(cv) * heat
-                              / (C_D_P * (double(g.exner_bg[i]) + double(sv.exner_pert[i])))
-                     + rate * double(theta[i]);
-            } else {
-                const R fac = R(C_D_V) * sv.rho[cond * ns + i] / cv / (R(C_D_P) * (g.exner_bg[i] + sv.exner_pert[i]));
-                yt = yt + wide(fac) * heat + rate * wide(theta[i]);
-            }
+            const float fac = float(C_D_V) * sv.rho[cond * ns + i] / cv / (float(C_D_P) * (g.exner_bg[i] + sv.exner_pert[i]));
+            yt = yt + wide(fac) * heat + rate * wide(theta[i]);
         }
-        st.rhotheta_v[i] = rk == 0 ? yt : 0.0 * st.rhotheta_v[i] + 1.0 * yt;
+        st.rhotheta_v[i] = yt;
     }
     if (p.n_const == 1) return;
     /* the other constituents: upstream flux.  The cell's edges, neighbours,
@@ -1242,43 +1403,42 @@ __global__ void __launch_bounds__(128) k_scalar_tend2(HGrid<R> g, StepParams p, 
      * of them. */
     int ej[6], nbj[6];
     bool sfj[6];
-    R uj[6], arj[6];
+    float uj[6], arj[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
         const bool on = j < n_edges;
         ej[j] = on ? g.adj[j * nc + c] : 0;
         nbj[j] = on ? g.adj_nbr[j * nc + c] : c;
         sfj[j] = on && g.adj_sign[j * nc + c] > 0;
-        uj[j] = on ? sv.u[(long long)l * ne + ej[j]] : R(0);
-        arj[j] = on ? g.area_h[(long long)l * ne + ej[j]] : R(0);
+        uj[j] = on ? sv.u[(long long)l * ne + ej[j]] : float(0);
+        arj[j] = on ? g.area_h[(long long)l * ne + ej[j]] : float(0);
     }
     const long long o = (long long)l * nc;
     for (int k = 0; k < p.n_const; ++k) {
         if (k == cond) continue;
-        const double new_w = rk == 1 ? 0.5 : 1.0, old_w = 1.0 - new_w;
-        const R *f = sv.rho + k * ns;
-        FluxSum<R> h;
-        const R fs = f[o + c];
+        const float *f = sv.rho + k * ns;
+        FluxSum<float> h;
+        const float fs = f[o + c];
 #pragma unroll
         for (int j = 0; j < 6; ++j) {
             if (j >= n_edges) continue;
-            const R ue = uj[j];
-            const R fv = ((ue >= R(0)) == sfj[j] ? fs : f[o + nbj[j]]) * ue;
-            const R a = fv * arj[j];
+            const float ue = uj[j];
+            const float fv = ((ue >= float(0)) == sfj[j] ? fs : f[o + nbj[j]]) * ue;
+            const float a = fv * arj[j];
             h.add(sfj[j] ? a : -a);
         }
         double cv = 0.0;
         if (oro) {
-            const R d_here = f[i];
+            const float d_here = f[i];
             if (l == nl - n_oro - 1) {
-                const R d_lo = w_lo <= R(0) ? d_here : f[i + nc];
+                const float d_lo = w_lo <= float(0) ? d_here : f[i + nc];
                 cv = wide(-d_lo * w_lo * area_lo);
             } else if (l == nl - 1) {
-                const R d_up = w_up <= R(0) ? f[i - nc] : d_here;
+                const float d_up = w_up <= float(0) ? f[i - nc] : d_here;
                 cv = wide(d_up * w_up * area_up);
             } else {
-                const R d_up = w_up <= R(0) ? f[i - nc] : d_here;
-                const R d_lo = w_lo <= R(0) ? d_here : f[i + nc];
+                const float d_up = w_up <= float(0) ? f[i - nc] : d_here;
+                const float d_lo = w_lo <= float(0) ? d_here : f[i + nc];
                 cv = wide(d_up * w_up * area_up - d_lo * w_lo * area_lo);
             }
         }
@@ -1290,11 +1450,11 @@ __global__ void __launch_bounds__(128) k_scalar_tend2(HGrid<R> g, StepParams p, 
             if (k == cond + 1) pt -= ns;
             y = y + pt_rates[pt + i];
         }
-        st.rho[k * ns + i] = rk == 0 ? y : old_w * st.rho[k * ns + i] + new_w * y;
+        st.rho[k * ns + i] = rk == 0 ? y : half_of(st.rho[k * ns + i] + y);
     }
 }
 
-/* ---- the same tendencies on the FP64 path, in three kernels.  FP64 issue
+/* ---- the same tendencies on the FP64 path (k_scalar_tend64), in three kernels.  FP64 issue
  * bounds them, so nothing is formed twice: the fluxes of an edge once
  * (k_edge_flux) instead of by both its cells in up to three layer passes, the
  * terrain corrections of a level once (k_level_corr) instead of by the cells

@@ -375,6 +375,18 @@ __global__ void k_waves_apply(VGrid vg, StepParams p, DState so, DState sn, Wave
 }
 
 /* ------------------------------------------------------------- tracers */
+/* layers (bits of held) that received a density, into one word of
+ * Present::by_const: one atomic at most per warp and word, from the threads of
+ * the warp that are here (a store per layer and warp cost k_tracers_solve_df
+ * 486 -> 884 us at RES_ID 7 with tracers everywhere) */
+__device__ __forceinline__ void mark_layers(unsigned *words, int word, unsigned held)
+{
+    const unsigned same = __match_any_sync(__activemask(), word);
+    held = __reduce_or_sync(same, held);
+    if ((threadIdx.x & 31) == __ffs(same) - 1 && (held & ~*(volatile unsigned *)(words + word)))
+        atomicOr(words + word, held);
+}
+
 struct TracerWork {
     const double *cp_ice, *cp_water; /* c_p of ice / liquid water at the cell temperature [L][Nc] */
     const double *inv_vol;           /* mixed path */
@@ -396,7 +408,8 @@ __device__ __forceinline__ double sink_velocity(const StepParams &p, int k, bool
  * count is a compile-time constant and the sweep stays in registers; NL = 0:
  * the layer count is vg.nl (at most CAP) and the sweep lives in local memory */
 template <int NL, int CAP, bool EXACT>
-__global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DState st, TracerWork tw, float *sh_rho)
+__global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DState st, TracerWork tw, float *sh_rho,
+                                Present present)
 {
     const int nc = vg.nc;
     const int nl = NL > 0 ? NL : vg.nl;
@@ -534,18 +547,30 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
     double *rn = sn.rho + k * ns;
     float *rs = sh_rho ? sh_rho + k * ns : nullptr;
     double x = rp[nl - 1];
+    unsigned held = 0; /* layers of a 32-layer group that receive a density */
     {
         const double v = EXACT ? (x < 0.0 ? 0.0 : x) : (nonneg<false>(x) ? x : 0.0);
         rn[(long long)(nl - 1) * nc + i] = v;
-        if (rs) rs[(long long)(nl - 1) * nc + i] = to_float(v);
+        if (rs) {
+            rs[(long long)(nl - 1) * nc + i] = to_float(v);
+            held = (is_zero(v) ? 0u : 1u) << ((nl - 1) & 31);
+        }
     }
 #pragma unroll
     for (int j = nl - 2; j >= 0; --j) {
         x = rp[j] - ep[j] * x;
         const double v = EXACT ? (x < 0.0 ? 0.0 : x) : (nonneg<false>(x) ? x : 0.0);
         rn[(long long)j * nc + i] = v;
-        if (rs) rs[(long long)j * nc + i] = to_float(v);
+        if (rs) {
+            rs[(long long)j * nc + i] = to_float(v);
+            if ((j & 31) == 31) {
+                mark_layers(present.by_const, 8 * k + (j >> 5) + 1, held);
+                held = 0;
+            }
+            held |= (is_zero(v) ? 0u : 1u) << (j & 31);
+        }
     }
+    if (rs) mark_layers(present.by_const, 8 * k, held);
 }
 
 /* sedimentation heating (rk 0 only), mixed path with FP64 eliminations:
@@ -765,7 +790,8 @@ __global__ void __launch_bounds__(32 * PCR_WARPS) k_waves_pcr(int nc, int nl, Wa
  * which the reduction overwrites only after the rows are built. */
 template <bool EXACT>
 __global__ void __launch_bounds__(32 * PCR_WARPS)
-    k_tracers_pcr(VGrid vg, StepParams p, DState so, DState sn, DState st, TracerWork tw, float *sh_rho)
+    k_tracers_pcr(VGrid vg, StepParams p, DState so, DState sn, DState st, TracerWork tw, float *sh_rho,
+                                Present present)
 {
     extern __shared__ double smem[];
     const int nc = vg.nc, nl = vg.nl, n = nl;
@@ -864,7 +890,10 @@ __global__ void __launch_bounds__(32 * PCR_WARPS)
         for (int j = row0; j < n; j += 32) {
             const double v = EXACT ? (x[j] < 0.0 ? 0.0 : x[j]) : (nonneg<false>(x[j]) ? x[j] : 0.0);
             rn[i + (long long)j * nc] = v;
-            if (rs) rs[i + (long long)j * nc] = to_float(v);
+            if (rs) {
+                rs[i + (long long)j * nc] = to_float(v);
+                if (!is_zero(v)) mark_layers(present.by_const, 8 * k + (j >> 5), 1u << (j & 31));
+            }
         }
     }
 }

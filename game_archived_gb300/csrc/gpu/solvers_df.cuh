@@ -35,6 +35,8 @@ namespace {
 /* threads per block of the double-float tracer solve; its elimination
  * coefficients live in shared memory, NL x TRACER_BLOCK (hi, lo) pairs each */
 constexpr int TRACER_BLOCK = 64;
+/* layers tested for a density at a time */
+constexpr int EMPTY_BATCH = 13;
 
 /* The column system A x = r of the tracer (rows as k_tracers_solve's mixed
  * path) is solved for the increment delta = x - rho_old: A delta = r - A
@@ -44,7 +46,8 @@ constexpr int TRACER_BLOCK = 64;
  * 53 bits (a double carried in double-float keeps 48). */
 template <int NL>
 __global__ void __launch_bounds__(TRACER_BLOCK) k_tracers_solve_df(VGrid vg, StepParams p, DState so, DState sn,
-                                                                   DState st, DfGrid dg, float *sh_rho)
+                                                                   DState st, DfGrid dg, float *sh_rho,
+                                                                   Present present)
 {
     /* the loops are not unrolled (the unrolled double-float sweep overflowed
      * the instruction cache), so the coefficients cannot be registers */
@@ -56,7 +59,10 @@ __global__ void __launch_bounds__(TRACER_BLOCK) k_tracers_solve_df(VGrid vg, Ste
     const int n_tr = p.n_const - 1;
     if (q >= (long long)n_tr * nc) return;
     const int t = threadIdx.x;
-    const int slot = (int)(q / nc), i = (int)(q - (long long)slot * nc);
+    /* the last slot (the vapour, in every column of a moist run) first: its
+     * solves start with the launch and the columns without condensates fill
+     * in behind them */
+    const int row = (int)(q / nc), slot = n_tr - 1 - row, i = (int)(q - (long long)row * nc);
     const int k = slot < p.n_cond ? slot : slot + 1; /* skip the main gas */
     bool has_sink;
     const double vsink = sink_velocity(p, k, has_sink);
@@ -69,11 +75,19 @@ __global__ void __launch_bounds__(TRACER_BLOCK) k_tracers_solve_df(VGrid vg, Ste
         /* a constituent absent from the column, old density and tendency 0 in
          * every layer (a cloud-free column's condensates): the system's
          * right-hand side is 0 and so is the new density, exactly */
-        bool empty = true;
+        const long long low = (long long)(nl - 1) * nc + i; /* tells most of the others */
+        bool empty = is_zero(ro[low]) && is_zero(tr[low]);
 #pragma unroll 1
-        for (int j = 0; j < nl && empty; ++j) {
-            const long long b = (long long)j * nc + i;
-            empty = is_zero(ro[b]) && is_zero(tr[b]);
+        for (int j0 = 0; j0 < nl && empty; j0 += EMPTY_BATCH) {
+            /* a batch of loads in flight per test */
+            unsigned long long any = 0;
+#pragma unroll
+            for (int d = 0; d < EMPTY_BATCH; ++d) {
+                if (j0 + d >= nl) continue;
+                const long long b = (long long)(j0 + d) * nc + i;
+                any |= (unsigned long long)(__double_as_longlong(ro[b]) | __double_as_longlong(tr[b]));
+            }
+            empty = (any << 1) == 0ULL;
         }
         if (empty) {
             double *rn = sn.rho + k * ns;
@@ -167,6 +181,8 @@ __global__ void __launch_bounds__(TRACER_BLOCK) k_tracers_solve_df(VGrid vg, Ste
     double *rn = sn.rho + k * ns;
     float *rs = sh_rho + k * ns;
     df x = df_zero();
+    static_assert(NL <= 32, "one word of layers");
+    unsigned held = 0;
 #pragma unroll 1
     for (int j = nl - 1; j >= 0; --j) {
         const float2 e2 = s_ep[j][t], r2 = s_rp[j][t];
@@ -176,7 +192,9 @@ __global__ void __launch_bounds__(TRACER_BLOCK) k_tracers_solve_df(VGrid vg, Ste
         const double v = nonneg<false>(xn) ? xn : 0.0;
         rn[b] = v;
         rs[b] = to_float(v);
+        held |= (is_zero(v) ? 0u : 1u) << j;
     }
+    mark_layers(present.by_const, 8 * k, held);
 }
 
 /* sedimentation heating (rk 0, column_solvers.c:455-462, 551-623): the

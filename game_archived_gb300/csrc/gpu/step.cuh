@@ -84,7 +84,7 @@ inline Views<double> views<double>(Context *c, StateMirror *sn)
 {
     Views<double> v{};
     v.sv = {sn->ds.rho, sn->ds.rhotheta_v, sn->ds.theta_v_pert, sn->ds.exner_pert, sn->ds.w, sn->ds.u};
-    v.sh = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    v.sh = Shadow{};
     return v;
 }
 template <>
@@ -99,6 +99,7 @@ inline Views<float> views<float>(Context *c, StateMirror *sn)
     v.sh.exner_pert = v.sh.theta_v_pert + ns;
     v.sh.w = v.sh.exner_pert + ns;
     v.sh.u = v.sh.w + (long long)(c->nl + 1) * c->nc;
+    v.sh.present = c->present;
     v.sv = {v.sh.rho, v.sh.rhotheta_v, v.sh.theta_v_pert, v.sh.exner_pert, v.sh.w, v.sh.u};
     return v;
 }
@@ -116,7 +117,7 @@ inline void launch_scalar_tend64(Context *c, const StepParams &p, const SView<do
     k_edge_flux<<<layer_grid(c->nl, c->ne, 256), 256, 0, s>>>(g, sv.rho + (long long)c->n_cond * c->ns, theta, sv.u, fm,
                                                              ft);
     c->kernel_launches += 2;
-    if (c->any_tilt) {
+    if (c->n_tilt) {
         const dim3 nb = layer_grid(c->n_oro, c->nc, 256);
         if (p.n_const > 1)
             k_level_corr<true><<<nb, 256, 0, s>>>(g, fm, ft, sv.u, cr, cr + nw, cr + 2 * nw);
@@ -278,24 +279,24 @@ void launch_tracers(Context *c, const StepParams &p, StateMirror *so, StateMirro
     if constexpr (!EXACT) {
         if (p.dfloat && mode == COLUMN_REGISTERS) {
             k_tracers_solve_df<NL_FIXED><<<nblocks(nsys, TRACER_BLOCK), TRACER_BLOCK, 0, strm>>>(
-                c->vg, p, so->ds, sn->ds, st->ds, c->dfg, sh.rho);
+                c->vg, p, so->ds, sn->ds, st->ds, c->dfg, sh.rho, sh.present);
             c->kernel_launches++;
             return;
         }
     }
     if (mode == COLUMN_REGISTERS)
         k_tracers_solve<NL_FIXED, NL_FIXED, EXACT><<<nblocks(nsys, 64), 64, 0, strm>>>(c->vg, p, so->ds, sn->ds,
-                                                                                        st->ds, tw, sh.rho);
+                                                                                        st->ds, tw, sh.rho, sh.present);
     else if (mode == COLUMN_LOCAL && c->nl <= SWEEP_SMALL)
         k_tracers_solve<0, SWEEP_SMALL, EXACT><<<nblocks(nsys, 64), 64, 0, strm>>>(c->vg, p, so->ds, sn->ds, st->ds,
-                                                                                    tw, sh.rho);
+                                                                                    tw, sh.rho, sh.present);
     else if (mode == COLUMN_LOCAL)
         k_tracers_solve<0, SWEEP_LARGE, EXACT><<<nblocks(nsys, 64), 64, 0, strm>>>(c->vg, p, so->ds, sn->ds, st->ds,
-                                                                                    tw, sh.rho);
+                                                                                    tw, sh.rho, sh.present);
     else
         k_tracers_pcr<EXACT><<<nblocks(nsys, PCR_WARPS), 32 * PCR_WARPS,
                                (size_t)PCR_WARPS * 6 * c->nl * sizeof(double), strm>>>(c->vg, p, so->ds, sn->ds,
-                                                                                       st->ds, tw, sh.rho);
+                                                                                       st->ds, tw, sh.rho, sh.present);
     c->kernel_launches++;
 }
 
@@ -317,6 +318,8 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
         const long long n_rho = (long long)c->n_const * ns, nw = (long long)(c->nl + 1) * c->nc,
                         nu = (long long)c->nl * c->ne;
         const long long pairs = (std::max(std::max(n_rho, nw), nu) + 1) / 2;
+        if (c->n_const > 1)
+            cudaMemsetAsync(c->present.by_layer, 0, ((size_t)c->nl + 8 * c->n_const) * sizeof(int), c->stream);
         k_make_shadow<<<nblocks(pairs, bs), bs, 0, c->stream>>>(n_rho, ns, nw, nu, sn->ds, v.sh);
         c->kernel_launches++;
     }
@@ -327,7 +330,7 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
         if constexpr (EXACT)
             k_pg_cells64<<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(g, p, v.sv, c->pg_cell64, c->grad_pi_v);
         else
-            k_pg_cells<<<nblocks(ns, bs), bs, 0, c->stream>>>(c->hg32, p, v.sv, c->pg_cell);
+            k_pg_cells<<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(c->hg32, p, v.sv, c->pg_cell, c->present);
         c->kernel_launches++;
     }
     {
@@ -403,14 +406,22 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
             if constexpr (EXACT) {
                 launch_scalar_tend64(c, p, v.sv, st->ds.rho, st->ds.rho, st->ds.rhotheta_v, theta, cpi, cpw, c->pt_rates,
                                      c->pt_heat, c->sed_heat, rk, irr);
-            } else if (p.irr) {
-                k_scalar_tend2<R, true><<<layer_grid(c->nl, c->nc, 128), 128, 0, c->stream>>>(
-                    g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, rk,
-                    irr);
             } else {
-                k_scalar_tend2<R, false><<<layer_grid(c->nl, c->nc, 128), 128, 0, c->stream>>>(
-                    g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, rk,
-                    irr);
+                auto flat = [&](auto kernel) {
+                    kernel<<<layer_grid(c->nl, c->nc, 128), 128, 0, c->stream>>>(
+                        g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, c->present,
+                        rk, irr);
+                };
+                auto tilt = [&](auto kernel) {
+                    kernel<<<layer_grid(c->nl, c->n_tilt, 128), 128, 0, c->stream>>>(
+                        g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, rk, irr,
+                        c->tilt_cells, c->n_tilt);
+                };
+                p.irr ? flat(k_scalar_tend32<true>) : flat(k_scalar_tend32<false>);
+                if (c->n_tilt) {
+                    p.irr ? tilt(k_scalar_tend_tilt<true>) : tilt(k_scalar_tend_tilt<false>);
+                    c->kernel_launches++;
+                }
             }
         }
         c->kernel_launches += EXACT ? 1 : 2; /* launch_scalar_tend64 counts its own */
