@@ -148,6 +148,37 @@ __device__ __forceinline__ double to_double(float x)
  * pipe) */
 __device__ __forceinline__ bool is_zero(double x) { return ((unsigned long long)__double_as_longlong(x) << 1) == 0ULL; }
 
+/* FP64 operations that stay behind the test that guards them: the compiler runs
+ * plain ones ahead of it and selects, and each issue holds the FP64 pipe for 16
+ * cycles */
+__device__ __forceinline__ double guarded_mul(double a, double b)
+{
+    double r;
+    asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+}
+__device__ __forceinline__ double guarded_add(double a, double b)
+{
+    double r;
+    asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+}
+__device__ __forceinline__ double guarded_fma(double a, double b, double c)
+{
+    double r;
+    asm volatile("fma.rn.f64 %0, %1, %2, %3;" : "=d"(r) : "d"(a), "d"(b), "d"(c));
+    return r;
+}
+
+/* half of x exactly, without an FP64 instruction for normal numbers whose half
+ * is normal, and zeros */
+__device__ __forceinline__ double half_of(double x)
+{
+    const int hi = __double2hiint(x);
+    if (((unsigned)(hi >> 20) & 0x7ffu) - 2u <= 2044u) return __hiloint2double(hi - 0x100000, __double2loint(x));
+    return is_zero(x) ? x : guarded_mul(0.5, x);
+}
+
 /* a double passed to either conversion would be narrowed silently */
 double to_double(double) = delete;
 float to_float(float) = delete;
