@@ -339,6 +339,9 @@ void substage_fwd(Context *c, AdjState *a, StepBufs<T> &B, int rk, bool first, c
                                                                                   B.zh[rk], B.zv[rk], B.fh[rk]);
             k_cell_kinetic<double><<<layer_grid(c->nl, c->nc, 256), 256, 0, st>>>(g, sn.u, sn.w, sn.rho, B.v2[rk],
                                                                                  B.fv[rk]);
+            k_level_terms<<<layer_grid(c->nl + 1, c->nc, 256), 256, 0, st>>>(
+                g, B.v2[rk], B.fv[rk], B.v2g[rk], c->level_q64, c->level_q64 + (long long)(c->nl + 1) * c->nc);
+            c->kernel_launches++;
         }
     } else if (adv) {
         fa_tri<T><<<nbk(a->ntri), 256, 0, st>>>(g, sn.u, B.tri[rk]);
@@ -349,7 +352,8 @@ void substage_fwd(Context *c, AdjState *a, StepBufs<T> &B, int rk, bool first, c
                                             B.v2g[rk], B.tend[0], B.tend[rk], moist ? sn.rho_all : nullptr);
     fa_mom_h<T><<<nbk(a->nu), 256, 0, st>>>(g, ap, adv, new_w, old_w, B.P, B.pgo, B.fh[rk], B.fv[rk], B.zh[rk],
                                             B.zv[rk], B.v2[rk], B.pvt[rk], B.v2g[rk], B.tend[0], B.tend[rk], so.u,
-                                            out.u);
+                                            out.u, c->level_q64,
+                                            c->level_q64 + (long long)(c->nl + 1) * c->nc);
     fa_theta<T><<<nbk(ns), 256, 0, st>>>(ns, sn.rho, sn.rt, B.theta[rk]);
     if constexpr (PLAIN) {
         const DState d = dview(a, rk ? B.sn1 : B.so);
@@ -410,7 +414,8 @@ void step_fwd(Context *c, AdjState *a, StepBufs<T> &B, const T *P_prev, const T 
     if constexpr (sizeof(T) == sizeof(double)) {
         const DState d = dview(a, B.so);
         const SView<double> sv{d.rho, d.rhotheta_v, d.theta_v_pert, d.exner_pert, d.w, d.u};
-        k_pg_cells64<<<layer_grid(c->nl, c->nc, 256), 256, 0, st>>>(g, a->p, sv, c->pg_cell64, c->grad_pi_v);
+        k_pg_cells64<<<layer_grid(c->nl, c->nc, 256), 256, 0, st>>>(g, a->p, sv, c->pg_cell64, c->grad_pi_v,
+                                                                    c->theta);
         fd_pgrad_v<<<layer_grid(c->nl - 1, c->nc, 256), 256, 0, st>>>(g, c->pg_cell64, c->grad_pi_v,
                                                                       a->n_const == 1, B.P);
         fd_pgrad_h<<<layer_grid(c->nl, c->ne, 256), 256, 0, st>>>(g, c->pg_cell64, c->grad_pi_v, a->n_const == 1,

@@ -395,7 +395,8 @@ __device__ __forceinline__ T a_vflux_h(const HGrid<double> &g, const T *flux_h, 
 template <class T>
 __global__ void fa_mom_h(HGrid<double> g, AParams ap, int adv, double new_w, double old_w, const T *P, const T *pg_old,
                          const T *flux_h, const T *flux_v, const T *zh, const T *zv, const T *v2, T *pvt, T *v2g,
-                         const T *tend_in, T *tend_out, const T *u_old, T *u_new)
+                         const T *tend_in, T *tend_out, const T *u_old, T *u_new, const double *q_hi,
+                         const double *q_lo)
 {
     const long long n = (long long)g.nl * g.ne;
     const long long i = gtid();
@@ -403,7 +404,10 @@ __global__ void fa_mom_h(HGrid<double> g, AParams ap, int adv, double new_w, dou
     const long long nw = (long long)(g.nl + 1) * g.nc, vi = nw + i;
     const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     if (adv) {
-        pvt[vi] = a_vflux_h(g, flux_h, flux_v, zh, zv, l, e);
+        if constexpr (sizeof(T) == sizeof(double))
+            pvt[vi] = vorticity_flux_levels(g, flux_h, q_hi, q_lo, zh, zv, l, e);
+        else
+            pvt[vi] = a_vflux_h(g, flux_h, flux_v, zh, zv, l, e);
         v2g[vi] = a_grad_h_pre(g, v2, v2g, l, e);
     }
     const double cur_hor = 0.5 + ap.impl_thermo_weight, old_hor = 1.0 - (0.5 + ap.impl_thermo_weight);
@@ -446,7 +450,7 @@ __global__ void fa_mom_v(HGrid<double> g, AParams ap, int adv, double new_w, dou
         tend_out[i] = tzero<T>();
         return;
     }
-    if (adv) v2g[i] = a_gv(g, v2, k, c);
+    if (adv && sizeof(T) != sizeof(double)) v2g[i] = a_gv(g, v2, k, c); /* FP64: k_level_terms */
     const double cur_ver = 1.0 - ap.impl_thermo_weight;
     T y = -cur_ver * P[i] + pvt[i] - 0.5 * v2g[i];
     if (rho_all) {

@@ -611,6 +611,8 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
     c->damp_inv = dalloc<double>(c, (size_t)(L - 1) * NC);
     c->damp_den = dalloc<double>(c, (size_t)(L - 1) * NC);
     c->pg_cell64 = dalloc<Quad>(c, NS);
+    c->level_q64 = dalloc<double>(c, (size_t)2 * (L + 1) * NC);
+    c->gas_share64 = dalloc<double>(c, NS);
     c->grad_pi_v = dalloc<double>(c, (size_t)(L + 1) * NC);
     {
         std::vector<double> iv(h_vol.size()), ia(h_areav.size());

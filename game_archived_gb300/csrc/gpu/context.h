@@ -105,6 +105,8 @@ struct Context {
     /* FP64 path: the same factors in double, and the vertical gradient of
      * Pi' at the inner interfaces [L+1][Nc] */
     Quad *pg_cell64 = nullptr;
+    double *level_q64 = nullptr;  /* k_level_terms' mass-flux factors [2][L+1][Nc] */
+    double *gas_share64 = nullptr; /* rho_gas / rho_total at rk 1 [L][Nc] */
     /* FP64 path: mass and rho theta_v fluxes of the edges [2][L][Ne], and the
      * terrain corrections of both and of the wind at the levels [3][L+1][Nc],
      * of the substage at hand (k_edge_flux, k_level_corr) */

@@ -48,21 +48,12 @@ __device__ __forceinline__ R grad_v(const HGrid<R> &g, const F *f, int k, int c)
     return div_tab(R(f[i - g.nc]) - R(f[i]), g.nd_v, g.r_nd_v, i);
 }
 
-/* the same for every inner interface of a field: formed once, where each is
- * read by up to twelve edges' gradients (grad_h_pre) and by the interface's
- * own momentum */
-__global__ void k_grad_v(HGrid<double> g, const double *f, double *out)
-{
-    const LayerPoint p = layer_point(g.nc);
-    if (p.in) out[p.i + g.nc] = grad_v(g, f, p.l + 1, p.x);
-}
-
 /* slopes are exactly 0 away from orography; no FP64 comparison */
 __device__ __forceinline__ bool zero_slope(double s) { return is_zero(s); }
 __device__ __forceinline__ bool zero_slope(float s) { return s == 0.0f; }
 
 /* horizontal gradient at edge e of layer l from the field and its vertical
- * gradients gv (k_grad_v): grad_h's operations in its order */
+ * gradients gv at the inner interfaces: grad_h's operations in its order */
 __device__ __forceinline__ double grad_h_pre(const HGrid<double> &g, double f_to, double f_fr, const double *gv, int l,
                                              int e, int fr, int to)
 {
@@ -707,25 +698,35 @@ __global__ void k_cell_kinetic(HGrid<R> g, const R *u, const R *w, const R *rho_
     }
 }
 
-/* modified TRSK vorticity flux at edge e of layer l (vorticity_flux.c:35-137) */
+/* x / 2; on the FP64 path without an FP64 instruction (exact, so where a
+ * product takes the factor does not change it) */
+__device__ __forceinline__ float halved(float x) { return 0.5f * x; }
+__device__ __forceinline__ double halved(double x) { return half_of(x); }
+
+/* modified TRSK sum of the vorticity flux at edge e of layer l
+ * (vorticity_flux.c:35-113) */
 template <typename R>
-__device__ __forceinline__ R vorticity_flux_h(const HGrid<R> &g, const R *flux_h, const R *flux_v, const R *zh,
-                                              const R *zv, int l, int e)
+__device__ __forceinline__ R trsk_sum(const HGrid<R> &g, const R *flux_h, const R *zv, int l, int e)
 {
     const long long ne = g.ne;
     const R *mf = flux_h + (long long)l * ne;
     const R *pv = zv + (long long)l * ne;
     const int fr = g.from[e], to = g.to[e];
     R out = R(0);
+    /* the middle edge of each side counts with the mean of two vorticities */
+    auto mean_term = [&](int j) {
+        if constexpr (sizeof(R) == sizeof(double))
+            return half_of(g.trsk_w[j * ne + e]) * mf[g.trsk_i[j * ne + e]] * (pv[g.trsk_m[j * ne + e]] + pv[e]);
+        else
+            return g.trsk_w[j * ne + e] * mf[g.trsk_i[j * ne + e]] * R(0.5) * (pv[g.trsk_m[j * ne + e]] + pv[e]);
+    };
     if (fr < N_PENT) {
         for (int j = 0; j < 4; ++j)
             out += g.trsk_w[j * ne + e] * mf[g.trsk_i[j * ne + e]] * pv[g.trsk_m[j * ne + e]];
     } else {
         for (int j = 0; j < 5; ++j) {
-            if (j == 2)
-                out += g.trsk_w[j * ne + e] * mf[g.trsk_i[j * ne + e]] * R(0.5) * (pv[g.trsk_m[j * ne + e]] + pv[e]);
-            else
-                out += g.trsk_w[j * ne + e] * mf[g.trsk_i[j * ne + e]] * pv[g.trsk_m[j * ne + e]];
+            if (j == 2) out += mean_term(j);
+            else out += g.trsk_w[j * ne + e] * mf[g.trsk_i[j * ne + e]] * pv[g.trsk_m[j * ne + e]];
         }
     }
     if (to < N_PENT) {
@@ -733,18 +734,60 @@ __device__ __forceinline__ R vorticity_flux_h(const HGrid<R> &g, const R *flux_h
             out += g.trsk_w[j * ne + e] * mf[g.trsk_i[j * ne + e]] * pv[g.trsk_m[j * ne + e]];
     } else {
         for (int j = 5; j < 10; ++j) {
-            if (j == 7)
-                out += g.trsk_w[j * ne + e] * mf[g.trsk_i[j * ne + e]] * R(0.5) * (pv[g.trsk_m[j * ne + e]] + pv[e]);
-            else
-                out += g.trsk_w[j * ne + e] * mf[g.trsk_i[j * ne + e]] * pv[g.trsk_m[j * ne + e]];
+            if (j == 7) out += mean_term(j);
+            else out += g.trsk_w[j * ne + e] * mf[g.trsk_i[j * ne + e]] * pv[g.trsk_m[j * ne + e]];
         }
     }
+    return out;
+}
+
+/* modified TRSK vorticity flux at edge e of layer l (vorticity_flux.c:35-137) */
+template <typename R>
+__device__ __forceinline__ R vorticity_flux_h(const HGrid<R> &g, const R *flux_h, const R *flux_v, const R *zh,
+                                              const R *zv, int l, int e)
+{
+    const long long ne = g.ne;
+    const int fr = g.from[e], to = g.to[e];
+    R out = trsk_sum(g, flux_h, zv, l, e);
     const R zt = zh[(long long)l * ne + e], zb = zh[(long long)(l + 1) * ne + e];
     const long long nc = g.nc;
-    out -= R(0.5) * ipw_at(g, 6, l, fr) * flux_v[l * nc + fr] * zt;
-    out -= R(0.5) * ipw_at(g, 6, l, to) * flux_v[l * nc + to] * zt;
-    out -= R(0.5) * ipw_at(g, 7, l, fr) * flux_v[(l + 1) * nc + fr] * zb;
-    out -= R(0.5) * ipw_at(g, 7, l, to) * flux_v[(l + 1) * nc + to] * zb;
+    out -= halved(ipw_at(g, 6, l, fr)) * flux_v[l * nc + fr] * zt;
+    out -= halved(ipw_at(g, 6, l, to)) * flux_v[l * nc + to] * zt;
+    out -= halved(ipw_at(g, 7, l, fr)) * flux_v[(l + 1) * nc + fr] * zb;
+    out -= halved(ipw_at(g, 7, l, to)) * flux_v[(l + 1) * nc + to] * zb;
+    return out;
+}
+
+/* What an edge's horizontal momentum reads of its two cells' levels, formed
+ * once per level instead of by each of the cell's six edges (FP64 path): the
+ * vertical gradient of v^2 at the inner interfaces, and the vertical mass
+ * flux times half the inner-product weight of the layer below (hi) and above
+ * (lo) the level, the factors of vorticity_flux.c:115-137. */
+__global__ void k_level_terms(HGrid<double> g, const double *v2, const double *flux_v, double *grad_v2, double *q_hi,
+                              double *q_lo)
+{
+    const LayerPoint p = layer_point(g.nc);
+    if (!p.in) return;
+    const int k = p.l, c = p.x;
+    const double f = flux_v[p.i];
+    if (k > 0 && k < g.nl) grad_v2[p.i] = grad_v(g, v2, k, c);
+    if (k < g.nl) q_hi[p.i] = half_of(ipw_at(g, 6, k, c)) * f;
+    if (k > 0) q_lo[p.i] = half_of(ipw_at(g, 7, k - 1, c)) * f;
+}
+
+/* vorticity_flux_h from them */
+__device__ __forceinline__ double vorticity_flux_levels(const HGrid<double> &g, const double *flux_h, const double *q_hi,
+                                                        const double *q_lo, const double *zh, const double *zv, int l,
+                                                        int e)
+{
+    const int fr = g.from[e], to = g.to[e];
+    const long long nc = g.nc, lc = l * nc;
+    double out = trsk_sum(g, flux_h, zv, l, e);
+    const double zt = zh[(long long)l * g.ne + e], zb = zh[(long long)(l + 1) * g.ne + e];
+    out -= q_hi[lc + fr] * zt;
+    out -= q_hi[lc + to] * zt;
+    out -= q_lo[lc + nc + fr] * zb;
+    out -= q_lo[lc + nc + to] * zb;
     return out;
 }
 
@@ -832,10 +875,10 @@ __global__ void k_pg_cells(HGrid<float> g, StepParams p, SView<float> s, float4 
 
 /* FP64 path: the same cell factors in double with the operations of
  * pgrad_h_parts / pgrad_v_parts (the dry build's density ratio is rho / rho =
- * 1 and is left out), and the vertical gradient of Pi' at the interface
- * above the cell.  Formed once per cell instead of once per edge and
+ * 1 and is left out), the vertical gradient of Pi' at the interface above
+ * the cell, and theta_v.  Formed once per cell instead of once per edge and
  * interface that reads it (up to eight times). */
-__global__ void k_pg_cells64(HGrid<double> g, StepParams p, SView<double> s, Quad *pc, double *grad_pi)
+__global__ void k_pg_cells64(HGrid<double> g, StepParams p, SView<double> s, Quad *pc, double *grad_pi, double *theta)
 {
     const LayerPoint pt = layer_point(g.nc);
     if (!pt.in) return;
@@ -844,6 +887,7 @@ __global__ void k_pg_cells64(HGrid<double> g, StepParams p, SView<double> s, Qua
     pc[i] = Quad{s.exner_pert[i], cdp * (g.theta_v_bg[i] + tp), cdp * tp,
                  p.n_const > 1 ? s.rho[p.n_cond * ns + i] / density_total_r(s.rho, p.n_const, ns, i) : 1.0};
     if (pt.l > 0) grad_pi[i] = grad_v(g, s.exner_pert, pt.l, pt.x);
+    theta[i] = s.rhotheta_v[i] / s.rho[p.n_cond * ns + i];
 }
 
 __device__ __forceinline__ double pgrad_h_cells(const HGrid<double> &g, const Quad *pc, const double *grad_pi, int l,
@@ -918,7 +962,7 @@ __device__ __forceinline__ float pgrad_v_packed(const HGrid<float> &g, float4 u,
 
 /* what the momentum kernels read of the first substage's pressure gradient
  * (mixed path: k_pg_cells; FP64 path: k_pg_cells64) and, FP64 path, of the
- * kinetic energy's vertical gradient (k_grad_v) */
+ * levels' terms (k_level_terms) and, at rk 1, rho_gas / rho_total */
 template <typename R>
 struct PgCells;
 template <>
@@ -928,7 +972,7 @@ struct PgCells<float> {
 template <>
 struct PgCells<double> {
     const Quad *cell;
-    const double *grad_pi, *grad_v2;
+    const double *grad_pi, *grad_v2, *q_hi, *q_lo, *gas_share;
 };
 
 /* ------------------------------------------------------- k_momentum_h
@@ -938,7 +982,8 @@ struct PgCells<double> {
  * the cell factors.  FP64 issue bounds the FP64 instantiation: with the
  * vertical gradients and cell factors formed once, the zero slopes skipped
  * and div_rcp for the distances it went from 182 to 101 us at RES_ID 5
- * with the mountain (789 to 378 us at RES_ID 6, flat, moist).  The wind update
+ * with the mountain (789 to 378 us at RES_ID 6, flat, moist), with the levels'
+ * terms formed once and the halves taken off the exponent to 89 (320).  The wind update
  * is FP64; u_shadow (mixed path) receives its FP32 copy. */
 template <typename R, bool ADV, bool PG>
 __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_momentum_h(HGrid<R> g, StepParams p, SView<R> sv, double *u_new, float *u_shadow, const double *u_old,
@@ -965,10 +1010,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
     }
     R pvt, v2g;
     if (ADV) {
-        pvt = vorticity_flux_h(g, flux_h, flux_v, zh, zv, l, e);
         if constexpr (sizeof(R) == sizeof(float)) {
+            pvt = vorticity_flux_h(g, flux_h, flux_v, zh, zv, l, e);
             v2g = grad_h(g, v2, l, e);
         } else {
+            pvt = vorticity_flux_levels(g, flux_h, pg.q_hi, pg.q_lo, zh, zv, l, e);
             const int fr = g.from[e], to = g.to[e];
             v2g = grad_h_pre(g, v2[(long long)l * g.nc + to], v2[(long long)l * g.nc + fr], pg.grad_v2, l, e, fr, to);
         }
@@ -980,12 +1026,15 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
     }
     constexpr bool F = sizeof(R) == sizeof(float);
     const R cur_hor = F ? R(p.cur_hor_f) : R(p.cur_hor), old_hor = F ? R(p.old_hor_f) : R(p.old_hor);
-    R y = old_hor * pgo - cur_hor * P + pvt - R(0.5) * v2g;
+    R y = old_hor * pgo - cur_hor * P + pvt - halved(v2g);
     /* friction acceleration of the diffusion branch, when it is active */
     if (fric_u) y = y + R(fric_u[i]);
     /* the pressure gradient is recomputed in substage 0 only, where the new
      * weight is 1 */
-    double t = PG ? wide(y) : old_w * tend_u[i] + new_w * wide(y);
+    double t;
+    if (PG) t = wide(y);
+    else if (F) t = old_w * tend_u[i] + new_w * wide(y);
+    else t = half_of(tend_u[i] + wide(y)); /* both weights 1/2 */
     tend_u[i] = t;
     const double un = u_old[i] + p.dt * t;
     u_new[i] = un;
@@ -1009,18 +1058,25 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
     if (ADV) {
         /* vertical part of the vorticity flux (vorticity_flux.c:143-183), all levels */
         const int n_edges = c < N_PENT ? 5 : 6;
-        const R vw = (k == 0 || k == nl) ? R(1) : R(0.5);
+        /* the weight 1/2 of the inner levels goes to every term (mixed path)
+         * or, exact in either place, to their sum */
+        const R vw = (k == 0 || k == nl || sizeof(R) == sizeof(double)) ? R(1) : R(0.5);
+        auto weight = [&](int j, int ll) {
+            if constexpr (sizeof(R) == sizeof(double)) return ipw_at(g, j, ll, c);
+            else return vw * ipw_at(g, j, ll, c);
+        };
         const R *z = zh + (long long)k * g.ne;
         if (k >= 1)
             for (int j = 0; j < n_edges; ++j) {
                 const int a = g.adj[j * g.nc + c];
-                pvt += vw * ipw_at(g, j, k - 1, c) * flux_h[(long long)(k - 1) * g.ne + a] * z[a];
+                pvt += weight(j, k - 1) * flux_h[(long long)(k - 1) * g.ne + a] * z[a];
             }
         if (k <= nl - 1)
             for (int j = 0; j < n_edges; ++j) {
                 const int a = g.adj[j * g.nc + c];
-                pvt += vw * ipw_at(g, j, k, c) * flux_h[(long long)k * g.ne + a] * z[a];
+                pvt += weight(j, k) * flux_h[(long long)k * g.ne + a] * z[a];
             }
+        if (sizeof(R) == sizeof(double) && k > 0 && k < nl) pvt = halved(pvt);
         pvt_v[i] = pvt;
     }
     if (k == 0 || k == nl) {
@@ -1047,9 +1103,14 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
         v2g = grad_v(g, v2, k, c);
         v2g_v[i] = v2g;
     } else {
-        v2g = v2g_v[i]; /* FP64 path: written by k_grad_v */
+        v2g = v2g_v[i]; /* FP64 path: written by k_level_terms */
     }
-    if (!PG && !dry) {
+    if constexpr (!PG && !F) {
+        if (!dry) {
+            d_up = pg.gas_share[i - g.nc] - R(1);
+            d_lo = pg.gas_share[i] - R(1);
+        }
+    } else if (!PG) {
         const long long ns = (long long)nl * g.nc;
         const long long up = (long long)(k - 1) * g.nc + c, lo = (long long)k * g.nc + c;
         d_up = sv.rho[p.n_cond * ns + up] / density_total_r(sv.rho, p.n_const, ns, up) - R(1);
@@ -1057,10 +1118,13 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
     }
     R pgc = (R(0.5) * (d_up + d_lo)) * g.gravity_m_v[i];
     const R cur_ver = sizeof(R) == sizeof(float) ? R(p.cur_ver_f) : R(p.cur_ver);
-    R y = -cur_ver * P + pvt - R(0.5) * v2g;
+    R y = -cur_ver * P + pvt - halved(v2g);
     if (fric_w) y = y + R(fric_w[i]);
     y = y + pgc;
-    double t = PG ? wide(y) : old_w * tend_w[i] + new_w * wide(y);
+    double t;
+    if (PG) t = wide(y);
+    else if (F) t = old_w * tend_w[i] + new_w * wide(y);
+    else t = half_of(tend_w[i] + wide(y)); /* both weights 1/2 */
     tend_w[i] = t;
 }
 
@@ -1095,6 +1159,17 @@ __global__ void k_theta(int nl, int nc, int n_cond, SView<R> sv, R *theta)
     const long long i = gtid();
     if (i >= ns) return;
     theta[i] = sv.rhotheta_v[i] / sv.rho[n_cond * ns + i];
+}
+
+/* FP64 path, rk 1: theta_v and rho_gas / rho_total of every cell, which two
+ * interfaces' condensate terms read */
+__global__ void k_theta_share(long long ns, int n_cond, int n_const, SView<double> sv, double *theta, double *share)
+{
+    const long long i = gtid();
+    if (i >= ns) return;
+    const double rg = sv.rho[n_cond * ns + i];
+    theta[i] = sv.rhotheta_v[i] / rg;
+    if (n_const > 1) share[i] = rg / density_total_r(sv.rho, n_const, ns, i);
 }
 
 /* Sum of edge fluxes of one cell.  R = double: plain double accumulation

@@ -144,7 +144,8 @@ inline PgCells<float> pg_cells<float>(Context *c)
 template <>
 inline PgCells<double> pg_cells<double>(Context *c)
 {
-    return {c->pg_cell64, c->grad_pi_v, c->w64.v2g_v};
+    return {c->pg_cell64, c->grad_pi_v, c->w64.v2g_v, c->level_q64, c->level_q64 + (long long)(c->nl + 1) * c->nc,
+            c->gas_share64};
 }
 
 template <typename R, bool ADV, bool PG>
@@ -328,7 +329,8 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
          * diffusion branch, which runs before it, changes none of its inputs) */
         ProfScope ps(c, "k_pg_cells");
         if constexpr (EXACT)
-            k_pg_cells64<<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(g, p, v.sv, c->pg_cell64, c->grad_pi_v);
+            k_pg_cells64<<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(g, p, v.sv, c->pg_cell64, c->grad_pi_v,
+                                                                                 c->theta);
         else
             k_pg_cells<<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(c->hg32, p, v.sv, c->pg_cell, c->present);
         c->kernel_launches++;
@@ -372,8 +374,9 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
             }
             c->kernel_launches += 3;
             if constexpr (EXACT) {
-                ProfScope ps(c, "k_grad_v");
-                k_grad_v<<<layer_grid(c->nl - 1, c->nc, bs), bs, 0, c->stream>>>(g, w.v2, w.v2g_v);
+                ProfScope ps(c, "k_level_terms");
+                k_level_terms<<<layer_grid(c->nl + 1, c->nc, bs), bs, 0, c->stream>>>(
+                    g, w.v2, w.flux_v, w.v2g_v, c->level_q64, c->level_q64 + (long long)(c->nl + 1) * c->nc);
                 c->kernel_launches++;
             }
         }
@@ -390,12 +393,18 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
                 cudaStreamWaitEvent(c->stream, c->ev_join, 0);
                 join_pending = false;
             }
+            if constexpr (EXACT) {
+                ProfScope ps(c, "k_theta");
+                k_theta_share<<<nblocks(ns, bs), bs, 0, c->stream>>>(ns, c->n_cond, c->n_const, v.sv, c->theta,
+                                                                     c->gas_share64);
+                c->kernel_launches++;
+            }
             launch_momentum_v<R, true, false>(c, p, v, st, new_w, old_w);
         }
         /* diffusion branch: temperature and mass diffusion */
         if (rk == 0 && (p.diff & DIFF_RAD_HS)) launch_held_suarez_radiation(c, so->ds);
         if (rk == 0 && p.diff) launch_diffusion_scalar(c, p, v.sv);
-        {
+        if constexpr (!EXACT) {
             ProfScope ps(c, "k_theta");
             k_theta<R><<<nblocks(ns, bs), bs, 0, c->stream>>>(c->nl, c->nc, c->n_cond, v.sv, theta);
         }
@@ -424,7 +433,7 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
                 }
             }
         }
-        c->kernel_launches += EXACT ? 1 : 2; /* launch_scalar_tend64 counts its own */
+        c->kernel_launches += EXACT ? 0 : 2; /* launch_scalar_tend64 counts its own */
         /* the tendency is final from here on: a host-in/host-out call copies
          * it out while the solvers run */
         if (rk == 1) {
