@@ -596,7 +596,7 @@ __global__ void ba_thomas(int nc, int nl_arg, const double *dden, const double *
         const long long q = (long long)j * nc + i;
         const double xb = div_rcp(wr_b[WR_SOL * m + q], dden[q], r_dden[q]);
         const double sub = j > 0 ? ee[q - nc] : 0.0; /* (A^T)_{j,j-1} = e_{j-1} */
-        const double den = j > 0 ? dd[q] - ep[j - 1] * sub : dd[q], inv = 1.0 / den;
+        const double den = j > 0 ? dd[q] - ep[j - 1] * sub : dd[q], inv = rcp_nr<2>(den);
         if (j < n - 1) ep[j] = div_rcp(cc[q], den, inv); /* (A^T)_{j,j+1} = c_j */
         rp[j] = div_rcp(j > 0 ? xb - rp[j - 1] * sub : xb, den, inv);
     }

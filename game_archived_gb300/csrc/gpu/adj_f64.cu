@@ -275,7 +275,8 @@ long long ck_stride(const AdjState *a) { return a->nblk + 3 * a->nv + (moist_of(
 /* the sound-wave solve with the FP64 step's kernels, its work kept on the
  * tape (wl, wr); the sweep also keeps the undamped solution, which the step
  * does not */
-void waves_fwd(Context *c, AdjState *a, int rk, DState so, DState sn, DState tend, double *wl, double *wr, DState out)
+void waves_fwd(Context *c, AdjState *a, int rk, DState so, DState sn, DState tend, const double *theta, double *wl,
+               double *wr, DState out)
 {
     const long long ns = a->ns, m = a->nwi;
     cudaStream_t st = c->stream;
@@ -285,7 +286,7 @@ void waves_fwd(Context *c, AdjState *a, int rk, DState so, DState sn, DState ten
     w.ep_expl = wl + WL_EPEXP * ns; w.thl = wl + WL_THL * ns;
     w.c = wr + WR_C * m; w.d = wr + WR_D * m; w.e = wr + WR_E * m; w.r = wr + WR_R * m;
     w.th_int = wr + WR_TH * m; w.rho_io = wr + WR_RIO * m; w.r_rho_io = wr + WR_RRIO * m;
-    k_waves_layer<true><<<nbk(ns), 256, 0, st>>>(c->vg, a->p, so, sn, tend, w, rk);
+    k_waves_layer<true><<<nbk(ns), 256, 0, st>>>(c->vg, a->p, so, sn, tend, w, rk, theta);
     k_waves_rows<<<layer_grid(c->nl - 1, c->nc, 256), 256, 0, st>>>(c->vg, a->p, so, tend, w);
     if (c->nl == 26)
         fa_waves_thomas_fixed<26><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, a->dden, a->r_dden, wr);
@@ -369,7 +370,8 @@ void substage_fwd(Context *c, AdjState *a, StepBufs<T> &B, int rk, bool first, c
     const T *str_gas = B.str[rk] + (long long)a->n_cond * ns;
     if constexpr (PLAIN) {
         waves_fwd(c, a, rk, dview(a, B.so), dview(a, rk ? B.sn1 : B.so),
-                  DState{B.str[rk], B.strt[rk], nullptr, nullptr, B.tend[rk], nullptr}, B.wl[rk], B.wr[rk],
+                  DState{B.str[rk], B.strt[rk], nullptr, nullptr, B.tend[rk], nullptr}, B.theta[rk], B.wl[rk],
+                  B.wr[rk],
                   dview(a, rk ? B.sn2 : B.sn1));
     } else {
         fa_waves_layer<T><<<nbk(ns), 256, 0, st>>>(vg, ap, rk, so, sn, str_gas, B.strt[rk], B.wl[rk]);
@@ -977,7 +979,7 @@ int adj_waves_backward(Context *c, StateMirror *so_m, StateMirror *sn_m, StateMi
     AState<double> so = view(a, so_m->dev), sn = view(a, sn_m->dev), out = view(a, a->B.sn2);
     double *wl = a->B.wl[0], *wr = a->B.wr[0];
     /* forward of the solver, keeping its work */
-    waves_fwd(c, a, rk, so_m->ds, sn_m->ds, st_m->ds, wl, wr, dview(a, a->B.sn2));
+    waves_fwd(c, a, rk, so_m->ds, sn_m->ds, st_m->ds, nullptr, wl, wr, dview(a, a->B.sn2));
     /* bars: the output bar moves to a work block, the input bar starts with
      * the pass-through fields */
     double *ob = a->Z.sn2, *ib = sn_bar->dev;

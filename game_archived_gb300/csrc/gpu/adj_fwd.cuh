@@ -670,7 +670,7 @@ __global__ void fa_waves_thomas_fixed(int nc, const double *dden, const double *
         const long long q = (long long)j * nc + i;
         const double dj = wr[WR_D * m + q], rj = wr[WR_R * m + q];
         const double cm = j > 0 ? wr[WR_C * m + q - nc] : 0.0;
-        const double den = j > 0 ? dj - ep[j - 1] * cm : dj, inv = 1.0 / den;
+        const double den = j > 0 ? dj - ep[j - 1] * cm : dj, inv = rcp_nr<2>(den);
         if (j < n - 1) ep[j] = div_rcp(wr[WR_E * m + q], den, inv);
         rp[j] = div_rcp(j > 0 ? rj - rp[j - 1] * cm : rj, den, inv);
     }

@@ -78,6 +78,10 @@ __device__ __forceinline__ double div_rcp(double x, double y, double r)
     const double q = __dmul_rn(x, r);
     return __fma_rn(__fma_rn(-q, y, x), r, q);
 }
+/* 1 / x correctly rounded (as div_rcp), from the hardware's seed: seven FP64
+ * issues and no branch.  Where the reciprocal only serves div_rcp, whose
+ * correction absorbs its last bits, rcp_nr<2> alone does. */
+__device__ __forceinline__ double rcp_full(double x) { return div_rcp(1.0, x, rcp_nr<2>(x)); }
 /* x / tab[i] with the reciprocals of tab in rtab on the FP64 path; the mixed
  * path divides in FP32 */
 __device__ __forceinline__ double div_tab(double x, const double *tab, const double *rtab, long long i)

@@ -85,16 +85,18 @@ __device__ __forceinline__ WaveCoeffs wave_coeffs(int rk, double ro, double rto,
 {
     const double pdw = 0.5, iro = 1.0 / ro;
     const double ao = div_rcp(-rto, ro * ro, iro * iro);
-    const double go = R_D / (C_D_V * rto) * (ebg + epo);
+    auto gamma = [&](double rt, double e) { return R_D / (C_D_V * rt) * (ebg + e); };
+    const double go = gamma(rto, epo);
     if (rk == 0) return {div_rcp(ao, vol, rv), div_rcp(iro, vol, rv), div_rcp(go, vol, rv)};
     const double an = div_rcp(-rtn, rn * rn, irn * irn);
-    const double gn = R_D / (C_D_V * rtn) * (ebg + epn);
+    const double gn = gamma(rtn, epn);
     return {div_rcp((1.0 - pdw) * ao + pdw * an, vol, rv), div_rcp((1.0 - pdw) * iro + pdw * irn, vol, rv),
             div_rcp((1.0 - pdw) * go + pdw * gn, vol, rv)};
 }
 
 template <bool EXACT>
-__global__ void k_waves_layer(VGrid vg, StepParams p, DState so, DState sn, DState st, WavesWork ww, int rk)
+__global__ void k_waves_layer(VGrid vg, StepParams p, DState so, DState sn, DState st, WavesWork ww, int rk,
+                              const double *theta)
 {
     const long long ns = (long long)vg.nl * vg.nc, b = gtid();
     if (b >= ns) return;
@@ -104,7 +106,8 @@ __global__ void k_waves_layer(VGrid vg, StepParams p, DState so, DState sn, DSta
     const double ro = so.rho[gp + b], rto = so.rhotheta_v[b];
     if (EXACT) {
         const double rv = vg.r_volume[b];
-        const double rn = sn.rho[gp + b], rtn = sn.rhotheta_v[b], irn = 1.0 / rn;
+        const double rn = sn.rho[gp + b], rtn = sn.rhotheta_v[b];
+        const double irn = rk != 0 || !theta ? 1.0 / rn : 0.0;
         const WaveCoeffs w = wave_coeffs(rk, ro, rto, vg.exner_bg[b], so.exner_pert[b], rn, rtn, irn,
                                          rk == 0 ? 0.0 : sn.exner_pert[b], vol, rv);
         const double str = st.rho[gp + b], strt = st.rhotheta_v[b], dtv = dt * vol;
@@ -115,7 +118,7 @@ __global__ void k_waves_layer(VGrid vg, StepParams p, DState so, DState sn, DSta
         ww.rt_expl[b] = rto + dt * strt;
         ww.tp_expl[b] = so.theta_v_pert[b] + dtv * (w.alpha * str + w.beta * strt);
         ww.ep_expl[b] = so.exner_pert[b] + dtv * w.gam * strt;
-        ww.thl[b] = div_rcp(rtn, rn, irn);
+        ww.thl[b] = theta ? theta[b] : div_rcp(rtn, rn, irn);
     } else {
         double alpha, beta, gam;
         const double iv = ww.inv_vol[b], iro = rcp_nr<1>(ro);
@@ -159,7 +162,7 @@ __global__ void k_waves_rows(VGrid vg, StepParams p, DState so, DState st, Waves
     const long long ns = (long long)nl * nc, gp = p.n_cond * ns;
     const long long b = q, lo = q + nc, wi = q + nc;
     const double dt = p.dt;
-    const double rho_io = 0.5 * (so.rho[gp + b] + so.rho[gp + lo]), r_rio = 1.0 / rho_io;
+    const double rho_io = 0.5 * (so.rho[gp + b] + so.rho[gp + lo]), r_rio = rcp_nr<2>(rho_io);
     const double rho_ie = 0.5 * (ww.rho_expl[b] + ww.rho_expl[lo]);
     const double tl_b = ww.thl[b], tl_lo = ww.thl[lo];
     const double th = 0.5 * (tl_b + tl_lo);
@@ -251,7 +254,7 @@ __global__ void k_waves_thomas(int nc, WavesWork ww)
         const double dj = ww.d[q], rj = ww.r[q];
         if (j == 0) {
             if (EXACT) {
-                const double inv = 1.0 / dj;
+                const double inv = rcp_nr<2>(dj);
                 ep[0] = div_rcp(ww.e[q], dj, inv);
                 rp[0] = div_rcp(rj, dj, inv);
             } else {
@@ -263,7 +266,7 @@ __global__ void k_waves_thomas(int nc, WavesWork ww)
             const double cm = ww.c[q - nc];
             const double den = dj - ep[j - 1] * cm;
             if (EXACT) {
-                const double inv = 1.0 / den;
+                const double inv = rcp_nr<2>(den);
                 if (j < n - 1) ep[j] = div_rcp(ww.e[q], den, inv);
                 rp[j] = div_rcp(rj - rp[j - 1] * cm, den, inv);
             } else {
@@ -347,7 +350,8 @@ __global__ void k_waves_apply(VGrid vg, StepParams p, DState so, DState sn, Wave
     else num = -ww.th_int[b - nc] * sol[b - nc] + ww.th_int[b] * sol[b];
     const double rt_new = EXACT ? ww.rt_expl[b] + div_rcp(dt * num, vg.volume[b], vg.r_volume[b])
                                 : ww.rt_expl[b] + dt * num * ww.inv_vol[b];
-    const double tp_new = (EXACT ? rt_new / r_new : rt_new * rcp_nr<1>(r_new)) - vg.theta_v_bg[b];
+    const double tp_new =
+        (EXACT ? div_rcp(rt_new, r_new, rcp_nr<2>(r_new)) : rt_new * rcp_nr<1>(r_new)) - vg.theta_v_bg[b];
     const double ep_new = so.exner_pert[b] + vg.volume[b] * ww.gam[b] * (rt_new - so.rhotheta_v[b]);
     sn.rho[gp + b] = r_new;
     sn.rhotheta_v[b] = rt_new;
@@ -403,6 +407,29 @@ __device__ __forceinline__ double sink_velocity(const StepParams &p, int k, bool
     return 0.0;
 }
 
+/* layers tested for a density at a time */
+constexpr int EMPTY_BATCH = 13;
+/* whether a constituent's old density and tendency are 0 in every layer of
+ * column i: the lowest layer first, which tells most of the others, then
+ * batches of loads in flight */
+__device__ __forceinline__ bool absent_from_column(const double *ro, const double *tr, int nl, int nc, int i)
+{
+    const long long low = (long long)(nl - 1) * nc + i;
+    bool empty = is_zero(ro[low]) && is_zero(tr[low]);
+#pragma unroll 1
+    for (int j0 = 0; j0 < nl && empty; j0 += EMPTY_BATCH) {
+        unsigned long long any = 0;
+#pragma unroll
+        for (int d = 0; d < EMPTY_BATCH; ++d) {
+            if (j0 + d >= nl) continue;
+            const long long b = (long long)(j0 + d) * nc + i;
+            any |= (unsigned long long)(__double_as_longlong(ro[b]) | __double_as_longlong(tr[b]));
+        }
+        empty = (any << 1) == 0ULL;
+    }
+    return empty;
+}
+
 /* vertical advection + sedimentation of constituent k in one column
  * (column_solvers.c:398-635); thread = (k-slot, column).  NL > 0: the layer
  * count is a compile-time constant and the sweep stays in registers; NL = 0:
@@ -417,7 +444,9 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
     const long long q = gtid();
     const int n_tr = p.n_const - 1;
     if (q >= (long long)n_tr * nc) return;
-    const int slot = (int)(q / nc), i = (int)(q - (long long)slot * nc);
+    /* FP64 path: the last slot (the vapour, in every column of a moist run)
+     * first, the columns without condensates fill in behind its solves */
+    const int row = (int)(q / nc), slot = EXACT ? n_tr - 1 - row : row, i = (int)(q - (long long)row * nc);
     const int k = slot < p.n_cond ? slot : slot + 1; /* skip the main gas */
     bool has_sink;
     const double vsink = sink_velocity(p, k, has_sink);
@@ -428,15 +457,9 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
     if (EXACT) {
         /* a constituent absent from the column, old density and tendency 0 in
          * every layer: so is the solution.  With the volumes' reciprocals
-         * and one division per row: RES_ID 6, cloud-free, 1088 -> 214 us;
-         * RES_ID 5 with clouds everywhere 221 -> 125 us */
-        bool empty = true;
-#pragma unroll 1
-        for (int j = 0; j < nl && empty; ++j) {
-            const long long b = i + (long long)j * nc;
-            empty = is_zero(ro[b]) && is_zero(tr[b]);
-        }
-        if (empty) {
+         * and one division per row: RES_ID 6, cloud-free, 1088 -> 103 us;
+         * RES_ID 5 with clouds everywhere 221 -> 120 us */
+        if (absent_from_column(ro, tr, nl, nc, i)) {
             double *rn = sn.rho + k * ns;
 #pragma unroll 1
             for (int j = 0; j < nl; ++j) rn[i + (long long)j * nc] = 0.0;
@@ -517,7 +540,7 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
         /* forward elimination */
         if (j == 0) {
             if (EXACT) {
-                const double inv = 1.0 / dj;
+                const double inv = rcp_nr<2>(dj);
                 ep[0] = div_rcp(ej, dj, inv);
                 rp[0] = div_rcp(rj, dj, inv);
             } else {
@@ -528,7 +551,7 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
         } else {
             const double den = dj - ep[j - 1] * c_prev;
             if (EXACT) {
-                const double inv = 1.0 / den;
+                const double inv = rcp_nr<2>(den);
                 if (j < nl - 1) ep[j] = div_rcp(ej, den, inv);
                 rp[j] = div_rcp(rj - rp[j - 1] * c_prev, den, inv);
             } else {
@@ -635,8 +658,7 @@ __global__ void k_tracers_sedheat(VGrid vg, StepParams p, DState so, DState sn, 
  * enthalpy fluxes of both its interfaces, twice the products of the walk down
  * a column but a layer count more threads (a walk of RES_ID 4's 2562 columns
  * fills 20 blocks); an absent condensate's flux is a zero and left out.
- * RES_ID 6, cloud-free: 328 -> 19 us; RES_ID 5 with clouds everywhere 128 ->
- * 38 us. */
+ * RES_ID 6, cloud-free: 328 -> 16 us. */
 __global__ void k_tracers_sedheat64(VGrid vg, StepParams p, DState so, DState sn, const double *temperature,
                                     TracerWork tw, double *sed_heat)
 {
@@ -659,6 +681,18 @@ __global__ void k_tracers_sedheat64(VGrid vg, StepParams p, DState so, DState sn
         const double cp = (k % 2 == 0) ? tw.cp_ice[up] : tw.cp_water[up];
         return cp * temperature[up] * fr;
     };
+    /* no condensate here or in the layers around: no arithmetic at all (the
+     * tests inside fe alone are run ahead of) */
+    unsigned long long any = 0;
+    for (int k = 0; k < n_cond; ++k) {
+        const double *r = so.rho + k * ns + b;
+        any |= (unsigned long long)(__double_as_longlong(r[0]) | (j > 0 ? __double_as_longlong(r[-nc]) : 0LL)
+                                    | (j < nl - 1 ? __double_as_longlong(r[nc]) : 0LL));
+    }
+    if ((any << 1) == 0ULL) {
+        sed_heat[b] = 0.0;
+        return;
+    }
     const double vol = vg.volume[b], rvol = vg.r_volume[b];
     double sh = 0.0;
 #pragma unroll 1

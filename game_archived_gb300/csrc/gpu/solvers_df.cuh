@@ -35,8 +35,6 @@ namespace {
 /* threads per block of the double-float tracer solve; its elimination
  * coefficients live in shared memory, NL x TRACER_BLOCK (hi, lo) pairs each */
 constexpr int TRACER_BLOCK = 64;
-/* layers tested for a density at a time */
-constexpr int EMPTY_BATCH = 13;
 
 /* The column system A x = r of the tracer (rows as k_tracers_solve's mixed
  * path) is solved for the increment delta = x - rho_old: A delta = r - A
@@ -75,21 +73,7 @@ __global__ void __launch_bounds__(TRACER_BLOCK) k_tracers_solve_df(VGrid vg, Ste
         /* a constituent absent from the column, old density and tendency 0 in
          * every layer (a cloud-free column's condensates): the system's
          * right-hand side is 0 and so is the new density, exactly */
-        const long long low = (long long)(nl - 1) * nc + i; /* tells most of the others */
-        bool empty = is_zero(ro[low]) && is_zero(tr[low]);
-#pragma unroll 1
-        for (int j0 = 0; j0 < nl && empty; j0 += EMPTY_BATCH) {
-            /* a batch of loads in flight per test */
-            unsigned long long any = 0;
-#pragma unroll
-            for (int d = 0; d < EMPTY_BATCH; ++d) {
-                if (j0 + d >= nl) continue;
-                const long long b = (long long)(j0 + d) * nc + i;
-                any |= (unsigned long long)(__double_as_longlong(ro[b]) | __double_as_longlong(tr[b]));
-            }
-            empty = (any << 1) == 0ULL;
-        }
-        if (empty) {
+        if (absent_from_column(ro, tr, nl, nc, i)) {
             double *rn = sn.rho + k * ns;
             float *rs = sh_rho + k * ns;
 #pragma unroll 1

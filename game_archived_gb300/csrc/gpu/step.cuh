@@ -187,7 +187,7 @@ static void launch_momentum(Context *c, const StepParams &p, const Views<R> &v, 
 /* implicit vertical sound waves (column_solvers.c:19-383) */
 template <bool EXACT>
 void launch_waves(Context *c, const StepParams &p, StateMirror *so, StateMirror *sn, StateMirror *st, int rk,
-                  const Shadow &sh)
+                  const Shadow &sh, const double *theta = nullptr)
 {
     const long long ns = c->ns;
     WavesWork ww = waves_work(c);
@@ -219,7 +219,7 @@ void launch_waves(Context *c, const StepParams &p, StateMirror *so, StateMirror 
     }
     {
         ProfScope ps(c, "k_waves_layer");
-        k_waves_layer<EXACT><<<nblocks(ns, 256), 256, 0, c->stream>>>(c->vg, p, so->ds, sn->ds, st->ds, ww, rk);
+        k_waves_layer<EXACT><<<nblocks(ns, 256), 256, 0, c->stream>>>(c->vg, p, so->ds, sn->ds, st->ds, ww, rk, theta);
     }
     {
         ProfScope ps(c, "k_waves_rows");
@@ -446,7 +446,7 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
             else
                 cudaEventRecord(c->ev_tend, c->stream);
         }
-        launch_waves<EXACT>(c, p, so, sn, st, rk, v.sh);
+        launch_waves<EXACT>(c, p, so, sn, st, rk, v.sh, EXACT ? c->theta : nullptr);
         if (rk == 0 && fork) {
             cudaEventRecord(c->ev_fork, c->stream);
             cudaStreamWaitEvent(c->stream2, c->ev_fork, 0);
