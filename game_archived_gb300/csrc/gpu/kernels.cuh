@@ -45,7 +45,7 @@ template <typename R, typename F>
 __device__ __forceinline__ R grad_v(const HGrid<R> &g, const F *f, int k, int c)
 {
     const long long i = (long long)k * g.nc + c;
-    return div_tab(R(f[i - g.nc]) - R(f[i]), g.nd_v, g.r_nd_v, i);
+    return div_tab(as<R>(f[i - g.nc]) - as<R>(f[i]), g.nd_v, g.r_nd_v, i);
 }
 
 /* slopes are exactly 0 away from orography; no FP64 comparison */
@@ -82,7 +82,7 @@ __device__ __forceinline__ R grad_h(const HGrid<R> &g, const F *f, int l, int e)
 {
     const int fr = g.from[e], to = g.to[e];
     const long long le = (long long)l * g.ne + e;
-    R out = div_tab(R(f[(long long)l * g.nc + to]) - R(f[(long long)l * g.nc + fr]), g.nd_h, g.r_nd_h, le);
+    R out = div_tab(as<R>(f[(long long)l * g.nc + to]) - as<R>(f[(long long)l * g.nc + fr]), g.nd_h, g.r_nd_h, le);
     if (l >= g.nl - g.n_oro) {
         /* a zero slope adds a zero */
         if (zero_slope(g.slope_h[le])) return out;
@@ -1028,7 +1028,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
     const R cur_hor = F ? R(p.cur_hor_f) : R(p.cur_hor), old_hor = F ? R(p.old_hor_f) : R(p.old_hor);
     R y = old_hor * pgo - cur_hor * P + pvt - halved(v2g);
     /* friction acceleration of the diffusion branch, when it is active */
-    if (fric_u) y = y + R(fric_u[i]);
+    if (fric_u) y = y + as<R>(fric_u[i]);
     /* the pressure gradient is recomputed in substage 0 only, where the new
      * weight is 1 */
     double t;
@@ -1119,7 +1119,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_mom
     R pgc = (R(0.5) * (d_up + d_lo)) * g.gravity_m_v[i];
     const R cur_ver = sizeof(R) == sizeof(float) ? R(p.cur_ver_f) : R(p.cur_ver);
     R y = -cur_ver * P + pvt - halved(v2g);
-    if (fric_w) y = y + R(fric_w[i]);
+    if (fric_w) y = y + as<R>(fric_w[i]);
     y = y + pgc;
     double t;
     if (PG) t = wide(y);

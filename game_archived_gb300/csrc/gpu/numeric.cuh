@@ -188,6 +188,13 @@ double to_double(double) = delete;
 float to_float(float) = delete;
 __device__ __forceinline__ double wide(float x) { return to_double(x); }
 __device__ __forceinline__ double wide(double x) { return x; }
+/* x in the horizontal precision R (to_float from double to float) */
+template <typename R, typename F>
+__device__ __forceinline__ R as(F x)
+{
+    if constexpr (sizeof(R) == sizeof(float) && sizeof(F) == sizeof(double)) return to_float(x);
+    else return x;
+}
 
 }  // namespace
 }  // namespace game
