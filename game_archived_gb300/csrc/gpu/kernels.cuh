@@ -846,8 +846,10 @@ __device__ __forceinline__ void pgrad_v_parts(const HGrid<R> &g, const StepParam
  * expressions of pgrad_h_parts / pgrad_v_parts, so that the first
  * substage's gradients gather two float4 per edge (or interface) instead of
  * some twenty scalars.  Read from the FP32 shadow of state_new, which the
- * first substage's pressure gradient reads. */
-__global__ void k_pg_cells(HGrid<float> g, StepParams p, SView<float> s, float4 *pc, Present present)
+ * first substage's pressure gradient reads.  Also the first substage's
+ * theta_v (k_theta) and the flags of the constituents each layer holds. */
+__global__ void k_pg_cells(HGrid<float> g, StepParams p, SView<float> s, float4 *pc, float *theta,
+                           Present present)
 {
     const LayerPoint pt = layer_point(g.nc);
     const long long ns = (long long)g.nl * g.nc, i = pt.i;
@@ -857,6 +859,7 @@ __global__ void k_pg_cells(HGrid<float> g, StepParams p, SView<float> s, float4 
         const float tp = s.theta_v_pert[i];
         pc[i] = make_float4(s.exner_pert[i], cdp * (g.theta_v_bg[i] + tp), cdp * tp,
                             s.rho[p.n_cond * ns + i] / density_total_r(s.rho, p.n_const, ns, i));
+        theta[i] = s.rhotheta_v[i] / s.rho[p.n_cond * ns + i];
         for (int k = 0; k < p.n_const; ++k) held |= (s.rho[k * ns + i] != 0.f) << k;
     }
     if (p.n_const == 1) return;

@@ -403,7 +403,10 @@ __global__ void __launch_bounds__(WAVES_BLOCK) k_waves_thomas_df(int nc, WavesWo
     }
 }
 
-__global__ void k_waves_apply_df(VGrid vg, StepParams p, DState so, DState sn, WavesWork ww, DfGrid dg, Shadow sh)
+/* theta: the next substage's theta_v from the shadow's rho theta_v and rho
+ * (k_theta's quotient) */
+__global__ void k_waves_apply_df(VGrid vg, StepParams p, DState so, DState sn, WavesWork ww, DfGrid dg, Shadow sh,
+                                 float *theta)
 {
     const int nc = vg.nc, nl = vg.nl;
     const long long ns = (long long)nl * nc;
@@ -438,8 +441,10 @@ __global__ void k_waves_apply_df(VGrid vg, StepParams p, DState so, DState sn, W
     sn.theta_v_pert[b] = df_to_double(tp_new);
     sn.exner_pert[b] = ep_new;
     if (sh.rho) {
-        sh.rho[gp + b] = to_float(r_new);
-        sh.rhotheta_v[b] = to_float(rt_new);
+        const float r32 = to_float(r_new), rt32 = to_float(rt_new);
+        sh.rho[gp + b] = r32;
+        sh.rhotheta_v[b] = rt32;
+        if (theta) theta[b] = rt32 / r32;
         sh.theta_v_pert[b] = tp_new.hi;
         sh.exner_pert[b] = to_float(ep_new);
     }

@@ -211,7 +211,8 @@ void launch_waves(Context *c, const StepParams &p, StateMirror *so, StateMirror 
             }
             {
                 ProfScope ps(c, "k_waves_apply");
-                k_waves_apply_df<<<nblocks(ns, 256), 256, 0, c->stream>>>(c->vg, p, so->ds, sn->ds, ww, c->dfg, sh);
+                k_waves_apply_df<<<nblocks(ns, 256), 256, 0, c->stream>>>(c->vg, p, so->ds, sn->ds, ww, c->dfg, sh,
+                                                                          rk == 0 ? c->theta32 : nullptr);
             }
             c->kernel_launches += 4;
             return;
@@ -332,7 +333,8 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
             k_pg_cells64<<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(g, p, v.sv, c->pg_cell64, c->grad_pi_v,
                                                                                  c->theta);
         else
-            k_pg_cells<<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(c->hg32, p, v.sv, c->pg_cell, c->present);
+            k_pg_cells<<<layer_grid(c->nl, c->nc, bs), bs, 0, c->stream>>>(c->hg32, p, v.sv, c->pg_cell, c->theta32,
+                                                                             c->present);
         c->kernel_launches++;
     }
     {
@@ -404,10 +406,14 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
         /* diffusion branch: temperature and mass diffusion */
         if (rk == 0 && (p.diff & DIFF_RAD_HS)) launch_held_suarez_radiation(c, so->ds);
         if (rk == 0 && p.diff) launch_diffusion_scalar(c, p, v.sv);
-        if constexpr (!EXACT) {
-            ProfScope ps(c, "k_theta");
-            k_theta<R><<<nblocks(ns, bs), bs, 0, c->stream>>>(c->nl, c->nc, c->n_cond, v.sv, theta);
-        }
+        /* theta_v: at rk 0 from k_pg_cells, at rk 1 from k_waves_apply_df or,
+         * without the double-float solve, here */
+        if constexpr (!EXACT)
+            if (rk == 1 && !(p.dfloat && column_mode(c, EXACT, c->nc) == COLUMN_REGISTERS)) {
+                ProfScope ps(c, "k_theta");
+                k_theta<R><<<nblocks(ns, bs), bs, 0, c->stream>>>(c->nl, c->nc, c->n_cond, v.sv, theta);
+                c->kernel_launches++;
+            }
         {
             ProfScope ps(c, "k_scalar_tend");
             IrrTerms irr{};
@@ -433,7 +439,7 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
                 }
             }
         }
-        c->kernel_launches += EXACT ? 0 : 2; /* launch_scalar_tend64 counts its own */
+        c->kernel_launches += EXACT ? 0 : 1; /* launch_scalar_tend64 counts its own */
         /* the tendency is final from here on: a host-in/host-out call copies
          * it out while the solvers run */
         if (rk == 1) {
