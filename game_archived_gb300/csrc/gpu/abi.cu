@@ -1503,7 +1503,7 @@ int inner_product_tangential(double *in_field_0, double *in_field_1, double *out
     double *a = c->dev_tmp[1], *b = c->dev_tmp[2], *o = c->dev_tmp[0];
     if (upload_field(in_field_0, a, c->map_vec, c->nv, c->nv)) return -1;
     if (upload_field(in_field_1, b, c->map_vec, c->nv, c->nv)) return -1;
-    op_inner_product_tangential(c, a, b, o);
+    op_inner_product_tangential(c, a, b, c->dev_tmp[3], o);
     if (download_field(out_field, o, c->map_s, c->ns, c->ns, 0, c->ns)) return -1;
     return finish();
 }

@@ -23,7 +23,7 @@ __global__ void k_op_grad_h(G g, const double *f, double *u, int with_correction
         u[i] = grad_h(g, f, l, e);
     } else {
         const int fr = g.from[e], to = g.to[e];
-        u[i] = (f[(long long)l * g.nc + to] - f[(long long)l * g.nc + fr]) / g.nd_h[i];
+        u[i] = div_tab(f[(long long)l * g.nc + to] - f[(long long)l * g.nc + fr], g.nd_h, g.r_nd_h, i);
     }
 }
 
@@ -122,7 +122,7 @@ __global__ void k_op_divv(G g, const double *in_u, const double *density, const 
             comp_v = d_up * up * g.area_v[(long long)l * nc + c] - d_lo * lo * g.area_v[(long long)(l + 1) * nc + c];
         }
     }
-    out[i] = 1.0 / g.volume[i] * (comp_h + comp_v);
+    out[i] = g.r_volume[i] * (comp_h + comp_v);
 }
 
 /* inner_product (inner_product.c:13-43) */
@@ -153,7 +153,8 @@ __global__ void k_op_rel_vort(G g, const double *u, const double *w, const doubl
         const int tf = g.dual_from[e], tt = g.dual_to[e];
         const long long kt = (long long)k * g.nt;
         const double af = g.dual_area_t[kt + tf], at = g.dual_area_t[kt + tt];
-        zv[(long long)k * g.ne + e] = (af * tri[kt + tf] + at * tri[kt + tt]) / (af + at);
+        zv[(long long)k * g.ne + e] = div_tab(af * tri[kt + tf] + at * tri[kt + tt], g.rhombus_area, g.r_rhombus_area,
+                                                 (long long)k * g.ne + e);
     }
 }
 
@@ -282,7 +283,7 @@ __global__ void k_op_add_vertical_divv(G g, const double *w, double *out)
     const double contra_upper = l == 0 ? 0.0 : w[up];
     const double contra_lower = l == g.nl - 1 ? 0.0 : w[lo];
     const double comp_v = contra_upper * g.area_v[up] - contra_lower * g.area_v[lo];
-    out[i] += 1 / g.volume[i] * comp_v;
+    out[i] += g.r_volume[i] * comp_v;
 }
 
 }  // namespace

@@ -82,7 +82,7 @@ void op_uv_at_edge(Context *c, const double *u, double *ue, double *ve);
 void op_edges_to_cells(Context *c, const double *ue, double *out);
 void op_curl_to_cells(Context *c, const double *zv, double *out);
 void op_edges_to_cells_lowest(Context *c, const double *ue, double *out);
-void op_inner_product_tangential(Context *c, const double *a, const double *b, double *out);
+void op_inner_product_tangential(Context *c, const double *a, const double *b, double *bt, double *out);
 int op_epv(Context *c, const double *pot_vort, DState s, double *epv);
 
 /* scatter of [k][Nc] device-order slices to reference order [k][Nc] and of

@@ -13,10 +13,11 @@
  *                     interval, turned to u/v, extrapolated to 10 m
  *   k_out_wind10_c    per column: 10 m wind at the cell, gusts
  *   divv_h, calc_rel_vort, calc_pot_vort (the step's operator kernels)
- *   k_curl_to_cells, k_uv_at_edge, k_edges_to_cells   model-layer winds and
+ *   k_curl_to_cells, k_tangential, k_edges_to_cells   model-layer winds and
  *                     vorticity at the cells
- *   k_epv_theta, grad, k_epv_pv, k_inner_tangential, k_epv_round   EPV
- *   k_out_plevels     per column: the six pressure levels
+ *   k_epv_theta, grad, k_epv_pv, k_tangential, k_inner_tangential,
+ *   k_epv_round       EPV
+ *   k_out_plevels     per column and level: the pressure levels
  * and k_latlon for the lat-lon interpolation of any set of [Nc] fields.
  */
 #include <algorithm>
@@ -101,6 +102,49 @@ __device__ __forceinline__ double tangential(const G &g, const double *u_layer, 
     double r = 0;
     for (int k = 0; k < 10; ++k) r += g.trsk_w[(long long)k * g.ne + e] * u_layer[g.trsk_i[(long long)k * g.ne + e]];
     return r;
+}
+
+/* layers per thread of k_tangential */
+constexpr int TAN_LAYERS = 7;
+
+/* the same of all layers u [L][Ne]; with TURN the two components turned to u
+ * and v at the edge (calc_uv_at_edge, averaging.c:152-174).  FP64 issue bounds it (20
+ * for the sum): a thread takes TAN_LAYERS layers of an edge, so that the
+ * edge's ten weights and neighbours are loaded and the sine and cosine of its
+ * direction are formed once for all of them (RES_ID 6, with the averages to the
+ * cells: 471 -> 288 us; epv_diagnostics, which sums it once per edge instead of
+ * twice, 817 -> 662 us). */
+template <bool TURN>
+__global__ void __launch_bounds__(128) k_tangential(G g, const double *direction, const double *u, double *out,
+                                                    double *out_v)
+{
+    const int e = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (e >= g.ne) return;
+    const int l0 = blockIdx.y * TAN_LAYERS, l1 = min(l0 + TAN_LAYERS, g.nl);
+    double w[10], co = 0, si = 0;
+    int id[10];
+#pragma unroll
+    for (int k = 0; k < 10; ++k) {
+        w[k] = g.trsk_w[(long long)k * g.ne + e];
+        id[k] = g.trsk_i[(long long)k * g.ne + e];
+    }
+    if (TURN) {
+        co = cos(direction[e]);
+        si = sin(direction[e]);
+    }
+    for (int l = l0; l < l1; ++l) {
+        const double *ul = u + (long long)l * g.ne;
+        double r = 0;
+#pragma unroll
+        for (int k = 0; k < 10; ++k) r += w[k] * ul[id[k]];
+        const long long i = (long long)l * g.ne + e;
+        if (TURN) {
+            out[i] = co * ul[e] - si * r;
+            out_v[i] = si * ul[e] + co * r;
+        } else {
+            out[i] = r;
+        }
+    }
 }
 
 /* per grid box: temperature, pressure, relative humidity in percent
@@ -334,17 +378,6 @@ __global__ void k_edges_to_cells_lowest(G g, const double *ue, double *out)
     out[i] = r;
 }
 
-/* calc_uv_at_edge (averaging.c:152-174) of the horizontal wind u [L][Ne] */
-__global__ void k_uv_at_edge(G g, OutGrid og, const double *u, double *ue, double *ve)
-{
-    const long long n = (long long)g.nl * g.ne, i = gtid();
-    if (i >= n) return;
-    const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
-    const double w0 = u[i];
-    const double w1 = tangential(g, u + (long long)l * g.ne, e);
-    passive_turn(w0, w1, -og.direction[e], &ue[i], &ve[i]);
-}
-
 /* theta_v' with the background added in the top layer only, the field whose
  * gradient epv_diagnostics takes (spatial_ops_for_output.c:113-118) */
 __global__ void k_epv_theta(VGrid vg, DState s, double *f)
@@ -379,11 +412,10 @@ __global__ void k_epv_pv(G g, VGrid vg, const double *pzh, const double *pzv, do
         const long long a = (long long)l * nc, b = (long long)(l + 1) * nc;
         const double zi = g.z_h[ih];
         const double lt = 0.5 * (zv[a + f] + zv[a + t]) - 0.5 * (zv[b + f] + zv[b + t]);
-        double upper, lower;
-        if (l == 0) upper = (0.5 * (zv[a + f] + zv[a + t]) - zi) / lt;
-        else upper = 0.5 * (g.z_h[ih - ne] - zi) / lt;
-        if (l == nl - 1) lower = (zi - 0.5 * (zv[b + f] + zv[b + t])) / lt;
-        else lower = 0.5 * (zi - g.z_h[ih + ne]) / lt;
+        const double r_lt = rcp_nr<2>(lt); /* for both quotients */
+        const double du = l == 0 ? 0.5 * (zv[a + f] + zv[a + t]) - zi : 0.5 * (g.z_h[ih - ne] - zi);
+        const double dl = l == nl - 1 ? zi - 0.5 * (zv[b + f] + zv[b + t]) : 0.5 * (zi - g.z_h[ih + ne]);
+        const double upper = div_rcp(du, lt, r_lt), lower = div_rcp(dl, lt, r_lt);
         out[i] = upper * pzh[(long long)l * ne + e] + lower * pzh[(long long)(l + 1) * ne + e];
     } else {
         const int k = row_of(i, nc), c = (int)(i - (long long)k * nc);
@@ -404,19 +436,19 @@ __global__ void k_epv_pv(G g, VGrid vg, const double *pzh, const double *pzv, do
 
 /* inner_product_tangential (spatial_ops_for_output.c:137-166): a given in
  * tangential components, all six edge slots (weight 0 in a pentagon's
- * sixth) */
-__global__ void k_inner_tangential(G g, const double *aw, const double *au, const double *bw, const double *bu,
+ * sixth); bt: the tangential components of b (k_tangential, once per edge
+ * instead of by each of its two cells) */
+__global__ void k_inner_tangential(G g, const double *aw, const double *au, const double *bw, const double *bt,
                                    double *out)
 {
     const long long ns = (long long)g.nl * g.nc, i = gtid();
     if (i >= ns) return;
     const int l = row_of(i, g.nc), c = (int)(i - (long long)l * g.nc);
-    const double *bl = bu + (long long)l * g.ne, *al = au + (long long)l * g.ne;
+    const double *bl = bt + (long long)l * g.ne, *al = au + (long long)l * g.ne;
     double r = 0;
     for (int j = 0; j < 6; ++j) {
         const int a = g.adj[(long long)j * g.nc + c];
-        const double tw = tangential(g, bl, a);
-        r += ipw_at(g, j, l, c) * al[a] * tw;
+        r += ipw_at(g, j, l, c) * al[a] * bl[a];
     }
     r += ipw_at(g, 6, l, c) * aw[i] * bw[i];
     r += ipw_at(g, 7, l, c) * aw[i + g.nc] * bw[i + g.nc];
@@ -432,16 +464,44 @@ struct PlIn {
 
 /* per column: vertical interpolation to the six pressure levels in ln p
  * between the layer nearest to the level and its neighbour, 9999 below the
- * lowest layer (write_output.c:766-825); out [6][Nc] */
+ * lowest layer (write_output.c:766-825); out [6][Nc].
+ *
+ * The nearest layer is the first minimum of |ln(level / p)|.  FP64 issue
+ * bounds the search (a division and a logarithm per layer and level), so the
+ * distances are first taken in FP32: where the least is ahead of every other
+ * layer's by more than the FP32 error (NEAR, a hundred times the rounding of
+ * logarithms up to 69), that layer is the FP64 minimum too and only its FP64
+ * distance is formed.  Elsewhere, and where a pressure is not a positive
+ * number of FP32's middle range, the level is searched in FP64.  A thread per
+ * level and column: the search is a chain of loads (RES_ID 6: 721 -> 168 us;
+ * 229 us with the six levels in one thread). */
 __global__ void k_out_plevels(int nc, int nl, PlIn in, PlOut o)
 {
-    const int i = (int)gtid();
-    if (i >= nc) return;
+    constexpr float NEAR = 1e-3f;
     const double levels[N_PRESSURE_LEVELS] = {20000, 30000, 50000, 70000, 85000, 92500};
-    for (int j = 0; j < N_PRESSURE_LEVELS; ++j) {
-        const double pl = levels[j];
-        int closest = 0;
-        double best = fabs(log(pl / in.p[i]));
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x), j = (int)blockIdx.y;
+    if (i >= nc) return;
+    const double pl = levels[j];
+    const float ln_level = logf((float)pl);
+    float d1 = INFINITY, d2 = INFINITY; /* least and second least distance */
+    int closest = 0;
+    bool fp32 = true;
+    for (int k = 0; k < nl; ++k) {
+        const float p = to_float(in.p[(long long)k * nc + i]);
+        fp32 = fp32 && p > 1e-30f && p < 1e30f;
+        const float d = fabsf(ln_level - logf(p));
+        if (d < d1) {
+            d2 = d1;
+            d1 = d;
+            closest = k;
+        } else {
+            d2 = fminf(d2, d);
+        }
+    }
+    const bool decided = fp32 && d2 - d1 > NEAR;
+    if (!decided) closest = 0;
+    double best = fabs(log(pl / in.p[(long long)closest * nc + i]));
+    if (!decided) {
         for (int k = 1; k < nl; ++k) {
             const double d = fabs(log(pl / in.p[(long long)k * nc + i]));
             if (d < best) {
@@ -449,22 +509,22 @@ __global__ void k_out_plevels(int nc, int nl, PlIn in, PlOut o)
                 closest = k;
             }
         }
-        int second = closest + 1;
-        if (pl < in.p[(long long)closest * nc + i]) second = closest - 1;
-        const long long oi = (long long)j * nc + i;
-        if ((closest == nl - 1 && second == nl) || second < 0) {
-            o.gh[oi] = o.t[oi] = o.rh[oi] = o.epv[oi] = o.relv[oi] = o.u[oi] = o.v[oi] = 9999;
-        } else {
-            const long long a = (long long)closest * nc + i, b = (long long)second * nc + i;
-            const double w = 1 - best / (fabs(log(in.p[a] / in.p[b])) + EPS_SEC);
-            o.gh[oi] = (w * in.gpot[a] + (1 - w) * in.gpot[b]) / G_MEAN_SFC_ABS;
-            o.t[oi] = w * in.t[a] + (1 - w) * in.t[b];
-            o.rh[oi] = w * in.rh[a] + (1 - w) * in.rh[b];
-            o.epv[oi] = w * in.epv[a] + (1 - w) * in.epv[b];
-            o.relv[oi] = w * in.relv[a] + (1 - w) * in.relv[b];
-            o.u[oi] = w * in.u[a] + (1 - w) * in.u[b];
-            o.v[oi] = w * in.v[a] + (1 - w) * in.v[b];
-        }
+    }
+    int second = closest + 1;
+    if (pl < in.p[(long long)closest * nc + i]) second = closest - 1;
+    const long long oi = (long long)j * nc + i;
+    if ((closest == nl - 1 && second == nl) || second < 0) {
+        o.gh[oi] = o.t[oi] = o.rh[oi] = o.epv[oi] = o.relv[oi] = o.u[oi] = o.v[oi] = 9999;
+    } else {
+        const long long a = (long long)closest * nc + i, b = (long long)second * nc + i;
+        const double w = 1 - best / (fabs(log(in.p[a] / in.p[b])) + EPS_SEC), w1 = 1 - w;
+        o.gh[oi] = (w * in.gpot[a] + w1 * in.gpot[b]) / G_MEAN_SFC_ABS;
+        o.t[oi] = w * in.t[a] + w1 * in.t[b];
+        o.rh[oi] = w * in.rh[a] + w1 * in.rh[b];
+        o.epv[oi] = w * in.epv[a] + w1 * in.epv[b];
+        o.relv[oi] = w * in.relv[a] + w1 * in.relv[b];
+        o.u[oi] = w * in.u[a] + w1 * in.u[b];
+        o.v[oi] = w * in.v[a] + w1 * in.v[b];
     }
 }
 
@@ -567,9 +627,14 @@ static OutBufs *ensure_obuf(Context *c)
 }
 
 /* ----------------------------------------------------------- operators */
+static dim3 tangential_grid(const Context *c)
+{
+    return dim3(nb(c->ne, 128), (unsigned)((c->nl + TAN_LAYERS - 1) / TAN_LAYERS));
+}
+
 void op_uv_at_edge(Context *c, const double *u, double *ue, double *ve)
 {
-    k_uv_at_edge<<<nb((long long)c->nl * c->ne), 256, 0, c->stream>>>(c->hg64, c->og, u, ue, ve);
+    k_tangential<true><<<tangential_grid(c), 128, 0, c->stream>>>(c->hg64, c->og.direction, u, ue, ve);
     c->kernel_launches++;
 }
 
@@ -591,11 +656,13 @@ void op_edges_to_cells_lowest(Context *c, const double *ue, double *out)
     c->kernel_launches++;
 }
 
-void op_inner_product_tangential(Context *c, const double *a, const double *b, double *out)
+/* bt: scratch [L][Ne] */
+void op_inner_product_tangential(Context *c, const double *a, const double *b, double *bt, double *out)
 {
     const long long off = (long long)(c->nl + 1) * c->nc;
-    k_inner_tangential<<<nb(c->ns), 256, 0, c->stream>>>(c->hg64, a, a + off, b, b + off, out);
-    c->kernel_launches++;
+    k_tangential<false><<<tangential_grid(c), 128, 0, c->stream>>>(c->hg64, nullptr, b + off, bt, nullptr);
+    k_inner_tangential<<<nb(c->ns), 256, 0, c->stream>>>(c->hg64, a, a + off, b, bt, out);
+    c->kernel_launches += 2;
 }
 
 int op_epv(Context *c, const double *pot_vort, DState s, double *epv)
@@ -609,7 +676,7 @@ int op_epv(Context *c, const double *pot_vort, DState s, double *epv)
      * the reference's calloc'd work array */
     CK(cudaMemsetAsync(b->grad, 0, (size_t)c->nv * sizeof(double), c->stream));
     op_grad(c, b->theta, b->grad, OP_GRAD_H | OP_GRAD_V | OP_GRAD_CON);
-    op_inner_product_tangential(c, b->pvmod, b->grad, epv);
+    op_inner_product_tangential(c, b->pvmod, b->grad, b->ue, epv);
     k_epv_round<<<nb(c->nc, 128), 128, 0, c->stream>>>(c->vg, s, b->theta);
     c->kernel_launches += 3;
     CK(cudaGetLastError());
@@ -667,7 +734,7 @@ int output_fields(Context *c, StateMirror *sm, const OutParams &p, const OutInpu
     PlOut po{f.geopotential_height, f.t_pl, f.rh_pl, f.epv_pl, f.u_pl, f.v_pl, f.rel_vort_pl};
     {
         ProfScope ps(c, "out_plevels");
-        k_out_plevels<<<nb(c->nc, 128), 128, 0, st>>>(c->nc, c->nl, pi, po);
+        k_out_plevels<<<dim3(nb(c->nc, 128), N_PRESSURE_LEVELS), 128, 0, st>>>(c->nc, c->nl, pi, po);
     }
     c->kernel_launches++;
     CK(cudaGetLastError());
