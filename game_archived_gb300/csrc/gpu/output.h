@@ -4,6 +4,8 @@
  * averaging.c:135-234) */
 #pragma once
 
+#include <functional>
+
 #include "context.h"
 #include "game_gb300.h"
 
@@ -41,8 +43,12 @@ struct OutInputs {
 };
 
 /* computes every field of f from the state mirror s; rounds the top layer
- * of s's theta_v_pert as (x + bg) - bg, as write_out does */
-int output_fields(Context *c, StateMirror *s, const OutParams &p, const OutInputs &in, const OutFields &f);
+ * of s's theta_v_pert as (x + bg) - bg, as write_out does.  done(k) is called
+ * after the launches of stage k, whose fields are then computed: 0 the surface,
+ * temperature, pressure and humidity, 1 the winds, vorticity and divergence,
+ * 2 the rest */
+int output_fields(Context *c, StateMirror *s, const OutParams &p, const OutInputs &in, const OutFields &f,
+                  const std::function<int(int)> &done);
 
 /* host inputs of one output pass, reference order (NULL where not needed) */
 struct OutHost {
