@@ -1207,8 +1207,9 @@ struct IrrTerms {
     const double *heating_diss, *temp_diff_heating, *radiation, *mass_diff;
 };
 
-/* The mixed path's tendencies at (cell, layer) of the columns without a sloping
- * edge (all of them on a flat grid), where the terrain corrections vanish.
+/* The mixed path's tendencies at (cell, layer) where the terrain corrections
+ * vanish: in the columns without a sloping edge (all of them on a flat grid)
+ * and above the terrain-following layers.
  * Edge fluxes are FP32 products, their divergences double-word FP32 sums
  * (FluxSum), the tendencies FP64.  The cell's edges, neighbours, orientation,
  * wind and face areas are loaded once for all constituents.
@@ -1220,18 +1221,14 @@ struct IrrTerms {
  * arithmetic; sums with exact zeros are left out, the rk 1 mean takes one
  * addition.  RES_ID 6 moist, cloud-free: 141 -> 85 us per launch. */
 template <bool IRR>
-__global__ void __launch_bounds__(128) k_scalar_tend32(HGrid<float> g, StepParams p, SView<float> sv, DState st,
-                                                       const float *theta, const float *cp_ice, const float *cp_water,
-                                                       const double *pt_rates, const double *pt_heat,
-                                                       const double *sed_heat, const double *inv_vol_tab,
-                                                       Present present, int rk, IrrTerms irr)
+__device__ __forceinline__ void scalar_tend_flat(const HGrid<float> &g, const StepParams &p, const SView<float> &sv,
+                                                 const DState &st, const float *theta, const float *cp_ice,
+                                                 const float *cp_water, const double *pt_rates, const double *pt_heat,
+                                                 const double *sed_heat, const double *inv_vol_tab,
+                                                 const Present &present, int rk, const IrrTerms &irr, int l, int c)
 {
     const long long ns = (long long)g.nl * g.nc;
-    const LayerPoint pt_ = layer_point(g.nc);
-    if (!pt_.in) return;
-    const long long i = pt_.i;
-    const int nl = g.nl, l = pt_.l, c = pt_.x;
-    if (g.tilt[c]) return; /* k_scalar_tend_tilt */
+    const long long i = (long long)l * g.nc + c;
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
     const int cond = p.n_cond;
@@ -1333,22 +1330,19 @@ __global__ void __launch_bounds__(128) k_scalar_tend32(HGrid<float> g, StepParam
     }
 }
 
-/* the same in the columns with a sloping edge (tilt_cells), with the terrain
- * corrections: the cell's edges are streamed one layer at a time, every
- * accumulator in the reference's order (layer l-1 before l, edges j = 0..5) */
+/* the same in the terrain-following layers of the columns with a sloping edge,
+ * with the terrain corrections: the cell's edges are streamed one layer at a
+ * time, every accumulator in the reference's order (layer l-1 before l, edges
+ * j = 0..5) */
 template <bool IRR>
-__global__ void __launch_bounds__(128) k_scalar_tend_tilt(HGrid<float> g, StepParams p, SView<float> sv,
-                                                          DState st, const float *theta, const float *cp_ice,
-                                                          const float *cp_water,
-                                                      const double *pt_rates, const double *pt_heat,
-                                                      const double *sed_heat, const double *inv_vol_tab, int rk,
-                                                      IrrTerms irr, const int *tilt_cells, int n_tilt)
+__device__ __forceinline__ void scalar_tend_tilt(const HGrid<float> &g, const StepParams &p, const SView<float> &sv,
+                                                 const DState &st, const float *theta, const float *cp_ice,
+                                                 const float *cp_water, const double *pt_rates, const double *pt_heat,
+                                                 const double *sed_heat, const double *inv_vol_tab, int rk,
+                                                 const IrrTerms &irr, int l, int c)
 {
     const long long ns = (long long)g.nl * g.nc;
-    const LayerPoint pt_ = layer_point(n_tilt);
-    if (!pt_.in) return;
     const int nl = g.nl, n_oro = g.n_oro;
-    const int l = pt_.l, c = tilt_cells[pt_.x];
     const long long i = (long long)l * g.nc + c;
     const long long nc = g.nc, ne = g.ne;
     const int n_edges = c < N_PENT ? 5 : 6;
@@ -1498,6 +1492,36 @@ __global__ void __launch_bounds__(128) k_scalar_tend_tilt(HGrid<float> g, StepPa
             y = y + pt_rates[pt + i];
         }
         st.rho[k * ns + i] = rk == 0 ? y : half_of(st.rho[k * ns + i] + y);
+    }
+}
+
+/* One launch for both: the first tilt_blocks blocks of a layer take the columns
+ * of tilt_cells, the others every cell and leave those out.  Two launches one
+ * after the other each wait for the latency of their gathers on a small grid
+ * (with the mountain and all constituents, RES_ID 4: 38 -> 28 us, RES_ID 7 628
+ * us either way); the tilted columns take the shorter way above the
+ * terrain-following layers.  64 registers (eight blocks per SM; 72 without the
+ * bound: 657 us at RES_ID 7) and no corrections compiled in for a flat grid
+ * (TILT = false; RES_ID 6, cloud-free: 96 -> 85 us). */
+template <bool IRR, bool TILT>
+__global__ void __launch_bounds__(128, 8) k_scalar_tend32(HGrid<float> g, StepParams p, SView<float> sv, DState st,
+                                                       const float *theta, const float *cp_ice, const float *cp_water,
+                                                       const double *pt_rates, const double *pt_heat,
+                                                       const double *sed_heat, const double *inv_vol_tab,
+                                                       Present present, int rk, IrrTerms irr, const int *tilt_cells,
+                                                       int n_tilt, int tilt_blocks)
+{
+    const int l = (int)blockIdx.y, b = (int)blockIdx.x, top = g.nl - g.n_oro - 1;
+    if (TILT && b < tilt_blocks) {
+        const int x = b * (int)blockDim.x + (int)threadIdx.x;
+        if (l < top || x >= n_tilt) return;
+        scalar_tend_tilt<IRR>(g, p, sv, st, theta, cp_ice, cp_water, pt_rates, pt_heat, sed_heat, inv_vol_tab, rk, irr, l,
+                              tilt_cells[x]);
+    } else {
+        const int c = (b - (TILT ? tilt_blocks : 0)) * (int)blockDim.x + (int)threadIdx.x;
+        if (c >= g.nc || (TILT && l >= top && g.tilt[c])) return;
+        scalar_tend_flat<IRR>(g, p, sv, st, theta, cp_ice, cp_water, pt_rates, pt_heat, sed_heat, inv_vol_tab, present, rk,
+                              irr, l, c);
     }
 }
 

@@ -422,21 +422,16 @@ void launch_step(Context *c, const StepParams &p, StateMirror *so, StateMirror *
                 launch_scalar_tend64(c, p, v.sv, st->ds.rho, st->ds.rho, st->ds.rhotheta_v, theta, cpi, cpw, c->pt_rates,
                                      c->pt_heat, c->sed_heat, rk, irr);
             } else {
-                auto flat = [&](auto kernel) {
-                    kernel<<<layer_grid(c->nl, c->nc, 128), 128, 0, c->stream>>>(
+                const int tilt_blocks = (int)nblocks(c->n_tilt, 128);
+                auto tend = [&](auto kernel) {
+                    kernel<<<dim3(tilt_blocks + nblocks(c->nc, 128), (unsigned)c->nl), 128, 0, c->stream>>>(
                         g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, c->present,
-                        rk, irr);
+                        rk, irr, c->tilt_cells, c->n_tilt, tilt_blocks);
                 };
-                auto tilt = [&](auto kernel) {
-                    kernel<<<layer_grid(c->nl, c->n_tilt, 128), 128, 0, c->stream>>>(
-                        g, p, v.sv, st->ds, theta, cpi, cpw, c->pt_rates, c->pt_heat, c->sed_heat, c->inv_vol, rk, irr,
-                        c->tilt_cells, c->n_tilt);
-                };
-                p.irr ? flat(k_scalar_tend32<true>) : flat(k_scalar_tend32<false>);
-                if (c->n_tilt) {
-                    p.irr ? tilt(k_scalar_tend_tilt<true>) : tilt(k_scalar_tend_tilt<false>);
-                    c->kernel_launches++;
-                }
+                if (c->n_tilt)
+                    p.irr ? tend(k_scalar_tend32<true, true>) : tend(k_scalar_tend32<false, true>);
+                else
+                    p.irr ? tend(k_scalar_tend32<true, false>) : tend(k_scalar_tend32<false, false>);
             }
         }
         c->kernel_launches += EXACT ? 0 : 1; /* launch_scalar_tend64 counts its own */
