@@ -444,9 +444,9 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
     const long long q = gtid();
     const int n_tr = p.n_const - 1;
     if (q >= (long long)n_tr * nc) return;
-    /* FP64 path: the last slot (the vapour, in every column of a moist run)
-     * first, the columns without condensates fill in behind its solves */
-    const int row = (int)(q / nc), slot = EXACT ? n_tr - 1 - row : row, i = (int)(q - (long long)row * nc);
+    /* the last slot (the vapour, in every column of a moist run) first, the
+     * columns without condensates fill in behind its solves */
+    const int row = (int)(q / nc), slot = n_tr - 1 - row, i = (int)(q - (long long)row * nc);
     const int k = slot < p.n_cond ? slot : slot + 1; /* skip the main gas */
     bool has_sink;
     const double vsink = sink_velocity(p, k, has_sink);
@@ -454,45 +454,60 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
     const double *ro = so.rho + k * ns;
     const double *tr = st.rho + k * ns;
     const long long bot = i + ns - nc;
-    if (EXACT) {
-        /* a constituent absent from the column, old density and tendency 0 in
-         * every layer: so is the solution.  With the volumes' reciprocals
-         * and one division per row: RES_ID 6, cloud-free, 1088 -> 103 us;
-         * RES_ID 5 with clouds everywhere 221 -> 120 us */
-        if (absent_from_column(ro, tr, nl, nc, i)) {
-            double *rn = sn.rho + k * ns;
+    /* a constituent absent from the column, old density and tendency 0 in
+     * every layer: so is the solution.  FP64, with the volumes' reciprocals
+     * and one division per row: RES_ID 6, cloud-free, 1088 -> 103 us;
+     * RES_ID 5 with clouds everywhere 221 -> 120 us.  Mixed, 80 layers,
+     * RES_ID 4, cloud-free, with the rows' inputs loaded a row ahead and blocks
+     * of one warp: 189 -> 121 us */
+    if (absent_from_column(ro, tr, nl, nc, i)) {
+        double *rn = sn.rho + k * ns;
+        float *rs = sh_rho ? sh_rho + k * ns : nullptr;
 #pragma unroll 1
-            for (int j = 0; j < nl; ++j) rn[i + (long long)j * nc] = 0.0;
-            return;
+        for (int j = 0; j < nl; ++j) {
+            rn[i + (long long)j * nc] = 0.0;
+            if (rs) rs[i + (long long)j * nc] = 0.f;
         }
+        return;
     }
     const double a_sfc = vg.area_v[(long long)nl * nc + i];
     double ep[NL > 0 ? NL : CAP], rp[NL > 0 ? NL : CAP];
     /* FP64 path: iw dt / V of the layer, shared by its flux terms */
     double gq = EXACT ? div_rcp(iw * dt, vg.volume[i], vg.r_volume[i]) : 0.0;
     double fi_prev = 0.0, fr_prev = 0.0, c_prev = 0.0;
+    /* what row j reads; where the layer count is a run-time one, a row ahead of
+     * its use (with a compile-time one the compiler places the loads) */
+    struct Row {
+        double ro, ro_lo, tr, wo, wn, ar, iv;
+    };
+    auto load = [&](int j) {
+        const long long b = i + (long long)j * nc;
+        return Row{ro[b], j < nl - 1 ? ro[b + nc] : 0.0, tr[b], so.w[b + nc], sn.w[b + nc], vg.area_v[b + nc],
+                   EXACT ? 0.0 : tw.inv_vol[b]};
+    };
+    Row next = load(0);
 #pragma unroll
     for (int j = 0; j < nl; ++j) {
+        const Row in = NL > 0 ? load(j) : next;
+        if (NL == 0 && j < nl - 1) next = load(j + 1);
         const long long b = i + (long long)j * nc;
         const double vol = EXACT ? vg.volume[b] : 0.0, rvol = EXACT ? vg.r_volume[b] : 0.0;
         double gq_next = 0.0;
         if (EXACT && j < nl - 1) gq_next = div_rcp(iw * dt, vg.volume[b + nc], vg.r_volume[b + nc]);
         /* mixed path: implicit and explicit weights are both 1/2, so every
          * flux term of row j carries the factor g = dt / (2 V_j) */
-        const double g = EXACT ? 0.0 : half_dt * tw.inv_vol[b];
+        const double g = EXACT ? 0.0 : half_dt * in.iv;
         /* flux at interface j (below layer j) */
         double fi = 0.0, fr = 0.0, cj = 0.0, ej = 0.0;
         if (j < nl - 1) {
-            const long long wi = b + nc;
-            double a_ = so.w[wi], b_ = sn.w[wi];
+            double a_ = in.wo, b_ = in.wn;
             if (has_sink) {
                 a_ -= vsink;
                 b_ -= vsink;
             }
-            const double ar = vg.area_v[wi];
-            a_ = ar * a_;
-            b_ = ar * b_;
-            const double dio = nonneg<EXACT>(b_) ? ro[b + nc] : ro[b];
+            a_ = in.ar * a_;
+            b_ = in.ar * b_;
+            const double dio = nonneg<EXACT>(b_) ? in.ro_lo : in.ro;
             fi = a_;
             fr = dio * b_;
             if (EXACT) {
@@ -504,7 +519,7 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
         }
         if (!EXACT) /* sub-diagonal of row j - 1, formed with row j's factor */
             c_prev = nonneg<EXACT>(fi_prev) ? 0.0 : g * fi_prev;
-        double dj, rj = ro[b] + dt * tr[b];
+        double dj, rj = in.ro + dt * in.tr;
         if (EXACT) {
             if (j == 0) {
                 dj = fi >= 0.0 ? 1.0 : 1.0 - gq * fi;

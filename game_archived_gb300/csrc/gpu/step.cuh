@@ -289,11 +289,14 @@ void launch_tracers(Context *c, const StepParams &p, StateMirror *so, StateMirro
     if (mode == COLUMN_REGISTERS)
         k_tracers_solve<NL_FIXED, NL_FIXED, EXACT><<<nblocks(nsys, 64), 64, 0, strm>>>(c->vg, p, so->ds, sn->ds,
                                                                                         st->ds, tw, sh.rho, sh.present);
+    /* sweeps in local memory: blocks of one warp, since a small grid's systems
+     * (80 layers, RES_ID 4: 80 warps of vapour) then lie on as many SMs (125 ->
+     * 121 us; the same at RES_ID 6) */
     else if (mode == COLUMN_LOCAL && c->nl <= SWEEP_SMALL)
-        k_tracers_solve<0, SWEEP_SMALL, EXACT><<<nblocks(nsys, 64), 64, 0, strm>>>(c->vg, p, so->ds, sn->ds, st->ds,
+        k_tracers_solve<0, SWEEP_SMALL, EXACT><<<nblocks(nsys, 32), 32, 0, strm>>>(c->vg, p, so->ds, sn->ds, st->ds,
                                                                                     tw, sh.rho, sh.present);
     else if (mode == COLUMN_LOCAL)
-        k_tracers_solve<0, SWEEP_LARGE, EXACT><<<nblocks(nsys, 64), 64, 0, strm>>>(c->vg, p, so->ds, sn->ds, st->ds,
+        k_tracers_solve<0, SWEEP_LARGE, EXACT><<<nblocks(nsys, 32), 32, 0, strm>>>(c->vg, p, so->ds, sn->ds, st->ds,
                                                                                     tw, sh.rho, sh.present);
     else
         k_tracers_pcr<EXACT><<<nblocks(nsys, PCR_WARPS), 32 * PCR_WARPS,
