@@ -110,6 +110,11 @@ struct StepBufs {
     T *pvt[2] = {}, *v2g[2] = {}, *tend[2] = {};
     T *theta[2] = {}, *str[2] = {}, *strt[2] = {};
     T *wl[2] = {}, *wr[2] = {};
+    /* one block of every array above but so, sn2, wl and wr, so that the
+     * backward step clears its bars with one memset; the last n_adv0 elements
+     * are substage 0's advection, which only a first step has */
+    T *block = nullptr;
+    long long n_block = 0, n_adv0 = 0;
 };
 
 }  // namespace
@@ -172,29 +177,44 @@ bool alloc_step(AdjState *a, StepBufs<T> &S)
         ok = ok && p;
     };
     A(S.so, a->nblk);
-    A(S.sn1, a->nblk);
     A(S.sn2, a->nblk);
-    if (a->n_const > 1) {
-        A(S.pre, PRE_OUT * a->ns);
-        A(S.sed, a->ns);
-    }
-    A(S.P, a->nv);
-    A(S.pgo, a->nv);
     for (int r = 0; r < 2; ++r) {
-        A(S.tri[r], a->ntri);
-        A(S.zh[r], a->nzh);
-        A(S.zv[r], a->nu);
-        A(S.fh[r], a->nu);
-        A(S.fv[r], a->nw);
-        A(S.v2[r], a->ns);
-        A(S.pvt[r], a->nv);
-        A(S.v2g[r], a->nv);
-        A(S.tend[r], a->nv);
-        A(S.theta[r], a->ns);
-        A(S.str[r], a->nrho);
-        A(S.strt[r], a->ns);
         A(S.wl[r], WL_N * a->ns);
         A(S.wr[r], WR_N * a->nwi);
+    }
+    /* the block: sized in a first pass, carved in a second */
+    for (int pass = 0; pass < 2 && ok; ++pass) {
+        long long at = 0;
+        auto B = [&](T *&p, long long n) {
+            if (pass) p = S.block + at;
+            at += (n + 31) / 32 * 32;
+        };
+        B(S.sn1, a->nblk);
+        if (a->n_const > 1) {
+            B(S.pre, PRE_OUT * a->ns);
+            B(S.sed, a->ns);
+        }
+        B(S.P, a->nv);
+        B(S.pgo, a->nv);
+        for (int r = 1; r >= 0; --r) {
+            B(S.pvt[r], a->nv);
+            B(S.v2g[r], a->nv);
+            B(S.tend[r], a->nv);
+            B(S.theta[r], a->ns);
+            B(S.str[r], a->nrho);
+            B(S.strt[r], a->ns);
+        }
+        for (int r = 1; r >= 0; --r) {
+            const long long start = at;
+            B(S.tri[r], a->ntri);
+            B(S.zh[r], a->nzh);
+            B(S.zv[r], a->nu);
+            B(S.fh[r], a->nu);
+            B(S.fv[r], a->nw);
+            B(S.v2[r], a->ns);
+            S.n_adv0 = at - start;
+        }
+        if (!pass) A(S.block, S.n_block = at);
     }
     return ok;
 }
@@ -477,28 +497,8 @@ void step_bwd(Context *c, AdjState *a, bool first, double *s2b, const double *P_
     /* zero all bars of the step */
     auto zero = [&](double *p, long long n) { cudaMemsetAsync(p, 0, (size_t)n * sizeof(double), st); };
     zero(sob, a->nblk);
-    zero(Z.sn1, a->nblk);
-    zero(Z.P, nv);
-    zero(Z.pgo, nv);
-    if (moist) {
-        zero(Z.pre, PRE_OUT * ns);
-        zero(Z.sed, ns);
-        zero(sed_prev_b, ns);
-    }
-    for (int r = 0; r < 2; ++r) {
-        zero(Z.tri[r], a->ntri);
-        zero(Z.zh[r], a->nzh);
-        zero(Z.zv[r], a->nu);
-        zero(Z.fh[r], a->nu);
-        zero(Z.fv[r], a->nw);
-        zero(Z.v2[r], ns);
-        zero(Z.pvt[r], nv);
-        zero(Z.v2g[r], nv);
-        zero(Z.tend[r], nv);
-        zero(Z.theta[r], ns);
-        zero(Z.str[r], a->nrho);
-        zero(Z.strt[r], ns);
-    }
+    zero(Z.block, first ? Z.n_block : Z.n_block - Z.n_adv0);
+    if (moist) zero(sed_prev_b, ns);
     if (pvt_next_b) ku_copy<double><<<nbk(nv), 256, 0, st>>>(nv, pvt_next_b, Z.pvt[1]);
     if (v2g_next_b) ku_copy<double><<<nbk(nv), 256, 0, st>>>(nv, v2g_next_b, Z.v2g[1]);
     if (moist && sed_next_b) ku_copy<double><<<nbk(ns), 256, 0, st>>>(ns, sed_next_b, Z.sed);
