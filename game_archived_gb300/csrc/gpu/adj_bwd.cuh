@@ -632,7 +632,7 @@ __global__ void ba_waves_rows(VGrid vg, StepParams p, AState<double> so, const d
     const long long ns = (long long)nl * nc, n = ns - nc, q = pt.i;
     const long long b = q, lo = q + nc, wi = q + nc;
     const double dt = p.dt;
-    const double *al = wl + WL_A * ns, *be = wl + WL_B * ns, *ga = wl + WL_G * ns, *rexp = wl + WL_REXP * ns;
+    const double *be = wl + WL_B * ns, *ga = wl + WL_G * ns, *rexp = wl + WL_REXP * ns;
     const double *epx = wl + WL_EPEXP * ns;
     const double r_rio = wr[WR_RRIO * n + q], th = wr[WR_TH * n + q];
     const double rho_ie = 0.5 * (rexp[b] + rexp[lo]);

@@ -971,11 +971,6 @@ int adj_waves_backward(Context *c, StateMirror *so_m, StateMirror *sn_m, StateMi
     AdjState *a = c->adj;
     if (set_params(c, a, p)) return -1;
     cudaStream_t st = c->stream;
-    const HGrid<double> &g = c->hg64;
-    (void)g;
-    const VGrid &vg = c->vg;
-    const AParams ap = a->ap;
-    const long long ns = a->ns;
     AState<double> so = view(a, so_m->dev), sn = view(a, sn_m->dev), out = view(a, a->B.sn2);
     double *wl = a->B.wl[0], *wr = a->B.wr[0];
     /* forward of the solver, keeping its work */

@@ -208,15 +208,6 @@ __device__ __forceinline__ double sat_pressure_water(double t)
     return r;
 }
 
-__device__ __forceinline__ double dsat_pressure_water_dT(double t)
-{
-    double tc = t - T_0;
-    if (tc > 100.0) tc = 100.0;
-    if (tc < 0.0) tc = 0.0;
-    double a = tc + 237.1;
-    return sat_pressure_water(t) * (4924.99 / (a * a) - 1.57 / (tc + 105.0));
-}
-
 __device__ __forceinline__ double sat_pressure_ice(double t)
 {
     double tc = t - T_0;
@@ -224,15 +215,6 @@ __device__ __forceinline__ double sat_pressure_ice(double t)
     if (tc > 0.0) tc = 0.0;
     double a = tc + 868.0;
     return exp(43.494 - 6545.8 / (tc + 278.0)) / (a * a);
-}
-
-__device__ __forceinline__ double dsat_pressure_ice_dT(double t)
-{
-    double tc = t - T_0;
-    if (tc < -80.0) tc = -80.0;
-    if (tc > 0.0) tc = 0.0;
-    double a = tc + 278.0;
-    return sat_pressure_ice(t) * (6545.8 / (a * a) - 2.0 / (tc + 868.0));
 }
 
 /* mass-weighted c_v (derived_quantities.c:97-115); cp_ice / cp_water are
