@@ -172,7 +172,10 @@ static T *dalloc(Context *c, size_t n)
 {
     void *p = nullptr;
     if (n == 0) n = 1;
-    if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) return nullptr;
+    if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) {
+        c->alloc_failed = true;
+        return nullptr;
+    }
     cudaMemset(p, 0, n * sizeof(T));
     c->owned.push_back({p, n * sizeof(T)});
     return (T *)p;
@@ -683,8 +686,11 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
         c->edge_flux64 = dalloc<double>(c, (size_t)2 * L * NE);
         c->level_corr64 = dalloc<double>(c, (size_t)3 * (L + 1) * NC);
     }
-    for (auto &b : c->owned)
-        if (!b.p) return fail("device allocation failed");
+    /* before the first kernel: none may run on a pointer that is missing */
+    if (c->alloc_failed) {
+        cudaGetLastError();
+        return fail("device allocation failed");
+    }
     if (make_f64_tables(c)) return -1;
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking));

@@ -76,6 +76,7 @@ struct Context {
     HGrid<float> hg32{};
     VGrid vg{};
     std::vector<DBuf> owned;
+    bool alloc_failed = false; /* an allocation of init_context failed */
 
     /* index maps device position -> reference position */
     int *map_state = nullptr;   /* state block, length state_len */
