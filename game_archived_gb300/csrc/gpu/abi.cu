@@ -1443,7 +1443,7 @@ int three_band_solver_gen_densities_adj(struct state *state_old, struct state *s
     if (rk_step == 0 && up_scal(irrev_bar, GAME_IRREV, "condensates_sediment_heat", sed_b)) return -1;
     StepParams p = params_from_config(c, config, delta_t);
     if (adj_gen_densities(c, p, &b.so, &b.sn, &b.st, b.temperature, rk_step, sed_b, &b.bso, &b.bsn, &b.bst, t_b))
-        return fail("three_band_solver_gen_densities_adj: more than 256 layers or a launch error");
+        return -1;
     if (download_state(state_old_bar, &b.bso, 1 | 16) || download_state(state_new_bar, &b.bsn, 1 | 16)
         || download_state(state_tendency_bar, &b.bst, 1))
         return -1;

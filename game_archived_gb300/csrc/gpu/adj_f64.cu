@@ -258,8 +258,11 @@ int ensure_adj(Context *c)
     for (int k = 0; k < 4; ++k)
         ok = ok && (a->tl_aux[k] = aalloc<Dual>(a, a->nv)) && (a->bar_aux[k] = aalloc<double>(a, a->nv))
              && (a->bar_aux_prev[k] = aalloc<double>(a, a->nv));
+    /* the tracer adjoint's work too: the backward sweep allocates nothing */
+    ok = ok && (c->n_const == 1 || tracer_adj_work(c));
     if (!ok) {
         adj_release_fn(c);
+        cudaGetLastError(); /* reported here, not by the next call */
         return fail("adjoint: device allocation failed");
     }
     return 0;
@@ -483,9 +486,9 @@ void waves_bwd(Context *c, AdjState *a, int rk, AState<double> so, AState<double
  * consumed) and, for a step that is not the model's first, the bars of the
  * lagged inputs; sed_prev_b (moist) receives the bar of the previous step's
  * sedimentation heat in every case. */
-void step_bwd(Context *c, AdjState *a, bool first, double *s2b, const double *P_next_b, const double *pvt_next_b,
-              const double *v2g_next_b, const double *sed_next_b, const double *sed_prev, double *sob,
-              double *P_prev_b, double *pvt_prev_b, double *v2g_prev_b, double *sed_prev_b)
+int step_bwd(Context *c, AdjState *a, bool first, double *s2b, const double *P_next_b, const double *pvt_next_b,
+             const double *v2g_next_b, const double *sed_next_b, const double *sed_prev, double *sob,
+             double *P_prev_b, double *pvt_prev_b, double *v2g_prev_b, double *sed_prev_b)
 {
     const HGrid<double> &g = c->hg64;
     const VGrid &vg = c->vg;
@@ -522,7 +525,7 @@ void step_bwd(Context *c, AdjState *a, bool first, double *s2b, const double *P_
             msn_b.ds = dview(a, out_b_blk);
             mst_b.ds = DState{Z.str[rk], nullptr, nullptr, nullptr, nullptr, nullptr};
             if (adj_gen_densities(c, a->p, &mso, &msn, &mst, B.pre, rk, Z.sed, &mso_b, &msn_b, &mst_b, Z.pre))
-                return;
+                return -1;
         }
         const long long gas = (long long)a->n_cond * ns;
         waves_bwd(c, a, rk, so, sn, out, B.str[rk] + gas, B.strt[rk], B.wl[rk], B.wr[rk], out_b, sob_v, sn_b,
@@ -568,6 +571,7 @@ void step_bwd(Context *c, AdjState *a, bool first, double *s2b, const double *P_
     if (moist) ba_prelude<<<nbk(ns), 256, 0, st>>>(vg, ap, so, Z.pre, sob_v);
     ba_rediag<<<nbk(ns), 256, 0, st>>>(ns, so.rho, so.rt, sob_v.tp, sob_v.rho, sob_v.rt);
     c->kernel_launches += moist ? 46 : 40;
+    return 0;
 }
 
 /* checkpoint slot of step start n: every ck_every-th step and the window's
@@ -896,10 +900,11 @@ int adj_window_backward(Context *c, const double *final_bar, double *init_bar)
         load_start<double>(c, a, n, a->B.so);
         const double *sed_prev = moist ? ck_aux(a, n, 3) : nullptr;
         step_fwd<double>(c, a, a->B, ck_aux(a, n, 0), ck_aux(a, n, 1), ck_aux(a, n, 2), sed_prev, first);
-        step_bwd(c, a, first, a->bar_state, have_next ? a->bar_aux[0] : nullptr,
-                 have_next ? a->bar_aux[1] : nullptr, have_next ? a->bar_aux[2] : nullptr,
-                 have_next_sed ? a->bar_aux[3] : nullptr, sed_prev, init_bar, a->bar_aux_prev[0],
-                 a->bar_aux_prev[1], a->bar_aux_prev[2], a->bar_aux_prev[3]);
+        if (step_bwd(c, a, first, a->bar_state, have_next ? a->bar_aux[0] : nullptr,
+                     have_next ? a->bar_aux[1] : nullptr, have_next ? a->bar_aux[2] : nullptr,
+                     have_next_sed ? a->bar_aux[3] : nullptr, sed_prev, init_bar, a->bar_aux_prev[0],
+                     a->bar_aux_prev[1], a->bar_aux_prev[2], a->bar_aux_prev[3]))
+            return -1;
         /* the step-start bar is the previous step's end-state bar */
         ku_copy<double><<<nbk(a->nblk), 256, 0, st>>>(a->nblk, init_bar, a->bar_state);
         for (int k = 0; k < 4; ++k) std::swap(a->bar_aux[k], a->bar_aux_prev[k]);

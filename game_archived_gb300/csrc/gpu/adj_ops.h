@@ -24,7 +24,7 @@ void op_pot_vort_adj(Context *c, const double *wind, const double *rho, const do
  * on entry (the tracers' new densities, zeroed on return); so_b (tracer
  * densities, w), st_b (tracer densities), sn_b (w) and t_b (temperature) are
  * accumulated; sed_b, the bar of the sedimentation heat, is read and zeroed
- * at rk 0.  Layer counts up to 256. */
+ * at rk 0.  Layer counts up to 256.  -1 with the error set on failure. */
 int adj_gen_densities(Context *c, const StepParams &p, StateMirror *so, StateMirror *sn, StateMirror *st,
                       const double *temperature, int rk, double *sed_b, StateMirror *so_b, StateMirror *sn_b,
                       StateMirror *st_b, double *t_b);

@@ -484,7 +484,7 @@ int adj_gen_densities(Context *c, const StepParams &p, StateMirror *so, StateMir
                       StateMirror *st_b, double *t_b)
 {
     if (c->n_const <= 1) return 0;
-    if (c->nl > 256) return -1;
+    if (c->nl > 256) return fail("three_band_solver_gen_densities_adj: more than 256 layers");
     const int n_tr = c->n_const - 1;
     const long long nsys = (long long)n_tr * c->nc, len = (long long)n_tr * c->ns;
     double *work = tracer_adj_work(c);
@@ -503,8 +503,9 @@ int adj_gen_densities(Context *c, const StepParams &p, StateMirror *so, StateMir
                                               st_b->ds, t_b);
     c->kernel_launches += 3;
     /* the forward overwrites the sedimentation heat at rk 0 */
-    if (rk == 0 && cudaMemsetAsync(sed_b, 0, (size_t)c->ns * sizeof(double), c->stream) != cudaSuccess) return -1;
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    if (rk == 0) CK(cudaMemsetAsync(sed_b, 0, (size_t)c->ns * sizeof(double), c->stream));
+    CK(cudaGetLastError());
+    return 0;
 }
 
 }  // namespace game

@@ -805,8 +805,12 @@ double *tracer_adj_work(Context *c)
 {
     if (c->tracer_adj) return c->tracer_adj;
     c->tracer_adj = dalloc<double>(c, 4 * (size_t)(c->n_const - 1) * (size_t)c->ns);
-    if (!c->tracer_adj) fail("device allocation of the tracer adjoint's work array failed");
-    else if (cudaDeviceSynchronize() != cudaSuccess) return nullptr; /* cleared before the stream uses it */
+    if (!c->tracer_adj) {
+        cudaGetLastError(); /* reported here, not by the next call */
+        fail("device allocation of the tracer adjoint's work array failed");
+    } else if (cudaDeviceSynchronize() != cudaSuccess) {
+        return nullptr; /* cleared before the stream uses it */
+    }
     return c->tracer_adj;
 }
 

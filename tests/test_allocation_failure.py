@@ -22,3 +22,61 @@ for k in [0, 1, total // 3, total // 2] + list(range(total - 24, total)):
     fake.fake_fail_malloc(-1, 0)
 assert init() == 0, error()
 """)
+
+
+def test_a_window_takes_its_memory_in_the_forward():
+    """The backward sweep of a moist window allocates nothing; a forward that
+    cannot have the memory fails, and the next call is not blamed for it."""
+    fakecuda.run("""
+_, m = make_model(3, 1, "jet_moist")
+g = abi.GpuModel(m, abi.FP64)
+final, bar, grad = (m.state_old.clone() for _ in range(3))
+g.window_forward(m.state_old, final, 100.0, 2)
+n = fake.fake_mallocs()
+g.window_backward(bar, grad)
+assert fake.fake_mallocs() == n, fake.fake_mallocs() - n
+g.close()
+
+for back in range(1, 4):        # the last allocations of the window's memory
+    g = abi.GpuModel(m, abi.FP64)
+    g.linear_combine_two_states(m.state_old, m.state_old, m.state_new, 1.0, 0.0)
+    if back == 1:
+        n = fake.fake_mallocs()
+        g.window_forward(m.state_old, final, 100.0, 2)
+        need = fake.fake_mallocs() - n
+    else:
+        fake.fake_fail_malloc(need - back, 0)
+        try:
+            g.window_forward(m.state_old, final, 100.0, 2)
+            assert False, back
+        except abi.GpuError as e:
+            assert "allocation" in str(e), e
+        fake.fake_fail_malloc(-1, 0)
+        g.linear_combine_two_states(m.state_old, m.state_old, m.state_new, 1.0, 0.0)
+    g.close()
+""")
+
+
+def test_a_failed_operator_adjoint_is_reported_once():
+    fakecuda.run("""
+_, m = make_model(3, 1, "jet_moist")
+g = abi.GpuModel(m, abi.FP64)
+args = [m.state_old, m.state_new, m.state_tendency, m.diagnostics, m.irrev]
+bars = [s.clone() for s in args]
+call = lambda: lib.three_band_solver_gen_densities_adj(m.state_old.ptr, m.state_new.ptr, m.state_tendency.ptr,
+    m.diagnostics.ptr, m.irrev.ptr, m.config.ptr, 100.0, 0, m.grid.ptr, *[b.ptr for b in bars])
+assert call() == 0, error()
+g.close()
+g = abi.GpuModel(m, abi.FP64)
+n = fake.fake_mallocs()
+assert call() == 0, error()
+n = fake.fake_mallocs() - n
+g.close()
+g = abi.GpuModel(m, abi.FP64)
+fake.fake_fail_malloc(n - 1, 0)
+assert call() != 0
+assert "tracer adjoint" in error(), error()
+fake.fake_fail_malloc(-1, 0)
+g.linear_combine_two_states(m.state_old, m.state_old, m.state_new, 1.0, 0.0)
+assert call() == 0, error()
+""")
