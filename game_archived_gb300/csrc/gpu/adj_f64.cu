@@ -163,7 +163,7 @@ T *aalloc(AdjState *a, long long n)
 {
     void *p = nullptr;
     if (cudaMalloc(&p, (size_t)(n > 0 ? n : 1) * sizeof(T)) != cudaSuccess) return nullptr;
-    cudaMemset(p, 0, (size_t)(n > 0 ? n : 1) * sizeof(T));
+    cudaMemsetAsync(p, 0, (size_t)(n > 0 ? n : 1) * sizeof(T), ctx()->stream);
     a->owned.push_back(p);
     return (T *)p;
 }

@@ -176,7 +176,10 @@ static T *dalloc(Context *c, size_t n)
         c->alloc_failed = true;
         return nullptr;
     }
-    cudaMemset(p, 0, n * sizeof(T));
+    /* cleared in the order of the stream that uses it (the default stream
+     * while there is none, waited for at the end of the initialisation): the
+     * context's streams do not wait for the default stream */
+    cudaMemsetAsync(p, 0, n * sizeof(T), c->stream);
     c->owned.push_back({p, n * sizeof(T)});
     return (T *)p;
 }
@@ -772,7 +775,7 @@ StateMirror *mirror(const void *host_state, int create)
         fail("device allocation of a state mirror failed");
         return nullptr;
     }
-    cudaMemset(m.dev, 0, (size_t)c->state_len * sizeof(double));
+    cudaMemsetAsync(m.dev, 0, (size_t)c->state_len * sizeof(double), c->stream);
     set_mirror_views(c, m);
     c->states[host_state] = m;
     return &c->states[host_state];
@@ -808,8 +811,6 @@ double *tracer_adj_work(Context *c)
     if (!c->tracer_adj) {
         cudaGetLastError(); /* reported here, not by the next call */
         fail("device allocation of the tracer adjoint's work array failed");
-    } else if (cudaDeviceSynchronize() != cudaSuccess) {
-        return nullptr; /* cleared before the stream uses it */
     }
     return c->tracer_adj;
 }

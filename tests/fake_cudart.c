@@ -17,7 +17,9 @@ enum { MEMORY_ALLOCATION = 2 };
 static long g_mallocs, g_fail_at = -1, g_launches;
 static size_t g_live;
 static err_t g_last;
+static int g_streams;
 static int g_handles;
+static long g_unordered; /* clears on the default stream once other streams exist */
 
 /* the n-th allocation from now (0 the next) fails, and every one after it
  * while keep is set; n < 0: none */
@@ -29,6 +31,7 @@ void fake_fail_malloc(long n, int keep)
 }
 long fake_mallocs(void) { return g_mallocs; }
 long fake_launches(void) { return g_launches; }
+long fake_unordered_clears(void) { return g_unordered; }
 size_t fake_live_bytes(void) { return g_live; }
 
 err_t cudaMalloc(void **p, size_t n)
@@ -55,8 +58,8 @@ err_t cudaFreeHost(void *p) { free(p); return 0; }
 err_t cudaHostGetDevicePointer(void **d, void *h, unsigned f) { (void)f; *d = h; return 0; }
 err_t cudaMemcpy(void *d, const void *s, size_t n, int kind) { (void)kind; memmove(d, s, n); return 0; }
 err_t cudaMemcpyAsync(void *d, const void *s, size_t n, int kind, void *st) { (void)kind; (void)st; memmove(d, s, n); return 0; }
-err_t cudaMemset(void *d, int v, size_t n) { memset(d, v, n); return 0; }
-err_t cudaMemsetAsync(void *d, int v, size_t n, void *st) { (void)st; memset(d, v, n); return 0; }
+err_t cudaMemsetAsync(void *d, int v, size_t n, void *st) { g_unordered += !st && g_streams > 0; memset(d, v, n); return 0; }
+err_t cudaMemset(void *d, int v, size_t n) { return cudaMemsetAsync(d, v, n, 0); }
 err_t cudaGetLastError(void) { err_t e = g_last; g_last = 0; return e; }
 const char *cudaGetErrorString(err_t e) { return e == MEMORY_ALLOCATION ? "out of memory" : e ? "error" : "no error"; }
 err_t cudaDeviceSynchronize(void) { return 0; }
@@ -64,8 +67,8 @@ err_t cudaGetDevice(int *d) { *d = 0; return 0; }
 err_t cudaSetDevice(int d) { (void)d; return 0; }
 err_t cudaGetSymbolAddress(void **p, const void *s) { (void)s; (void)p; return g_last = 13; }
 static err_t handle(void **h) { *h = (void *)(size_t)(++g_handles); return 0; }
-err_t cudaStreamCreateWithFlags(void **s, unsigned f) { (void)f; return handle(s); }
-err_t cudaStreamDestroy(void *s) { (void)s; return 0; }
+err_t cudaStreamCreateWithFlags(void **s, unsigned f) { (void)f; ++g_streams; return handle(s); }
+err_t cudaStreamDestroy(void *s) { (void)s; --g_streams; return 0; }
 err_t cudaStreamSynchronize(void *s) { (void)s; return 0; }
 err_t cudaStreamWaitEvent(void *s, void *e, unsigned f) { (void)s; (void)e; (void)f; return 0; }
 err_t cudaStreamIsCapturing(void *s, int *c) { (void)s; *c = 0; return 0; }

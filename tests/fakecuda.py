@@ -20,7 +20,7 @@ from game_archived_gb300 import abi, native
 from helpers import make_model
 fake = ctypes.CDLL({so!r})
 fake.fake_fail_malloc.argtypes = [ctypes.c_long, ctypes.c_int]
-for f in ("fake_mallocs", "fake_launches"):
+for f in ("fake_mallocs", "fake_launches", "fake_unordered_clears"):
     getattr(fake, f).restype = ctypes.c_long
 fake.fake_live_bytes.restype = ctypes.c_size_t
 lib = native.gpu()

@@ -80,3 +80,20 @@ fake.fake_fail_malloc(-1, 0)
 g.linear_combine_two_states(m.state_old, m.state_old, m.state_new, 1.0, 0.0)
 assert call() == 0, error()
 """)
+
+
+def test_new_buffers_are_cleared_on_the_stream_that_uses_them():
+    """The library's streams do not wait for the default stream: a clear there
+    could wipe what a kernel or an upload has written meanwhile."""
+    fakecuda.run("""
+_, m = make_model(3, 1, "jet_moist")
+g = abi.GpuModel(m, abi.FP64)
+g.linear_combine_two_states(m.state_old, m.state_old, m.state_new, 1.0, 0.0)
+g.manage_rkhevi(100.0, 0.0)
+final, bar, grad = (m.state_old.clone() for _ in range(3))
+g.window_forward(m.state_old, final, 100.0, 2)
+g.window_backward(bar, grad)
+m.config["momentum_diff_h"] = 1
+g.manage_rkhevi(100.0, 0.0)
+assert fake.fake_unordered_clears() == 0, fake.fake_unordered_clears()
+""")
