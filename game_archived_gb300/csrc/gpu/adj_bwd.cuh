@@ -594,11 +594,11 @@ __global__ void ba_thomas(int nc, int nl_arg, const double *dden, const double *
 #pragma unroll
     for (int j = 0; j < n; ++j) {
         const long long q = (long long)j * nc + i;
-        const double xb = div_rcp(wr_b[WR_SOL * m + q], dden[q], r_dden[q]);
+        const double xb = div_sweep(wr_b[WR_SOL * m + q], dden[q], r_dden[q]);
         const double sub = j > 0 ? ee[q - nc] : 0.0; /* (A^T)_{j,j-1} = e_{j-1} */
-        const double den = j > 0 ? dd[q] - ep[j - 1] * sub : dd[q], inv = rcp_nr<2>(den);
-        if (j < n - 1) ep[j] = div_rcp(cc[q], den, inv); /* (A^T)_{j,j+1} = c_j */
-        rp[j] = div_rcp(j > 0 ? xb - rp[j - 1] * sub : xb, den, inv);
+        const double den = j > 0 ? dd[q] - ep[j - 1] * sub : dd[q], inv = rcp_sweep(den);
+        if (j < n - 1) ep[j] = div_sweep(cc[q], den, inv); /* (A^T)_{j,j+1} = c_j */
+        rp[j] = div_sweep(j > 0 ? xb - rp[j - 1] * sub : xb, den, inv);
     }
     double lam_next = 0.0, x_next = 0.0;
 #pragma unroll

@@ -670,9 +670,9 @@ __global__ void fa_waves_thomas_fixed(int nc, const double *dden, const double *
         const long long q = (long long)j * nc + i;
         const double dj = wr[WR_D * m + q], rj = wr[WR_R * m + q];
         const double cm = j > 0 ? wr[WR_C * m + q - nc] : 0.0;
-        const double den = j > 0 ? dj - ep[j - 1] * cm : dj, inv = rcp_nr<2>(den);
-        if (j < n - 1) ep[j] = div_rcp(wr[WR_E * m + q], den, inv);
-        rp[j] = div_rcp(j > 0 ? rj - rp[j - 1] * cm : rj, den, inv);
+        const double den = j > 0 ? dj - ep[j - 1] * cm : dj, inv = rcp_sweep(den);
+        if (j < n - 1) ep[j] = div_sweep(wr[WR_E * m + q], den, inv);
+        rp[j] = div_sweep(j > 0 ? rj - rp[j - 1] * cm : rj, den, inv);
     }
     double x = 0.0;
 #pragma unroll
@@ -680,7 +680,7 @@ __global__ void fa_waves_thomas_fixed(int nc, const double *dden, const double *
         const long long q = (long long)j * nc + i;
         x = j < n - 1 ? rp[j] - ep[j] * x : rp[j];
         wr[WR_X * m + q] = x;
-        wr[WR_SOL * m + q] = div_rcp(x, dden[q], r_dden[q]);
+        wr[WR_SOL * m + q] = div_sweep(x, dden[q], r_dden[q]);
     }
 }
 

@@ -344,9 +344,9 @@ __global__ void ka_gen_solve(int nc, int nl_arg, int n_tr, int n_cond, TracerRow
         const long long o = (long long)j * nc;
         dd[j] = dx[o];
         const double cm = j > 0 ? cc[o - nc] : 0.0, r = ry[o];
-        const double den = j > 0 ? dd[j] - ep[j - 1] * cm : dd[j], inv = rcp_nr<2>(den);
-        ep[j] = j < nl - 1 ? div_rcp(ee[o], den, inv) : 0.0;
-        rp[j] = div_rcp(j > 0 ? r - rp[j - 1] * cm : r, den, inv);
+        const double den = j > 0 ? dd[j] - ep[j - 1] * cm : dd[j], inv = rcp_sweep(den);
+        ep[j] = j < nl - 1 ? div_sweep(ee[o], den, inv) : 0.0;
+        rp[j] = div_sweep(j > 0 ? r - rp[j - 1] * cm : r, den, inv);
     }
     double x = 0.0;
 #pragma unroll
@@ -362,9 +362,9 @@ __global__ void ka_gen_solve(int nc, int nl_arg, int n_tr, int n_cond, TracerRow
         const double g = rp[j] < 0.0 ? 0.0 : rn_b[o];
         rn_b[o] = 0.0;
         const double sub = j > 0 ? ee[o - nc] : 0.0;
-        const double den = j > 0 ? dd[j] - ep[j - 1] * sub : dd[j], inv = rcp_nr<2>(den);
-        ep[j] = j < nl - 1 ? div_rcp(cc[o], den, inv) : 0.0;
-        rp[j] = div_rcp(j > 0 ? g - rp[j - 1] * sub : g, den, inv);
+        const double den = j > 0 ? dd[j] - ep[j - 1] * sub : dd[j], inv = rcp_sweep(den);
+        ep[j] = j < nl - 1 ? div_sweep(cc[o], den, inv) : 0.0;
+        rp[j] = div_sweep(j > 0 ? g - rp[j - 1] * sub : g, den, inv);
     }
     double y = 0.0;
 #pragma unroll

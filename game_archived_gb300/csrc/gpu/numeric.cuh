@@ -41,8 +41,12 @@ inline dim3 layer_grid(int layers, int n, int bs) { return dim3((unsigned)((n + 
  * once per column: k_tracers_pcr was slower with the other (181 -> 216 us). */
 __device__ __forceinline__ int row_of(long long i, int n) { return (int)((unsigned)i / (unsigned)n); }
 
-/* FP64 reciprocal for the mixed path (the FP64 path divides exactly as the
- * reference).  The seed is the hardware's approximate reciprocal (PTX
+/* x == +-0 by an integer test (an FP64 comparison would issue on the FP64
+ * pipe) */
+__device__ __forceinline__ bool is_zero(double x) { return ((unsigned long long)__double_as_longlong(x) << 1) == 0ULL; }
+
+/* FP64 reciprocal for the mixed path, and for the FP64 path's quotients that
+ * div_rcp and div_sweep correct.  The seed is the hardware's approximate reciprocal (PTX
  * rcp.approx.ftz.f64; relative error below 2^-20, measured on GB300 over
  * 2^20 inputs spanning 1e-300..1e300), refined by Newton-Raphson steps
  * r <- r + r (1 - x r), each of which squares the relative error: one step
@@ -70,18 +74,53 @@ __device__ __forceinline__ double rcp_nr(double x)
  * elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
  * Dev. 34, 1990; Brisebarre, Muller and Raina, "Accelerating correctly
  * rounded floating-point division when the divisor is known in advance",
- * IEEE Trans. Computers 53, 2004).  Equal to x / y for finite operands away
- * from the ends of the exponent range (tested), in three FP64 issues
- * instead of the division's eight or more, without its branch. */
+ * IEEE Trans. Computers 53, 2004), in three FP64 issues instead of the
+ * division's eight or more, without its branch.  The theorem holds while
+ * dividend and quotient are far from the ends of the exponent range (their
+ * exponents within 500 of 0; the divisor's is then within 1000); elsewhere,
+ * so for subnormal, infinite and NaN operands, divisors of 0 and overflows,
+ * the call divides.  The test is four integer instructions beside FP64 ones
+ * that issue at 1/64 of their rate: no kernel's time moved with it, but for
+ * the column sweeps' (div_sweep).  Equal to x / y bit for bit where r is the
+ * correctly rounded reciprocal (tested on the device).  With a reciprocal an
+ * ulp off (rcp_nr<2>, a product of two) the same but for quotients as close
+ * to the middle of two doubles as any, by divisors next to the end of their
+ * binade, where one ulp is possible. */
+__device__ __noinline__ double div_ieee(double x, double y) { return x / y; }
+__device__ __forceinline__ bool mid_range(double x)
+{
+    return ((unsigned)__double2hiint(x) & 0x7ff00000u) - (523u << 20) <= 1000u << 20;
+}
 __device__ __forceinline__ double div_rcp(double x, double y, double r)
 {
     const double q = __dmul_rn(x, r);
-    return __fma_rn(__fma_rn(-q, y, x), r, q);
+    double z = __fma_rn(__fma_rn(-q, y, x), r, q);
+    if (!mid_range(q) || !mid_range(x)) z = is_zero(q) && is_zero(x) ? q : div_ieee(x, y);
+    return z;
 }
-/* 1 / x correctly rounded (as div_rcp), from the hardware's seed: seven FP64
- * issues and no branch.  Where the reciprocal only serves div_rcp, whose
- * correction absorbs its last bits, rcp_nr<2> alone does. */
+/* 1 / x as div_rcp gives it, from the hardware's seed.  Where the reciprocal
+ * only serves div_rcp, whose correction absorbs its last bits, rcp_nr<2>
+ * alone does. */
 __device__ __forceinline__ double rcp_full(double x) { return div_rcp(1.0, x, rcp_nr<2>(x)); }
+/* The same in the column sweeps, whose unrolled rows hold a column in
+ * registers: a call at every quotient costs them (RES_ID 6, k_tracers_solve
+ * 102 -> 177 us, k_waves_thomas 53 -> 86 us), so a selection takes its place:
+ * x r itself where it is zero, subnormal, infinite or NaN, and the seed as the
+ * reciprocal of a pivot that is zero, infinite or NaN.  IEEE's result for
+ * those too (a subnormal pivot counts as 0, one above 2^1022 as infinite);
+ * one ulp is possible where the quotient is subnormal or the dividend below
+ * 2^-900. */
+__device__ __forceinline__ double div_sweep(double x, double y, double r)
+{
+    const double q = __dmul_rn(x, r);
+    const double z = __fma_rn(__fma_rn(-q, y, x), r, q);
+    return ((unsigned)__double2hiint(q) & 0x7ff00000u) - 0x100000u <= 0x7fd00000u ? z : q;
+}
+__device__ __forceinline__ double rcp_sweep(double x)
+{
+    const double seed = rcp_nr<0>(x), r = rcp_nr<2>(x);
+    return ((unsigned)__double2hiint(seed) & 0x7ff00000u) - 0x100000u <= 0x7fd00000u ? r : seed;
+}
 /* x / tab[i] with the reciprocals of tab in rtab on the FP64 path; the mixed
  * path divides in FP32 */
 __device__ __forceinline__ double div_tab(double x, const double *tab, const double *rtab, long long i)
@@ -148,9 +187,6 @@ __device__ __forceinline__ double to_double(float x)
     const unsigned long long f = ((unsigned long long)m << (52 - p)) & 0xfffffffffffffULL;
     return __hiloint2double((int)(sign | ((unsigned)(p + 874) << 20) | (unsigned)(f >> 32)), (int)(unsigned)f);
 }
-/* x == +-0 by an integer test (an FP64 comparison would issue on the FP64
- * pipe) */
-__device__ __forceinline__ bool is_zero(double x) { return ((unsigned long long)__double_as_longlong(x) << 1) == 0ULL; }
 
 /* FP64 operations that stay behind the test that guards them: the compiler runs
  * plain ones ahead of it and selects, and each issue holds the FP64 pipe for 16

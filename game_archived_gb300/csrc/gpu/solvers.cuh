@@ -254,9 +254,9 @@ __global__ void k_waves_thomas(int nc, WavesWork ww)
         const double dj = ww.d[q], rj = ww.r[q];
         if (j == 0) {
             if (EXACT) {
-                const double inv = rcp_nr<2>(dj);
-                ep[0] = div_rcp(ww.e[q], dj, inv);
-                rp[0] = div_rcp(rj, dj, inv);
+                const double inv = rcp_sweep(dj);
+                ep[0] = div_sweep(ww.e[q], dj, inv);
+                rp[0] = div_sweep(rj, dj, inv);
             } else {
                 const double inv = rcp_nr<2>(dj);
                 ep[0] = ww.e[q] * inv;
@@ -266,9 +266,9 @@ __global__ void k_waves_thomas(int nc, WavesWork ww)
             const double cm = ww.c[q - nc];
             const double den = dj - ep[j - 1] * cm;
             if (EXACT) {
-                const double inv = rcp_nr<2>(den);
-                if (j < n - 1) ep[j] = div_rcp(ww.e[q], den, inv);
-                rp[j] = div_rcp(rj - rp[j - 1] * cm, den, inv);
+                const double inv = rcp_sweep(den);
+                if (j < n - 1) ep[j] = div_sweep(ww.e[q], den, inv);
+                rp[j] = div_sweep(rj - rp[j - 1] * cm, den, inv);
             } else {
                 const double inv = rcp_nr<2>(den);
                 if (j < n - 1) ep[j] = ww.e[q] * inv;
@@ -279,7 +279,7 @@ __global__ void k_waves_thomas(int nc, WavesWork ww)
     /* damping: divide by 1 + dt * coefficient (mixed path: multiply by the
      * tabulated reciprocal) */
     auto damp = [&](double x, long long q) {
-        return EXACT ? div_rcp(x, ww.damp_den[q], ww.damp_inv[q]) : x * ww.damp_inv[q];
+        return EXACT ? div_sweep(x, ww.damp_den[q], ww.damp_inv[q]) : x * ww.damp_inv[q];
     };
     double x = rp[n - 1];
     ww.r[(long long)(n - 1) * nc + i] = damp(x, (long long)(n - 1) * nc + i);
@@ -473,7 +473,7 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
     const double a_sfc = vg.area_v[(long long)nl * nc + i];
     double ep[NL > 0 ? NL : CAP], rp[NL > 0 ? NL : CAP];
     /* FP64 path: iw dt / V of the layer, shared by its flux terms */
-    double gq = EXACT ? div_rcp(iw * dt, vg.volume[i], vg.r_volume[i]) : 0.0;
+    double gq = EXACT ? div_sweep(iw * dt, vg.volume[i], vg.r_volume[i]) : 0.0;
     double fi_prev = 0.0, fr_prev = 0.0, c_prev = 0.0;
     /* what row j reads; where the layer count is a run-time one, a row ahead of
      * its use (with a compile-time one the compiler places the loads) */
@@ -493,7 +493,7 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
         const long long b = i + (long long)j * nc;
         const double vol = EXACT ? vg.volume[b] : 0.0, rvol = EXACT ? vg.r_volume[b] : 0.0;
         double gq_next = 0.0;
-        if (EXACT && j < nl - 1) gq_next = div_rcp(iw * dt, vg.volume[b + nc], vg.r_volume[b + nc]);
+        if (EXACT && j < nl - 1) gq_next = div_sweep(iw * dt, vg.volume[b + nc], vg.r_volume[b + nc]);
         /* mixed path: implicit and explicit weights are both 1/2, so every
          * flux term of row j carries the factor g = dt / (2 V_j) */
         const double g = EXACT ? 0.0 : half_dt * in.iv;
@@ -523,17 +523,17 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
         if (EXACT) {
             if (j == 0) {
                 dj = fi >= 0.0 ? 1.0 : 1.0 - gq * fi;
-                rj += div_rcp(ew * dt * fr, vol, rvol);
+                rj += div_sweep(ew * dt * fr, vol, rvol);
             } else if (j == nl - 1) {
                 dj = fi_prev >= 0.0 ? 1.0 + gq * fi_prev : 1.0;
-                if (has_sink) dj += div_rcp(iw * vsink * dt * a_sfc, vol, rvol);
-                rj += div_rcp(-ew * dt * fr_prev, vol, rvol);
-                if (has_sink) rj += div_rcp(-ew * vsink * dt * ro[bot] * a_sfc, vol, rvol);
+                if (has_sink) dj += div_sweep(iw * vsink * dt * a_sfc, vol, rvol);
+                rj += div_sweep(-ew * dt * fr_prev, vol, rvol);
+                if (has_sink) rj += div_sweep(-ew * vsink * dt * ro[bot] * a_sfc, vol, rvol);
             } else {
                 dj = 1.0;
                 if (fi_prev >= 0.0) dj += gq * fi_prev;
                 if (fi < 0.0) dj -= gq * fi;
-                rj += div_rcp(ew * dt * (-fr_prev + fr), vol, rvol);
+                rj += div_sweep(ew * dt * (-fr_prev + fr), vol, rvol);
             }
         } else {
             if (j == 0) {
@@ -555,9 +555,9 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
         /* forward elimination */
         if (j == 0) {
             if (EXACT) {
-                const double inv = rcp_nr<2>(dj);
-                ep[0] = div_rcp(ej, dj, inv);
-                rp[0] = div_rcp(rj, dj, inv);
+                const double inv = rcp_sweep(dj);
+                ep[0] = div_sweep(ej, dj, inv);
+                rp[0] = div_sweep(rj, dj, inv);
             } else {
                 const double inv = rcp_nr<2>(dj);
                 ep[0] = ej * inv;
@@ -566,9 +566,9 @@ __global__ void k_tracers_solve(VGrid vg, StepParams p, DState so, DState sn, DS
         } else {
             const double den = dj - ep[j - 1] * c_prev;
             if (EXACT) {
-                const double inv = rcp_nr<2>(den);
-                if (j < nl - 1) ep[j] = div_rcp(ej, den, inv);
-                rp[j] = div_rcp(rj - rp[j - 1] * c_prev, den, inv);
+                const double inv = rcp_sweep(den);
+                if (j < nl - 1) ep[j] = div_sweep(ej, den, inv);
+                rp[j] = div_sweep(rj - rp[j - 1] * c_prev, den, inv);
             } else {
                 const double inv = rcp_nr<2>(den);
                 if (j < nl - 1) ep[j] = ej * inv;

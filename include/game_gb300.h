@@ -105,14 +105,18 @@ int game_gpu_event_elapsed(int a, int b, float *ms);
 int game_gpu_profile(int on);
 int game_gpu_profile_count(void);
 int game_gpu_profile_get(int i, const char **name, double *ms, long long *launches);
-/* the mixed path's numeric primitives beside the CUDA operations they stand
+/* the step's numeric primitives beside the CUDA operations they stand
  * for, over n host values (for tests; no context needed): op 0 / 1 the
  * Newton-refined FP64 reciprocal with 1 / 2 steps, 2 IEEE 1.0 / x, 3 / 4
  * double -> float by integer operations / by the conversion instruction,
  * 5 / 6 float -> double likewise, 7 the double-float split and join of x,
  * 8 the double-float reciprocal, 9 / 10 double-float product / sum of in[i]
- * and in[n + i]; in and out are double arrays except the float side of ops
- * 3 to 6 */
+ * and in[n + i]; of the FP64 path, with x = in[i] and y = in[n + i], 11 / 12
+ * the quotient by a reciprocal at hand with 1.0 / y / with op 1's, 13 x / y,
+ * 14 that quotient by y y with the square of 1.0 / y, 15 x / (y y), 16 the
+ * reciprocal, 17 / 18 the half of x by its exponent / 0.5 x, 19 / 20 x^3 and
+ * x^4, 21 the column sweeps' quotient; in and out are double arrays except
+ * the float side of ops 3 to 6 */
 int game_gpu_numerics(int op, const void *in, void *out, long long n);
 /* ---- health check and checkpoints (no counterpart in the reference's
  * library interface; see each) ---- */
