@@ -76,8 +76,7 @@ struct HGrid {
     const R *dual_area_t;   /* [L][Nt] */
     const R *dual_z_t;      /* [L][Nt] */
     /* FP64 path only (null in the FP32 copy): reciprocals of grid quantities
-     * for div_rcp (0 where the quantity is 0), and products of grid
-     * quantities in the operators' order */
+     * for div_rcp, and products of grid quantities in the operators' order */
     const R *r_nd_v, *r_area_v;             /* [L+1][Nc] */
     const R *r_volume;                      /* [L][Nc] */
     const R *r_nd_h;                        /* [L][Ne] */

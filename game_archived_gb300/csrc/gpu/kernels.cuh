@@ -48,7 +48,11 @@ __device__ __forceinline__ R grad_v(const HGrid<R> &g, const F *f, int k, int c)
     return div_tab(as<R>(f[i - g.nc]) - as<R>(f[i]), g.nd_v, g.r_nd_v, i);
 }
 
-/* slopes are exactly 0 away from orography; no FP64 comparison */
+/* Slopes and height differences are exactly 0 away from orography, and what
+ * they multiply is left out there (tests on integers: no FP64 comparison): a
+ * zero for finite values; a field that is infinite or NaN in a neighbouring
+ * layer does not become a NaN through it.  ALL: nothing is left out (the
+ * single operators, whose NaN are the reference's for any field). */
 __device__ __forceinline__ bool zero_slope(double s) { return is_zero(s); }
 __device__ __forceinline__ bool zero_slope(float s) { return s == 0.0f; }
 
@@ -77,7 +81,7 @@ __device__ __forceinline__ double grad_h_pre(const HGrid<double> &g, double f_to
 /* horizontal gradient at edge e of layer l, with the terrain-following
  * covariant -> contravariant correction in the orography layers
  * (gradient_operators.c:14-33, averaging.c:14-39 and :113-133) */
-template <typename R, typename F>
+template <bool ALL = false, typename R, typename F>
 __device__ __forceinline__ R grad_h(const HGrid<R> &g, const F *f, int l, int e)
 {
     const int fr = g.from[e], to = g.to[e];
@@ -85,7 +89,7 @@ __device__ __forceinline__ R grad_h(const HGrid<R> &g, const F *f, int l, int e)
     R out = div_tab(as<R>(f[(long long)l * g.nc + to]) - as<R>(f[(long long)l * g.nc + fr]), g.nd_h, g.r_nd_h, le);
     if (l >= g.nl - g.n_oro) {
         /* a zero slope adds a zero */
-        if (zero_slope(g.slope_h[le])) return out;
+        if (!ALL && zero_slope(g.slope_h[le])) return out;
         R c = ipw_at(g, 6, l, fr) * grad_v(g, f, l, fr);
         c += ipw_at(g, 6, l, to) * grad_v(g, f, l, to);
         if (l < g.nl - 1) {
@@ -99,7 +103,7 @@ __device__ __forceinline__ R grad_h(const HGrid<R> &g, const F *f, int l, int e)
 }
 
 /* horizontal covariant wind component (averaging.c:97-111) */
-template <typename R, typename F>
+template <bool ALL = false, typename R, typename F>
 __device__ __forceinline__ R hor_covariant(const HGrid<R> &g, const F *u, const F *w, int l, int e)
 {
     const long long le = (long long)l * g.ne + e;
@@ -107,7 +111,7 @@ __device__ __forceinline__ R hor_covariant(const HGrid<R> &g, const F *u, const 
     if (l >= g.nl - g.n_oro) {
         const R slope = g.slope_h[le];
         /* a zero slope adds a zero */
-        if (zero_slope(slope)) return r;
+        if (!ALL && zero_slope(slope)) return r;
         const int fr = g.from[e], to = g.to[e];
         R c = ipw_at(g, 6, l, fr) * R(w[(long long)l * g.nc + fr]);
         c += ipw_at(g, 6, l, to) * R(w[(long long)l * g.nc + to]);
@@ -523,7 +527,7 @@ __global__ void k_make_shadow(long long n_rho, long long ns, long long nw, long 
 
 /* ------------------------------------------------------- k_tri_vort
  * vertical relative vorticity on triangles (vorticities.c:167-222) */
-template <typename R>
+template <typename R, bool ALL = false>
 __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_tri_vort(HGrid<R> g, const R *u, R *tri_vort)
 {
     const LayerPoint pt_ = layer_point(g.nt);
@@ -543,7 +547,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_tri
             double vel = u[le];
             if (l >= g.nl - g.n_oro) {
                 const double zh = g.z_h[le], dz = g.dual_z_t[i] - zh;
-                if (!is_zero(dz)) {
+                if (ALL || !is_zero(dz)) {
                     const bool above = __double_as_longlong(dz) > 0 || l == g.nl - 1;
                     const long long lo_e = above ? le - g.ne : le + g.ne;
                     const double r = above ? -g.r_dz_h[le] : g.r_dz_h[le + g.ne];
@@ -578,7 +582,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == sizeof(float) ? 8 : 1) k_tri
 }
 
 /* tangential relative vorticity at level k, edge e (vorticities.c:104-165) */
-template <typename R>
+template <bool ALL = false, typename R>
 __device__ __forceinline__ R rel_vort_tangential(const HGrid<R> &g, const R *u, const R *w, int k, int e)
 {
     const int nl = g.nl;
@@ -588,12 +592,12 @@ __device__ __forceinline__ R rel_vort_tangential(const HGrid<R> &g, const R *u, 
     if constexpr (sizeof(R) == sizeof(double)) inv_area = g.r_dual_area_h[ke];
     else inv_area = R(1) / g.dual_area_h[ke];
     if (k == nl) {
-        R c2 = hor_covariant(g, u, w, k - 1, e);
+        R c2 = hor_covariant<ALL>(g, u, w, k - 1, e);
         return inv_area * g.nd_h[(long long)(k - 1) * g.ne + e] * c2;
     }
     const int fr = g.from[e], to = g.to[e];
-    R c0 = hor_covariant(g, u, w, k, e);
-    R c2 = hor_covariant(g, u, w, k - 1, e);
+    R c0 = hor_covariant<ALL>(g, u, w, k, e);
+    R c2 = hor_covariant<ALL>(g, u, w, k - 1, e);
     return inv_area * (-g.nd_h[(long long)k * g.ne + e] * c0
                        + g.nd_v[(long long)k * g.nc + fr] * w[(long long)k * g.nc + fr]
                        + g.nd_h[(long long)(k - 1) * g.ne + e] * c2
@@ -792,7 +796,7 @@ __device__ __forceinline__ void pgrad_h_parts(const HGrid<R> &g, const StepParam
     const int fr = g.from[e], to = g.to[e];
     const long long cf = (long long)l * g.nc + fr, ct = (long long)l * g.nc + to;
     const R cdp = R(C_D_P);
-    nl = grad_h(g, s.exner_pert, l, e);
+    nl = grad_h<true>(g, s.exner_pert, l, e);
     R s_to = cdp * (g.theta_v_bg[ct] + s.theta_v_pert[ct]), s_fr = cdp * (g.theta_v_bg[cf] + s.theta_v_pert[cf]);
     nl = (R(0.5) * (s_to + s_fr)) * nl;
     l_term = (R(0.5) * (cdp * s.theta_v_pert[ct] + cdp * s.theta_v_pert[cf])) * g.exner_bg_grad_h[(long long)l * g.ne + e];

@@ -20,7 +20,7 @@ __global__ void k_op_grad_h(G g, const double *f, double *u, int with_correction
     if (i >= n) return;
     const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     if (with_correction) {
-        u[i] = grad_h(g, f, l, e);
+        u[i] = grad_h<true>(g, f, l, e);
     } else {
         const int fr = g.from[e], to = g.to[e];
         u[i] = div_tab(f[(long long)l * g.nc + to] - f[(long long)l * g.nc + fr], g.nd_h, g.r_nd_h, i);
@@ -148,7 +148,7 @@ __global__ void k_op_rel_vort(G g, const double *u, const double *w, const doubl
     const long long n = (long long)(g.nl + 1) * g.ne, i = gtid();
     if (i >= n) return;
     const int k = row_of(i, g.ne), e = (int)(i - (long long)k * g.ne);
-    zh[i] = rel_vort_tangential(g, u, w, k, e);
+    zh[i] = rel_vort_tangential<true>(g, u, w, k, e);
     if (k < g.nl) {
         const int tf = g.dual_from[e], tt = g.dual_to[e];
         const long long kt = (long long)k * g.nt;
@@ -345,7 +345,7 @@ void op_inner_product(Context *c, const double *a, const double *b, double *out)
 void op_rel_vort(Context *c, const double *wind, double *tri, double *curl)
 {
     const long long off = (long long)(c->nl + 1) * c->nc, coff = (long long)(c->nl + 1) * c->ne;
-    k_tri_vort<double><<<dim3(nb(c->nt), (unsigned)c->nl), 256, 0, c->stream>>>(c->hg64, wind + off, tri);
+    k_tri_vort<double, true><<<dim3(nb(c->nt), (unsigned)c->nl), 256, 0, c->stream>>>(c->hg64, wind + off, tri);
     k_op_rel_vort<<<nb(coff), 256, 0, c->stream>>>(c->hg64, wind + off, wind, tri, curl, curl + coff);
     c->kernel_launches += 2;
 }

@@ -13,7 +13,7 @@ namespace {
 __global__ void k_reciprocal(long long n, const double *x, double *r)
 {
     const long long i = gtid();
-    if (i < n) r[i] = x[i] != 0.0 ? 1.0 / x[i] : 0.0;
+    if (i < n) r[i] = 1.0 / x[i];
 }
 
 /* of z_h(k-1) - z_h(k), the edge heights' differences (vorticities.c:200-214) */
