@@ -235,13 +235,15 @@ __global__ void k_op_lincomb(long long n, const double *a, const double *b, doub
 }
 
 /* 1 a + 0 b, the time loop's copy of the new state to the old one
- * (coordinator.c:305): a where b is finite, the general form's NaN elsewhere,
- * without its three FP64 issues per value (67 of 86 us at RES_ID 6; 8 mixed
+ * (coordinator.c:305): a where b is finite (+0 for an a of -0 unless b is
+ * negative too), the general form's NaN elsewhere, without its three FP64 issues per value (67 of 86 us at RES_ID 6; 8 mixed
  * steps 10.06 -> 9.72 ms).
  * Four values a thread by two 16-byte accesses per array. */
-__device__ __forceinline__ double keep_if_finite(double a, double b)
+__device__ __forceinline__ double one_a_zero_b(double a, double b)
 {
-    return (__double2hiint(b) & 0x7ff00000) == 0x7ff00000 ? guarded_fma(0.0, b, a) : a;
+    if ((__double2hiint(b) & 0x7ff00000) == 0x7ff00000) return guarded_fma(0.0, b, a);
+    if (is_zero(a)) return __hiloint2double(__double2hiint(a) & __double2hiint(b) & (int)0x80000000u, 0);
+    return a;
 }
 __global__ void k_op_copy_state(long long n, const double *a, const double *b, double *o)
 {
@@ -251,10 +253,10 @@ __global__ void k_op_copy_state(long long n, const double *a, const double *b, d
         for (int h = 0; h < 4; h += 2) {
             const double2 x = *reinterpret_cast<const double2 *>(a + i + h);
             const double2 y = *reinterpret_cast<const double2 *>(b + i + h);
-            *reinterpret_cast<double2 *>(o + i + h) = make_double2(keep_if_finite(x.x, y.x), keep_if_finite(x.y, y.y));
+            *reinterpret_cast<double2 *>(o + i + h) = make_double2(one_a_zero_b(x.x, y.x), one_a_zero_b(x.y, y.y));
         }
     } else {
-        for (long long q = i; q < n; ++q) o[q] = keep_if_finite(a[q], b[q]);
+        for (long long q = i; q < n; ++q) o[q] = one_a_zero_b(a[q], b[q]);
     }
 }
 __global__ void k_op_lincomb_theta(VGrid vg, int n_cond, DState o)

@@ -73,3 +73,21 @@ def test_pressure_gradient(setup):
     got = m.forcings["pressure_gradient_acc_neg_nl"].copy()
     o.manage_pressure_gradient(s)
     _same(got, m.forcings["pressure_gradient_acc_neg_nl"])
+
+
+def test_state_copy_is_the_linear_combination(setup):
+    """coefficients 1 and 0, the time loop's copy: 1 a + 0 b bit for bit, signed
+    zeros, infinities and NaN of either State included"""
+    m, g, _ = setup
+    v = np.array([0.0, -0.0, 1.5, -2.5, np.inf, -np.inf, np.nan, 5e-324, -5e-324])
+    a, b, out = m.state_old.clone(), m.state_old.clone(), m.state_old.clone()
+    for f in ("rho", "rhotheta_v", "exner_pert", "wind"):
+        n = a[f].size
+        a[f][:] = np.resize(np.repeat(v, v.size), n)
+        b[f][:] = np.resize(np.tile(v, v.size), n)
+    g.linear_combine_two_states(a, b, out, 1.0, 0.0)
+    for f in ("rho", "rhotheta_v", "exner_pert", "wind"):
+        with np.errstate(all="ignore"):
+            want = 1.0 * a[f] + 0.0 * b[f]
+        same = (out[f].view(np.uint64) == want.view(np.uint64)) | (np.isnan(out[f]) & np.isnan(want))
+        assert same.all(), (f, a[f][~same][:5], b[f][~same][:5], out[f][~same][:5])
