@@ -109,7 +109,7 @@ struct StepBufs {
     T *tri[2] = {}, *zh[2] = {}, *zv[2] = {}, *fh[2] = {}, *fv[2] = {}, *v2[2] = {};
     T *pvt[2] = {}, *v2g[2] = {}, *tend[2] = {};
     T *theta[2] = {}, *str[2] = {}, *strt[2] = {};
-    T *wl[2] = {}, *wr[2] = {};
+    T *wl[2] = {}, *wr[2] = {}; /* the bars': [0] alone */
     /* one block of every array above but so, sn2, wl and wr, so that the
      * backward step clears its bars with one memset; the last n_adv0 elements
      * are substage 0's advection, which only a first step has */
@@ -169,7 +169,7 @@ T *aalloc(AdjState *a, long long n)
 }
 
 template <class T>
-bool alloc_step(AdjState *a, StepBufs<T> &S)
+bool alloc_step(AdjState *a, StepBufs<T> &S, int waves)
 {
     bool ok = true;
     auto A = [&](T *&p, long long n) {
@@ -178,7 +178,7 @@ bool alloc_step(AdjState *a, StepBufs<T> &S)
     };
     A(S.so, a->nblk);
     A(S.sn2, a->nblk);
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < waves; ++r) {
         A(S.wl[r], WL_N * a->ns);
         A(S.wr[r], WR_N * a->nwi);
     }
@@ -248,7 +248,9 @@ int ensure_adj(Context *c)
     a->ntri = (long long)c->nl * c->nt;
     a->nzh = (long long)(c->nl + 1) * c->ne;
     a->nwi = (long long)(c->nl - 1) * c->nc;
-    bool ok = alloc_step(a, a->B) && alloc_step(a, a->Z) && alloc_step(a, a->D);
+    /* the tape keeps the sound-wave work of both substages, the bars have one
+     * substage's at a time (waves_bwd) */
+    bool ok = alloc_step(a, a->B, 2) && alloc_step(a, a->Z, 1) && alloc_step(a, a->D, 2);
     ok = ok && (a->rn_b = aalloc<double>(a, a->ns)) && (a->rtn_b = aalloc<double>(a, a->ns))
          && (a->db = aalloc<double>(a, a->nwi)) && (a->br = aalloc<double>(a, BR_N * a->nwi));
     ok = ok && (a->dden = aalloc<double>(a, a->nwi)) && (a->r_dden = aalloc<double>(a, a->nwi))
@@ -311,8 +313,8 @@ void waves_fwd(Context *c, AdjState *a, int rk, DState so, DState sn, DState ten
     w.th_int = wr + WR_TH * m; w.rho_io = wr + WR_RIO * m; w.r_rho_io = wr + WR_RRIO * m;
     k_waves_layer<true><<<nbk(ns), 256, 0, st>>>(c->vg, a->p, so, sn, tend, w, rk, theta);
     k_waves_rows<<<layer_grid(c->nl - 1, c->nc, 256), 256, 0, st>>>(c->vg, a->p, so, tend, w);
-    if (c->nl == 26)
-        fa_waves_thomas_fixed<26><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, a->dden, a->r_dden, wr);
+    if (c->nl == NL_FIXED)
+        fa_waves_thomas_fixed<NL_FIXED><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, a->dden, a->r_dden, wr);
     else
         fa_waves_thomas<double><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, wr);
     w.r = wr + WR_SOL * m; /* what the step leaves in r */
@@ -332,8 +334,8 @@ void tracers_fwd(Context *c, AdjState *a, int rk, DState so, DState out, double 
         c->kernel_launches++;
     }
     const DState tend{str, nullptr, nullptr, nullptr, nullptr, nullptr};
-    if (c->nl == 26)
-        k_tracers_solve<26, 26, true><<<nbk(nsys, 64), 64, 0, st>>>(c->vg, a->p, so, out, tend, tw, nullptr, Present{});
+    if (c->nl == NL_FIXED)
+        k_tracers_solve<NL_FIXED, NL_FIXED, true><<<nbk(nsys, 64), 64, 0, st>>>(c->vg, a->p, so, out, tend, tw, nullptr, Present{});
     else
         k_tracers_solve<0, MAX_L, true><<<nbk(nsys, 64), 64, 0, st>>>(c->vg, a->p, so, out, tend, tw, nullptr, Present{});
     c->kernel_launches++;
@@ -403,11 +405,10 @@ void substage_fwd(Context *c, AdjState *a, StepBufs<T> &B, int rk, bool first, c
         fa_waves_apply<T><<<nbk(ns), 256, 0, st>>>(vg, ap, so, B.wl[rk], B.wr[rk], out);
     }
     c->kernel_launches += adv ? 11 : 8;
-    if (moist) {
-        if constexpr (PLAIN) {
-            tracers_fwd(c, a, rk, dview(a, B.so), dview(a, rk ? B.sn2 : B.sn1), B.str[rk], B.pre, B.sed);
-            return;
-        }
+    if (!moist) return;
+    if constexpr (PLAIN) {
+        tracers_fwd(c, a, rk, dview(a, B.so), dview(a, rk ? B.sn2 : B.sn1), B.str[rk], B.pre, B.sed);
+    } else {
         if (rk == 0) {
             fa_sedheat<T><<<nbk(c->nc, 128), 128, 0, st>>>(vg, a->p, so, out.w, B.pre, B.sed);
             c->kernel_launches++;
@@ -470,8 +471,8 @@ void waves_bwd(Context *c, AdjState *a, int rk, AState<double> so, AState<double
     const dim3 cells = layer_grid(c->nl, c->nc, 256);
     ba_apply_state<<<cells, 256, 0, st>>>(vg, so, wl, wr, out, out_b, a->rn_b, a->rtn_b, a->db, so_b, wl_b, wr_b);
     ba_apply_rho<<<cells, 256, 0, st>>>(vg, a->p.dt, wr, a->rn_b, a->rtn_b, a->db, wl_b, wr_b);
-    if (c->nl == 26)
-        ba_thomas<26, 26><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, a->r_dden, wr, wr_b);
+    if (c->nl == NL_FIXED)
+        ba_thomas<NL_FIXED, NL_FIXED><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, a->r_dden, wr, wr_b);
     else
         ba_thomas<0, MAX_L><<<nbk(c->nc, 64), 64, 0, st>>>(c->nc, c->nl, a->dden, a->r_dden, wr, wr_b);
     ba_waves_rows<<<layer_grid(c->nl - 1, c->nc, 256), 256, 0, st>>>(vg, a->p, so, wl, wr, wr_b, a->br, so_b, tend_w_b);

@@ -493,8 +493,8 @@ int adj_gen_densities(Context *c, const StepParams &p, StateMirror *so, StateMir
     const dim3 boxes(nb(c->nc, 128), (unsigned)c->nl, (unsigned)n_tr);
     ka_gen_rows<<<boxes, 128, 0, c->stream>>>(c->vg, p, so->ds, sn->ds, st->ds, w);
     const unsigned cols = nb(nsys, 64);
-    if (c->nl == 26)
-        ka_gen_solve<26, 26><<<cols, 64, 0, c->stream>>>(c->nc, c->nl, n_tr, c->n_cond, w, sn_b->ds);
+    if (c->nl == NL_FIXED)
+        ka_gen_solve<NL_FIXED, NL_FIXED><<<cols, 64, 0, c->stream>>>(c->nc, c->nl, n_tr, c->n_cond, w, sn_b->ds);
     else if (c->nl <= 64)
         ka_gen_solve<0, 64><<<cols, 64, 0, c->stream>>>(c->nc, c->nl, n_tr, c->n_cond, w, sn_b->ds);
     else

@@ -613,7 +613,6 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
     c->energy_buf = dalloc<double>(c, 3 * (size_t)NS);
     c->wv_layer = dalloc<double>(c, 8 * (size_t)NS);
     c->wv_rows = dalloc<double>(c, 7 * (size_t)(L - 1) * NC);
-    c->damp_dc = dalloc<double>(c, (size_t)(L - 1) * NC);
     c->damp_inv = dalloc<double>(c, (size_t)(L - 1) * NC);
     c->damp_den = dalloc<double>(c, (size_t)(L - 1) * NC);
     c->pg_cell64 = dalloc<Quad>(c, NS);

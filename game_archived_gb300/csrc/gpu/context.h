@@ -164,11 +164,10 @@ struct Context {
         int launches; /* kernels in the graph */
     };
     std::map<GraphKey, GraphEntry> graphs;
-    /* Klemp damping coefficient of every inner interface [L-1][Nc] and
-     * 1 / (1 + dt * coefficient) for the values in damp_key (start height,
-     * maximum coefficient, dt) */
-    double *damp_dc = nullptr, *damp_inv = nullptr;
-    double *damp_den = nullptr; /* 1 + dt * coefficient */
+    /* 1 + dt * Klemp damping coefficient of every inner interface [L-1][Nc]
+     * and its reciprocal, for the values in damp_key (start height, maximum
+     * coefficient, dt) */
+    double *damp_den = nullptr, *damp_inv = nullptr;
     float2 *damp_inv_df = nullptr; /* damp_inv as double-float pairs */
     double damp_key[3] = {-1.0, -1.0, -1.0};
     /* grid terms of the mixed-path sound-wave rows [6][L-1][Nc] */

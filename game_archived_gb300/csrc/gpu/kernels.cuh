@@ -1695,6 +1695,9 @@ __global__ void __launch_bounds__(128)
 
 /* per-thread column sweeps of the adjoint hold at most this many layers */
 constexpr int MAX_L = 64;
+/* the layer count the register-resident column sweeps are compiled for
+ * (NO_OF_LAYERS of every GAME configuration) */
+constexpr int NL_FIXED = 26;
 
 }  // namespace
 }  // namespace game

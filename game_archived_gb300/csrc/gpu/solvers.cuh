@@ -49,12 +49,12 @@ struct WavesWork {
     const double *geo;
 };
 
-/* Klemp (2008) damping coefficient at inner interface j + 1 of every column
+/* 1 + dt times the Klemp (2008) damping coefficient at inner interface j + 1 of every column
  * (column_solvers.c:285-298).  It depends on the grid and the two damping
  * parameters only, so it is tabulated once per parameter pair instead of
  * once per substage. */
-__global__ void k_damping_table(VGrid vg, double start_height, double coeff_max, double dt, double *dc, double *den,
-                                double *inv_den, float2 *inv_den_df)
+__global__ void k_damping_table(VGrid vg, double start_height, double coeff_max, double dt, double *den, double *inv_den,
+                                float2 *inv_den_df)
 {
     const long long n = (long long)(vg.nl - 1) * vg.nc, q = gtid();
     if (q >= n) return;
@@ -65,7 +65,6 @@ __global__ void k_damping_table(VGrid vg, double start_height, double coeff_max,
         const double s = sin(0.5 * M_PI * zad / (vg.z_v[0] - start_height));
         r = coeff_max * (s * s);
     }
-    dc[q] = r;
     den[q] = 1.0 + dt * r;
     const double inv = 1.0 / den[q];
     inv_den[q] = inv;

@@ -29,9 +29,6 @@ inline Work<double> &work<double>(Context *c) { return c->w64; }
 template <>
 inline Work<float> &work<float>(Context *c) { return c->w32; }
 
-/* the layer count the register-resident column sweeps are compiled for
- * (NO_OF_LAYERS of every GAME configuration) */
-constexpr int NL_FIXED = 26;
 /* capacities of the local-memory sweeps for other layer counts */
 constexpr int SWEEP_SMALL = 64, SWEEP_LARGE = 256;
 /* the mixed path solves a batch of fewer systems than this with the warp
