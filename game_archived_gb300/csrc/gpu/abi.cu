@@ -265,6 +265,7 @@ int run_device_step(Context *c, const StepParams &p, StateMirror *so, StateMirro
     /* the damping table is read by the step's kernels: bring it up to date
      * outside any graph, before the first launch */
     if (launch_damping_table(c, p)) return -1;
+    if (c->precision == PREC_FP64 && ensure_f64(c, true)) return -1;
     auto launch = [&]() {
         return c->precision == PREC_FP64 ? launch_step_f64(c, p, so, sn, st) : launch_step_mixed(c, p, so, sn, st);
     };
@@ -680,7 +681,7 @@ static int grad_parts(double *in_field, double *out_field, struct grid *grid, in
     double *f = c->dev_tmp[0], *v = c->dev_tmp[1];
     if (upload_field(in_field, f, c->map_s, c->ns, c->ns)) return -1;
     if (vec_op_prologue(out_field, v)) return -1;
-    op_grad(c, f, v, parts);
+    if (op_grad(c, f, v, parts)) return -1;
     if (download_field(out_field, v, c->map_vec, c->nv, c->nv, 0, c->nv)) return -1;
     return finish();
 }
@@ -796,7 +797,7 @@ static int rel_vort_common(double *velocity_field, double *density_field, struct
     const long long ntri = (long long)c->nl * c->nt;
     double *wind = c->dev_tmp[0], *rel = c->dev_tmp[1], *tri = c->dev_tmp[2], *pv = c->dev_tmp[3];
     if (upload_field(velocity_field, wind, c->map_vec, c->nv, c->nv)) return -1;
-    op_rel_vort(c, wind, tri, rel);
+    if (op_rel_vort(c, wind, tri, rel)) return -1;
     if (download_field(member<double>(diagnostics, GAME_DIAGNOSTICS, "rel_vort_on_triangles"), tri, c->map_tri, ntri,
                        ntri, 0, ntri)) return -1;
     CK(cudaStreamSynchronize(c->stream));
@@ -998,7 +999,7 @@ int manage_pressure_gradient(struct state *state, struct grid *grid, struct dual
     if (up_vec(forcings, GAME_FORCINGS, "pressure_gradient_acc_neg_l", l)) return -1;
     if (up_vec(forcings, GAME_FORCINGS, "pgrad_acc_old", old)) return -1;
     StepParams p = params_from_config(c, config, 1.0);
-    sub_pressure_gradient(c, p, &b.sn, nl, l, old, b.decel);
+    if (sub_pressure_gradient(c, p, &b.sn, nl, l, old, b.decel)) return -1;
     if (down_vec(forcings, GAME_FORCINGS, "pgrad_acc_old", old)) return -1;
     if (down_vec(forcings, GAME_FORCINGS, "pressure_gradient_acc_neg_nl", nl)) return -1;
     if (down_vec(forcings, GAME_FORCINGS, "pressure_gradient_acc_neg_l", l)) return -1;
@@ -1050,11 +1051,11 @@ int vector_tendencies_expl(struct state *state, struct state *state_tendency, st
         double *wind = b.sn.ds.w, *rho_gas = b.sn.ds.rho + (long long)c->n_cond * ns;
         if (up_vec(diagnostics, GAME_DIAGNOSTICS, "flux_density", flux)) return -1;
         op_scalar_times_vector(c, rho_gas, wind, flux, OP_STV_H | OP_STV_V);
-        op_rel_vort(c, wind, b.tri, rel);
+        if (op_rel_vort(c, wind, b.tri, rel)) return -1;
         op_pot_vort(c, rel, rho_gas, pv);
         op_vorticity_flux(c, flux, pv, pvt);
         op_inner_product(c, wind, wind, b.v2);
-        op_grad(c, b.v2, v2g, OP_GRAD_H | OP_GRAD_V | OP_GRAD_CON);
+        if (op_grad(c, b.v2, v2g, OP_GRAD_H | OP_GRAD_V | OP_GRAD_CON)) return -1;
         if (down_vec(diagnostics, GAME_DIAGNOSTICS, "flux_density", flux)) return -1;
         if (download_field(vec_of(diagnostics, GAME_DIAGNOSTICS, "rel_vort_on_triangles"), b.tri, c->map_tri, ntri,
                            ntri, 0, ntri))
@@ -1097,8 +1098,9 @@ int scalar_tendencies_expl(struct state *state_old, struct state *state, struct 
         if (up_scal(irrev, GAME_IRREV, "condensates_sediment_heat", b.sed_heat)) return -1;
     }
     StepParams p = params_from_config(c, config, delta_t);
-    sub_scalar_tendencies(c, p, &b.sn, &b.st, rk_step, b.theta, b.cp_ice, b.cp_water, b.pt_rates, b.pt_heat,
-                          b.sed_heat);
+    if (sub_scalar_tendencies(c, p, &b.sn, &b.st, rk_step, b.theta, b.cp_ice, b.cp_water, b.pt_rates, b.pt_heat,
+                              b.sed_heat))
+        return -1;
     if (download_state(state_tendency, &b.st, 1 | 2)) return -1;
     return finish();
 }
@@ -1341,7 +1343,7 @@ int calc_pot_vort_adj(double *velocity_field, double *density_field, double *pot
     double *wind = v[0], *rho = v[1], *rel = v[2], *pv = v[3], *pvb = v[4], *zero_u = v[5], *wb = v[6], *rb = v[7],
            *trib = v[8];
     if (up(velocity_field, wind, c->map_vec, c->nv) || up(density_field, rho, c->map_s, c->ns)) return -1;
-    op_rel_vort(c, wind, c->sub.tri, rel);
+    if (op_rel_vort(c, wind, c->sub.tri, rel)) return -1;
     op_pot_vort(c, rel, rho, pv);
     if (up(pot_vort_bar, pvb, c->map_curl, c->ncurl) || up(velocity_field_bar, wb, c->map_vec, c->nv)
         || up(density_field_bar, rb, c->map_s, c->ns))

@@ -229,6 +229,7 @@ void adj_release_fn(Context *c)
 
 int ensure_adj(Context *c)
 {
+    if (ensure_f64(c, true)) return -1;
     if (c->adj) return 0;
     if (c->n_const != 1 && c->n_const != 6)
         return fail("adjoint: the adjoint and tangent-linear models cover the dry build and the moist build of six "

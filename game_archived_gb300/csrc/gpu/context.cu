@@ -615,10 +615,6 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
     c->wv_rows = dalloc<double>(c, 7 * (size_t)(L - 1) * NC);
     c->damp_inv = dalloc<double>(c, (size_t)(L - 1) * NC);
     c->damp_den = dalloc<double>(c, (size_t)(L - 1) * NC);
-    c->pg_cell64 = dalloc<Quad>(c, NS);
-    c->level_q64 = dalloc<double>(c, (size_t)2 * (L + 1) * NC);
-    c->gas_share64 = dalloc<double>(c, NS);
-    c->grad_pi_v = dalloc<double>(c, (size_t)(L + 1) * NC);
     {
         std::vector<double> iv(h_vol.size()), ia(h_areav.size());
         for (size_t k = 0; k < iv.size(); ++k) iv[k] = 1.0 / h_vol[k];
@@ -673,27 +669,11 @@ int init_context(int res_id, int n_layers, int moisture_on, const void *grid_p, 
     };
     work(c->w64, double(0));
     work(c->w32, float(0));
-    {
-        /* the FP64 path's tables: reciprocals and products of grid quantities */
-        HGrid<double> &g = c->hg64;
-        g.r_nd_v = dalloc<double>(c, (size_t)(L + 1) * NC);
-        g.r_nd_h = dalloc<double>(c, (size_t)L * NE);
-        g.r_dual_area_h = dalloc<double>(c, (size_t)(L + 1) * NE);
-        g.r_dual_area_t = dalloc<double>(c, (size_t)L * NT);
-        g.r_dz_h = dalloc<double>(c, (size_t)(L + 1) * NE);
-        g.rhombus_area = dalloc<double>(c, (size_t)L * NE);
-        g.r_rhombus_area = dalloc<double>(c, (size_t)L * NE);
-        g.tri_circ = dalloc<double>(c, (size_t)3 * L * NT);
-        g.corr_w = dalloc<double>(c, (size_t)6 * NS);
-        c->edge_flux64 = dalloc<double>(c, (size_t)2 * L * NE);
-        c->level_corr64 = dalloc<double>(c, (size_t)3 * (L + 1) * NC);
-    }
     /* before the first kernel: none may run on a pointer that is missing */
     if (c->alloc_failed) {
         cudaGetLastError();
         return fail("device allocation failed");
     }
-    if (make_f64_tables(c)) return -1;
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
@@ -800,6 +780,42 @@ int ensure_diff_buffers(Context *c)
     };
     for (auto &w : want)
         if (!(*w.p = dalloc<double>(c, w.n))) return fail("device allocation of the diffusion fields failed");
+    return 0;
+}
+
+int ensure_f64(Context *c, bool work)
+{
+    if (c->f64_tables && (!work || c->f64_work)) return 0;
+    HGrid<double> &g = c->hg64;
+    const size_t NS = (size_t)c->ns, V = (size_t)(c->nl + 1) * c->nc, U = (size_t)c->nl * c->ne;
+    const size_t Z = (size_t)(c->nl + 1) * c->ne, T = (size_t)c->nl * c->nt;
+    bool ok = true;
+    auto want = [&](auto *&p, size_t n) {
+        using E = std::remove_const_t<std::remove_reference_t<decltype(*p)>>;
+        if (!p) ok = (p = dalloc<E>(c, n)) && ok;
+    };
+    if (!c->f64_tables) {
+        want(g.r_nd_v, V); want(g.r_nd_h, U); want(g.r_dual_area_h, Z); want(g.r_dual_area_t, T);
+        want(g.r_dz_h, Z); want(g.rhombus_area, U); want(g.r_rhombus_area, U); want(g.tri_circ, 3 * T);
+    }
+    if (work) {
+        want(c->pg_cell64, NS); want(c->level_q64, 2 * V); want(c->gas_share64, NS); want(c->grad_pi_v, V);
+        want(c->edge_flux64, 2 * U);
+        if (c->n_tilt) { /* the terrain corrections of the tilted columns */
+            want(g.corr_w, 6 * NS);
+            want(c->level_corr64, 3 * V);
+        }
+    }
+    if (!ok) {
+        cudaGetLastError(); /* reported here, not by the next call */
+        return fail("device allocation of the FP64 path's tables and work arrays failed");
+    }
+    if (!c->f64_tables && make_f64_tables(c)) return -1;
+    c->f64_tables = true;
+    if (work && !c->f64_work) {
+        if (c->n_tilt && make_f64_corr_weights(c)) return -1;
+        c->f64_work = true;
+    }
     return 0;
 }
 

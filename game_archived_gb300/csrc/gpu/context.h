@@ -105,6 +105,7 @@ struct Context {
     float4 *pg_cell = nullptr;
     /* FP64 path: the same factors in double, and the vertical gradient of
      * Pi' at the inner interfaces [L+1][Nc] */
+    bool f64_tables = false, f64_work = false; /* ensure_f64 */
     Quad *pg_cell64 = nullptr;
     double *level_q64 = nullptr;  /* k_level_terms' mass-flux factors [2][L+1][Nc] */
     double *gas_share64 = nullptr; /* rho_gas / rho_total at rk 1 [L][Nc] */
@@ -269,9 +270,17 @@ int upload_field(const double *host, double *dev, const int *map, long long n, l
 int download_field(double *host, const double *dev, const int *map, long long n, long long host_len,
                    long long host_lo, long long host_hi);
 
-/* the FP64 path's reciprocal and product tables of the context's grid
- * (tables_f64.cu), from the tables already on the device */
+/* the FP64 path's reciprocal and product tables of the context's grid and
+ * its terrain-correction weights (tables_f64.cu), from the tables already on
+ * the device */
 int make_f64_tables(Context *c);
+int make_f64_corr_weights(Context *c);
+/* these tables (the operators, the output pass) and with work the work arrays
+ * of the FP64 step too (the step, the tendencies, the adjoint), before their
+ * first use and outside any graph: a run that stays mixed has neither, 47
+ * doubles per cell and layer less (38 on a flat grid; RES_ID 7 with the
+ * mountain: 1.6 GB) */
+int ensure_f64(Context *c, bool work);
 
 /* the mixed step's lagged fields in its FP32 work arrays (aux.cu), from and to
  * device vector fields [w (L+1) Nc][u L Ne] of doubles: P the pressure

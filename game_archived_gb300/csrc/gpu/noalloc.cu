@@ -8,8 +8,9 @@
  * next step overlapping the current one, other libraries' work) would stall
  * all of them for one diagnostic; and an application that has handed its
  * device memory to its own pool up front has nothing left for a library to
- * take.  The context-based entry points allocate only in game_gpu_init, but
- * they need that context and host buffers; this entry point needs neither.
+ * take.  The context-based entry points allocate in game_gpu_init (and once
+ * more where a call first needs more: another State, the FP64 step, an adjoint
+ * window, an output pass) and need host buffers; this entry point does neither.
  *
  * Scratch.  The reduction needs, per field, one (hi, lo) pair of doubles per
  * block and one counter.  They live in the file-scope array below, fixed at

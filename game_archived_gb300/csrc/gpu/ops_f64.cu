@@ -304,13 +304,15 @@ void op_add_vertical_divv(Context *c, const double *vec, double *out)
     c->kernel_launches++;
 }
 
-void op_grad(Context *c, const double *f, double *vec, int parts)
+int op_grad(Context *c, const double *f, double *vec, int parts)
 {
+    if (ensure_f64(c, false)) return -1;
     double *w = vec, *u = vec + (long long)(c->nl + 1) * c->nc;
     if (parts & OP_GRAD_V) k_op_grad_v<<<nb((long long)(c->nl - 1) * c->nc), 256, 0, c->stream>>>(c->hg64, f, w);
     if (parts & OP_GRAD_H)
         k_op_grad_h<<<nb((long long)c->nl * c->ne), 256, 0, c->stream>>>(c->hg64, f, u, (parts & OP_GRAD_CON) ? 1 : 0);
     c->kernel_launches += 2;
+    return 0;
 }
 
 void op_cov_to_con(Context *c, double *vec)
@@ -344,12 +346,14 @@ void op_inner_product(Context *c, const double *a, const double *b, double *out)
     c->kernel_launches++;
 }
 
-void op_rel_vort(Context *c, const double *wind, double *tri, double *curl)
+int op_rel_vort(Context *c, const double *wind, double *tri, double *curl)
 {
+    if (ensure_f64(c, false)) return -1;
     const long long off = (long long)(c->nl + 1) * c->nc, coff = (long long)(c->nl + 1) * c->ne;
     k_tri_vort<double, true><<<dim3(nb(c->nt), (unsigned)c->nl), 256, 0, c->stream>>>(c->hg64, wind + off, tri);
     k_op_rel_vort<<<nb(coff), 256, 0, c->stream>>>(c->hg64, wind + off, wind, tri, curl, curl + coff);
     c->kernel_launches += 2;
+    return 0;
 }
 
 void op_pot_vort(Context *c, const double *rel, const double *rho, double *pv)

@@ -105,9 +105,10 @@ __global__ void k_sub_cp_tables(long long ns, const double *t, double *cp_ice, d
 
 }  // namespace
 
-void sub_pressure_gradient(Context *c, const StepParams &p, StateMirror *s, double *p_nl, double *p_l, double *pg_old,
-                           double *decel)
+int sub_pressure_gradient(Context *c, const StepParams &p, StateMirror *s, double *p_nl, double *p_l, double *pg_old,
+                          double *decel)
 {
+    if (ensure_f64(c, false)) return -1;
     const long long nv = c->nv;
     SView<double> sv{s->ds.rho, s->ds.rhotheta_v, s->ds.theta_v_pert, s->ds.exner_pert, s->ds.w, s->ds.u};
     if (!p.first_step) k_sub_neg_sum<<<nblocks(nv, 256), 256, 0, c->stream>>>(nv, p_nl, p_l, pg_old);
@@ -115,6 +116,7 @@ void sub_pressure_gradient(Context *c, const StepParams &p, StateMirror *s, doub
     k_sub_decel<<<nblocks(c->ns, 256), 256, 0, c->stream>>>(c->ns, s->ds.rho, c->n_const, c->n_cond, 0, decel);
     if (p.first_step) k_sub_neg_sum<<<nblocks(nv, 256), 256, 0, c->stream>>>(nv, p_nl, p_l, pg_old);
     c->kernel_launches += 3;
+    return 0;
 }
 
 void sub_condensates_v(Context *c, StateMirror *s, double *decel, double *cond_v)
@@ -142,15 +144,17 @@ void sub_cp_tables(Context *c, const double *temperature, double *cp_ice, double
     c->kernel_launches++;
 }
 
-void sub_scalar_tendencies(Context *c, const StepParams &p, StateMirror *sn, StateMirror *st, int rk, double *theta,
-                           const double *cp_ice, const double *cp_water, const double *pt_rates,
-                           const double *pt_heat, const double *sed_heat)
+int sub_scalar_tendencies(Context *c, const StepParams &p, StateMirror *sn, StateMirror *st, int rk, double *theta,
+                          const double *cp_ice, const double *cp_water, const double *pt_rates,
+                          const double *pt_heat, const double *sed_heat)
 {
+    if (ensure_f64(c, true)) return -1;
     const Views<double> v = views<double>(c, sn);
     k_theta<double><<<nblocks(c->ns, 256), 256, 0, c->stream>>>(c->nl, c->nc, c->n_cond, v.sv, theta);
     launch_scalar_tend64(c, p, v.sv, st->ds.rho, st->ds.rho, st->ds.rhotheta_v, theta, cp_ice, cp_water, pt_rates,
                          pt_heat, sed_heat, rk, IrrTerms{});
     c->kernel_launches++;
+    return 0;
 }
 
 int sub_ver_waves(Context *c, const StepParams &p, StateMirror *so, StateMirror *sn, StateMirror *st, int rk)

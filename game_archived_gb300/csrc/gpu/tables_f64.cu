@@ -69,21 +69,27 @@ __global__ void k_corr_w(HGrid<double> g, double *w)
 int make_f64_tables(Context *c)
 {
     const HGrid<double> &g = c->hg64;
+    cudaStream_t st = c->stream;
     const long long nwc = (long long)(c->nl + 1) * c->nc, nze = (long long)(c->nl + 1) * c->ne;
     const long long nue = (long long)c->nl * c->ne, ntt = (long long)c->nl * c->nt;
     auto rcp = [&](long long n, const double *x, const double *r) {
-        k_reciprocal<<<(unsigned)((n + 255) / 256), 256>>>(n, x, const_cast<double *>(r));
+        k_reciprocal<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, x, const_cast<double *>(r));
     };
     rcp(nwc, g.nd_v, g.r_nd_v);
     rcp(nue, g.nd_h, g.r_nd_h);
     rcp(nze, g.dual_area_h, g.r_dual_area_h);
     rcp(ntt, g.dual_area_t, g.r_dual_area_t);
-    k_r_dz_h<<<layer_grid(c->nl + 1, c->ne, 256), 256>>>(g, const_cast<double *>(g.r_dz_h));
-    k_rhombus_area<<<layer_grid(c->nl, c->ne, 256), 256>>>(g, const_cast<double *>(g.rhombus_area),
-                                              const_cast<double *>(g.r_rhombus_area));
-    k_tri_circ<<<layer_grid(c->nl, c->nt, 256), 256>>>(g, const_cast<double *>(g.tri_circ));
-    k_corr_w<<<layer_grid(c->nl, c->nc, 256), 256>>>(g, const_cast<double *>(g.corr_w));
-    CK(cudaDeviceSynchronize());
+    k_r_dz_h<<<layer_grid(c->nl + 1, c->ne, 256), 256, 0, st>>>(g, const_cast<double *>(g.r_dz_h));
+    k_rhombus_area<<<layer_grid(c->nl, c->ne, 256), 256, 0, st>>>(g, const_cast<double *>(g.rhombus_area),
+                                                                  const_cast<double *>(g.r_rhombus_area));
+    k_tri_circ<<<layer_grid(c->nl, c->nt, 256), 256, 0, st>>>(g, const_cast<double *>(g.tri_circ));
+    CK(cudaGetLastError());
+    return 0;
+}
+
+int make_f64_corr_weights(Context *c)
+{
+    k_corr_w<<<layer_grid(c->nl, c->nc, 256), 256, 0, c->stream>>>(c->hg64, const_cast<double *>(c->hg64.corr_w));
     CK(cudaGetLastError());
     return 0;
 }

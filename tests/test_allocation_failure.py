@@ -97,3 +97,42 @@ m.config["momentum_diff_h"] = 1
 g.manage_rkhevi(100.0, 0.0)
 assert fake.fake_unordered_clears() == 0, fake.fake_unordered_clears()
 """)
+
+
+def test_a_mixed_run_holds_nothing_of_the_fp64_path():
+    """the FP64 path's tables come with the first operator that reads them, its
+    work arrays with the first FP64 step, once; without memory for them that
+    call fails and the mixed step goes on"""
+    fakecuda.run("""
+for mountain in (False, True):
+    _, m = make_model(3, 1, "jet_moist", mountain=mountain)
+    lay = m.layout
+    g = abi.GpuModel(m, abi.MIXED, resident=True)
+    for s in (m.state_old, m.state_new, m.state_tendency):
+        g.sync_to_device(s)
+    bytes_ = fake.fake_live_bytes
+    n, start = fake.fake_mallocs(), bytes_()
+    for _ in range(2):
+        g.manage_rkhevi(100.0, 0.0)
+    assert fake.fake_mallocs() - n <= 1 and bytes_() == start, (fake.fake_mallocs() - n, bytes_() - start)
+    lib.game_gpu_set_precision(abi.FP64)
+    fake.fake_fail_malloc(3, 0)
+    try:
+        g.manage_rkhevi(100.0, 0.0)
+        assert False
+    except abi.GpuError as e:
+        assert "FP64 path" in str(e), e
+    fake.fake_fail_malloc(-1, 0)
+    lib.game_gpu_set_precision(abi.MIXED)
+    g.manage_rkhevi(100.0, 0.0)
+    lib.game_gpu_set_precision(abi.FP64)
+    g.manage_rkhevi(100.0, 0.0)
+    per_box = (bytes_() - start) / 8 / (lay.nl * lay.nc)
+    assert (46 if mountain else 37) < per_box < (50 if mountain else 40), per_box
+    n = fake.fake_mallocs()
+    g.manage_rkhevi(100.0, 0.0)
+    lib.game_gpu_set_precision(abi.MIXED)
+    g.manage_rkhevi(100.0, 0.0)
+    assert fake.fake_mallocs() == n
+    g.close()
+""")
