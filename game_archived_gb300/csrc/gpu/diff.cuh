@@ -34,6 +34,15 @@
  *                    every density, their divergences
  * Device layout: scalar [L][Nc], vector [w (L+1)][Nc] then [u L][Ne],
  * triangle [L][Nt].
+ *
+ * Conversions between the carried doubles and R go by the instruction: a few
+ * per point, whose FP64 issue hides behind the gathers, while the integer form
+ * (to_float) lengthens every chain (RES_ID 6, mixed: kd_wdiff_b 39.2 -> 31.8 us,
+ * kd_dissipation 38.7 -> 34.9, kd_sdiff_coeff 28.8 -> 23.5, kd_fric_h 183 -> 168;
+ * RES_ID 3: kd_n2_adv 24.6 -> 18.4).  The two kernels that gain from the integer
+ * form keep it: the scalar fluxes, which take up to ten temperatures per edge
+ * (RES_ID 6 with the mountain, 190 us against 277), and kd_hor_visc (39.4
+ * against 43.0).
  */
 #pragma once
 
@@ -145,9 +154,9 @@ __global__ void kd_n2_adv(HGrid<R> g, SView<R> sv, DiffBufs b, DiffScratch<R> s)
         return g.gravity_m_v[(long long)k * nc + c] * (scal * gr);
     };
     if (l == 0)
-        b.n2[i] = wide(nsq(1));
+        b.n2[i] = double(nsq(1));
     else if (l < nl - 1)
-        b.n2[i] = wide(ipw_at(g, 6, l, c) * nsq(l) + ipw_at(g, 7, l, c) * nsq(l + 1));
+        b.n2[i] = double(ipw_at(g, 6, l, c) * nsq(l) + ipw_at(g, 7, l, c) * nsq(l + 1));
     /* advection of the TKE */
     const int n_edges = c < N_PENT ? 5 : 6;
     R r = R(0);
@@ -155,8 +164,8 @@ __global__ void kd_n2_adv(HGrid<R> g, SView<R> sv, DiffBufs b, DiffScratch<R> s)
         const int e = g.adj[j * nc + c];
         r += ipw_at(g, j, l, c) * grad_h(g, b.tke, l, e) * sv.u[(long long)l * g.ne + e];
     }
-    const R a_top = l >= 1 ? grad_v(g, b.tke, l, c) : as<R>(b.ph_tb[c]);
-    const R a_bot = l + 1 <= nl - 1 ? grad_v(g, b.tke, l + 1, c) : as<R>(b.ph_tb[nc + c]);
+    const R a_top = l >= 1 ? grad_v(g, b.tke, l, c) : R(b.ph_tb[c]);
+    const R a_bot = l + 1 <= nl - 1 ? grad_v(g, b.tke, l + 1, c) : R(b.ph_tb[nc + c]);
     r += ipw_at(g, 6, l, c) * a_top * sv.w[i];
     r += ipw_at(g, 7, l, c) * a_bot * sv.w[i + nc];
     s.adv[i] = r;
@@ -169,11 +178,11 @@ __global__ void kd_tke(long long ns, int gas, R dt, R mean_velocity_area, SView<
     const long long i = gtid();
     if (i >= ns) return;
     const R rg = sv.rho[gas * ns + i];
-    const R decay = R(8.0 * (PI_ * PI_)) / mean_velocity_area * as<R>(b.visc[i]) / rg;
-    const R tke = as<R>(b.tke[i]);
-    R t = tke + dt * (-s.adv[i] + as<R>(b.hdiss[i]) / rg - decay * tke);
+    const R decay = R(8.0 * (PI_ * PI_)) / mean_velocity_area * R(b.visc[i]) / rg;
+    const R tke = R(b.tke[i]);
+    R t = tke + dt * (-s.adv[i] + R(b.hdiss[i]) / rg - decay * tke);
     if (t < R(0)) t = R(0);
-    b.tke[i] = wide(t);
+    b.tke[i] = double(t);
 }
 
 /* hor_viscosity (effective_diff_coeffs.c:19-112) at the cells: vint is the
@@ -283,7 +292,7 @@ __device__ __forceinline__ R vert_hor_viscosity(const HGrid<R> &g, const DiffBuf
     const long long f1 = (long long)k * nc + g.from[e], t1 = (long long)k * nc + g.to[e];
     const R *kv = s.kvt;
     R mdc = R(0.25) * (kv[f0] + kv[t0] + kv[f1] + kv[t1]);
-    const R molecular_viscosity = R(0.25) * (as<R>(b.mol[f0]) + as<R>(b.mol[t0]) + as<R>(b.mol[f1]) + as<R>(b.mol[t1]));
+    const R molecular_viscosity = R(0.25) * (R(b.mol[f0]) + R(b.mol[t0]) + R(b.mol[f1]) + R(b.mol[t1]));
     mdc += molecular_viscosity;
     return R(0.25) * (rg[f0] + rg[t0] + rg[f1] + rg[t1]) * mdc;
 }
@@ -295,7 +304,7 @@ __device__ __forceinline__ R dv_hdz(const HGrid<R> &g, const DiffGrid<R> &dg, co
                                     int k, int e)
 {
     const long long ne = g.ne;
-    if (k == 0) return as<R>(b.dvdz_top[e]);
+    if (k == 0) return R(b.dvdz_top[e]);
     if (k == g.nl) {
         const long long q = (long long)(g.nl - 1) * ne + e, sfc = (long long)g.nl * g.nc;
         return sv.u[q] / (g.z_h[q] - R(0.5) * (dg.z_v[sfc + g.from[e]] + dg.z_v[sfc + g.to[e]]));
@@ -323,7 +332,7 @@ __global__ void kd_fric_h(HGrid<R> g, DiffGrid<R> dg, int n_const, int gas, SVie
         const R cu = curl_of_vorticity(g, dg, s, l, e);
         fa = (gr - cu) / (R(0.5) * (density_total_r(sv.rho, n_const, ns, f) + density_total_r(sv.rho, n_const, ns, t)));
     } else {
-        fa = as<R>(b.fric[nw + i]);
+        fa = R(b.fric[nw + i]);
     }
     if (V) {
         const R *rg = sv.rho + gas * ns;
@@ -335,7 +344,7 @@ __global__ void kd_fric_h(HGrid<R> g, DiffGrid<R> dg, int n_const, int gas, SVie
               / delta_z
               / (R(0.5) * (density_total_r(sv.rho, n_const, ns, f) + density_total_r(sv.rho, n_const, ns, t)));
     }
-    b.fric[nw + i] = wide(fa);
+    b.fric[nw + i] = double(fa);
 }
 
 /* diffusion of w, step a (momentum_diff_diss.c:137-150 and 153-166):
@@ -353,9 +362,9 @@ __global__ void kd_wdiff_a(HGrid<R> g, DiffGrid<R> dg, int gas, SView<R> sv, Dif
     const R lo = l == nl - 1 ? R(0) : sv.w[(long long)(l + 1) * nc + c];
     const R comp_v = up * g.area_v[(long long)l * nc + c] - lo * g.area_v[(long long)(l + 1) * nc + c];
     const R dwdz = R(0) + R(1) / g.volume[i] * comp_v;
-    const R kv = tke2vert(as<R>(b.tke[i]), as<R>(b.n2[i]), dg.layer_thickness[i]);
+    const R kv = tke2vert(R(b.tke[i]), R(b.n2[i]), dg.layer_thickness[i]);
     s.kvt[i] = kv;
-    const R mdc = as<R>(b.mol[i]) + kv;
+    const R mdc = R(b.mol[i]) + kv;
     s.s1[i] = sv.rho[gas * ns + i] * mdc * dwdz;
     s.s2[i] = ipw_at(g, 6, l, c) * sv.w[(long long)l * nc + c] + ipw_at(g, 7, l, c) * sv.w[(long long)(l + 1) * nc + c];
 }
@@ -368,7 +377,7 @@ __global__ void kd_wdiff_b(HGrid<R> g, DiffBufs b, DiffScratch<R> s)
     if (i >= n) return;
     const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     const long long o = (long long)l * g.nc;
-    s.flx[i] = R(0.5) * (as<R>(b.visc[o + g.from[e]]) + as<R>(b.visc[o + g.to[e]])) * grad_h(g, s.s2, l, e);
+    s.flx[i] = R(0.5) * (R(b.visc[o + g.from[e]]) + R(b.visc[o + g.to[e]])) * grad_h(g, s.s2, l, e);
 }
 
 /* step c (:184): divergence of the diffusive flux */
@@ -394,7 +403,7 @@ __global__ void kd_wdiff_d(HGrid<R> g, int n_const, SView<R> sv, DiffBufs b, Dif
     R fa = (s.s1[up] - s.s1[lo]) / g.nd_v[(long long)k * nc + c];
     fa += R(0.5) * (s.s3[up] + s.s3[lo]);
     fa = fa / (R(0.5) * (density_total_r(sv.rho, n_const, ns, up) + density_total_r(sv.rho, n_const, ns, lo)));
-    b.fric[(long long)k * nc + c] = wide(fa);
+    b.fric[(long long)k * nc + c] = double(fa);
 }
 
 /* simple_dissipation_rate (momentum_diff_diss.c:296-310) */
@@ -409,11 +418,11 @@ __global__ void kd_dissipation(HGrid<R> g, int n_const, SView<R> sv, DiffBufs b)
     R r = R(0);
     for (int j = 0; j < n_edges; ++j) {
         const long long vi = (long long)l * g.ne + g.adj[j * nc + c];
-        r += ipw_at(g, j, l, c) * sv.u[vi] * as<R>(b.fric[nw + vi]);
+        r += ipw_at(g, j, l, c) * sv.u[vi] * R(b.fric[nw + vi]);
     }
-    r += ipw_at(g, 6, l, c) * sv.w[i] * as<R>(b.fric[i]);
-    r += ipw_at(g, 7, l, c) * sv.w[i + nc] * as<R>(b.fric[i + nc]);
-    b.hdiss[i] = wide(-density_total_r(sv.rho, n_const, ns, i) * r);
+    r += ipw_at(g, 6, l, c) * sv.w[i] * R(b.fric[i]);
+    r += ipw_at(g, 7, l, c) * sv.w[i + nc] * R(b.fric[i + nc]);
+    b.hdiss[i] = double(-density_total_r(sv.rho, n_const, ns, i) * r);
 }
 
 /* ------------------------------------------------- Held-Suarez forcing */
@@ -435,7 +444,7 @@ __global__ void kd_pbl_hs_cell(HGrid<R> g, DiffGrid<R> dg, int gas, int moist, c
     s.hs_p[i] = p;
     if (l == nl - 1) {
         const R lapse = R(0.0065);
-        const R temp_lowest_layer = as<R>(temperature[i]);
+        const R temp_lowest_layer = R(temperature[i]);
         const R temp_surface = temp_lowest_layer + lapse * (dg.z_scalar[i] - dg.z_v[(long long)nl * g.nc + c]);
         R gas_constant = R(R_D);
         if (moist) {
@@ -462,8 +471,8 @@ __global__ void kd_pbl_hs(HGrid<R> g, SView<R> sv, DiffBufs b, DiffScratch<R> s)
     const R pressure = R(0.5) * (s.hs_p[o + g.from[e]] + s.hs_p[o + g.to[e]]);
     const R pressure_sfc = R(0.5) * (s.hs_ps[g.from[e]] + s.hs_ps[g.to[e]]);
     const R sigma = pressure / pressure_sfc, sigma_b = R(0.7);
-    const R fa = as<R>(b.fric[nw + i]) + -R(1.0 / 86400.0) * fmax(R(0), (sigma - sigma_b) / (R(1) - sigma_b)) * sv.u[i];
-    b.fric[nw + i] = wide(fa);
+    const R fa = R(b.fric[nw + i]) + -R(1.0 / 86400.0) * fmax(R(0), (sigma - sigma_b) / (R(1) - sigma_b)) * sv.u[i];
+    b.fric[nw + i] = double(fa);
 }
 
 /* Held-Suarez radiative forcing (src/radiation/held_suar.c:18-56), FP64 on
@@ -509,8 +518,8 @@ __global__ void kd_sdiff_coeff(long long ns, int n_cond, int moist, const R *lt,
 {
     const long long i = gtid();
     if (i >= ns) return;
-    const R mch = as<R>(b.visc[i]) / sv.rho[n_cond * ns + i];
-    const R mcv = as<R>(b.mol[i]) + tke2vert(as<R>(b.tke[i]), as<R>(b.n2[i]), lt[i]);
+    const R mch = R(b.visc[i]) / sv.rho[n_cond * ns + i];
+    const R mcv = R(b.mol[i]) + tke2vert(R(b.tke[i]), R(b.n2[i]), lt[i]);
     s.mch[i] = mch;
     s.mcv[i] = mcv;
     R cv = R(0);

@@ -45,7 +45,7 @@ template <typename R, typename F>
 __device__ __forceinline__ R grad_v(const HGrid<R> &g, const F *f, int k, int c)
 {
     const long long i = (long long)k * g.nc + c;
-    return div_tab(as<R>(f[i - g.nc]) - as<R>(f[i]), g.nd_v, g.r_nd_v, i);
+    return div_tab(R(f[i - g.nc]) - R(f[i]), g.nd_v, g.r_nd_v, i);
 }
 
 /* Slopes and height differences are exactly 0 away from orography, and what
@@ -86,7 +86,7 @@ __device__ __forceinline__ R grad_h(const HGrid<R> &g, const F *f, int l, int e)
 {
     const int fr = g.from[e], to = g.to[e];
     const long long le = (long long)l * g.ne + e;
-    R out = div_tab(as<R>(f[(long long)l * g.nc + to]) - as<R>(f[(long long)l * g.nc + fr]), g.nd_h, g.r_nd_h, le);
+    R out = div_tab(R(f[(long long)l * g.nc + to]) - R(f[(long long)l * g.nc + fr]), g.nd_h, g.r_nd_h, le);
     if (l >= g.nl - g.n_oro) {
         /* a zero slope adds a zero */
         if (!ALL && zero_slope(g.slope_h[le])) return out;

@@ -146,9 +146,11 @@ __device__ __forceinline__ bool nonneg(double x)
  * from FP64 results, to keep the conversion off the FP64 pipe (one warp
  * instruction per 16 cycles).  No case may use the conversion instruction: the
  * compiler runs it ahead of the test that guards it, so a fallback costs every
- * value its FP64 issue.  Without it k_make_shadow's FP64 issue falls from 16 us
- * to 0 and its time from 37 to 34 us, k_cell_prepare_f32's from 31 to 5 us and
- * 59.5 to 57.7 us, the scalar tendencies take 141 us for 147 (RES_ID 6). */
+ * value its FP64 issue.  RES_ID 6, against the form with a fallback in the same
+ * tree: k_make_shadow 39.0 -> 36.1 us, k_cell_prepare_f32 58.7 -> 56.6 us.
+ * Where a kernel converts a value or two per point beside gathers that wait
+ * for L2, the instruction's issue hides and the longer code does not: most of
+ * the diffusion kernels convert by the instruction (diff.cuh). */
 __device__ __forceinline__ float to_float(double x)
 {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x), m = b & 0xfffffffffffffULL;
