@@ -681,7 +681,7 @@ static int grad_parts(double *in_field, double *out_field, struct grid *grid, in
     double *f = c->dev_tmp[0], *v = c->dev_tmp[1];
     if (upload_field(in_field, f, c->map_s, c->ns, c->ns)) return -1;
     if (vec_op_prologue(out_field, v)) return -1;
-    if (op_grad(c, f, v, parts)) return -1;
+    if (op_grad(c, f, v, parts, true)) return -1;
     if (download_field(out_field, v, c->map_vec, c->nv, c->nv, 0, c->nv)) return -1;
     return finish();
 }
@@ -797,7 +797,7 @@ static int rel_vort_common(double *velocity_field, double *density_field, struct
     const long long ntri = (long long)c->nl * c->nt;
     double *wind = c->dev_tmp[0], *rel = c->dev_tmp[1], *tri = c->dev_tmp[2], *pv = c->dev_tmp[3];
     if (upload_field(velocity_field, wind, c->map_vec, c->nv, c->nv)) return -1;
-    if (op_rel_vort(c, wind, tri, rel)) return -1;
+    if (op_rel_vort(c, wind, tri, rel, true)) return -1;
     if (download_field(member<double>(diagnostics, GAME_DIAGNOSTICS, "rel_vort_on_triangles"), tri, c->map_tri, ntri,
                        ntri, 0, ntri)) return -1;
     CK(cudaStreamSynchronize(c->stream));
@@ -1051,11 +1051,11 @@ int vector_tendencies_expl(struct state *state, struct state *state_tendency, st
         double *wind = b.sn.ds.w, *rho_gas = b.sn.ds.rho + (long long)c->n_cond * ns;
         if (up_vec(diagnostics, GAME_DIAGNOSTICS, "flux_density", flux)) return -1;
         op_scalar_times_vector(c, rho_gas, wind, flux, OP_STV_H | OP_STV_V);
-        if (op_rel_vort(c, wind, b.tri, rel)) return -1;
+        if (op_rel_vort(c, wind, b.tri, rel, true)) return -1;
         op_pot_vort(c, rel, rho_gas, pv);
         op_vorticity_flux(c, flux, pv, pvt);
         op_inner_product(c, wind, wind, b.v2);
-        if (op_grad(c, b.v2, v2g, OP_GRAD_H | OP_GRAD_V | OP_GRAD_CON)) return -1;
+        if (op_grad(c, b.v2, v2g, OP_GRAD_H | OP_GRAD_V | OP_GRAD_CON, true)) return -1;
         if (down_vec(diagnostics, GAME_DIAGNOSTICS, "flux_density", flux)) return -1;
         if (download_field(vec_of(diagnostics, GAME_DIAGNOSTICS, "rel_vort_on_triangles"), b.tri, c->map_tri, ntri,
                            ntri, 0, ntri))
@@ -1343,7 +1343,7 @@ int calc_pot_vort_adj(double *velocity_field, double *density_field, double *pot
     double *wind = v[0], *rho = v[1], *rel = v[2], *pv = v[3], *pvb = v[4], *zero_u = v[5], *wb = v[6], *rb = v[7],
            *trib = v[8];
     if (up(velocity_field, wind, c->map_vec, c->nv) || up(density_field, rho, c->map_s, c->ns)) return -1;
-    if (op_rel_vort(c, wind, c->sub.tri, rel)) return -1;
+    if (op_rel_vort(c, wind, c->sub.tri, rel, true)) return -1;
     op_pot_vort(c, rel, rho, pv);
     if (up(pot_vort_bar, pvb, c->map_curl, c->ncurl) || up(velocity_field_bar, wb, c->map_vec, c->nv)
         || up(density_field_bar, rb, c->map_s, c->ns))
@@ -1489,7 +1489,7 @@ int epv_diagnostics(double *pot_vort, struct state *state, double *epv, struct g
     if (upload_field(host_tvp, tvp, c->map_s, c->ns, c->ns)) return -1;
     DState s{};
     s.theta_v_pert = tvp;
-    if (op_epv(c, pv, s, o)) return -1;
+    if (op_epv(c, pv, s, o, true)) return -1;
     if (download_field(epv, o, c->map_s, c->ns, c->ns, 0, c->ns)) return -1;
     /* the top layer of theta_v_pert as the reference leaves it */
     if (download_field(host_tvp, tvp, c->map_s, c->ns, c->ns, 0, c->nc)) return -1;

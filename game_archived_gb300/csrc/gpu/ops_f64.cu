@@ -14,13 +14,14 @@ namespace {
 
 using G = HGrid<double>;
 
+template <bool ALL>
 __global__ void k_op_grad_h(G g, const double *f, double *u, int with_correction)
 {
     const long long n = (long long)g.nl * g.ne, i = gtid();
     if (i >= n) return;
     const int l = row_of(i, g.ne), e = (int)(i - (long long)l * g.ne);
     if (with_correction) {
-        u[i] = grad_h<true>(g, f, l, e);
+        u[i] = grad_h<ALL>(g, f, l, e);
     } else {
         const int fr = g.from[e], to = g.to[e];
         u[i] = div_tab(f[(long long)l * g.nc + to] - f[(long long)l * g.nc + fr], g.nd_h, g.r_nd_h, i);
@@ -143,12 +144,13 @@ __global__ void k_op_inner(G g, const double *aw, const double *au, const double
 }
 
 /* calc_rel_vort (vorticities.c:104-165): tangential [L+1][Ne], rhombus [L][Ne] */
+template <bool ALL>
 __global__ void k_op_rel_vort(G g, const double *u, const double *w, const double *tri, double *zh, double *zv)
 {
     const long long n = (long long)(g.nl + 1) * g.ne, i = gtid();
     if (i >= n) return;
     const int k = row_of(i, g.ne), e = (int)(i - (long long)k * g.ne);
-    zh[i] = rel_vort_tangential<true>(g, u, w, k, e);
+    zh[i] = rel_vort_tangential<ALL>(g, u, w, k, e);
     if (k < g.nl) {
         const int tf = g.dual_from[e], tt = g.dual_to[e];
         const long long kt = (long long)k * g.nt;
@@ -304,13 +306,14 @@ void op_add_vertical_divv(Context *c, const double *vec, double *out)
     c->kernel_launches++;
 }
 
-int op_grad(Context *c, const double *f, double *vec, int parts)
+int op_grad(Context *c, const double *f, double *vec, int parts, bool all)
 {
     if (ensure_f64(c, false)) return -1;
     double *w = vec, *u = vec + (long long)(c->nl + 1) * c->nc;
     if (parts & OP_GRAD_V) k_op_grad_v<<<nb((long long)(c->nl - 1) * c->nc), 256, 0, c->stream>>>(c->hg64, f, w);
+    auto grad_h = all ? k_op_grad_h<true> : k_op_grad_h<false>;
     if (parts & OP_GRAD_H)
-        k_op_grad_h<<<nb((long long)c->nl * c->ne), 256, 0, c->stream>>>(c->hg64, f, u, (parts & OP_GRAD_CON) ? 1 : 0);
+        grad_h<<<nb((long long)c->nl * c->ne), 256, 0, c->stream>>>(c->hg64, f, u, (parts & OP_GRAD_CON) ? 1 : 0);
     c->kernel_launches += 2;
     return 0;
 }
@@ -346,12 +349,14 @@ void op_inner_product(Context *c, const double *a, const double *b, double *out)
     c->kernel_launches++;
 }
 
-int op_rel_vort(Context *c, const double *wind, double *tri, double *curl)
+int op_rel_vort(Context *c, const double *wind, double *tri, double *curl, bool all)
 {
     if (ensure_f64(c, false)) return -1;
     const long long off = (long long)(c->nl + 1) * c->nc, coff = (long long)(c->nl + 1) * c->ne;
-    k_tri_vort<double, true><<<dim3(nb(c->nt), (unsigned)c->nl), 256, 0, c->stream>>>(c->hg64, wind + off, tri);
-    k_op_rel_vort<<<nb(coff), 256, 0, c->stream>>>(c->hg64, wind + off, wind, tri, curl, curl + coff);
+    auto tri_vort = all ? k_tri_vort<double, true> : k_tri_vort<double, false>;
+    auto rel_vort = all ? k_op_rel_vort<true> : k_op_rel_vort<false>;
+    tri_vort<<<layer_grid(c->nl, c->nt, 256), 256, 0, c->stream>>>(c->hg64, wind + off, tri);
+    rel_vort<<<nb(coff), 256, 0, c->stream>>>(c->hg64, wind + off, wind, tri, curl, curl + coff);
     c->kernel_launches += 2;
     return 0;
 }

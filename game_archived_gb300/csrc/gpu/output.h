@@ -89,7 +89,7 @@ void op_edges_to_cells(Context *c, const double *ue, double *out);
 void op_curl_to_cells(Context *c, const double *zv, double *out);
 void op_edges_to_cells_lowest(Context *c, const double *ue, double *out);
 void op_inner_product_tangential(Context *c, const double *a, const double *b, double *bt, double *out);
-int op_epv(Context *c, const double *pot_vort, DState s, double *epv);
+int op_epv(Context *c, const double *pot_vort, DState s, double *epv, bool all); /* all: as op_grad's */
 
 /* scatter of [k][Nc] device-order slices to reference order [k][Nc] and of
  * the pressure-level fields [6][Nc] to the reference's [Nc][6], into dst

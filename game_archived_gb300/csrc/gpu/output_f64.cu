@@ -683,7 +683,7 @@ void op_inner_product_tangential(Context *c, const double *a, const double *b, d
     c->kernel_launches += 2;
 }
 
-int op_epv(Context *c, const double *pot_vort, DState s, double *epv)
+int op_epv(Context *c, const double *pot_vort, DState s, double *epv, bool all)
 {
     OutBufs *b = ensure_obuf(c);
     if (!b) return -1;
@@ -693,7 +693,7 @@ int op_epv(Context *c, const double *pot_vort, DState s, double *epv)
     /* the gradient leaves the top and surface levels untouched: zero, as
      * the reference's calloc'd work array */
     CK(cudaMemsetAsync(b->grad, 0, (size_t)c->nv * sizeof(double), c->stream));
-    if (op_grad(c, b->theta, b->grad, OP_GRAD_H | OP_GRAD_V | OP_GRAD_CON)) return -1;
+    if (op_grad(c, b->theta, b->grad, OP_GRAD_H | OP_GRAD_V | OP_GRAD_CON, all)) return -1;
     op_inner_product_tangential(c, b->pvmod, b->grad, b->ue, epv);
     k_epv_round<<<nb(c->nc, 128), 128, 0, c->stream>>>(c->vg, s, b->theta);
     c->kernel_launches += 3;
@@ -734,7 +734,7 @@ int output_fields(Context *c, StateMirror *sm, const OutParams &p, const OutInpu
     {
         ProfScope ps(c, "out_divv_vort");
         op_divv(c, s.w, nullptr, nullptr, f.divv_h, 0);
-        if (op_rel_vort(c, s.w, b->tri, b->rel)) return -1;
+        if (op_rel_vort(c, s.w, b->tri, b->rel, false)) return -1;
         op_curl_to_cells(c, b->rel + (long long)(c->nl + 1) * c->ne, f.rel_vort);
     }
     {
@@ -749,7 +749,7 @@ int output_fields(Context *c, StateMirror *sm, const OutParams &p, const OutInpu
     {
         ProfScope ps(c, "out_epv");
         op_pot_vort(c, b->rel, s.rho + (long long)p.n_cond * S, b->pv);
-        if (op_epv(c, b->pv, s, f.epv)) return -1;
+        if (op_epv(c, b->pv, s, f.epv, false)) return -1;
     }
     PlIn pi{P, c->gravity_potential, T, RH, f.epv, f.u, f.v, f.rel_vort};
     PlOut po{f.geopotential_height, f.t_pl, f.rh_pl, f.epv_pl, f.u_pl, f.v_pl, f.rel_vort_pl};
