@@ -483,7 +483,7 @@ __global__ void fa_rediag(VGrid vg, AState<T> s)
     if (i < ns) s.tp[i] = s.rt[i] / s.rho[i] - vg.theta_v_bg[i];
 }
 
-/* mass and rho theta_v tendencies of the dry build (k_scalar_tend2, main
+/* mass and rho theta_v tendencies of the dry build (k_scalar_tend64, main
  * gas), new weight 1 in both substages */
 template <class T>
 __global__ void fa_scalar(HGrid<double> g, const T *rho, const T *theta, const T *u, T *st_rho, T *st_rt)

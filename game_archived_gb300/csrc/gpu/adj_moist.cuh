@@ -425,7 +425,7 @@ __global__ void ba_prelude(VGrid vg, AParams ap, AState<double> s, const double 
 }
 
 /* ------------------------------------------------- moist scalar tendencies
- * k_scalar_tend2 (kernels.cuh) with R = double: the main gas's mass flux and
+ * k_scalar_tend64 (kernels.cuh): the main gas's mass flux and
  * rho theta_v flux as fa_scalar, plus the phase-transition rates, the
  * c_v-weighted diabatic heating, and the non-main constituents' upstream
  * fluxes with their rk 1 blend 0.5 old + 0.5 new.  str = [C][L][Nc]. */

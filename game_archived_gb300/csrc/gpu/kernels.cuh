@@ -135,9 +135,9 @@ __device__ __forceinline__ double density_total(const double *rho, int n_const, 
 
 /* ------------------------------------------------------ thermodynamics
  * src/constituents/dictionary.c (FP64 on both paths) */
-/* t^3 and t^4 with the products' rounding errors carried along (TwoProd), each
- * rounded once: what the reference's pow(t, n) returns, at five or six FP64
- * instructions instead of some 150 */
+/* t^3 and t^4 with the products' rounding errors carried along (TwoProd):
+ * correctly rounded (tested), the reference's pow(t, n) to its last bit, at five
+ * or six FP64 instructions instead of some 150 */
 __device__ __forceinline__ double cube(double t)
 {
     const double s = t * t, se = __fma_rn(t, t, -s), p = s * t;
@@ -1482,12 +1482,13 @@ __device__ __forceinline__ void scalar_tend_tilt(const HGrid<float> &g, const St
 }
 
 /* One launch for both: the first tilt_blocks blocks of a layer take the columns
- * of tilt_cells, the others every cell and leave those out.  Two launches one
- * after the other each wait for the latency of their gathers on a small grid
- * (with the mountain and all constituents, RES_ID 4: 38 -> 28 us, RES_ID 7 628
- * us either way); the tilted columns take the shorter way above the
- * terrain-following layers.  64 registers (eight blocks per SM; 72 without the
- * bound: 657 us at RES_ID 7) and no corrections compiled in for a flat grid
+ * of tilt_cells, the others every cell and leave those out; the tilted columns
+ * take the shorter way above the terrain-following layers.  Against one kernel
+ * that decides per cell, with the mountain and all constituents: RES_ID 6 202 ->
+ * 172 us, RES_ID 3 and 4, where both wait for the latency of their gathers, 21 ->
+ * 24 and 24 -> 28 us (two launches one after the other 38).  64 registers (eight
+ * blocks per SM; 72 without the bound, which spills 48 bytes of the tilted form:
+ * 657 against 628 us at RES_ID 7) and no corrections compiled in for a flat grid
  * (TILT = false; RES_ID 6, cloud-free: 96 -> 85 us). */
 template <bool IRR, bool TILT>
 __global__ void __launch_bounds__(128, 8) k_scalar_tend32(HGrid<float> g, StepParams p, SView<float> sv, DState st,

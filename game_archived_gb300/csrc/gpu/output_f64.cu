@@ -467,7 +467,7 @@ struct PlIn {
     const double *p, *gpot, *t, *rh, *epv, *u, *v, *relv;
 };
 
-/* per column: vertical interpolation to the six pressure levels in ln p
+/* per column and pressure level: vertical interpolation in ln p
  * between the layer nearest to the level and its neighbour, 9999 below the
  * lowest layer (write_output.c:766-825); out [6][Nc].
  *

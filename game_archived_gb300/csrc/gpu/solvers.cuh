@@ -15,12 +15,14 @@
  * tracers (column_solvers.c:385-639)
  *   k_tracers_solve per (constituent, column): rows built on the fly, Thomas
  *                   sweep in registers, clipping
- *   k_tracers_sedheat per column: sedimentation enthalpy flux
- *                   divergence, accumulated over the condensates in the
+ *   k_tracers_sedheat64 per (layer, column), k_tracers_sedheat (mixed path
+ *                   with FP64 eliminations) per column: sedimentation enthalpy
+ *                   flux divergence, accumulated over the condensates in the
  *                   reference's order
  *
- * EXACT = true keeps the reference's operation order bit for bit (FP64
- * parity path); EXACT = false (mixed path) multiplies by precomputed
+ * EXACT = true keeps the reference's operation order (FP64 parity path), its
+ * quotients by reciprocals at hand where one serves several (div_rcp,
+ * div_sweep: IEEE's results); EXACT = false (mixed path) multiplies by precomputed
  * reciprocals of the grid metrics and of repeated denominators, which moves
  * results by a few ulps but removes most FP64 divisions.
  */
