@@ -236,7 +236,6 @@ int import_aux(const void *diag, const void *forc, const void *irrev)
     Context *c = ctx();
     if (diag == g_bound.aux_diag && forc == g_bound.aux_forc && irrev == g_bound.aux_irrev) return 0;
     const long long nv = c->nv, ns = c->ns;
-    const long long woff = (long long)(c->nl + 1) * c->nc;
     double *t0 = c->dev_tmp[0], *t1 = c->dev_tmp[1];
     /* P = nl + l */
     if (upload_field(member<double>(forc, GAME_FORCINGS, "pressure_gradient_acc_neg_nl"), t0, c->map_vec, nv, nv)) return -1;
@@ -245,15 +244,11 @@ int import_aux(const void *diag, const void *forc, const void *irrev)
     if (upload_field(member<double>(forc, GAME_FORCINGS, "pot_vort_tend"), t2, c->map_vec, nv, nv)) return -1;
     if (upload_field(member<double>(forc, GAME_FORCINGS, "v_squared_grad"), t3, c->map_vec, nv, nv)) return -1;
     /* flux_density: the TOA/surface vertical entries are never written by the step */
-    CK(cudaStreamSynchronize(c->stream));
-    double *fl = nullptr;
-    CK(cudaMalloc(&fl, (size_t)nv * sizeof(double)));
+    double *fl = c->wv_layer; /* scratch of the step's solves, 8 S >= nv */
     if (upload_field(member<double>(diag, GAME_DIAGNOSTICS, "flux_density"), fl, c->map_vec, nv, nv)) return -1;
     aux_sum_to_work(c, t0, t1, t2, t3, fl, nullptr, nullptr);
     if (upload_field(member<double>(irrev, GAME_IRREV, "condensates_sediment_heat"), c->sed_heat, c->map_s, ns, ns)) return -1;
     CK(cudaStreamSynchronize(c->stream));
-    cudaFree(fl);
-    (void)woff;
     g_bound.aux_diag = diag;
     g_bound.aux_forc = forc;
     g_bound.aux_irrev = irrev;
